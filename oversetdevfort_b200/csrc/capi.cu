@@ -215,6 +215,7 @@ int create_resources(ovs_ctx* c, const ovs_dims* dims) {
   OVS_CUDA_TRY(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   OVS_CUDA_TRY(cudaEventCreate(&c->ev0));
   OVS_CUDA_TRY(cudaEventCreate(&c->ev1));
+  for (cudaEvent_t& e : c->ev_poll) OVS_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   int st;
   const size_t N = c->N;
   for (int f = 0; f < OVS_F_COUNT; ++f) {
@@ -287,6 +288,7 @@ int ovs_destroy(ovs_ctx* c) {
   if (c->h_async_cfl) cudaFreeHost(c->h_async_cfl);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  for (cudaEvent_t e : c->ev_poll) if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   cudaGetLastError();
   delete c;

@@ -19,7 +19,7 @@
 // sol += sum y_j v_j).  All scalars live on the device; every dot product is
 // a fixed-grid, fixed-order FP64 reduction (last-block-done), so results are
 // bit-identical from run to run.  The host only polls the "done" word once
-// per batch of iterations.
+// per batch of iterations, a batch behind the launches.
 #include "ovs_internal.cuh"
 
 #include <algorithm>
@@ -56,7 +56,8 @@ __device__ __forceinline__ void ld4(const double* p, double v[4]) {
 template <typename A, typename B, bool ACC64> struct AccT { using type = double; };
 template <> struct AccT<float, float, false> { using type = float; };
 
-// MODE 0: y = A x ; MODE 1: y = P^-1 A x ; MODE 2: y = b - A x
+// MODE 0: y = A x ; MODE 1: y = P^-1 A x (times *scale, if given) ; MODE 2:
+// y = b - A x
 // Block systems: NG groups of 4 values per slot, one lane per group.
 //   NS   (NG=4): groups rows u1,u2,u3,p over columns (u1,u2,u3,p)
 //   NSVOF(NG=6): + row phi over (u1,u2,u3,phi), + column phi into (u1,u2,u3,p)
@@ -70,7 +71,8 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
                                                 const int* __restrict__ colidx, const TM* __restrict__ vals,
                                                 const TX* __restrict__ x, TY* __restrict__ y,
                                                 const TM* __restrict__ pre, const double* __restrict__ b,
-                                                const int* __restrict__ rows = nullptr, long nrows = 0) {
+                                                const int* __restrict__ rows = nullptr, long nrows = 0,
+                                                const double* __restrict__ scale = nullptr) {
   using AT = typename AccT<TM, TX, ACC64>::type;
   constexpr int NV = 4 * NG;
   constexpr int RPW = 32 / NG;  // rows per warp
@@ -173,6 +175,7 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
     } else {
       z = yv * (AT)pre[(size_t)10 * N + row];
     }
+    if (scale) z *= (AT)__ldg(scale);
   } else if (MODE == 2) {
     z = (AT)b[(size_t)g * N + row] - yv;
   }
@@ -184,10 +187,10 @@ __global__ void __launch_bounds__(SPMV_THREADS)
 spmv_block_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                   const TM* __restrict__ vals, const TX* __restrict__ x, TY* __restrict__ y,
                   const TM* __restrict__ pre, const double* __restrict__ b,
-                  const int* __restrict__ done) {
+                  const int* __restrict__ done, const double* __restrict__ scale) {
   if (done && *done) return;
   const long wglob = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  spmv_block_warp<NG, TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b);
+  spmv_block_warp<NG, TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b, nullptr, 0, scale);
 }
 
 // the same product over a list of rows (a partition's interior or boundary
@@ -208,7 +211,8 @@ __device__ __forceinline__ void spmv_scalar_warp(long wglob, int N, const int* _
                                                  const int* __restrict__ colidx, const TM* __restrict__ vals,
                                                  const TX* __restrict__ x, TY* __restrict__ y,
                                                  const TM* __restrict__ pre, const double* __restrict__ b,
-                                                 const int* __restrict__ rows = nullptr, long nrows = 0) {
+                                                 const int* __restrict__ rows = nullptr, long nrows = 0,
+                                                 const double* __restrict__ scale = nullptr) {
   using AT = typename AccT<TM, TX, ACC64>::type;
   const int lane = threadIdx.x & 31;
   const int sub = lane >> 3, k = lane & 7;
@@ -233,8 +237,12 @@ __device__ __forceinline__ void spmv_scalar_warp(long wglob, int N, const int* _
   a += __shfl_xor_sync(0xffffffffu, a, 1);
   if (!active || k != 0) return;
   AT z = a;
-  if (MODE == 1) z = a * (AT)pre[row];
-  else if (MODE == 2) z = (AT)b[row] - a;
+  if (MODE == 1) {
+    z = a * (AT)pre[row];
+    if (scale) z *= (AT)__ldg(scale);
+  } else if (MODE == 2) {
+    z = (AT)b[row] - a;
+  }
   y[row] = (TY)z;
 }
 
@@ -243,10 +251,10 @@ __global__ void __launch_bounds__(SPMV_THREADS)
 spmv_scalar_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                    const TM* __restrict__ vals, const TX* __restrict__ x, TY* __restrict__ y,
                    const TM* __restrict__ pre, const double* __restrict__ b,
-                   const int* __restrict__ done) {
+                   const int* __restrict__ done, const double* __restrict__ scale) {
   if (done && *done) return;
   const long wglob = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  spmv_scalar_warp<TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b);
+  spmv_scalar_warp<TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b, nullptr, 0, scale);
 }
 
 template <typename TM, typename TX, typename TY, int MODE>
@@ -284,7 +292,7 @@ int launch_spmv_rows(ovs_ctx* c, int sys, const TM* vals, const double* x, doubl
 
 template <typename TM, typename TX, typename TY, int MODE, bool ACC64 = true>
 int launch_spmv(ovs_ctx* c, int sys, const TM* vals, const TX* x, TY* y, const TM* pre,
-                const double* b, const int* done) {
+                const double* b, const int* done, const double* scale = nullptr) {
   const int N = c->N;
   int rpw = sys == OVS_SYS_NS ? 8 : (sys == OVS_SYS_NSVOF ? 5 : 4);
   long warps = ((long)N + rpw - 1) / rpw;
@@ -292,19 +300,19 @@ int launch_spmv(ovs_ctx* c, int sys, const TM* vals, const TX* x, TY* y, const T
   if (sys == OVS_SYS_NS)
     {
       spmv_block_kernel<4, TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
-          N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
+          N, c->rowptr, c->colidx, vals, x, y, pre, b, done, scale);
       ++c->launches;
     }
   else if (sys == OVS_SYS_NSVOF)
     {
       spmv_block_kernel<6, TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
-          N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
+          N, c->rowptr, c->colidx, vals, x, y, pre, b, done, scale);
       ++c->launches;
     }
   else
     {
       spmv_scalar_kernel<TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
-          N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
+          N, c->rowptr, c->colidx, vals, x, y, pre, b, done, scale);
       ++c->launches;
     }
   OVS_CUDA_TRY(cudaGetLastError());
@@ -455,6 +463,7 @@ gm_start_kernel(int N, int nf, int sys, const double* __restrict__ rhs, const TM
     gm->unorm0 = un;
     gm->epsnrm = tol * un;
     gm->e[0] = un;
+    gm->sc[0] = 1.0;
     gm->iks = 0;
     gm->done = (un == 0.0) ? 1 : 0;
     gm->breakdown = (un == 0.0) ? 1 : 0;
@@ -506,19 +515,17 @@ gm_normalize_kernel(const TW* w, TV* v, size_t n, GmresDev* gm, int first) {
   for (size_t i = 4 * n4 + t0; i < n; i += stride) v[i] = (TV)((double)w[i] / d);
 }
 
-// H(k+1,k) = sqrt(beta), Givens rotations of column k, e update, exit test
+// H(k+1,k) = unorm, Givens rotations of column k (Hk[0..k), rotated in
+// place; cs, sn: the earlier rotations), e update, exit test
 // (SparseGMRES_NS.f90:289-327); one thread
-__device__ void givens_step(GmresDev* gm, int k) {
-  const int ld = gm->kspace + 1;
-  double* Hk = gm->H + (size_t)(k - 1) * ld;
-  const double unorm = sqrt(gm->beta);
-  Hk[k] = unorm;
+__device__ void givens_step(GmresDev* gm, int k, double unorm, double* Hk, const double* cs, const double* sn) {
+  double cur = Hk[0];
   for (int jk = 1; jk <= k - 1; ++jk) {
-    const double tmp = gm->cs[jk - 1] * Hk[jk - 1] + gm->sn[jk - 1] * Hk[jk];
-    Hk[jk] = -gm->sn[jk - 1] * Hk[jk - 1] + gm->cs[jk - 1] * Hk[jk];
-    Hk[jk - 1] = tmp;
+    const double nxt = Hk[jk];
+    Hk[jk - 1] = cs[jk - 1] * cur + sn[jk - 1] * nxt;
+    cur = -sn[jk - 1] * cur + cs[jk - 1] * nxt;
   }
-  const double a = Hk[k - 1], b = Hk[k];
+  const double a = cur, b = unorm;
   const double tmp = sqrt(a * a + b * b);
   if (tmp == 0.0) {
     // column k of H is zero (P^-1 A v_k has no component outside
@@ -531,14 +538,15 @@ __device__ void givens_step(GmresDev* gm, int k) {
     gm->breakdown = 1;
     return;
   }
-  gm->cs[k - 1] = a / tmp;
-  gm->sn[k - 1] = b / tmp;
+  const double c = a / tmp, sg = b / tmp;
+  gm->cs[k - 1] = c;
+  gm->sn[k - 1] = sg;
   Hk[k - 1] = tmp;
-  Hk[k] = 0.0;
-  const double t2 = gm->cs[k - 1] * gm->e[k - 1] + gm->sn[k - 1] * gm->e[k];
-  gm->e[k] = -gm->sn[k - 1] * gm->e[k - 1] + gm->cs[k - 1] * gm->e[k];
-  gm->e[k - 1] = t2;
-  const double er = fabs(gm->e[k]);
+  const double ek = gm->e[k - 1];
+  gm->e[k - 1] = c * ek + sg * gm->e[k];
+  const double en = -sg * ek + c * gm->e[k];
+  gm->e[k] = en;
+  const double er = fabs(en);
   gm->ercheck = er;
   gm->iks = k;
   const bool conv = (er <= gm->epsnrm) && (k >= gm->kmin);
@@ -641,365 +649,339 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
     }
     for (size_t i = 4 * n4 + t0; i < n; i += stride) w[i] = (TV)((double)w[i] / unorm);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) givens_step(gm, k);
-}
-
-// Sizes of the on-chip Gram-Schmidt kernel (gm_mgs_onchip_kernel below):
-// 512 threads (16 warps); each warp owns the TMEM lanes of its quarter
-// (warp % 4) and a quarter of the 512 columns (warp / 4), so every thread
-// holds 128 32-bit columns: 32 groups of 4 FP32 values, or 16 groups of 4
-// FP64 values split into low and high words.
-constexpr int ONCHIP_THREADS = 512;
-constexpr int TMEM_COLS = 512;
-constexpr int TMEM_COLS_PER_THREAD = 128;
-template <typename TV> struct TmemGeom {
-  static constexpr int words = (int)(sizeof(TV) / 4);              // columns per value
-  static constexpr int gpp = 16 / (4 * words);                     // groups per 16-column piece
-  static constexpr int pieces = TMEM_COLS_PER_THREAD / 16;         // pieces per thread
-  static constexpr int groups = pieces * gpp;                      // groups per thread
-  static constexpr int cap = 4 * groups * ONCHIP_THREADS;          // values per block
-};
-
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(addr));
-}
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15, %16};\n"
-      :
-      : "r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]));
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// group gi of a 16-column piece <-> 4 values
-__device__ __forceinline__ void unpack_group(const uint32_t (&r)[16], int gi, float*, double a[4]) {
-#pragma unroll
-  for (int e = 0; e < 4; ++e) a[e] = (double)__uint_as_float(r[4 * gi + e]);
-}
-__device__ __forceinline__ void unpack_group(const uint32_t (&r)[16], int gi, double*, double a[4]) {
-#pragma unroll
-  for (int e = 0; e < 4; ++e) a[e] = __hiloint2double((int)r[8 * gi + 2 * e + 1], (int)r[8 * gi + 2 * e]);
-}
-__device__ __forceinline__ void pack_group(uint32_t (&r)[16], int gi, float*, const double a[4]) {
-#pragma unroll
-  for (int e = 0; e < 4; ++e) r[4 * gi + e] = __float_as_uint((float)a[e]);
-}
-__device__ __forceinline__ void pack_group(uint32_t (&r)[16], int gi, double*, const double a[4]) {
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    r[8 * gi + 2 * e] = (uint32_t)__double2loint(a[e]);
-    r[8 * gi + 2 * e + 1] = (uint32_t)__double2hiint(a[e]);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    gm->sc[k] = 1.0;
+    givens_step(gm, k, unorm, gm->H + (size_t)(k - 1) * (gm->kspace + 1), gm->cs, gm->sn);
   }
 }
 
-// The on-chip kernel indexes 32-bit within its block's chunk, from base
-// pointers at the chunk start.  ld4m loads the group at local index li (a
-// multiple of 4) or, when !ok, the chunk's first group; the load itself is
-// unconditional so a thread keeps several in flight.  Values at or beyond
-// the chunk end nl, and all four when !ok, come back as zero.  The group
-// stays in the storage type until it is used.
-template <typename TV> struct Vec4;
-template <> struct Vec4<float> { using type = float4; };
-template <> struct Vec4<double> { struct type { double x, y, z, w; }; };
-template <typename TV>
-__device__ __forceinline__ typename Vec4<TV>::type ld4m(const TV* p, int li, int nl, bool ok) {
-  typename Vec4<TV>::type v;
-  const TV* q = p + (ok ? li : 0);
-  if constexpr (sizeof(TV) == 4) {
-    v = *reinterpret_cast<const float4*>(q);
-  } else {
-    const double2 a = reinterpret_cast<const double2*>(q)[0], b = reinterpret_cast<const double2*>(q)[1];
-    v.x = a.x; v.y = a.y; v.z = b.x; v.w = b.y;
+// ------------------------------------------------- Gram-Schmidt, one kernel
+// The orthogonalization of Arnoldi step k (w = P^-1 A v_k, written to basis
+// slot k by the SpMV launch before it) with the coefficients of modified
+// Gram-Schmidt and one grid-wide barrier instead of one per coefficient.
+// MGS takes h_j = v_j . (w - sum_{i<j} h_i v_i), that is
+//   (I + L) h = V^T w,   L_ji = v_j . v_i (j > i),
+// so V^T w and the new row of L (v_k . v_j) are all the reductions a step
+// needs: the inverse compact WY form of MGS (Swirydowicz, Langou, Ananthan,
+// Yang, Thomas, "Low synchronization Gram-Schmidt and generalized minimal
+// residual algorithms", 2021).  T = (I + L)^-1 grows by a row per step.
+//   phase A  every v_j is read once, for both dots (FP64 products and sums);
+//   barrier  every block adds the partial dots in the same order and forms h;
+//   phase B  w -= sum_j h_j v_j and |w|^2, the last block to finish adds the
+//            norm and does the Givens step and T's new row.
+// w stays unnormalized: gm->sc[j] = 1 / |w| belongs to slot j, and the SpMV
+// (linear in its vector), the dots and the coefficients carry it, which
+// saves the barrier and the pass over w that a division would need.
+// Each basis vector is read twice per step, as in MGS; the bound is that
+// traffic (two vectors a step at 6.4 TB/s) for long vectors and the chain
+// launch - dots - barrier - h - update - tail for short ones.
+//
+// A warp owns sub-chunks of 32 V values.  Phase A takes JG vectors at a
+// time: all their loads in flight, 2 JG sums per lane, reduced over the
+// lanes by halving (16 shuffles for 16 sums) into the warp's accumulators in
+// shared memory.  Phase B visits the sub-chunks in reverse, so that what
+// phase A read last is still in L2.  V = 4 (256-bit loads in FP64) where it
+// gives every warp of the grid a sub-chunk, V = 1 for shorter vectors; there
+// the JG groups of a sub-chunk are also spread over `js` warps.
+constexpr int ORTH_THREADS = 512;
+constexpr int ORTH_WARPS = ORTH_THREADS / 32;
+constexpr int JG = 8;
+
+// V values at index i (a multiple of V), zero at and beyond n.  Plain loads:
+// the slot being orthogonalized is rewritten by the thread that reads it.
+template <int V, typename TV>
+__device__ __forceinline__ void orth_ld(const TV* __restrict__ p, size_t i, size_t n, TV (&x)[V]) {
+  if (V == 4 && i + 4 <= n) {
+    if constexpr (V == 4 && sizeof(TV) == 8) {
+      asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p + i));
+    } else if constexpr (V == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(p + i);
+      x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    }
+    return;
   }
-  if (!ok || li + 4 > nl) {
-    if (!ok || li >= nl) v.x = 0;
-    if (!ok || li + 1 >= nl) v.y = 0;
-    if (!ok || li + 2 >= nl) v.z = 0;
-    if (!ok || li + 3 >= nl) v.w = 0;
+#pragma unroll
+  for (int q = 0; q < V; ++q) x[q] = i + q < n ? p[i + q] : (TV)0;
+}
+
+// Sums over the 32 lanes of 2 JG = 16 values per lane: lane l (even) ends up
+// with the sum of value 8 b4 + 4 b3 + 2 b2 + b1 (b the bits of l).
+__device__ __forceinline__ double lanes_sum16(double (&p)[16], int lane) {
+#pragma unroll
+  for (int half = 8, off = 16; half >= 1; half >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double send = up ? p[i] : p[i + half], keep = up ? p[i + half] : p[i];
+      p[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
   }
+  return p[0] + __shfl_xor_sync(0xffffffffu, p[0], 1);
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-template <typename TV>
-__device__ __forceinline__ void st4l(TV* p, int li, int nl, const double v[4]) {
-  if (li + 4 <= nl) { st4v(p + li, v); return; }
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    if (li + q < nl) p[li + q] = (TV)v[q];
-}
-template <typename V4> __device__ __forceinline__ void widen(const V4& v, double a[4]) {
-  a[0] = (double)v.x; a[1] = (double)v.y; a[2] = (double)v.z; a[3] = (double)v.w;
-}
-// Gram-Schmidt step on one group: a -= beta * p (rounded to TV), dot term
-template <typename TV, typename V4>
-__device__ __forceinline__ double mgs_apply(double a[4], const V4& p, const V4& y, double beta, bool sub,
-                                            bool self) {
-  if (sub) {
-    double pv[4];
-    widen(p, pv);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) a[q] = (double)(TV)(a[q] - beta * pv[q]);
-  }
-  if (self) return a[0] * a[0] + a[1] * a[1] + a[2] * a[2] + a[3] * a[3];
-  double yv[4];
-  widen(y, yv);
-  return a[0] * yv[0] + a[1] * yv[1] + a[2] * yv[2] + a[3] * yv[3];
+
+// shared memory of a step: the warps' sums (2 kk each), a, g, h, h sc, cs, sn
+inline size_t orth_smem(int k) {
+  const size_t kk = ((size_t)k + JG - 1) / JG * JG;
+  return sizeof(double) * ((2 * ORTH_WARPS + 6) * kk + 2);
 }
 
-// FP32 basis: the update w -= beta * v_{j-1} runs in FP32 (one FMA with
-// beta rounded to FP32; w is stored in FP32 either way) and only the dot
-// product is formed in FP64: the products of two FP32 values are exact in
-// FP64 and are summed there.  Two conversions per value instead of five.
-__device__ __forceinline__ double mgs_apply_f(float a[4], const float4& p, const float4& y, float bf, bool sub,
-                                              bool self) {
-  if (sub) {
-    a[0] = fmaf(-bf, p.x, a[0]); a[1] = fmaf(-bf, p.y, a[1]);
-    a[2] = fmaf(-bf, p.z, a[2]); a[3] = fmaf(-bf, p.w, a[3]);
-  }
-  const double a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3];
-  if (self) return a0 * a0 + a1 * a1 + a2 * a2 + a3 * a3;
-  return a0 * (double)y.x + a1 * (double)y.y + a2 * (double)y.z + a3 * (double)y.w;
-}
-
-// The chunk of w owned by a block is cut into pieces of 16 columns per
-// thread: piece p holds groups p*gpp .. p*gpp+gpp-1 of every thread, group g
-// of thread t at local index 4*(g*512 + t), so each load instruction of a
-// warp covers contiguous memory.  Pieces 0..7 live in tensor memory, the
-// next `spieces` in dynamic shared memory (one 32 KB slot each), the rest
-// stay in global memory (w's own basis slot).
-template <typename TV> struct PieceLoads {
-  typename Vec4<TV>::type p[TmemGeom<TV>::gpp], y[TmemGeom<TV>::gpp];
-};
-template <typename TV> struct PieceGeom {
-  static constexpr int values = 4 * TmemGeom<TV>::gpp * ONCHIP_THREADS;   // values per piece
-  static constexpr int bytes = values * (int)sizeof(TV);                   // 32 KB
-};
-__device__ __forceinline__ int piece_li(int p, int gi, int gpp) {
-  return 4 * ((p * gpp + gi) * ONCHIP_THREADS + (int)threadIdx.x);
-}
-
-// Global loads of v_{j-1} (pp, null in step 1) and v_j (yp, null in step
-// k+1) for one piece, all issued before any is used.
-template <typename TV>
-__device__ __forceinline__ void issue_piece(PieceLoads<TV>& L, const TV* pp, const TV* yp, int p, int nl) {
-  using Geo = TmemGeom<TV>;
-#pragma unroll
-  for (int gi = 0; gi < Geo::gpp; ++gi) {
-    const int li = piece_li(p, gi, Geo::gpp);
-    const bool ok = li < nl;
-    if (pp) L.p[gi] = ld4m(pp, li, nl, ok);
-    if (yp) L.y[gi] = ld4m(yp, li, nl, ok);
-  }
-}
-
-// One Gram-Schmidt step on group gi of a piece whose w values are in r
-// (the 16 columns of the piece, as stored in tensor memory).
-template <typename TV>
-__device__ __forceinline__ double step_group(uint32_t (&r)[16], int gi, const PieceLoads<TV>& L, double beta,
-                                             bool sub, bool self) {
-  if constexpr (sizeof(TV) == 4) {
-    float f[4] = {__uint_as_float(r[4 * gi]), __uint_as_float(r[4 * gi + 1]), __uint_as_float(r[4 * gi + 2]),
-                  __uint_as_float(r[4 * gi + 3])};
-    const double s = mgs_apply_f(f, L.p[gi], L.y[gi], (float)beta, sub, self);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) r[4 * gi + e] = __float_as_uint(f[e]);
-    return s;
-  } else {
-    double a[4];
-    unpack_group(r, gi, (TV*)nullptr, a);
-    const double s = mgs_apply<TV>(a, L.p[gi], L.y[gi], beta, sub, self);
-    pack_group(r, gi, (TV*)nullptr, a);
-    return s;
-  }
-}
-
-// the piece's 16 columns from / to shared or global memory
-template <typename TV>
-__device__ __forceinline__ void mem_to_cols(const TV* base, int p, int nl, bool global, uint32_t (&r)[16]) {
-  using Geo = TmemGeom<TV>;
-#pragma unroll
-  for (int gi = 0; gi < Geo::gpp; ++gi) {
-    const int li = piece_li(p, gi, Geo::gpp);
-    double a[4];
-    if (global) widen(ld4m(base, li, nl, li < nl), a);
-    else ld4v(base + 4 * (gi * ONCHIP_THREADS + (int)threadIdx.x), a);
-    pack_group(r, gi, (TV*)nullptr, a);
-  }
-}
-template <typename TV>
-__device__ __forceinline__ void cols_to_mem(TV* base, int p, int nl, bool global, const uint32_t (&r)[16]) {
-  using Geo = TmemGeom<TV>;
-#pragma unroll
-  for (int gi = 0; gi < Geo::gpp; ++gi) {
-    const int li = piece_li(p, gi, Geo::gpp);
-    double a[4];
-    unpack_group(r, gi, (TV*)nullptr, a);
-    if (global) { if (li < nl) st4l(base, li, nl, a); }
-    else st4v(base + 4 * (gi * ONCHIP_THREADS + (int)threadIdx.x), a);
-  }
-}
-
-// Gram-Schmidt of one Arnoldi iteration with w held on chip (w = P^-1 A v_k
-// already written to basis slot k by the SpMV launch before it).  One block
-// of 512 threads per SM; block b owns a contiguous chunk of w (a multiple of
-// 4 values) and keeps it, for all k+1 steps, in tensor memory (all 512
-// columns of the SM, used as plain storage), then in dynamic shared memory;
-// only what does not fit there stays in global memory.  Each step then
-// streams v_{j-1} and v_j alone, two pieces at a time with all their loads
-// in flight together.  The steps, their order and the fixed-order reductions
-// follow gm_arnoldi_kernel (FP32 basis: see mgs_apply_f); entries at and
-// beyond n are never touched.  Every block allocates its tensor memory after
-// the done test and frees it on the one exit path below.
-template <typename TV>
-__global__ void __launch_bounds__(ONCHIP_THREADS, 1)
-gm_mgs_onchip_kernel(TV* V, size_t ld, size_t n, int k, GmresDev* gm, double* part, size_t chunk, int spieces) {
-  using Geo = TmemGeom<TV>;
-  using PG = PieceGeom<TV>;
+template <typename TV, int V>
+__global__ void __launch_bounds__(ORTH_THREADS, 1)
+gm_orthog_kernel(TV* basis, size_t ld, size_t n, int k, GmresDev* gm, double* part, double* T, int nsc, int js) {
   cg::grid_group grid = cg::this_grid();
   if (gm->done) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TV* ws = reinterpret_cast<TV*>(smem_raw);
-  __shared__ double sh[32];
-  __shared__ double sbeta;
-  __shared__ uint32_t tmem_base_sh;
-  const int G = gridDim.x, b = blockIdx.x, t = threadIdx.x, wid = t >> 5;
-  if (wid == 0) {
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&tmem_base_sh);
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tbase = tmem_base_sh;
-  // this warp's lanes (quarter wid % 4) and columns (slot wid / 4)
-  const uint32_t taddr = tbase + ((uint32_t)(32 * (wid & 3)) << 16) + (uint32_t)(TMEM_COLS_PER_THREAD * (wid >> 2));
-  const size_t c0 = (size_t)b * chunk;
-  const int nl = c0 < n ? (int)((c0 + chunk < n ? c0 + chunk : n) - c0) : 0;   // values of this chunk
-  const int np = (nl + PG::values - 1) / PG::values;                            // pieces of this chunk
-  const int ponchip = Geo::pieces + spieces;                                    // pieces held on chip
-  TV* wb = V + ld * (size_t)k + c0;
-  // w into tensor and shared memory
-#pragma unroll 1
-  for (int p = 0; p < np && p < ponchip; ++p) {
-    uint32_t r[16];
-    mem_to_cols(wb, p, nl, true, r);
-    if (p < Geo::pieces) tmem_st16(taddr + 16 * p, r);
-    else cols_to_mem(ws + (size_t)(p - Geo::pieces) * PG::values, p, nl, false, r);
-  }
-  tmem_wait_st();
-  double beta = 0.0;
-  PieceLoads<TV> L0, L1;
-  for (int j = 1; j <= k + 1; ++j) {
-    const bool sub = j >= 2, self = j == k + 1;
-    const TV* pp = sub ? V + ld * (size_t)(j - 2) + c0 : nullptr;
-    const TV* yp = self ? nullptr : V + ld * (size_t)(j - 1) + c0;
-    double sacc = 0.0;
-#pragma unroll 1
-    for (int p0 = 0; p0 < np; p0 += 2) {
-      issue_piece(L0, pp, yp, p0, nl);
-      if (p0 + 1 < np) issue_piece(L1, pp, yp, p0 + 1, nl);
+  extern __shared__ __align__(16) double orth_sm[];
+  __shared__ double sh[ORTH_WARPS];
+  __shared__ int is_last;
+  const int kk = (k + JG - 1) / JG * JG, ncol = 2 * k - 1;   // columns: k dots with w, k - 1 with v_k
+  double* acc = orth_sm;                    // [ORTH_WARPS][2 kk]
+  double* as = acc + 2 * ORTH_WARPS * kk;   // V^T w
+  double* gs = as + kk;                     // row k of L
+  double* hh = gs + kk;                     // the coefficients
+  double* hs = hh + kk;                     // times the slots' scales
+  double* cs = hs + kk;
+  double* sn = cs + kk;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int G = gridDim.x, b = blockIdx.x, W = G * ORTH_WARPS;
+  const int gw = wid * G + b;               // short vectors spread over the blocks first
+  const TV* vk = basis + ld * (size_t)(k - 1);
+  TV* w = basis + ld * (size_t)k;
+  double* nrm = part;                       // G partial norms
+  double* col = part + G;                   // [ncol][G] partial dots
+  double* my = acc + 2 * kk * wid;
+  for (int c = lane; c < 2 * kk; c += 32) my[c] = 0.0;
+  __syncwarp();
+  // ---- phase A
+  const int slot = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+  for (long it = gw; it < (long)nsc * js; it += W) {
+    const int sc = (int)(it / js), jj = (int)(it - (long)sc * js);
+    const size_t i = ((size_t)sc * 32 + lane) * V;
+    TV wv[V], kv[V];
+    orth_ld<V>(w, i, n, wv);
+    orth_ld<V>(vk, i, n, kv);
+    for (int j0 = jj * JG; j0 < k; j0 += js * JG) {
+      TV x[JG][V];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int p = p0 + h;
-        if (p >= np) break;
-        const PieceLoads<TV>& L = h ? L1 : L0;
-        uint32_t r[16];
-        const bool in_tmem = p < Geo::pieces, in_smem = !in_tmem && p < ponchip;
-        TV* sbase = ws + (size_t)(p - Geo::pieces) * PG::values;
-        if (in_tmem) {
-          tmem_ld16(taddr + 16 * p, r);
-          tmem_wait_ld();
-        } else {
-          mem_to_cols(in_smem ? sbase : wb, p, nl, !in_smem, r);
-        }
+      for (int u = 0; u < JG; ++u) orth_ld<V>(basis + ld * (size_t)min(j0 + u, k - 1), i, n, x[u]);
+      double p[2 * JG];
 #pragma unroll
-        for (int gi = 0; gi < Geo::gpp; ++gi) sacc += step_group<TV>(r, gi, L, beta, sub, self);
-        if (sub) {
-          if (in_tmem) tmem_st16(taddr + 16 * p, r);
-          else cols_to_mem(in_smem ? sbase : wb, p, nl, !in_smem, r);
+      for (int u = 0; u < JG; ++u) {
+        p[u] = p[JG + u] = 0.0;
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          p[u] += (double)wv[q] * (double)x[u][q];
+          p[JG + u] += (double)kv[q] * (double)x[u][q];
         }
       }
-    }
-    tmem_wait_st();
-    const double bp = block_sum(sacc, sh);
-    double* pb = part + (size_t)(j & 1) * G;
-    if (t == 0) pb[b] = bp;
-    grid.sync();
-    // every block adds the partials in the same order (lane-strided, then a
-    // fixed butterfly; lane 0's value is used), so all see the same beta
-    if (t < 32) {
-      double v = 0.0;
-      for (int q = t; q < G; q += 32) v += __ldcg(pb + q);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (t == 0) sbeta = v;
-    }
-    __syncthreads();
-    beta = sbeta;
-    if (b == 0 && t == 0) {
-      gm->H[(size_t)(k - 1) * (gm->kspace + 1) + (j - 1)] = beta;
-      gm->beta = beta;
+      const double s = lanes_sum16(p, lane);
+      if (!(lane & 1)) my[(slot < JG ? 0 : kk - JG) + j0 + slot] += s;
     }
   }
-  // normalize into basis slot k (SparseGMRES_NS.f90:291-294), Givens update
-  const double unorm = sqrt(beta);
-  const double d = unorm != 0.0 ? unorm : 1.0;
-#pragma unroll 1
-  for (int p = 0; p < np; ++p) {
-    uint32_t r[16];
-    const bool in_tmem = p < Geo::pieces, in_smem = !in_tmem && p < ponchip;
-    if (in_tmem) {
-      tmem_ld16(taddr + 16 * p, r);
-      tmem_wait_ld();
-    } else {
-      mem_to_cols(in_smem ? ws + (size_t)(p - Geo::pieces) * PG::values : wb, p, nl, !in_smem, r);
-    }
-#pragma unroll
-    for (int gi = 0; gi < Geo::gpp; ++gi) {
-      const int li = piece_li(p, gi, Geo::gpp);
-      double a[4];
-      unpack_group(r, gi, (TV*)nullptr, a);
-      a[0] /= d; a[1] /= d; a[2] /= d; a[3] /= d;
-      if (li < nl) st4l(wb, li, nl, a);
-    }
-  }
-  // release the tensor memory (every access to it has completed above)
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  if (wid == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TMEM_COLS));
-  if (b == 0 && t == 0) givens_step(gm, k);
-}
-
-// back-substitution (SparseGMRES_NS.f90:341-346); single thread
-__global__ void gm_backsub_kernel(GmresDev* gm) {
-  const int iks = gm->iks, ld = gm->kspace + 1;
-  for (int jk = iks; jk >= 1; --jk) {
-    const double y = gm->e[jk - 1] / gm->H[(size_t)(jk - 1) * ld + (jk - 1)];
-    gm->y[jk - 1] = y;
-    for (int lk = 1; lk <= jk - 1; ++lk) gm->e[lk - 1] = gm->e[lk - 1] - y * gm->H[(size_t)(jk - 1) * ld + (lk - 1)];
+  for (int c = threadIdx.x; c < ncol; c += ORTH_THREADS) {
+    const int o = c < k ? c : kk + c - k;
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < ORTH_WARPS; ++q) s += acc[2 * kk * q + o];
+    col[(size_t)c * G + b] = s;
+  }
+  grid.sync();
+  // ---- the dots, added over the blocks in the same order everywhere (four
+  // columns of a warp's share in flight)
+  const double sk = gm->sc[k - 1];
+  for (int c0 = wid; c0 < ncol; c0 += 4 * ORTH_WARPS) {
+    double s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = c0 + u * ORTH_WARPS;
+      s[u] = 0.0;
+      if (c < ncol)
+        for (int q = lane; q < G; q += 32) s[u] += __ldcg(col + (size_t)c * G + q);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = c0 + u * ORTH_WARPS;
+      const double t = warp_sum(s[u]);
+      if (lane == 0 && c < ncol) {
+        if (c < k) as[c] = t * gm->sc[c];
+        else gs[c - k] = t * sk * gm->sc[c - k];
+      }
+    }
+  }
+  __syncthreads();
+  // ---- h = T V^T w (rows 0..k-2 of T; the last row is direct)
+  const int ks = gm->kspace;
+  for (int j0 = wid; j0 < k - 1; j0 += 4 * ORTH_WARPS) {
+    double s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = j0 + u * ORTH_WARPS;
+      s[u] = 0.0;
+      if (j < k - 1)
+        for (int c = lane; c < j; c += 32) s[u] += __ldcg(T + (size_t)j * ks + c) * as[c];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = j0 + u * ORTH_WARPS;
+      const double t = warp_sum(s[u]);
+      if (lane == 0 && j < k - 1) {
+        hh[j] = as[j] + t;
+        hs[j] = hh[j] * gm->sc[j];
+      }
+    }
+  }
+  __syncthreads();
+  if (wid == 0) {
+    double t = 0.0;
+    for (int j = lane; j < k - 1; j += 32) t += gs[j] * hh[j];
+    t = warp_sum(t);
+    if (lane == 0) {
+      hh[k - 1] = as[k - 1] - t;
+      hs[k - 1] = hh[k - 1] * sk;
+    }
+  }
+  __syncthreads();
+  // ---- phase B: the update and its norm
+  double na = 0.0;
+  const int cnt = gw < nsc ? (nsc - gw + W - 1) / W : 0;
+  for (int r = cnt - 1; r >= 0; --r) {
+    const size_t i = ((size_t)(gw + (long)r * W) * 32 + lane) * V;
+    TV wv[V];
+    orth_ld<V>(w, i, n, wv);
+    constexpr int JB = V == 1 ? 2 * JG : JG;
+    for (int j0 = 0; j0 < k; j0 += JB) {
+      TV x[JB][V];
+#pragma unroll
+      for (int u = 0; u < JB; ++u) orth_ld<V>(basis + ld * (size_t)min(j0 + u, k - 1), i, n, x[u]);
+#pragma unroll
+      for (int u = 0; u < JB; ++u) {
+        const TV h = j0 + u < k ? (TV)hs[j0 + u] : (TV)0;
+#pragma unroll
+        for (int q = 0; q < V; ++q) wv[q] = fma(-h, x[u][q], wv[q]);
+      }
+    }
+    if (V == 4 && i + 4 <= n) {
+      if constexpr (V == 4) {
+        const double d[4] = {(double)wv[0], (double)wv[1], (double)wv[2], (double)wv[3]};
+        st4v(w + i, d);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < V; ++q)
+        if (i + q < n) w[i + q] = wv[q];
+    }
+#pragma unroll
+    for (int q = 0; q < V; ++q) na += (double)wv[q] * (double)wv[q];
+  }
+  na = warp_sum(na);
+  if (lane == 0) sh[wid] = na;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int q = 0; q < ORTH_WARPS; ++q) s += sh[q];
+    nrm[b] = s;
+    __threadfence();
+    is_last = atomicAdd(&gm->counter, 1) == G - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  // ---- the last block: norm, Givens rotations (one thread, its data staged
+  // in shared memory) and the new row of T (the other warps)
+  double* Hk = gm->H + (size_t)(k - 1) * (ks + 1);
+  for (int j = threadIdx.x; j < k - 1; j += ORTH_THREADS) { cs[j] = gm->cs[j]; sn[j] = gm->sn[j]; }
+  if (wid == 0) {
+    double s = 0.0;
+    for (int q = lane; q < G; q += 32) s += __ldcg(nrm + q);
+    s = warp_sum(s);
+    if (lane == 0) sh[0] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double unorm = sqrt(sh[0]);
+    gm->counter = 0;
+    gm->beta = sh[0];
+    gm->sc[k] = unorm != 0.0 ? 1.0 / unorm : 1.0;
+    givens_step(gm, k, unorm, hh, cs, sn);
+  } else if (wid > 0 && k > 1) {
+    // t_c = -(g_c + sum_{j>c} g_j T_jc), T's diagonal being 1; up to eight
+    // threads share a column's sum
+    const int cols = k - 1, t = threadIdx.x - 32, parts = max(1, min(8, (ORTH_THREADS - 32) / cols));
+    for (int u = t; u < cols * parts; u += ORTH_THREADS - 32) {
+      const int q = u / cols, c = u - q * cols;
+      double s = q == 0 ? gs[c] : 0.0;
+#pragma unroll 4
+      for (int j = c + 1 + q; j < cols; j += parts) s += gs[j] * __ldcg(T + (size_t)j * ks + c);
+      acc[u] = s;
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += ORTH_THREADS) Hk[j] = hh[j];
+  const int parts = k > 1 ? max(1, min(8, (ORTH_THREADS - 32) / (k - 1))) : 0;
+  for (int c = threadIdx.x; c < k - 1; c += ORTH_THREADS) {
+    double s = 0.0;
+    for (int q = 0; q < parts; ++q) s += acc[q * (k - 1) + c];
+    T[(size_t)(k - 1) * ks + c] = -s;
   }
 }
 
-// sol += sum_j y_j v_j (SparseGMRES_NS.f90:349-352)
+// back-substitution (SparseGMRES_NS.f90:341-346): one block, thread l holds
+// e(l); the columns of H are loaded eight at a time ahead of the steps that
+// use them.  y_j comes out times the scale of slot j.
+constexpr int BACKSUB_THREADS = 416;
+static_assert(BACKSUB_THREADS >= OVS_MAX_KSPACE, "one thread per unknown");
+__global__ void __launch_bounds__(BACKSUB_THREADS) gm_backsub_kernel(GmresDev* gm) {
+  __shared__ double ys;
+  const int iks = gm->iks, ld = gm->kspace + 1, t = threadIdx.x;
+  double e = t < iks ? gm->e[t] : 0.0;
+  for (int j1 = iks; j1 > 0; j1 -= 8) {
+    double h[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int j = j1 - 1 - u;
+      h[u] = j >= 0 && t <= j ? gm->H[(size_t)j * ld + t] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int j = j1 - 1 - u;
+      if (j < 0) break;
+      if (t == j) ys = e / h[u];
+      __syncthreads();
+      const double y = ys;
+      if (t == j) gm->y[j] = y * gm->sc[j];
+      else if (t < j) e = e - y * h[u];
+      __syncthreads();
+    }
+  }
+}
+
+// sol += sum_j y_j v_j (SparseGMRES_NS.f90:349-352), eight vectors' loads in
+// flight per value
 template <typename TV>
-__global__ void gm_update_kernel(double* __restrict__ sol, const TV* __restrict__ basis, size_t n, size_t ld,
-                                 const GmresDev* __restrict__ gm) {
+__global__ void __launch_bounds__(256)
+gm_update_kernel(double* __restrict__ sol, const TV* __restrict__ basis, size_t n, size_t ld,
+                 const GmresDev* __restrict__ gm) {
+  __shared__ double y[OVS_MAX_KSPACE];
   const int iks = gm->iks;
+  for (int j = threadIdx.x; j < iks; j += blockDim.x) y[j] = gm->y[j];
+  __syncthreads();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double s = sol[i];
-    for (int j = 0; j < iks; ++j) s = s + gm->y[j] * (double)basis[(size_t)j * ld + i];
+    int j = 0;
+    for (; j + 8 <= iks; j += 8) {
+      TV x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = __ldcs(basis + (size_t)(j + u) * ld + i);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s = s + y[j + u] * (double)x[u];
+    }
+    for (; j < iks; ++j) s = s + y[j] * (double)basis[(size_t)j * ld + i];
     sol[i] = s;
   }
 }
@@ -1027,15 +1009,17 @@ int ensure_basis(ovs_ctx* c, int prec, size_t bytes) {
   return OVS_OK;
 }
 
-// Launch plan of one Arnoldi iteration.  Default: the preconditioned SpMV
-// as an ordinary launch, then gm_mgs_onchip_kernel (one 512-thread block
-// per SM, cooperative).  fused = 1 (environment OVS_ARNOLDI_FUSED=1, or when
-// the on-chip kernel cannot be made co-resident): gm_arnoldi_kernel alone.
+// Launch plan of the Arnoldi iterations of a cycle.  Default: the
+// preconditioned SpMV as an ordinary launch, then gm_orthog_kernel (one
+// 512-thread block per SM at most, cooperative).  fused = 1 (environment
+// OVS_ARNOLDI_FUSED=1, or when the blocks cannot be made co-resident):
+// gm_arnoldi_kernel alone.
 struct ArnoldiPlan {
   bool fused = false;
   int grid = 0;
-  size_t chunk = 0, smem_bytes = 0;
-  int spieces = 0;
+  bool wide = false;   // V = 4
+  int nsc = 0;         // sub-chunks of 32 V values
+  double* T = nullptr;
 };
 
 template <typename TM, typename TV, bool ACC64>
@@ -1049,39 +1033,47 @@ ArnoldiKern<TM, TV, ACC64> fused_kernel(int sys) {
   return gm_arnoldi_kernel<TM, TV, OVS_SYS_TEM, ACC64>;
 }
 
+template <typename TV>
+auto orthog_kernel(bool wide) {
+  return wide ? gm_orthog_kernel<TV, 4> : gm_orthog_kernel<TV, 1>;
+}
+
+// warps that share a sub-chunk's groups of vectors at step k
+inline int orth_split(const ArnoldiPlan& pl, int k, int sms) {
+  const int groups = (k + JG - 1) / JG, room = std::max(1, sms * ORTH_WARPS / std::max(1, pl.nsc));
+  return std::min(groups, room);
+}
+
 template <typename TM, typename TV, bool ACC64>
-int plan_arnoldi(ovs_ctx* c, int sys, size_t n, bool want_fused, ArnoldiPlan* pl) {
+int plan_arnoldi(ovs_ctx* c, int sys, size_t n, int kspace, bool want_fused, ArnoldiPlan* pl) {
   int st;
-  if ((st = ovs_ensure((void**)&c->coop_part, sizeof(double) * 2 * OVS_COOP_MAX_BLOCKS))) return st;
+  // the partial sums (fused variant: two per block; gm_orthog_kernel: 2 k per
+  // block), then T, kspace x kspace; kept by the context, grown when needed
+  const size_t parts = std::max((size_t)2 * OVS_COOP_MAX_BLOCKS, (size_t)2 * kspace * c->num_sms);
+  const size_t need = sizeof(double) * (parts + (size_t)kspace * kspace);
+  if (c->coop_bytes < need) {
+    if (c->coop_part) cudaFree(c->coop_part);
+    c->coop_part = nullptr;
+    c->coop_bytes = 0;
+    if ((st = ovs_ensure((void**)&c->coop_part, need))) return st;
+    c->coop_bytes = need;
+  }
+  pl->T = c->coop_part + parts;
   pl->fused = want_fused;
   if (!want_fused) {
-    const int G = c->num_sms;
-    const size_t chunk = ((n + G - 1) / G + 3) & ~(size_t)3;
-    const size_t rcap = (size_t)TmemGeom<TV>::cap;
-    int optin = 0;
-    OVS_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    const size_t pv = PieceGeom<TV>::values, pbytes = PieceGeom<TV>::bytes;
-    const size_t max_sp = optin > 2048 ? (size_t)(optin - 2048) / pbytes : 0;   // room for static smem
-    const size_t want = chunk > rcap ? (chunk - rcap + pv - 1) / pv : 0;
-    const size_t sp = want < max_sp ? want : max_sp;
-    // The kernel takes all 512 tensor-memory columns of its SM, so two of
-    // its blocks must never share an SM (the second allocation would wait
-    // for the first block, which waits for it in grid.sync): request more
-    // than half of the SM's shared memory and require exactly one block.
-    const size_t min_bytes = 118784;
-    const size_t bytes = sp * pbytes > min_bytes ? sp * pbytes : min_bytes;
-    auto kern = gm_mgs_onchip_kernel<TV>;
-    if ((size_t)optin >= bytes + 512 && chunk < ((size_t)1 << 30)) {
-      OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-      int per_sm = 0;
-      OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ONCHIP_THREADS, bytes));
-      if (per_sm == 1) {
-        pl->grid = G;
-        pl->chunk = chunk;
-        pl->spieces = (int)sp;
-        pl->smem_bytes = bytes;
-        return OVS_OK;
-      }
+    // V = 4 once it gives every warp of the chip a sub-chunk
+    pl->wide = n >= (size_t)128 * ORTH_WARPS * c->num_sms;
+    const size_t per = pl->wide ? 128 : 32, nsc = (n + per - 1) / per;
+    auto kern = orthog_kernel<TV>(pl->wide);
+    const size_t bytes = orth_smem(kspace);
+    int per_sm = 0;
+    OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ORTH_THREADS, bytes));
+    if (per_sm >= 1 && nsc < ((size_t)1 << 31)) {
+      pl->nsc = (int)nsc;
+      const long items = (long)nsc * orth_split(*pl, kspace, c->num_sms);
+      pl->grid = (int)std::min((long)c->num_sms, (items + ORTH_WARPS - 1) / ORTH_WARPS);
+      return OVS_OK;
     }
     pl->fused = true;
   }
@@ -1111,14 +1103,14 @@ int launch_arnoldi(ovs_ctx* c, int sys, const ArnoldiPlan& pl, const TM* vals, c
     return OVS_OK;
   }
   int st = launch_spmv<TM, TV, TV, 1, ACC64>(c, sys, vals, V + ld * (size_t)(k - 1), V + ld * (size_t)k, pre,
-                                               nullptr, &gm->done);
+                                               nullptr, &gm->done, gm->sc + (k - 1));
   if (st) return st;
-  int kk = k;
-  size_t ldv = ld, nn = n, ch = pl.chunk;
-  int sp = pl.spieces;
-  void* args[] = {&V, &ldv, &nn, &kk, &gm, &part, &ch, &sp};
-  OVS_CUDA_TRY(cudaLaunchCooperativeKernel((void*)gm_mgs_onchip_kernel<TV>, pl.grid, ONCHIP_THREADS, args,
-                                           pl.smem_bytes, c->stream));
+  int kk = k, nsc = pl.nsc, js = orth_split(pl, k, c->num_sms);
+  size_t ldv = ld, nn = n;
+  double* T = pl.T;
+  void* args[] = {&V, &ldv, &nn, &kk, &gm, &part, &T, &nsc, &js};
+  OVS_CUDA_TRY(cudaLaunchCooperativeKernel((void*)orthog_kernel<TV>(pl.wide), pl.grid, ORTH_THREADS, args,
+                                           orth_smem(k), c->stream));
   ++c->launches;
   return OVS_OK;
 }
@@ -1161,20 +1153,26 @@ int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol,
   OVS_CUDA_TRY(cudaGetLastError());
   // one Arnoldi iteration per step (see ArnoldiPlan)
   ArnoldiPlan pl;
-  if ((st = plan_arnoldi<TM, TV, ACC64>(c, sys, n, c->arnoldi_fused, &pl))) return st;
-  const int batch = N > 200000 ? 4 : 16;
-  int k = 1;
-  for (; k <= kspace;) {
+  if ((st = plan_arnoldi<TM, TV, ACC64>(c, sys, n, kspace, c->arnoldi_fused, &pl))) return st;
+  // the host reads the done word of a batch while the next one runs; what is
+  // queued after the end of the cycle returns at once
+  const int batch = N > 200000 ? 4 : 8;
+  c->h_pinned[0] = c->h_pinned[1] = 0;
+  for (int k = 1, q = 0; k <= kspace; ++q) {
     const int kend = (k + batch - 1 < kspace) ? k + batch - 1 : kspace;
     for (; k <= kend; ++k)
       if ((st = launch_arnoldi<TM, TV, ACC64>(c, sys, pl, vals, pre, V, ld, n, k))) return st;
-    OVS_CUDA_TRY(cudaMemcpyAsync(c->h_pinned, &gm->done, sizeof(int), cudaMemcpyDeviceToHost, s));
-    OVS_CUDA_TRY(cudaStreamSynchronize(s));
-    if (c->h_pinned[0]) break;
+    if (k > kspace) break;
+    OVS_CUDA_TRY(cudaMemcpyAsync(c->h_pinned + (q & 1), &gm->done, sizeof(int), cudaMemcpyDeviceToHost, s));
+    OVS_CUDA_TRY(cudaEventRecord(c->ev_poll[q & 1], s));
+    if (q > 0) {
+      OVS_CUDA_TRY(cudaEventSynchronize(c->ev_poll[(q - 1) & 1]));
+      if (c->h_pinned[(q - 1) & 1]) break;
+    }
   }
-  gm_backsub_kernel<<<1, 1, 0, s>>>(gm);
+  gm_backsub_kernel<<<1, BACKSUB_THREADS, 0, s>>>(gm);
   ++c->launches;
-  gm_update_kernel<TV><<<ovs_grid(n, 256, 4 * c->num_sms * 8), 256, 0, s>>>(sol, V, n, ld, gm);
+  gm_update_kernel<TV><<<ovs_grid(n, 256, 8 * c->num_sms), 256, 0, s>>>(sol, V, n, ld, gm);
   ++c->launches;
   OVS_CUDA_TRY(cudaGetLastError());
   if (info) {
@@ -1228,11 +1226,16 @@ int profile_krylov_t(ovs_ctx* c, int what, int sys, int reps, double* ms) {
   int km[2] = {kspace, 1};
   OVS_CUDA_TRY(cudaMemcpyAsync(&gm->kspace, km, sizeof(km), cudaMemcpyHostToDevice, c->stream));
   OVS_CUDA_TRY(cudaMemsetAsync(&gm->done, 0, sizeof(int), c->stream));
-  OVS_CUDA_TRY(cudaMemsetAsync(&gm->epsnrm, 0, sizeof(double), c->stream));
+  // no exit test passes, and the slots hold what they hold
+  const double eps = -1.0;
+  const std::vector<double> ones(OVS_MAX_KSPACE + 1, 1.0);
+  OVS_CUDA_TRY(cudaMemcpyAsync(&gm->epsnrm, &eps, sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  OVS_CUDA_TRY(cudaMemcpyAsync(gm->sc, ones.data(), sizeof(gm->sc), cudaMemcpyHostToDevice, c->stream));
   const TM* vals = as<TM>(S.vals);
   const TM* pre = as<TM>(S.binv);
   ArnoldiPlan pl;
-  if ((st = plan_arnoldi<TM, TM, ACC64>(c, sys, n, what == OVS_PROF_ARNOLDI_FUSED, &pl))) return st;
+  if ((st = plan_arnoldi<TM, TM, ACC64>(c, sys, n, kspace, what == OVS_PROF_ARNOLDI_FUSED, &pl))) return st;
+  OVS_CUDA_TRY(cudaMemsetAsync(pl.T, 0, sizeof(double) * kspace * kspace, c->stream));
   auto run = [&]() -> int {
     if (what == OVS_PROF_SPMV) {
       st = launch_spmv<TM, TM, TM, 1, ACC64>(c, sys, vals, V, V + ld, pre, nullptr, nullptr);

@@ -54,6 +54,7 @@ struct GmresDev {
   double y[OVS_MAX_KSPACE];
   double partials[OVS_RED_BLOCKS];
   double scal[8];     // misc scalar results (norms)
+  double sc[OVS_MAX_KSPACE + 1];   // scale of each basis slot (1 / norm of what it holds)
 };
 
 // one boundary of setBCs_NSVOF / setBCs_Tem with its types (read by FACE_ID)
@@ -78,6 +79,7 @@ struct ovs_ctx {
   int num_sms = 148;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev_poll[2] = {nullptr, nullptr};   // the done word of a batch of Krylov iterations has arrived
   int N = 0, E = 0, nshl = 0;
   // mesh
   int* ien = nullptr;        // E*nshl, element-major, 0-based
@@ -176,7 +178,8 @@ struct ovs_ctx {
   double* work64 = nullptr;              // 3 vectors of 5N doubles (b, r, x)
   float* work32 = nullptr;               // 1 vector of 5N floats
   double* wvec = nullptr;                // FP64 vector under orthogonalization
-  double* coop_part = nullptr;           // partial sums of the cooperative Arnoldi kernels
+  double* coop_part = nullptr;           // partial sums of the cooperative Arnoldi kernels, then T = (I + L)^-1
+  size_t coop_bytes = 0;                 //   (rows of kspace, strictly lower part)
   bool arnoldi_fused = false;            // one-launch Arnoldi variant (env OVS_ARNOLDI_FUSED=1)
   // status words: [0] negative DetJ count, [1] non-finite flag, [3] face column missing from a row
   int* flags = nullptr;
