@@ -434,7 +434,7 @@ __device__ __forceinline__ void element_geometry(const RA& r, const LA& lo, T g[
 
 // pass 1, NS-only: IntElmAss_NS_overset's Gauss loop with e3LHS_3D_fluid_Old /
 // e3Rhs_3D_fluid (quirks: uprime = 0, kap_dc = NS_kdc_a, tauBar = 0)
-template <typename T, typename RA, typename LA>
+template <typename T, bool MAT = true, typename RA, typename LA>
 __device__ void summarize_ns(const SumArgs& a, const RA& r, const LA& lo, bool target, T* o,
                              double& tamax, T& detj_out) {
   const ovs_params& p = a.p;
@@ -499,10 +499,11 @@ __device__ void summarize_ns(const SumArgs& a, const RA& r, const LA& lo, bool t
     }
   }
   using L = Lay<OVS_ASM_NS>;
+  T* orh = o + (MAT ? L::RHS0 : 0);
 #pragma unroll
-  for (int n = 0; n < 4; ++n) put4(o + L::RHS0 + 4 * n, ru[n][0], ru[n][1], ru[n][2], rp[n]);
-  put4(o + L::C0, KA, KB, MM, (T)0);
-  if constexpr (!std::is_same<T, Dual>::value)
+  for (int n = 0; n < 4; ++n) put4(orh + 4 * n, ru[n][0], ru[n][1], ru[n][2], rp[n]);
+  if constexpr (MAT) put4(o + L::C0, KA, KB, MM, (T)0);
+  if constexpr (MAT && !std::is_same<T, Dual>::value)
     block_sums<T, OVS_ASM_NS>(q, g, target ? w : (T)0, (T)p.almi, fact2, rho, o);
 }
 
@@ -654,7 +655,7 @@ __device__ __forceinline__ void nsvof_node_terms(const T (&g)[4][3], const T (&d
 // pass 1, NS+VOF quench (src/solveQuenching.f90:295-523), one thread per
 // element: geometry and gradients, the four Gauss points (nsvof_point),
 // then the residual rows, the element constants and the block sums
-template <typename T, typename RA, typename LA>
+template <typename T, bool MAT = true, typename RA, typename LA>
 __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, bool fluid, T* o,
                                 double& tamax, T& detj_out) {
   using W = typename Wide<T>::type;
@@ -709,11 +710,13 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
       rh[5 * n + 3] = rp[n]; rh[5 * n + 4] = rf[n];
     }
 #pragma unroll
-    for (int k = 0; k < 20; k += 4) put4(o + L::RHS0 + k, rh[k], rh[k + 1], rh[k + 2], rh[k + 3]);
+    for (int k = 0; k < 20; k += 4) put4(o + (MAT ? L::RHS0 : 0) + k, rh[k], rh[k + 1], rh[k + 2], rh[k + 3]);
   }
-  put4(o + L::C0, KA, KB, MM, KDP);
-  put4(o + L::C0 + 4, dphi[0], dphi[1], dphi[2], (T)0);
-  if constexpr (!std::is_same<T, Dual>::value)
+  if constexpr (MAT) {
+    put4(o + L::C0, KA, KB, MM, KDP);
+    put4(o + L::C0 + 4, dphi[0], dphi[1], dphi[2], (T)0);
+  }
+  if constexpr (MAT && !std::is_same<T, Dual>::value)
     block_sums<T, OVS_ASM_NSVOF>(q, g, fluid ? w : (T)0, (T)p.almi, (T)(p.alfi * p.delt * p.gami), (T)0, o);
 }
 
@@ -725,7 +728,7 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
 // elements take uadv = dSe = trc = 0, which turns the fluid block formula
 // into the solid one.  The adjoint instantiation (dual numbers) needs the
 // residual only and skips the matrix.
-template <typename T, typename RA, typename LA>
+template <typename T, bool MAT = true, typename RA, typename LA>
 __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool fluid, T* o,
                               double& tamax, T& detj_out) {
   using W = typename Wide<T>::type;
@@ -797,7 +800,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
     T kdcT = 0;
     if (kdc_on && fluid) kdcT = (T)p.tem_kdc * fabs(res) * iv.sGG * iv.tref;
     const T dSe = (cpw - cpa) * mdot + ((cpw - cpa) * (Ti - ts) - lh) * dmdT;
-    if constexpr (!std::is_same<T, Dual>::value) {
+    if constexpr (MAT && !std::is_same<T, Dual>::value) {
       const T uq[3] = {fluid ? uadv[0] : (T)0, fluid ? uadv[1] : (T)0, fluid ? uadv[2] : (T)0};
       const T dSq = fluid ? dSe : (T)0, trq = fluid ? tauT * rcp : (T)0;
       T cq[4];
@@ -823,7 +826,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
       for (int n = 0; n < 4; ++n) rt[n] += w * (-N[n] * rcp * rTi - hk * gdT[n]);
     }
   }
-  if constexpr (!std::is_same<T, Dual>::value) {
+  if constexpr (MAT && !std::is_same<T, Dual>::value) {
 #pragma unroll
     for (int ia = 0; ia < 4; ++ia)
 #pragma unroll
@@ -831,7 +834,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
         o[4 * ia + ib] = K[ia][ib] + HK * (g[ia][0] * g[ib][0] + g[ia][1] * g[ib][1] + g[ia][2] * g[ib][2]);
   }
 #pragma unroll
-  for (int n = 0; n < 4; ++n) o[Lay<OVS_ASM_TEM>::RHS0 + n] = rt[n];
+  for (int n = 0; n < 4; ++n) o[(MAT ? Lay<OVS_ASM_TEM>::RHS0 : 0) + n] = rt[n];
 }
 
 // -------------------------------------------------- pass 2: block expansion
@@ -1016,10 +1019,13 @@ template <typename T, int KIND, bool SMEMREC> struct SumBlocks { static constexp
 // blocks and 10.2 ms at 4)
 template <int KIND> struct SumBlocks<double, KIND, true> { static constexpr int v = 2; };
 
-template <typename T, int KIND, bool SMEMREC>
-__global__ void __launch_bounds__(128, (SumBlocks<T, KIND, SMEMREC>::v))
+// MAT false (vector-only pass): the summary is the residual rows alone, 4 NF
+// values per element.
+template <typename T, int KIND, bool SMEMREC, bool MAT = true>
+__global__ void __launch_bounds__(128, (MAT ? SumBlocks<T, KIND, SMEMREC>::v : SMEMREC ? 3 : 1))
 element_summary_kernel(const SumArgs a) {
   using L = Lay<KIND>;
+  constexpr int SW = MAT ? L::SW : 4 * L::NF;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   double tamax = 0.0;   // the element's largest taua over its points (CflPerPoint: largest CFL number)
   int nbad = 0;
@@ -1033,11 +1039,11 @@ element_summary_kernel(const SumArgs a) {
       if constexpr (KIND == OVS_ASM_NS) {
         const bool target = ((a.p.subdomain_flag & 1) && eid == a.p.elm_id_set[0]) ||
                             ((a.p.subdomain_flag & 2) && eid == a.p.elm_id_set[1]);
-        summarize_ns<T>(a, r, lo, target, o, tamax, detj);
+        summarize_ns<T, MAT>(a, r, lo, target, o, tamax, detj);
       } else if constexpr (KIND == OVS_ASM_NSVOF) {
-        summarize_nsvof<T>(a, r, lo, eid == a.p.fluid_elm_id, o, tamax, detj);
+        summarize_nsvof<T, MAT>(a, r, lo, eid == a.p.fluid_elm_id, o, tamax, detj);
       } else {
-        summarize_tem<T>(a, r, lo, eid == a.p.fluid_elm_id, o, tamax, detj);
+        summarize_tem<T, MAT>(a, r, lo, eid == a.p.fluid_elm_id, o, tamax, detj);
       }
     };
     if constexpr (SMEMREC && sizeof(T) == 8) {
@@ -1055,27 +1061,27 @@ element_summary_kernel(const SumArgs a) {
           col[(size_t)(n * 16 + 2 * k + 1) * 128] = v.y;
         }
       }
-      run(SmemRecs<T>{col}, ZeroRecs<T>{}, reinterpret_cast<T*>(a.sum) + (size_t)e * L::SW);
+      run(SmemRecs<T>{col}, ZeroRecs<T>{}, reinterpret_cast<T*>(a.sum) + (size_t)e * SW);
     } else {
       T r[4][16], lo[4][4];
 #pragma unroll
       for (int n = 0; n < 4; ++n) load_rec(rec, nodes[n], r[n], lo[n]);
       if constexpr (KIND == OVS_ASM_TEM) {
-        T o[L::SW];
+        T o[SW];
         run(r, lo, o);
-        // 20 values per tet: 5 groups of 4 (256-bit stores in FP64, the
+        // 20 values per tet (vector-only: 4): groups of 4 (256-bit stores in FP64, the
         // summary 32-byte aligned; 2.45 against 2.52 ms at 128^3)
-        T* dst = reinterpret_cast<T*>(a.sum) + (size_t)e * L::SW;
+        T* dst = reinterpret_cast<T*>(a.sum) + (size_t)e * SW;
         if constexpr (sizeof(T) == 8) {
 #pragma unroll
-          for (int k = 0; k < L::SW; k += 4) put4(dst + k, o[k], o[k + 1], o[k + 2], o[k + 3]);
+          for (int k = 0; k < SW; k += 4) put4(dst + k, o[k], o[k + 1], o[k + 2], o[k + 3]);
         } else {
-          store_row<L::SW>(dst, o);
+          store_row<SW>(dst, o);
         }
       } else {
         // NS / NS+VOF write their summary with vector stores as its parts
         // are formed
-        run(r, lo, reinterpret_cast<T*>(a.sum) + (size_t)e * L::SW);
+        run(r, lo, reinterpret_cast<T*>(a.sum) + (size_t)e * SW);
       }
     }
     if (!(detj > (T)0)) nbad = 1;
@@ -1274,7 +1280,7 @@ assemble_rows_kernel(const AsmArgs a) {
       s4_n = __ldg(a.n2s + rn.z + lane);
     }
     // ---------------- row write with the Dirichlet treatment
-    if (a.mat) {
+    {
       if (lane < deg) cib[lane] = ib0;
       if (lane + 32 < deg) cib[lane + 32] = ib1;
       for (int s = lane + 64; s < deg; s += 32) cib[s] = __ldg(a.ibc + cols[s]);
@@ -1500,7 +1506,7 @@ __device__ __forceinline__ void gather_row(const AsmArgs& a, const int4 rr, cons
     }
     __syncwarp();
     // output tasks (entry j, group g): the entry's pieces added in order
-    if (a.mat && deg > 0) {
+    if (deg > 0) {
       const int nt = (nsl + (wd ? 1 : 0)) * NG;
       for (int q = lane; q < nt; q += 32) {
         const int j = q / NG, g = q - j * NG;
@@ -1618,7 +1624,7 @@ __device__ __forceinline__ void gather_row_il(const AsmArgs& a, const int4 rr, c
         }
       }
     }
-    if (offl && a.mat) write_block<T, NV>(out + (size_t)s * NV, acc, masks, ibA, ibB, false, cnt);
+    if (offl) write_block<T, NV>(out + (size_t)s * NV, acc, masks, ibA, ibB, false, cnt);
     if (o0 == 0) {
       if (diagl) {
 #pragma unroll
@@ -1628,7 +1634,7 @@ __device__ __forceinline__ void gather_row_il(const AsmArgs& a, const int4 rr, c
       }
       __syncwarp();
       constexpr int NG = NV >= 4 ? NV / 4 : 1;
-      if (a.mat && deg > 0 && lane < NG) {
+      if (deg > 0 && lane < NG) {
         constexpr int GW = NV >= 4 ? 4 : 1;
         T v4[GW];
 #pragma unroll
@@ -1682,6 +1688,44 @@ __global__ void __launch_bounds__(128) gather_rows_kernel(const AsmArgs a) {
                                     lane);
     else
       gather_row<T, KIND, false>(a, __ldg(a.row_rec + t), sum, Lay<KIND>::SW, nullptr, nullptr, gw[wid], masks, lane);
+}
+
+// Row pass of a vector-only assembly (tets and hexahedra): 8 lanes per node
+// add the element residuals of the node's elements, lane l the elements l,
+// l + 8, ... of its ascending list, then the lanes' sums by halving, an order
+// fixed by the mesh.  The residual evaluations of a Newton loop ask for no
+// matrix; the full row pass formed every block for them (48x48x96 cells x6
+// tets, FP64, both passes: 2.19 ms; this way 0.63 ms).
+template <typename T, int NF>
+__global__ void __launch_bounds__(256) residual_rows_kernel(const AsmArgs a, int nshl, bool tem) {
+  const int lane = threadIdx.x & 31, l8 = lane & 7;
+  const int A = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 3);
+  const bool on = A < a.N;
+  const T* sum = reinterpret_cast<const T*>(a.rec);
+  T r[NF];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) r[f] = (T)0;
+  if (on) {
+    const int ep = __ldg(a.n2e_ptr + A), ee = __ldg(a.n2e_ptr + A + 1);
+    for (int q = ep + l8; q < ee; q += 8) {
+      const int pk = __ldg(a.n2e + q);
+      const T* p = sum + ((size_t)(pk >> 3) * nshl + (pk & 7)) * NF;
+#pragma unroll
+      for (int f = 0; f < NF; ++f) r[f] += __ldg(p + f);
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) r[f] += __shfl_xor_sync(0xffffffffu, r[f], o);
+  if (!on || l8 >= NF) return;
+  T v = r[0];
+#pragma unroll
+  for (int f = 1; f < NF; ++f) v = l8 == f ? r[f] : v;
+  const unsigned bit = tem ? TB : (l8 < 3 ? 1u << l8 : (l8 == 3 ? PB : FB));
+  if (__ldg(a.ibc + A) & bit) v = (T)0;
+  if (!isfinite((double)v)) atomicOr(a.flags + 1, 1);
+  reinterpret_cast<T*>(a.rhs)[(size_t)l8 * a.N + A] = v;
 }
 
 // ---------------------------------------------------------- tiled row pass
@@ -1868,9 +1912,38 @@ int launch_tiled(ovs_ctx* c, const AsmArgs& a) {
   return OVS_OK;
 }
 
+template <typename T, int NF>
+int launch_residual_rows(ovs_ctx* c, const AsmArgs& a, bool tem) {
+  residual_rows_kernel<T, NF><<<ovs_grid((size_t)c->N * 8, 256, 1 << 30), 256, 0, c->stream>>>(a, c->nshl, tem);
+  ++c->launches;
+  OVS_CUDA_TRY(cudaGetLastError());
+  return OVS_OK;
+}
+
+// vector-only pass: the element residuals, then their sums per node.  The
+// node records stay in registers unless the option asks for shared memory:
+// without the matrix values that is the faster one in FP64 too (NS+VOF, both
+// kernels and the alpha stage: 3.33 against 3.69 ms at 128^3, 0.41 against
+// 0.45 ms at 48x48x96).
+template <typename T, int KIND>
+int launch_residual(ovs_ctx* c, const AsmArgs& a, const SumArgs& sa) {
+  if (sizeof(T) == 8 && c->elem_smem > 0) {
+    const size_t esm = sizeof(T) * 64 * 128;
+    OVS_CUDA_TRY(cudaFuncSetAttribute(element_summary_kernel<T, KIND, true, false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esm));
+    element_summary_kernel<T, KIND, true, false><<<(sa.E + 127) / 128, 128, esm, c->stream>>>(sa);
+  } else {
+    element_summary_kernel<T, KIND, false, false><<<(sa.E + 127) / 128, 128, 0, c->stream>>>(sa);
+  }
+  ++c->launches;
+  OVS_CUDA_TRY(cudaGetLastError());
+  return launch_residual_rows<T, Lay<KIND>::NF>(c, a, KIND == OVS_ASM_TEM);
+}
+
 // parts: bit 0 the element pass, bit 1 the row pass
 template <typename T, int KIND>
 int launch_assemble(ovs_ctx* c, const AsmArgs& a, const SumArgs& sa, int parts = 3) {
+  if (!a.mat) return launch_residual<T, KIND>(c, a, sa);
   // pass 1: element summaries
   if (parts & 1) {
     if (sizeof(T) == 8 && (c->elem_smem > 0 || (c->elem_smem < 0 && KIND == OVS_ASM_NSVOF))) {

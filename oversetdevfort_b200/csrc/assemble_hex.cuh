@@ -111,13 +111,14 @@ __device__ __forceinline__ void store_n(T* dst, const T* v, int n) {
 }
 
 // element pass, NS+VOF quench on a hex (src/solveQuenching.f90:295-523);
-// TC: write the compact records of the tensor-core matrix pass instead
-template <typename T, bool TC = false>
+// TC: write the compact records of the tensor-core matrix pass instead; MAT
+// false (vector-only pass): the residual rows alone
+template <typename T, bool TC = false, bool MAT = true>
 __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const T lo[8][4], bool fluid,
                                     T* out, double& tamax, int& nbad) {
   using W = typename Wide<T>::type;
   using L = HexLay<OVS_ASM_NSVOF>;
-  constexpr int RHS0 = TC ? HexTcLay::RHS0 : L::RHS0;
+  constexpr int RHS0 = !MAT ? 0 : TC ? HexTcLay::RHS0 : L::RHS0;
   const T fact2 = (T)(p.alfi * p.delt * p.gami);
   const T taut = (T)(4.0 / (p.delt * p.delt));
   const T rhoa = (T)p.rhoa, rhow = (T)p.rhow, ts = (T)p.ts;
@@ -220,7 +221,8 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
     const T mupk = mu + kdc;
     const T dmdi = dmd * ira;
     const T wf = fluid ? w : (T)0;   // solid elements contribute nothing
-    if constexpr (TC) {
+    if constexpr (!MAT) {
+    } else if constexpr (TC) {
       T rec[HexTcLay::GPW];
 #pragma unroll
       for (int k = 0; k < 3; ++k)
@@ -294,7 +296,7 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
 
 // element pass, temperature on a hex (src/solveQuenching.f90:712-856);
 // record layout of this pass: xd(0:2) u(3:5) um(6:8) phi(9) T(10) rT(11)
-template <typename T>
+template <typename T, bool MAT = true>
 __device__ void hex_summarize_tem(const ovs_params& p, const T r[8][16], const T lo[8][4], bool fluid, T* out,
                                   double& tamax, int& nbad) {
   using W = typename Wide<T>::type;
@@ -391,16 +393,16 @@ __device__ void hex_summarize_tem(const ovs_params& p, const T r[8][16], const T
 #pragma unroll
       for (int n = 0; n < 8; ++n) rt[n] += w * (-N[n] * rcp * rTi - hk * gdT[n]);
     }
-    store_n(out + gp * L::GPW, rec, L::GPW);
+    if constexpr (MAT) store_n(out + gp * L::GPW, rec, L::GPW);
   }
 #pragma unroll
-  for (int n = 0; n < 8; ++n) out[L::RHS0 + n] = rt[n];
+  for (int n = 0; n < 8; ++n) out[(MAT ? L::RHS0 : 0) + n] = rt[n];
 }
 
-template <typename T, int KIND, bool TC = false>
+template <typename T, int KIND, bool TC = false, bool MAT = true>
 __global__ void __launch_bounds__(64) hex_element_kernel(const SumArgs a) {
   using L = HexLay<KIND>;
-  constexpr int SW = TC ? HexTcLay::SW : L::SW;
+  constexpr int SW = !MAT ? 8 * L::NF : TC ? HexTcLay::SW : L::SW;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   double tamax = 0.0;   // the element's largest taua over its points
   int nbad = 0;
@@ -411,8 +413,8 @@ __global__ void __launch_bounds__(64) hex_element_kernel(const SumArgs a) {
     for (int n = 0; n < 8; ++n) load_rec(rec, a.ien[8 * (size_t)e + n], r[n], lo[n]);
     const bool fluid = __ldg(a.elm_id + e) == a.p.fluid_elm_id;
     T* out = reinterpret_cast<T*>(a.sum) + (size_t)e * SW;
-    if constexpr (KIND == OVS_ASM_NSVOF) hex_summarize_nsvof<T, TC>(a.p, r, lo, fluid, out, tamax, nbad);
-    else hex_summarize_tem<T>(a.p, r, lo, fluid, out, tamax, nbad);
+    if constexpr (KIND == OVS_ASM_NSVOF) hex_summarize_nsvof<T, TC, MAT>(a.p, r, lo, fluid, out, tamax, nbad);
+    else hex_summarize_tem<T, MAT>(a.p, r, lo, fluid, out, tamax, nbad);
   }
   double cfl = (double)a.p.delt * sqrt(tamax);   // as the tet element pass
 #pragma unroll
@@ -920,7 +922,7 @@ __global__ void __launch_bounds__(128) hex_rows_kernel(const AsmArgs a) {
     }
     // row write with the Dirichlet treatment (as for the tets)
     const unsigned ibA = a.ibc[A];
-    if (a.mat) {
+    {
       T* outp = reinterpret_cast<T*>(a.vals) + (size_t)rp * NV;
       const T cnt = (T)ne;
       if constexpr (NV >= 4) {
@@ -966,6 +968,12 @@ __global__ void __launch_bounds__(128) hex_rows_kernel(const AsmArgs a) {
 
 template <typename T, int KIND>
 int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int parts) {
+  if (!a0.mat) {   // vector-only pass, as for the tets
+    hex_element_kernel<T, KIND, false, false><<<(sa.E + 63) / 64, 64, 0, c->stream>>>(sa);
+    ++c->launches;
+    OVS_CUDA_TRY(cudaGetLastError());
+    return launch_residual_rows<T, HexLay<KIND>::NF>(c, a0, KIND == OVS_ASM_TEM);
+  }
   constexpr bool can_tc = std::is_same<T, float>::value && KIND == OVS_ASM_NSVOF;
   const bool tc = can_tc && c->hex_tc;
   AsmArgs a = a0;

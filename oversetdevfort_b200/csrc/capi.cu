@@ -781,37 +781,7 @@ int ovs_residual_norms(ovs_ctx* c, int prec, double r[4]) {
   if (!c || !r || (prec != OVS_FP64 && prec != OVS_FP32)) return OVS_ERR_ARG;
   int st;
   if ((st = ovs_activate(c))) return st;
-  r[0] = r[1] = r[2] = r[3] = 0.0;
-  const size_t N = c->N;
-  // momentum/continuity/VOF from the NS+VOF system if assembled, else NS
-  int fs = c->sys[OVS_SYS_NSVOF][prec].rhs ? OVS_SYS_NSVOF : (c->sys[OVS_SYS_NS][prec].rhs ? OVS_SYS_NS : 0);
-  double* tmp = nullptr;
-  OVS_CUDA_TRY(cudaMallocAsync(&tmp, sizeof(double) * 5 * N, c->stream));
-  auto sumsq = [&](int sys, int f0, int nf, double* out) -> int {
-    const size_t n = N * nf;
-    if (prec == OVS_FP64)
-      {
-        copy_convert_kernel<double, double><<<ovs_grid(n, 256, 1 << 30), 256, 0, c->stream>>>(
-            (const double*)c->sys[sys][prec].rhs + N * f0, tmp, n);
-        ++c->launches;
-      }
-    else
-      {
-        copy_convert_kernel<float, double><<<ovs_grid(n, 256, 1 << 30), 256, 0, c->stream>>>(
-            (const float*)c->sys[sys][prec].rhs + N * f0, tmp, n);
-        ++c->launches;
-      }
-    return ovs_dot_impl(c, tmp, tmp, n, out);
-  };
-  if (fs) {
-    if ((st = sumsq(fs, 0, 3, &r[0]))) return st;
-    if ((st = sumsq(fs, 3, 1, &r[1]))) return st;
-    if (fs == OVS_SYS_NSVOF && (st = sumsq(fs, 4, 1, &r[2]))) return st;
-  }
-  if (c->sys[OVS_SYS_TEM][prec].rhs && (st = sumsq(OVS_SYS_TEM, 0, 1, &r[3]))) return st;
-  OVS_CUDA_TRY(cudaFreeAsync(tmp, c->stream));
-  OVS_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return OVS_OK;
+  return ovs_resnorm_impl(c, prec, r);
 }
 
 int ovs_profile(ovs_ctx* c, int what, int system, int precision, int reps, double* avg_ms) {

@@ -1260,8 +1260,68 @@ int ovs_profile_krylov(ovs_ctx* c, int what, int sys, int prec, int reps, double
   return profile_krylov_t<float, false>(c, what, sys, reps, ms);
 }
 
-int ovs_dot_impl(ovs_ctx* c, const double* a, const double* b, size_t n, double* out) {
-  return dot64(c, a, b, n, out);
+// calculate_residual: the sums of squares of the four residual fields (rhs:
+// nfs N flow values - u, p and, for nfs = 5, phi - and N temperature values;
+// either may be null), all in one launch with the fixed order of every
+// reduction here (one launch and one read-back: a copy, a dot and a wait per
+// field were 8 launches and 4 waits).
+template <typename T>
+__global__ void __launch_bounds__(OVS_RED_THREADS)
+resnorm_kernel(const T* __restrict__ flow, int nfs, const T* __restrict__ tem, size_t N, GmresDev* gm) {
+  __shared__ double sh[32];
+  __shared__ int is_last;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  auto add = [&](const T* p, size_t n, double& acc) {
+    for (size_t i = t0; i < n; i += stride) acc += (double)p[i] * (double)p[i];
+  };
+  if (flow) {
+    add(flow, 3 * N, s[0]);
+    add(flow + 3 * N, N, s[1]);
+    if (nfs == 5) add(flow + 4 * N, N, s[2]);
+  }
+  if (tem) add(tem, N, s[3]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double p = block_sum(s[k], sh);
+    if (threadIdx.x == 0) gm->partials[(size_t)k * OVS_RED_BLOCKS + blockIdx.x] = p;
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    is_last = atomicAdd(&gm->counter, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    double v = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+      v += __ldcg(gm->partials + (size_t)k * OVS_RED_BLOCKS + b);
+    const double t = block_sum(v, sh);
+    if (threadIdx.x == 0) gm->scal[k] = t;
+  }
+  if (threadIdx.x == 0) gm->counter = 0;
+}
+
+int ovs_resnorm_impl(ovs_ctx* c, int prec, double r[4]) {
+  // momentum/continuity/VOF from the NS+VOF system if assembled, else NS
+  const int fs = c->sys[OVS_SYS_NSVOF][prec].rhs ? OVS_SYS_NSVOF : OVS_SYS_NS;
+  const void *flow = c->sys[fs][prec].rhs, *tem = c->sys[OVS_SYS_TEM][prec].rhs;
+  const int nfs = ovs_sys_nf(fs);
+  const int grid = ovs_grid((size_t)c->N * 3, OVS_RED_THREADS, OVS_RED_BLOCKS);
+  if (prec == OVS_FP64)
+    resnorm_kernel<double><<<grid, OVS_RED_THREADS, 0, c->stream>>>(as<double>(flow), nfs, as<double>(tem),
+                                                                    (size_t)c->N, c->gm);
+  else
+    resnorm_kernel<float><<<grid, OVS_RED_THREADS, 0, c->stream>>>(as<float>(flow), nfs, as<float>(tem),
+                                                                   (size_t)c->N, c->gm);
+  ++c->launches;
+  OVS_CUDA_TRY(cudaGetLastError());
+  OVS_CUDA_TRY(cudaMemcpyAsync(c->h_pinned_d, c->gm->scal, sizeof(double) * 4, cudaMemcpyDeviceToHost, c->stream));
+  OVS_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  memcpy(r, c->h_pinned_d, sizeof(double) * 4);
+  return OVS_OK;
 }
 
 int ovs_precond_setup(ovs_ctx* c, int sys, int prec) {

@@ -52,7 +52,7 @@ struct GmresDev {
   double e[OVS_MAX_KSPACE + 1];
   double cs[OVS_MAX_KSPACE], sn[OVS_MAX_KSPACE];
   double y[OVS_MAX_KSPACE];
-  double partials[OVS_RED_BLOCKS];
+  double partials[4 * OVS_RED_BLOCKS];
   double scal[8];     // misc scalar results (norms)
   double sc[OVS_MAX_KSPACE + 1];   // scale of each basis slot (1 / norm of what it holds)
 };
@@ -244,8 +244,6 @@ int ovs_solve_impl(ovs_ctx* c, int sys, int mode, double rtol, int kspace,
 int ovs_round_impl(ovs_ctx* c, int sys);
 int ovs_update_impl(ovs_ctx* c, int sys);
 int ovs_resnorm_impl(ovs_ctx* c, int prec, double r[4]);
-int ovs_dot_impl(ovs_ctx* c, const double* a, const double* b, size_t n,
-                 double* out);
 int ovs_profile_assemble(ovs_ctx* c, int kernel, int prec, int reps, double* ms, int parts);
 int ovs_residual_vjp_impl(ovs_ctx* c, int kernel, const double* cot_host, double* grad_host);
 int ovs_gmres_transposed_impl(ovs_ctx* c, int sys, const double* drhs, double tol, int kspace, int kmin,
