@@ -25,7 +25,6 @@
 //     stores.
 // Gauss-point physics is recomputed by each of the element's nshl rows
 // instead of being staged through HBM.
-#include "dual.cuh"
 #include "ovs_internal.cuh"
 
 #include <math.h>
@@ -116,30 +115,21 @@ template <typename T> struct ZeroRecs {
 
 // SMEMREC (FP64 only): the node records through shared memory (a 3-block
 // register bound) instead of registers (255 registers, 2 blocks)
-// Type of the VOF value and of the property blend: FP64 for the FP32 and
-// FP64 routines, the dual number itself for the adjoint.
-template <typename T> struct Wide { using type = double; };
-template <> struct Wide<Dual> { using type = Dual; };
-
 // VOF field at tet Gauss point g in FP64 from the record value (slot k)
 // plus its rounding remainder (lo[.][3]): sum_a N_a phi_a, in node order
 template <typename T, typename RA, typename LA>
-__device__ __forceinline__ typename Wide<T>::type gp_phi(const RA& r, const LA& lo, int k, int g) {
-  using W = typename Wide<T>::type;
+__device__ __forceinline__ double gp_phi(const RA& r, const LA& lo, int k, int g) {
   const double a = 0.5854101966249685, b = 0.1381966011250105;
   const double xi = (g == 0) ? a : b, eta = (g == 1) ? a : b, ze = (g == 2) ? a : b;
   const double N[4] = {xi, eta, ze, 1.0 - xi - eta - ze};
-  W s = 0.0;
+  double s = 0.0;
 #pragma unroll
-  for (int n = 0; n < 4; ++n) s += ((W)r[n][k] + (W)lo[n][3]) * N[n];
+  for (int n = 0; n < 4; ++n) s += ((double)r[n][k] + (double)lo[n][3]) * N[n];
   return s;
 }
 
 // the clamp of prop_interp (src/e3int.f90:4-13): phic = min(max(phi, 0), 1)
 __device__ __forceinline__ double clamp01(double x) { return fmax(fmin(x, 1.0), 0.0); }
-__device__ __forceinline__ Dual clamp01(const Dual& x) {
-  return x.v < 0.0 ? Dual(0.0) : (x.v > 1.0 ? Dual(1.0) : x);
-}
 
 // store NV (multiple of 4) register values to 16-byte aligned shared memory
 template <int NV>
@@ -398,11 +388,9 @@ __device__ __forceinline__ void block_sums(const T (&q)[4][Lay<KIND>::GQ], const
 template <typename T, int KIND> struct CflPerPoint { static constexpr bool v = false; };
 template <> struct CflPerPoint<float, OVS_ASM_NSVOF> { static constexpr bool v = true; };
 
-// 1 / sqrt(x): the reciprocal square root (FP64, FP32), and for the dual
-// numbers of the adjoint the quotient
+// 1 / sqrt(x): the reciprocal square root
 __device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
 __device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
-__device__ __forceinline__ Dual inv_sqrt(const Dual& x) { return 1.0 / sqrt(x); }
 
 struct SumArgs {
   const void* rec;
@@ -503,7 +491,7 @@ __device__ void summarize_ns(const SumArgs& a, const RA& r, const LA& lo, bool t
 #pragma unroll
   for (int n = 0; n < 4; ++n) put4(orh + 4 * n, ru[n][0], ru[n][1], ru[n][2], rp[n]);
   if constexpr (MAT) put4(o + L::C0, KA, KB, MM, (T)0);
-  if constexpr (MAT && !std::is_same<T, Dual>::value)
+  if constexpr (MAT)
     block_sums<T, OVS_ASM_NS>(q, g, target ? w : (T)0, (T)p.almi, fact2, rho, o);
 }
 
@@ -546,10 +534,9 @@ __device__ __forceinline__ void nsvof_point(const ovs_params& p, bool fluid, con
                                             const T (&G)[3][3], T GG, T trG, T w, const T (&du)[3][3],
                                             const T (&dp)[3], const T (&dphi)[3], T divu, const T (&svis)[4],
                                             const T (&gdphi)[4], const T (&ui)[3], const T (&umi)[3],
-                                            const T (&aci)[3], T pri, typename Wide<T>::type phid, T rphii, T Ti,
+                                            const T (&aci)[3], T pri, double phid, T rphii, T Ti,
                                             T* q, T& KA, T& KB, T& MM, T& KDP, T (&ru)[4][3], T (&rp)[4],
                                             T (&rf)[4], double& tamax, const PointInv<T>& iv) {
-  using W = typename Wide<T>::type;
   const T fact2 = (T)(p.alfi * p.delt * p.gami);
   const T taut = iv.taut;
   const T rhoa = (T)p.rhoa, rhow = (T)p.rhow, ts = (T)p.ts;
@@ -557,7 +544,7 @@ __device__ __forceinline__ void nsvof_point(const ovs_params& p, bool fluid, con
   const bool kdc_on = fabs(p.ns_kdc_w) + fabs(p.ns_kdc_a) > 0.0;
   const bool kdcphi_on = fabs(p.lsc_kdc) > 0.0;
   const T phii = (T)phid;
-  const W phicd = clamp01(phid);
+  const double phicd = clamp01(phid);
   const T phic = (T)phicd;
   T mdot, dmd;
   if (Ti > ts) {
@@ -658,7 +645,6 @@ __device__ __forceinline__ void nsvof_node_terms(const T (&g)[4][3], const T (&d
 template <typename T, bool MAT = true, typename RA, typename LA>
 __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, bool fluid, T* o,
                                 double& tamax, T& detj_out) {
-  using W = typename Wide<T>::type;
   const ovs_params& p = a.p;
   T g[4][3], G[3][3], detj, GG, trG;
   element_geometry<T>(r, lo, g, G, detj, GG, trG);
@@ -695,7 +681,7 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
       aci[d] = r[0][9 + d] * N[0] + r[1][9 + d] * N[1] + r[2][9 + d] * N[2] + r[3][9 + d] * N[3];
     }
     const T pri = r[0][12] * N[0] + r[1][12] * N[1] + r[2][12] * N[2] + r[3][12] * N[3];
-    const W phid = gp_phi<T>(r, lo, 13, gp);   // VOF in FP64 for the 1000:1 property blend
+    const double phid = gp_phi<T>(r, lo, 13, gp);   // VOF in FP64 for the 1000:1 property blend
     const T rphii = r[0][14] * N[0] + r[1][14] * N[1] + r[2][14] * N[2] + r[3][14] * N[3];
     const T Ti = r[0][15] * N[0] + r[1][15] * N[1] + r[2][15] * N[2] + r[3][15] * N[3];
     nsvof_point<T>(p, fluid, N, g, G, GG, trG, w, du, dp, dphi, divu, svis, gdphi, ui, umi, aci, pri, phid, rphii, Ti,
@@ -716,7 +702,7 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
     put4(o + L::C0, KA, KB, MM, KDP);
     put4(o + L::C0 + 4, dphi[0], dphi[1], dphi[2], (T)0);
   }
-  if constexpr (MAT && !std::is_same<T, Dual>::value)
+  if constexpr (MAT)
     block_sums<T, OVS_ASM_NSVOF>(q, g, fluid ? w : (T)0, (T)p.almi, (T)(p.alfi * p.delt * p.gami), (T)0, o);
 }
 
@@ -726,12 +712,10 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
 //   K(a,b) += w (Na + trc ca) (rcp (fact1 Nb + fact2 cb) - fact2 dSe Nb)
 // with trc = tauT rho cp, c_n = uadv . grad N_n, then K(a,b) += HK gab; solid
 // elements take uadv = dSe = trc = 0, which turns the fluid block formula
-// into the solid one.  The adjoint instantiation (dual numbers) needs the
-// residual only and skips the matrix.
+// into the solid one.
 template <typename T, bool MAT = true, typename RA, typename LA>
 __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool fluid, T* o,
                               double& tamax, T& detj_out) {
-  using W = typename Wide<T>::type;
   const ovs_params& p = a.p;
   T g[4][3], G[3][3], detj, GG, trG;
   element_geometry<T>(r, lo, g, G, detj, GG, trG);
@@ -758,7 +742,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
   for (int gp = 0; gp < 4; ++gp) {
     T N[4];
     tet_shape<T>(gp, N);
-    const W phid = gp_phi<T>(r, lo, 9, gp);
+    const double phid = gp_phi<T>(r, lo, 9, gp);
     const T Ti = r[0][10] * N[0] + r[1][10] * N[1] + r[2][10] * N[2] + r[3][10] * N[3];
     const T rTi = r[0][11] * N[0] + r[1][11] * N[1] + r[2][11] * N[2] + r[3][11] * N[3];
     T ui[3], umi[3];
@@ -767,7 +751,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
       ui[d] = r[0][3 + d] * N[0] + r[1][3 + d] * N[1] + r[2][3 + d] * N[2] + r[3][3 + d] * N[3];
       umi[d] = r[0][6 + d] * N[0] + r[1][6 + d] * N[1] + r[2][6 + d] * N[2] + r[3][6 + d] * N[3];
     }
-    const W phicd = clamp01(phid);
+    const double phicd = clamp01(phid);
     const T phic = (T)phicd;
     T mdot, dmdT;
     if (Ti > ts) {
@@ -800,7 +784,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
     T kdcT = 0;
     if (kdc_on && fluid) kdcT = (T)p.tem_kdc * fabs(res) * iv.sGG * iv.tref;
     const T dSe = (cpw - cpa) * mdot + ((cpw - cpa) * (Ti - ts) - lh) * dmdT;
-    if constexpr (MAT && !std::is_same<T, Dual>::value) {
+    if constexpr (MAT) {
       const T uq[3] = {fluid ? uadv[0] : (T)0, fluid ? uadv[1] : (T)0, fluid ? uadv[2] : (T)0};
       const T dSq = fluid ? dSe : (T)0, trq = fluid ? tauT * rcp : (T)0;
       T cq[4];
@@ -826,7 +810,7 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
       for (int n = 0; n < 4; ++n) rt[n] += w * (-N[n] * rcp * rTi - hk * gdT[n]);
     }
   }
-  if constexpr (MAT && !std::is_same<T, Dual>::value) {
+  if constexpr (MAT) {
 #pragma unroll
     for (int ia = 0; ia < 4; ++ia)
 #pragma unroll
@@ -1971,15 +1955,20 @@ int launch_assemble(ovs_ctx* c, const AsmArgs& a, const SumArgs& sa, int parts =
 
 // ------------------------------------------------ adjoint of the residual
 // VJP of the assembled residual (the RHS the row pass writes, FP64) with
-// respect to the nodal state.  One thread per element recomputes the
-// element's residual rows on dual numbers once per nodal input of the
-// element (Gauss-point quantities are recomputed, not stored) and contracts
-// the tangent rows with the cotangent, which is zero on Dirichlet rows (the
-// row pass writes 0 there).  A node pass then sums the element terms in
+// respect to the nodal state, in reverse mode.  One thread per element
+// contracts the element's residual rows with the cotangent (zero on Dirichlet
+// rows, where the row pass writes 0), which leaves one scalar per Gauss point,
+// and walks that point's formulas backwards: the adjoint of every
+// intermediate, then of the fields at the point (spread to the nodes by the
+// shape values), of the gradients and of the geometry.  Nothing is stored
+// between assembly and adjoint.  A node pass sums the element terms in
 // ascending element id (deterministic) and applies the alpha-stage chain
 // factors: x+d_a = xg + ..., u_a = .. + alfi ug, p, phi_a = .. + alfi phig,
 // T_a = .. + alfi Tg, a_a = .. + almi acg, phidot_a = .. + almi rphig,
 // Tdot_a = .. + almi rTg (src/solveQuenching.f90:26-37).
+// The cost is a few residual evaluations per element (196,608 tets: NS+VOF
+// 0.21 ms, T 0.07 ms); the forward-mode form evaluated the residual on dual
+// numbers once per nodal input, 52 times for NS+VOF (24 ms for both).
 struct VjpArgs {
   const double* rec;      // FP64 alpha-stage records of the kernel's layout
   const int* ien;
@@ -1991,35 +1980,412 @@ struct VjpArgs {
   ovs_params p;
 };
 
+// element terms per node, in the order of the output fields below
 template <int KIND> struct VjpMap;
-// record slot, output field (OVS_VJP_* order), chain factor kind (0: 1, 1: alfi, 2: almi)
-template <> struct VjpMap<OVS_ASM_NSVOF> {
-  static constexpr int NC = 13;
-  __device__ static int slot(int q) { const int s[13] = {0, 1, 2, 3, 4, 5, 12, 13, 15, 9, 10, 11, 14}; return s[q]; }
-};
-template <> struct VjpMap<OVS_ASM_TEM> {
-  static constexpr int NC = 9;
-  __device__ static int slot(int q) { const int s[9] = {0, 1, 2, 3, 4, 5, 9, 10, 11}; return s[q]; }
-};
+template <> struct VjpMap<OVS_ASM_NSVOF> { static constexpr int NC = 13; };   // x(3) u(3) p phi T a(3) phidot
+template <> struct VjpMap<OVS_ASM_TEM> { static constexpr int NC = 9; };      // x(3) u(3) phi T Tdot
+// output field (OVS_VJP_* order) and chain factor kind (0: 1, 1: alfi, 2: almi)
 static const int h_vjp_out_nsvof[13] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12};
 static const int h_vjp_fac_nsvof[13] = {0, 0, 0, 1, 1, 1, 0, 1, 1, 2, 2, 2, 2};
 static const int h_vjp_out_tem[9] = {0, 1, 2, 3, 4, 5, 7, 8, 13};
 static const int h_vjp_fac_tem[9] = {0, 0, 0, 1, 1, 1, 1, 1, 2};
 
+// phase change at a point: mdot and its factor, as the residual routines take
+// them; the adjoint of mdot goes to phic and T
+struct PhasePoint {
+  double phic, mdot, dm_dphi, dm_dT;
+};
+__device__ __forceinline__ PhasePoint phase_point(const ovs_params& p, double phid, double Ti) {
+  PhasePoint q;
+  q.phic = clamp01(phid);
+  const double d = (Ti - p.ts) / p.ts;
+  const bool hot = Ti > p.ts;
+  const double c = hot ? p.c_evap * p.rhow : p.c_cond * p.rhoa;
+  const double share = hot ? 1.0 - q.phic : q.phic;
+  q.mdot = c * share * d;
+  q.dm_dphi = (hot ? -c : c) * d;
+  q.dm_dT = c * share / p.ts;
+  return q;
+}
+
+// adjoint of the geometry: from gb (of the gradients), Gb (of G) and db (of
+// DetJ) to the node coordinates, in the first three terms of each node
+template <int NC>
+__device__ __forceinline__ void vjp_geometry(const double (&g)[4][3], double detj, const double (&gb)[4][3],
+                                             const double (&Gb)[3][3], double db, double* out) {
+  double Bb[3][3], X[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      double t = gb[k][i] - gb[3][i];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) t += (Gb[i][j] + Gb[j][i]) * g[k][j];
+      Bb[k][i] = t;
+    }
+  // B = A^-1 (rows g_0..g_2): dB = -B dA B, d DetJ = DetJ tr(B dA)
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int l = 0; l < 3; ++l) X[k][l] = Bb[k][0] * g[l][0] + Bb[k][1] * g[l][1] + Bb[k][2] * g[l][2];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double s3 = 0.0;
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      const double ab = db * detj * g[l][i] - (g[0][i] * X[0][l] + g[1][i] * X[1][l] + g[2][i] * X[2][l]);
+      out[l * NC + i] = ab;
+      s3 -= ab;
+    }
+    out[3 * NC + i] = s3;
+  }
+}
+
+__device__ void vjp_nsvof(const ovs_params& p, const double (&r)[4][16], const double (&vv)[4][5], double* out) {
+  constexpr int NC = VjpMap<OVS_ASM_NSVOF>::NC;
+  const ZeroRecs<double> lo;
+  double g[4][3], G[3][3], detj, GG, trG;
+  element_geometry<double>(r, lo, g, G, detj, GG, trG);
+  const double w = detj * (0.25 / 6.0);
+  double du[3][3], dp[3], dphi[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      du[i][j] = r[0][3 + i] * g[0][j] + r[1][3 + i] * g[1][j] + r[2][3 + i] * g[2][j] + r[3][3 + i] * g[3][j];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    dp[j] = r[0][12] * g[0][j] + r[1][12] * g[1][j] + r[2][12] * g[2][j] + r[3][12] * g[3][j];
+    dphi[j] = r[0][13] * g[0][j] + r[1][13] * g[1][j] + r[2][13] * g[2][j] + r[3][13] * g[3][j];
+  }
+  const double divu = du[0][0] + du[1][1] + du[2][2];
+  // cotangent contractions with the gradients
+  double D[3][3], Q[3], R[3], hs[3], sn[4];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) sn[n] = vv[n][0] + vv[n][1] + vv[n][2];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      D[i][j] = vv[0][i] * g[0][j] + vv[1][i] * g[1][j] + vv[2][i] * g[2][j] + vv[3][i] * g[3][j];
+    Q[j] = vv[0][3] * g[0][j] + vv[1][3] * g[1][j] + vv[2][3] * g[2][j] + vv[3][3] * g[3][j];
+    R[j] = vv[0][4] * g[0][j] + vv[1][4] * g[1][j] + vv[2][4] * g[2][j] + vv[3][4] * g[3][j];
+    hs[j] = sn[0] * g[0][j] + sn[1] * g[1][j] + sn[2] * g[2][j] + sn[3] * g[3][j];
+  }
+  const double B = D[0][0] + D[1][1] + D[2][2];
+  double SV = 0.0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) SV += hs[j] * (du[j][k] + du[k][j]);
+  const double RdP = R[0] * dphi[0] + R[1] * dphi[1] + R[2] * dphi[2];
+  const double irhoa = 1.0 / p.rhoa, ira = irhoa - 1.0 / p.rhow, itrG = 1.0 / trG, iGG = 1.0 / GG;
+  const double isGG = sqrt(iGG), taut = 4.0 / (p.delt * p.delt);
+  const bool kdc_on = fabs(p.ns_kdc_w) + fabs(p.ns_kdc_a) > 0.0, kdcphi_on = fabs(p.lsc_kdc) > 0.0;
+  // adjoints gathered over the points
+  double wb = 0.0, SVb = 0.0, GGb = 0.0, itrGb = 0.0, divb = 0.0;
+  double dub[3][3], dpb[3], dfb[3], Db[3][3], Qb[3], Rb[3], Gb[3][3], nb[4][10];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dpb[i] = dfb[i] = Qb[i] = Rb[i] = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) dub[i][j] = Db[i][j] = Gb[i][j] = 0.0;
+  }
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int k = 0; k < 10; ++k) nb[n][k] = 0.0;
+#pragma unroll 1
+  for (int gp = 0; gp < 4; ++gp) {
+    double N[4];
+    tet_shape<double>(gp, N);
+    auto at = [&](int k) { return r[0][k] * N[0] + r[1][k] * N[1] + r[2][k] * N[2] + r[3][k] * N[3]; };
+    double uadv[3], a[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      uadv[d] = at(3 + d) - at(6 + d);
+      a[d] = at(9 + d) - p.gravvec[d];
+    }
+    const double pri = at(12), phid = at(13), rphii = at(14), Ti = at(15);
+    // the point's formulas, as nsvof_point
+    const PhasePoint ph = phase_point(p, phid, Ti);
+    const bool inside = !(phid < 0.0 || phid > 1.0), hot = Ti > p.ts;
+    const double dmd_dT = !inside ? 0.0 : (hot ? -p.c_evap * p.rhow : p.c_cond * p.rhoa) / p.ts * p.c_dmdot;
+    const double dmdi = dmd_dT * (Ti - p.ts) * ira;
+    const double vdot = ph.mdot * ira;
+    const double rho = p.rhow * (1.0 - ph.phic) + p.rhoa * ph.phic, mu = p.muw * (1.0 - ph.phic) + p.mua * ph.phic;
+    const double lam = -2.0 / 3.0 * mu;
+    double acc[3], rL[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      acc[i] = a[i] + du[i][0] * uadv[0] + du[i][1] * uadv[1] + du[i][2] * uadv[2];
+      rL[i] = rho * acc[i] + dp[i];
+    }
+    const double res = rphii + (uadv[0] * dphi[0] + uadv[1] * dphi[1] + uadv[2] * dphi[2]) + phid * vdot - ph.mdot * irhoa;
+    const double taua = quad_uGu<double>(uadv, G), irho = 1.0 / rho, nu = mu * irho;
+    const double taud = nu * nu * 12.0 * GG, is = rsqrt(taut + taua + taud), tauM = irho * is;
+    const double tauLS = rsqrt(taut + taua), sq = sqrt(taua + taud), tauC = rho * sq * itrG;
+    double lw = 0.0, srr = 0.0;
+    const double rr = rL[0] * rL[0] + rL[1] * rL[1] + rL[2] * rL[2];
+    if (kdc_on) {
+      lw = (double)low_word(p.ns_kdc_w * (1.0 - ph.phic) + p.ns_kdc_a * ph.phic);
+      srr = sqrt(rr * iGG);
+    }
+    const double mupk = mu + lw * srr, kdphi = kdcphi_on ? p.lsc_kdc * fabs(res) * isGG : 0.0;
+    const double Z = divu - vdot, F = pri - tauC * Z - lam * divu;
+    double A[3], C[3], P = 0.0, V = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      A[i] = vv[0][i] * N[0] + vv[1][i] * N[1] + vv[2][i] * N[2] + vv[3][i] * N[3];
+      C[i] = D[i][0] * uadv[0] + D[i][1] * uadv[1] + D[i][2] * uadv[2];
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) { P += vv[n][3] * N[n]; V += vv[n][4] * N[n]; }
+    const double uR = uadv[0] * R[0] + uadv[1] * R[1] + uadv[2] * R[2];
+    const double CrL = C[0] * rL[0] + C[1] * rL[1] + C[2] * rL[2], QrL = Q[0] * rL[0] + Q[1] * rL[1] + Q[2] * rL[2];
+    wb += -rho * (A[0] * acc[0] + A[1] * acc[1] + A[2] * acc[2]) + B * F - mupk * SV - rho * tauM * CrL - P * Z -
+          tauM * QrL - (V + tauLS * uR) * res - kdphi * RdP + V * dmdi * tauC * Z;
+    // ---- backwards
+    const double Fb = w * B;
+    double rhob = -w * tauM * CrL, mub = -w * SV + 2.0 / 3.0 * Fb * divu, ub[3];
+    SVb -= w * mupk;
+    const double tMb = -w * (rho * CrL + QrL), Zb = w * (V * dmdi * tauC - P) - Fb * tauC;
+    const double tCb = (w * V * dmdi - Fb) * Z;
+    double resb = -w * (V + tauLS * uR);
+    const double kdpb = -w * RdP;
+    if (kdcphi_on) {
+      resb += res > 0.0 ? kdpb * p.lsc_kdc * isGG : (res < 0.0 ? -kdpb * p.lsc_kdc * isGG : 0.0);
+      GGb -= 0.5 * kdpb * kdphi * iGG;
+    }
+    const double kdcb = srr > 0.0 ? -w * SV * lw * 0.5 / srr : 0.0;   // of rr / GG
+    GGb -= kdcb * rr * iGG * iGG;
+    double tab = -0.5 * tauLS * tauLS * tauLS * (-w * uR * res);
+    const double isb = tMb * irho, sumb = -0.5 * is * is * is * isb;
+    double irhob = tMb * is;
+    const double sqb = sq > 0.0 ? tCb * rho * itrG / (2.0 * sq) : 0.0;
+    rhob += tCb * sq * itrG;
+    itrGb += tCb * rho * sq;
+    tab += sumb + sqb;
+    const double tdb = sumb + sqb, nub = tdb * 24.0 * nu * GG;
+    GGb += tdb * 12.0 * nu * nu;
+    mub += nub * irho;
+    irhob += nub * mu;
+    rhob -= irhob * irho * irho;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      Db[i][i] += w * F;
+      const double Cb = -w * rho * tauM * rL[i];
+      const double rLb = -w * tauM * (rho * C[i] + Q[i]) + 2.0 * rL[i] * kdcb * iGG;
+      const double t1b = rLb - w * A[i];
+      Qb[i] -= w * tauM * rL[i];
+      dpb[i] += rLb;
+      rhob += t1b * acc[i];
+      const double ab = t1b * rho;   // of acceleration + convection
+#pragma unroll
+      for (int n = 0; n < 4; ++n) nb[n][6 + i] += N[n] * ab;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        Db[i][j] += Cb * uadv[j];
+        dub[i][j] += ab * uadv[j];
+        Gb[i][j] += tab * uadv[i] * uadv[j];
+      }
+      ub[i] = resb * dphi[i] - w * tauLS * res * R[i] + 2.0 * tab * (G[i][0] * uadv[0] + G[i][1] * uadv[1] + G[i][2] * uadv[2]);
+      Rb[i] -= w * (tauLS * res * uadv[i] + kdphi * dphi[i]);
+      dfb[i] += resb * uadv[i] - w * kdphi * R[i];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const double Cb = -w * rho * tauM * rL[i];
+        const double rLb = -w * tauM * (rho * C[i] + Q[i]) + 2.0 * rL[i] * kdcb * iGG;
+        ub[j] += Cb * D[i][j] + (rLb - w * A[i]) * rho * du[i][j];
+      }
+    divb += Zb - Fb * lam;
+    const double vb = -Zb + resb * phid, mb = vb * ira - resb * irhoa;
+    double phicb = rhob * (p.rhoa - p.rhow) + mub * (p.mua - p.muw) + mb * ph.dm_dphi;
+    const double Tb = mb * ph.dm_dT + w * V * tauC * Z * ira * dmd_dT;
+    const double phib = resb * vdot + (inside ? phicb : 0.0);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) nb[n][d] += N[n] * ub[d];
+      nb[n][3] += N[n] * Fb;
+      nb[n][4] += N[n] * phib;
+      nb[n][5] += N[n] * Tb;
+      nb[n][9] += N[n] * resb;
+    }
+  }
+  // ---- gradients and geometry
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    dub[i][i] += divb;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) dub[i][j] += SVb * (hs[i] + hs[j]);
+  }
+  GGb *= 2.0;
+  const double trb = -itrGb * itrG * itrG;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    Gb[i][i] += trb;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) Gb[i][j] += GGb * G[i][j];
+  }
+  double gb[4][3];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      double t = vv[n][3] * Qb[j] + vv[n][4] * Rb[j] + r[n][12] * dpb[j] + r[n][13] * dfb[j];
+      double hb = 0.0;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        t += vv[n][i] * Db[i][j] + r[n][3 + i] * dub[i][j];
+        hb += du[j][i] + du[i][j];
+      }
+      gb[n][j] = t + sn[n] * SVb * hb;
+    }
+    double* o = out + n * NC;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      o[3 + i] = nb[n][i] + dub[i][0] * g[n][0] + dub[i][1] * g[n][1] + dub[i][2] * g[n][2];
+      o[9 + i] = nb[n][6 + i];
+    }
+    o[6] = nb[n][3] + dpb[0] * g[n][0] + dpb[1] * g[n][1] + dpb[2] * g[n][2];
+    o[7] = nb[n][4] + dfb[0] * g[n][0] + dfb[1] * g[n][1] + dfb[2] * g[n][2];
+    o[8] = nb[n][5];
+    o[12] = nb[n][9];
+  }
+  vjp_geometry<NC>(g, detj, gb, Gb, wb * (0.25 / 6.0), out);
+}
+
+// record layout of the temperature pass: xd(0:2) u(3:5) um(6:8) phi(9) T(10) rT(11)
+__device__ void vjp_tem(const ovs_params& p, const double (&r)[4][16], const double (&vv)[4][1], bool fluid,
+                        double* out) {
+  constexpr int NC = VjpMap<OVS_ASM_TEM>::NC;
+  const ZeroRecs<double> lo;
+  double g[4][3], G[3][3], detj, GG, trG;
+  element_geometry<double>(r, lo, g, G, detj, GG, trG);
+  const double w = detj * (0.25 / 6.0);
+  double dT[3], R[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    dT[j] = r[0][10] * g[0][j] + r[1][10] * g[1][j] + r[2][10] * g[2][j] + r[3][10] * g[3][j];
+    R[j] = vv[0][0] * g[0][j] + vv[1][0] * g[1][j] + vv[2][0] * g[2][j] + vv[3][0] * g[3][j];
+  }
+  const double RdT = R[0] * dT[0] + R[1] * dT[1] + R[2] * dT[2];
+  const double iGG = 1.0 / GG, isGG = sqrt(iGG), taut = 4.0 / (p.delt * p.delt), dcp = p.cpw - p.cpa;
+  const double tk = fabs(p.tem_kdc) > 0.0 ? p.tem_kdc / p.tref : 0.0;
+  double wb = 0.0, GGb = 0.0, dTb[3] = {0, 0, 0}, Rb[3] = {0, 0, 0}, Gb[3][3], nb[4][6];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) Gb[i][j] = 0.0;
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) nb[n][k] = 0.0;
+#pragma unroll 1
+  for (int gp = 0; gp < 4; ++gp) {
+    double N[4];
+    tet_shape<double>(gp, N);
+    auto at = [&](int k) { return r[0][k] * N[0] + r[1][k] * N[1] + r[2][k] * N[2] + r[3][k] * N[3]; };
+    const double phid = at(9), Ti = at(10), rTi = at(11);
+    double V = 0.0;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) V += vv[n][0] * N[n];
+    double ub[3] = {0, 0, 0}, phib = 0.0, Tb = 0.0, rTb;
+    if (fluid) {
+      const double uadv[3] = {at(3) - at(6), at(4) - at(7), at(5) - at(8)};
+      const PhasePoint ph = phase_point(p, phid, Ti);
+      const double rho = p.rhow * (1.0 - ph.phic) + p.rhoa * ph.phic, cp = p.cpw * (1.0 - ph.phic) + p.cpa * ph.phic;
+      const double hk = p.kappaw * (1.0 - ph.phic) + p.kappaa * ph.phic;
+      const double rcp = (p.rhow * p.cpw) * (1.0 - ph.phic) + (p.rhoa * p.cpa) * ph.phic;
+      const double lat = dcp * (Ti - p.ts) - p.lh, udT = uadv[0] * dT[0] + uadv[1] * dT[1] + uadv[2] * dT[2];
+      const double res = rcp * (rTi + udT) - lat * ph.mdot, taua = quad_uGu<double>(uadv, G);
+      const double ircp = 1.0 / (rho * cp), kk = hk * ircp, is = rsqrt(taua + taut + kk * kk * 12.0 * GG), tauT = ircp * is;
+      const double hkd = hk + tk * fabs(res) * isGG;
+      const double uR = uadv[0] * R[0] + uadv[1] * R[1] + uadv[2] * R[2];
+      wb += -(V + rcp * tauT * uR) * res - hkd * RdT;
+      // ---- backwards
+      const double hkb = -w * RdT;
+      double resb = -w * (V + rcp * tauT * uR);
+      resb += res > 0.0 ? hkb * tk * isGG : (res < 0.0 ? -hkb * tk * isGG : 0.0);
+      GGb -= 0.5 * hkb * tk * fabs(res) * isGG * iGG;
+      const double rcpb = -w * tauT * uR * res + resb * (rTi + udT);
+      const double tTb = -w * rcp * uR * res, sumb = -0.5 * is * is * is * tTb * ircp;
+      const double kkb = sumb * 24.0 * kk * GG, ircpb = tTb * is + kkb * hk;
+      GGb += sumb * 12.0 * kk * kk;
+      const double pb = -ircpb * ircp * ircp;   // of rho cp
+      const double mb = -resb * lat;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        ub[i] = -w * rcp * tauT * res * R[i] + resb * rcp * dT[i] +
+                2.0 * sumb * (G[i][0] * uadv[0] + G[i][1] * uadv[1] + G[i][2] * uadv[2]);
+        Rb[i] -= w * (rcp * tauT * res * uadv[i] + hkd * dT[i]);
+        dTb[i] += resb * rcp * uadv[i] - w * hkd * R[i];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) Gb[i][j] += sumb * uadv[i] * uadv[j];
+      }
+      const double phicb = pb * (cp * (p.rhoa - p.rhow) + rho * (p.cpa - p.cpw)) + (hkb + kkb * ircp) * (p.kappaa - p.kappaw) +
+                           rcpb * (p.rhoa * p.cpa - p.rhow * p.cpw) + mb * ph.dm_dphi;
+      phib = phid < 0.0 || phid > 1.0 ? 0.0 : phicb;
+      Tb = -resb * dcp * ph.mdot + mb * ph.dm_dT;
+      rTb = resb * rcp;
+    } else {
+      const double rcp = p.rhos * p.cps;
+      wb += -V * rcp * rTi - p.kappas * RdT;
+      rTb = -w * V * rcp;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        Rb[i] -= w * p.kappas * dT[i];
+        dTb[i] -= w * p.kappas * R[i];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) nb[n][d] += N[n] * ub[d];
+      nb[n][3] += N[n] * phib;
+      nb[n][4] += N[n] * Tb;
+      nb[n][5] += N[n] * rTb;
+    }
+  }
+  double gb[4][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) Gb[i][j] += 2.0 * GGb * G[i][j];
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) gb[n][j] = vv[n][0] * Rb[j] + r[n][10] * dTb[j];
+    double* o = out + n * NC;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[3 + i] = nb[n][i];
+    o[6] = nb[n][3];
+    o[7] = nb[n][4] + dTb[0] * g[n][0] + dTb[1] * g[n][1] + dTb[2] * g[n][2];
+    o[8] = nb[n][5];
+  }
+  vjp_geometry<NC>(g, detj, gb, Gb, wb * (0.25 / 6.0), out);
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(128) residual_vjp_kernel(const VjpArgs a) {
-  using L = Lay<KIND>;
-  using M = VjpMap<KIND>;
-  constexpr int NF = L::NF;
+  constexpr int NF = Lay<KIND>::NF, NC = VjpMap<KIND>::NC;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= a.E) return;
   const int4 nd = __ldg(reinterpret_cast<const int4*>(a.ien) + e);
   const int nodes[4] = {nd.x, nd.y, nd.z, nd.w};
-  double r[4][16], lo[4][4];
+  const bool fluid = __ldg(a.elm_id + e) == a.p.fluid_elm_id;
+  double* out = a.ge + (size_t)e * 4 * NC;
+  if (KIND == OVS_ASM_NSVOF && !fluid) {   // solid elements contribute nothing
+    for (int q = 0; q < 4 * NC; ++q) out[q] = 0.0;
+    return;
+  }
+  double r[4][16], lo[4][4], vv[4][NF];
 #pragma unroll
   for (int n = 0; n < 4; ++n) load_rec(a.rec, nodes[n], r[n], lo[n]);
-  const bool fluid = __ldg(a.elm_id + e) == a.p.fluid_elm_id;
-  double vv[4][NF];
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const unsigned ib = __ldg(a.ibc + nodes[m]);
@@ -2029,32 +2395,8 @@ __global__ void __launch_bounds__(128) residual_vjp_kernel(const VjpArgs a) {
       vv[m][f] = (ib & bit) ? 0.0 : a.cot[(size_t)f * a.N + nodes[m]];
     }
   }
-  SumArgs sa;
-  sa.p = a.p;
-  for (int n = 0; n < 4; ++n) {
-    for (int q = 0; q < M::NC; ++q) {
-      Dual rd[4][16], ld[4][4];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) rd[m][k] = Dual(r[m][k]);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) ld[m][k] = Dual(lo[m][k]);
-      }
-      rd[n][M::slot(q)].d = 1.0;
-      Dual o[L::SW];
-      double cfl = 0.0;
-      Dual detj;
-      if constexpr (KIND == OVS_ASM_NSVOF) summarize_nsvof<Dual>(sa, rd, ld, fluid, o, cfl, detj);
-      else summarize_tem<Dual>(sa, rd, ld, fluid, o, cfl, detj);
-      double acc = 0.0;
-#pragma unroll
-      for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int f = 0; f < NF; ++f) acc += vv[m][f] * o[L::RHS0 + NF * m + f].d;
-      a.ge[((size_t)e * 4 + n) * M::NC + q] = acc;
-    }
-  }
+  if constexpr (KIND == OVS_ASM_NSVOF) vjp_nsvof(a.p, r, vv, out);
+  else vjp_tem(a.p, r, vv, fluid, out);
 }
 
 struct VjpGatherArgs {
@@ -2063,23 +2405,31 @@ struct VjpGatherArgs {
   const double* ge;
   double* grad;           // OVS_VJP_COUNT*N field-major
   int N, NC;
-  int out[16];
-  double fac[16];
+  int q[OVS_VJP_COUNT];   // the element term of an output field, -1: zero
+  double fac[OVS_VJP_COUNT];
 };
 
-__global__ void vjp_gather_kernel(const VjpGatherArgs a) {
-  const int A = blockIdx.x * blockDim.x + threadIdx.x;
-  if (A >= a.N) return;
-  double s[16];
-  for (int q = 0; q < a.NC; ++q) s[q] = 0.0;
-  for (int k = a.n2e_ptr[A]; k < a.n2e_ptr[A + 1]; ++k) {
-    const int packed = a.n2e[k];
-    const double* g = a.ge + ((size_t)(packed >> 3) * 4 + (packed & 7)) * a.NC;
-    for (int q = 0; q < a.NC; ++q) s[q] += g[q];
+// 16 lanes per node, lane q adds term q of the node's elements in ascending
+// order; the block's 16 nodes leave field by field (128 contiguous bytes)
+__global__ void __launch_bounds__(256) vjp_gather_kernel(const VjpGatherArgs a) {
+  __shared__ double sm[16][17];
+  const int q = threadIdx.x & 15, nl = threadIdx.x >> 4, A = blockIdx.x * 16 + nl;
+  double s = 0.0;
+  if (A < a.N && q < a.NC) {
+    const int k1 = __ldg(a.n2e_ptr + A + 1);
+#pragma unroll 4
+    for (int k = __ldg(a.n2e_ptr + A); k < k1; ++k) {
+      const int packed = __ldg(a.n2e + k);
+      s += __ldg(a.ge + ((size_t)(packed >> 3) * 4 + (packed & 7)) * a.NC + q);
+    }
   }
-  for (int f = 0; f < OVS_VJP_COUNT; ++f) a.grad[(size_t)f * a.N + A] = 0.0;
-  for (int q = 0; q < a.NC; ++q) a.grad[(size_t)a.out[q] * a.N + A] = a.fac[q] * s[q];
+  sm[q][nl] = s;
+  __syncthreads();
+  const int f = nl, B = blockIdx.x * 16 + q;   // field, node
+  if (f < OVS_VJP_COUNT && B < a.N)
+    a.grad[(size_t)f * a.N + B] = a.q[f] < 0 ? 0.0 : a.fac[f] * sm[a.q[f]][q];
 }
+static_assert(OVS_VJP_COUNT <= 16, "one lane group per output field");
 
 #include "assemble_hex.cuh"
 
@@ -2347,12 +2697,13 @@ int ovs_residual_vjp_impl(ovs_ctx* c, int kernel, const double* cot_host, double
   ga.grad = c->vjp_grad;
   ga.N = c->N;
   ga.NC = NC;
+  for (int f = 0; f < OVS_VJP_COUNT; ++f) { ga.q[f] = -1; ga.fac[f] = 0.0; }
   for (int q = 0; q < NC; ++q) {
-    const int fk = tem ? h_vjp_fac_tem[q] : h_vjp_fac_nsvof[q];
-    ga.out[q] = tem ? h_vjp_out_tem[q] : h_vjp_out_nsvof[q];
-    ga.fac[q] = fk == 0 ? 1.0 : (fk == 1 ? c->params.alfi : c->params.almi);
+    const int f = tem ? h_vjp_out_tem[q] : h_vjp_out_nsvof[q], fk = tem ? h_vjp_fac_tem[q] : h_vjp_fac_nsvof[q];
+    ga.q[f] = q;
+    ga.fac[f] = fk == 0 ? 1.0 : (fk == 1 ? c->params.alfi : c->params.almi);
   }
-  vjp_gather_kernel<<<ovs_grid(c->N, 128, 1 << 30), 128, 0, s>>>(ga);
+  vjp_gather_kernel<<<(c->N + 15) / 16, 256, 0, s>>>(ga);
   ++c->launches;
   OVS_CUDA_TRY(cudaGetLastError());
   OVS_CUDA_TRY(cudaMemcpyAsync(grad_host, c->vjp_grad, sizeof(double) * N * OVS_VJP_COUNT, cudaMemcpyDeviceToHost, s));

@@ -97,11 +97,10 @@ __device__ __forceinline__ T hex_geometry(int gp, const T r[8][16], const T lo[8
 }
 
 template <typename T>
-__device__ __forceinline__ typename Wide<T>::type hex_phi(const T r[8][16], const T lo[8][4], int k, int gp) {
-  using W = typename Wide<T>::type;
-  W s = 0.0;
+__device__ __forceinline__ double hex_phi(const T r[8][16], const T lo[8][4], int k, int gp) {
+  double s = 0.0;
 #pragma unroll
-  for (int a = 0; a < 8; ++a) s += ((W)r[a][k] + (W)lo[a][3]) * hex_N<double>(gp, a);
+  for (int a = 0; a < 8; ++a) s += ((double)r[a][k] + (double)lo[a][3]) * hex_N<double>(gp, a);
   return s;
 }
 
@@ -116,7 +115,6 @@ __device__ __forceinline__ void store_n(T* dst, const T* v, int n) {
 template <typename T, bool TC = false, bool MAT = true>
 __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const T lo[8][4], bool fluid,
                                     T* out, double& tamax, int& nbad) {
-  using W = typename Wide<T>::type;
   using L = HexLay<OVS_ASM_NSVOF>;
   constexpr int RHS0 = !MAT ? 0 : TC ? HexTcLay::RHS0 : L::RHS0;
   const T fact2 = (T)(p.alfi * p.delt * p.gami);
@@ -171,9 +169,9 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
       Ti += r[a][15] * N[a];
     }
     const T divu = du[0][0] + du[1][1] + du[2][2];
-    const W phid = hex_phi<T>(r, lo, 13, gp);
+    const double phid = hex_phi<T>(r, lo, 13, gp);
     const T phii = (T)phid;
-    const W phicd = clamp01(phid);
+    const double phicd = clamp01(phid);
     const T phic = (T)phicd;
     T mdot, dmd;
     if (Ti > ts) {
@@ -299,7 +297,6 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
 template <typename T, bool MAT = true>
 __device__ void hex_summarize_tem(const ovs_params& p, const T r[8][16], const T lo[8][4], bool fluid, T* out,
                                   double& tamax, int& nbad) {
-  using W = typename Wide<T>::type;
   using L = HexLay<OVS_ASM_TEM>;
   const T fact2 = (T)(p.alfi * p.gami * p.delt);
   const T ts = (T)p.ts, cpw = (T)p.cpw, cpa = (T)p.cpa, lh = (T)p.lh;
@@ -337,8 +334,8 @@ __device__ void hex_summarize_tem(const ovs_params& p, const T r[8][16], const T
     T gdT[8];
 #pragma unroll
     for (int n = 0; n < 8; ++n) gdT[n] = g[n][0] * dT[0] + g[n][1] * dT[1] + g[n][2] * dT[2];
-    const W phid = hex_phi<T>(r, lo, 9, gp);
-    const W phicd = clamp01(phid);
+    const double phid = hex_phi<T>(r, lo, 9, gp);
+    const double phicd = clamp01(phid);
     const T phic = (T)phicd;
     T mdot, dmdT;
     if (Ti > ts) {
