@@ -564,21 +564,6 @@ def run_ours(args, world, rank, local_rank, dist):
             prof[f"asm_{kn}_{nm}_ms"] = ctx.profile(F.OVS_PROF_ASSEMBLE, kern, prec, 5)
             prof[f"asm_{kn}_{nm}_elements_ms"] = ctx.profile(F.OVS_PROF_ASSEMBLE_ELEMENTS, kern, prec, 5)
             prof[f"asm_{kn}_{nm}_rows_ms"] = ctx.profile(F.OVS_PROF_ASSEMBLE_ROWS, kern, prec, 5)
-    # the row-pass variants, same box, same data: the chunked pass (element
-    # blocks reduced through shared memory, summaries staged by cp.async),
-    # the tiled pass (summaries staged per row tile by bulk copies) and the
-    # gather pass (the default, last)
-    rows_ab = {}
-    for vn, opts in (("chunked", ((F.OVS_OPT_ROWS_TILED, 0), (F.OVS_OPT_ROWS_GATHER, 0))),
-                     ("tiled", ((F.OVS_OPT_ROWS_TILED, 1), (F.OVS_OPT_ROWS_GATHER, 1))),
-                     ("gather", ((F.OVS_OPT_ROWS_TILED, 0), (F.OVS_OPT_ROWS_GATHER, 1)))):
-        for o, v in opts:
-            ctx.set_option(o, v)
-        for prec, nm in ((F.OVS_FP64, "fp64"), (F.OVS_FP32, "fp32")):
-            for kern, kn in ((F.OVS_ASM_NSVOF, "nsvof"), (F.OVS_ASM_TEM, "tem")):
-                ctx.assemble(kern, 6, prec)
-                rows_ab[f"{kn}_{nm}_{vn}_ms"] = ctx.profile(F.OVS_PROF_ASSEMBLE_ROWS, kern, prec, 5)
-    prof["rows_variants"] = rows_ab
     # the FP64 element pass with the node records in registers against
     # shared memory (the default takes shared memory for NS+VOF, registers
     # for T)
@@ -603,7 +588,7 @@ def run_ours(args, world, rank, local_rank, dist):
     pa_ach = pass64 / (prof["asm_nsvof_fp64_ms"] * 1e-3) / 1e9
     row_ach = pass64 / (prof["asm_nsvof_fp64_rows_ms"] * 1e-3) / 1e9
     dpt, dpt_src = ncu_dram_per_tet("assembly_nsvof_fp64_quench48_dram.md", 663552)
-    roof_asm = {"kernel": "element_summary_kernel + gather_rows_kernel <double, NSVOF>: one NS+VOF assembly "
+    roof_asm = {"kernel": "element_summary_kernel + edge_rows_kernel <double, NSVOF>: one NS+VOF assembly "
                           "pass (MAT+VEC), the dominant work of the step",
                 "bound": "hbm", "achieved": pa_ach, "peak": hbm, "unit": "GB/s", "frac": pa_ach / hbm,
                 "traffic": dpt * E if dpt else None, "traffic_source": dpt_src, "peak_kind": peak_kind,
@@ -625,7 +610,7 @@ def run_ours(args, world, rank, local_rank, dist):
                                     "peak_kind": "measured live (ovs_measure_fp64_peak, FP64 FMA)",
                                     "source": fpt_src}
     pass32 = assembly_pass_bytes(E, N, nnz, 4)
-    roof_asm32 = {"kernels": "element_summary_kernel + gather_rows_kernel <float, NSVOF>", "bound": "hbm",
+    roof_asm32 = {"kernels": "element_summary_kernel + edge_rows_kernel <float, NSVOF>", "bound": "hbm",
                   "achieved": pass32 / (prof["asm_nsvof_fp32_ms"] * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                   "algorithmic_bytes": pass32, "avg_ms": prof["asm_nsvof_fp32_ms"], "peak_kind": peak_kind}
     roof_asm32["frac"] = roof_asm32["achieved"] / hbm

@@ -109,24 +109,15 @@ enum {
                                   0 (default, the faster one measured; env OVS_HEX_TC=1 sets 1): the
                                   CUDA-core row expansion */
   OVS_OPT_ARNOLDI_FUSED = 2,   /* 1: one-launch Arnoldi variant (default 0; env OVS_ARNOLDI_FUSED=1) */
-  OVS_OPT_ROWS_STAGED = 3,     /* chunked tet row pass (OVS_OPT_ROWS_GATHER = 0), NS and NS+VOF kernels: 1
-                                  (default) stages each chunk's element summaries in shared memory with
-                                  asynchronous copies; 0 (env OVS_ROWS_STAGED=0) reads them from global memory
-                                  lane by lane */
+  OVS_OPT_ROWS_STAGED = 3,     /* accepted, without effect (as are 5, 6 and 7): one pass over the edges serves
+                                  every tet mesh, where there were variants to choose from */
   OVS_OPT_ELEM_SMEM = 4,       /* FP64 tet element pass: 0 (env OVS_ELEM_SMEM=0) holds the node records in
                                   registers, 1 (env OVS_ELEM_SMEM=1) in shared memory; -1 (default) shared
                                   memory for NS+VOF and registers for NS and T, the faster of the two
                                   measured for each */
-  OVS_OPT_ROWS_GATHER = 5,     /* tet row pass without tiles (OVS_OPT_ROWS_TILED = 0): 1 (default) every lane
-                                  gathers whole blocks of the row by the contribution lists built with the
-                                  pattern, reading the summaries from global memory; 0 (env
-                                  OVS_ROWS_GATHER=0) the chunked pass, element blocks reduced through shared
-                                  memory */
-  OVS_OPT_ROWS_TILED = 6,      /* tet row pass: 1 (env OVS_ROWS_TILED=1) one CTA per tile of rows, the tile's
-                                  element summaries staged in shared memory by bulk copies, then gathered as
-                                  above; 0 (default, the faster one measured) the untiled passes */
-  OVS_OPT_TILE_ELEMS = 7,      /* element budget of a row tile (default 96, env OVS_TILE_ELEMS; 4..4000);
-                                  rows with more elements take the untiled gather pass */
+  OVS_OPT_ROWS_GATHER = 5,     /* accepted, without effect */
+  OVS_OPT_ROWS_TILED = 6,      /* accepted, without effect */
+  OVS_OPT_TILE_ELEMS = 7,      /* accepted for 4..4000, without effect */
   OVS_OPT_MIXED_OUTER = 8      /* OVS_MIXED solves: m > 0 (default 30, env OVS_MIXED_OUTER; up to 200) a
                                   flexible GMRES(m) outer in FP64 whose directions are preconditioned by one
                                   FP32 GMRES cycle each; 0 the restarted refinement (one FP32 cycle on the

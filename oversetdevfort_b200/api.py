@@ -146,8 +146,9 @@ class Context:
 
     def set_option(self, option: int, value: int):
         """A kernel-variant option of this context (OVS_OPT_*: HEX_TC,
-        ARNOLDI_FUSED, ROWS_STAGED, ELEM_SMEM, ROWS_GATHER, ROWS_TILED,
-        TILE_ELEMS); see include/ovs.h for the values."""
+        ARNOLDI_FUSED, ELEM_SMEM, MIXED_OUTER; the former row-pass variants
+        ROWS_STAGED, ROWS_GATHER, ROWS_TILED, TILE_ELEMS are accepted without
+        effect); see include/ovs.h for the values."""
         F.check(self.lib.ovs_set_option(self.h, option, int(value)), "ovs_set_option")
 
     def set_faces(self, bf):

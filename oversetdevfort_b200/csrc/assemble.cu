@@ -8,23 +8,20 @@
 // BCLhs_tem, src/BCLhs_3D.f90) and the scatter (FillSparseMat_*,
 // LocaltoGlobalNSVOF_3D).
 //
-// Scheme (row owner, deterministic, atomic-free):
-//   * one warp owns one CSR row, i.e. one node A;
-//   * phase 1: lane l takes the l-th element of A's element list (sorted by
-//     element id) and evaluates A's row of that element's matrix, i.e. the
-//     nshl node-pair blocks (A, b), plus A's residual entries, from the
-//     gathered node records; results go to shared memory;
-//   * phase 2: the warp adds the element rows into a shared accumulator of
-//     A's CSR slots, element by element in ascending element id, so every
-//     slot is summed in the same order on every run;
+// Scheme (deterministic, atomic-free):
+//   * element pass: one thread per element evaluates its Gauss points once and
+//     writes a compact summary, the sums every block of its matrix is formed
+//     from, and its residual rows;
+//   * edge pass (tets): the work of an off-diagonal entry (A, B) is the list of
+//     elements holding both nodes, in ascending order, the same list for
+//     (B, A); a pair of lanes takes the two entries of an edge, expands one
+//     block per element from the summaries and writes its block; 8 lanes per
+//     node do the same for the diagonal block and the residual (hexahedra: a
+//     row pass of their own, assemble_hex.cuh);
 //   * the Dirichlet treatment of the reference zeroes element rows/columns
 //     and puts 1 on the element diagonal; both commute with the sum, so they
-//     are applied once at the row write: masked entries are 0, a constrained
-//     diagonal entry equals the number of elements around A;
-//   * the row (contiguous in the CSR value array) is written with vector
-//     stores.
-// Gauss-point physics is recomputed by each of the element's nshl rows
-// instead of being staged through HBM.
+//     are applied once at the write: masked entries are 0, a constrained
+//     diagonal entry equals the number of elements around A.
 #include "ovs_internal.cuh"
 
 #include <math.h>
@@ -47,15 +44,16 @@ struct AsmArgs {
   const int* n2e;
   const unsigned* n2s;    // slots of each entry's element nodes in the row
   const int4* row_rec;    // per row in processing order: {A, rowptr[A], n2e_ptr[A], deg | sd << 8 | ne << 16}
-  const int* cptr;        // off-diagonal contribution lists (tets): offsets per CSR entry
-  const int* clist;       //   entries (e << 4) | (la << 2) | b
+  const int4* edge_rec;   // edges (tets): {A, B, slot of (A, B), slot of (B, A)}, tile by tile of rows
+  const unsigned* edge_ptr;   //   offsets into edge_list, one per edge and the end
+  const unsigned* edge_list;  //   (e << 4) | (local node of A << 2) | local node of B
+  const unsigned* tile_edge;  // first edge of every tile of OVS_TILE_ROWS rows, and the end
   void* vals;             // nnz*NV
   void* rhs;              // NF*N field-major
   const void* kbuf;       // hex tensor-core block values (E x 64 x 24), or null
   int* flags;             // [0] non-positive DetJ count, [1] non-finite residual
   unsigned long long* cfl_bits;
   int N;
-  int nrows;              // row records the row pass visits (N, or the rows a tile cannot hold)
   int mat, vec;
   int max_deg;
   ovs_params p;
@@ -251,30 +249,36 @@ __device__ __forceinline__ void cfl_max(unsigned long long* bits, double v) {
 // row) expands A's row of each element matrix from the summaries.  Inactive
 // elements (solid on the NS+VOF pass, non-target on the NS pass) store zero
 // sums and zero residuals, which makes every expanded block exactly zero.
-// NS / NS+VOF: the Gauss-point sums of the block formulas (see
-// expand_block), which pass 1 forms once per element:
-//   [0, ND0)     per (row node a, column node b), PW values at PW (4a + b):
-//                NS+VOF {S_ab, L1_ab + E_ab, PL_ab, V_ab}, NS {S_ab}
-//   [ND0, C0)    per node n, 8 values: grad N_n (3), PR_n, T_n, U_n, Q_n, 0
-//   [C0, RHS0)   KA KB MM, then NS+VOF: KDP dphi (3) 0; NS: 0
-//   [RHS0, SW)   the residual, NF values per node
-// (PR_n is both P_b and R_a of the block formulas, U_n both U_b and W_a)
-//   TEM  : the 4x4 element matrix itself, row-major (a, b) | residual 4 = 20
-//          (a scalar system: its element matrix is smaller than the
-//          Gauss-point records it would be expanded from)
+// NS / NS+VOF: the Gauss-point sums of the block formulas (see form_block),
+// which pass 1 forms once per element, in groups of 4 values that a lane of
+// the edge pass reads with one load each:
+//   [0, ND0)    per (row node a, column node b), PW values at PW (4a + b):
+//               NS+VOF {S_ab, L1_ab + E_ab, PL_ab, V_ab}, NS {S_ab}
+//   [ND0, T0)   per node n: grad N_n (3) and U_n (NS: 0)
+//   [T0, C0)    T_n (4), Q_n (4)
+//   [C0, RHS0)  NS+VOF KA KB MM KDP dphi (3) PR; NS KA KB MM PR
+//   [RHS0, SW)  the residual: (u1, u2, u3, p) of every node, then NS+VOF phi (4)
+// (PR = fact2 w, the sum of fact2 w N_n over the points, the same for every
+// node; U_n is both U_b and W_a of the block formulas)
+//   TEM  : the element matrix itself (a scalar system: smaller than what it
+//          would be expanded from) as K_ab, K_ba of the six edges a < b (12),
+//          then K_aa and the residual of every node (8)
 // GQ: the values pass 1 keeps per Gauss point for the sums: uadv (3) and
 // rt = rho tauM; NS+VOF: uadv (3) rho rt tauLS src eps ufac plfac (the
 // factors of the phase-change terms).
 template <int KIND> struct Lay;
 template <> struct Lay<OVS_ASM_NS> {
-  static constexpr int PW = 1, ND0 = 16, C0 = 48, RHS0 = 52, SW = 68, NF = 4, NV = 16, GQ = 4;
+  static constexpr int PW = 1, ND0 = 16, T0 = 32, C0 = 40, RHS0 = 44, SW = 60, NF = 4, NV = 16, GQ = 4;
 };
 template <> struct Lay<OVS_ASM_NSVOF> {
-  static constexpr int PW = 4, ND0 = 64, C0 = 96, RHS0 = 104, SW = 124, NF = 5, NV = 24, GQ = 10;
+  static constexpr int PW = 4, ND0 = 64, T0 = 80, C0 = 88, RHS0 = 96, SW = 116, NF = 5, NV = 24, GQ = 10;
 };
 template <> struct Lay<OVS_ASM_TEM> {
-  static constexpr int SW = 20, RHS0 = 16, NF = 1, NV = 1;
+  static constexpr int SW = 20, RHS0 = 12, NF = 1, NV = 1;
 };
+
+// number of the edge {a, b} of a tet, a < b in the order 01 02 03 12 13 23
+__device__ __forceinline__ constexpr int tet_edge(int a, int b) { return a * (5 - a) / 2 + b - 1; }
 
 // 4 values of an element summary (global memory; 16-byte aligned in FP32,
 // 32-byte aligned in FP64, where every 4-value group of a summary sits on
@@ -295,22 +299,22 @@ __device__ __forceinline__ void put4(double* d, double a, double b, double c, do
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(d), "d"(a), "d"(b), "d"(c), "d"(e));
 }
 
-// The Gauss-point sums of the NS / NS+VOF block formulas (expand_block)
+// The Gauss-point sums of the NS / NS+VOF block formulas (form_block)
 // from the per-point values q (layout GQ above), the shape gradients g and
 // the weight w, written to the summary o: with c_n = uadv . grad N_n,
 //   S_ab  = sum w rho (Na + rt ca)(fact1 Nb + fact2 cb)
 //   L1_ab = sum w (Na + tauLS ca)(fact1 Nb + fact2 cb + fact2 Nb src)
 //   E_ab  = sum eps Na Nb      PL_ab = -sum plfac Na Nb
 //   V_ab  = sum fact2 w (Na + tauLS ca) Nb
-//   PR_n  = sum fact2 w Nn     T_n = sum w rt (fact1 Nn + fact2 cn)
-//   U_n   = sum ufac Nn        Q_n = sum fact2 w rt cn
+//   U_n   = sum ufac Nn        T_n = sum w rt (fact1 Nn + fact2 cn)
+//   Q_n   = sum fact2 w rt cn
 // (rho = rho_ns on the NS pass).  Each sum is formed once per element here
 // instead of once per block in the row pass.  block_sums_row writes the
 // pairs of row node a and node a's record (a may vary per lane: the
 // per-node values are picked by selects, which fold for a constant a).
 template <typename T, int KIND>
 __device__ __forceinline__ void block_sums_row(const T (&q)[4][Lay<KIND>::GQ], const T (&g)[4][3], T w, T fact1,
-                                               T fact2, T rho_ns, int a, T* o) {
+                                               T fact2, T rho_ns, int a, T* o, T (&tq)[8]) {
   using L = Lay<KIND>;
   constexpr bool vof = KIND == OVS_ASM_NSVOF;
   T c[4][4];
@@ -347,14 +351,13 @@ __device__ __forceinline__ void block_sums_row(const T (&q)[4][Lay<KIND>::GQ], c
   } else {
     put4(o + L::PW * 4 * a, S[0], S[1], S[2], S[3]);
   }
-  T PR = 0, Tn = 0, U = 0, Q = 0;
+  T Tn = 0, U = 0, Q = 0;
 #pragma unroll
   for (int gp = 0; gp < 4; ++gp) {
     T N[4];
     tet_shape<T>(gp, N);
     const T Nn = pick4<T>(N, a), cn = pick4<T>(c[gp], a);
     const T rt = vof ? q[gp][4] : q[gp][3];
-    PR += fact2 * w * Nn;
     Tn += w * rt * (fact1 * Nn + fact2 * cn);
     Q += fact2 * w * rt * cn;
     if constexpr (vof) U += q[gp][8] * Nn;
@@ -365,16 +368,20 @@ __device__ __forceinline__ void block_sums_row(const T (&q)[4][Lay<KIND>::GQ], c
     const T col[4] = {g[0][d], g[1][d], g[2][d], g[3][d]};
     ga[d] = pick4<T>(col, a);
   }
-  put4(o + L::ND0 + 8 * a, ga[0], ga[1], ga[2], PR);
-  put4(o + L::ND0 + 8 * a + 4, Tn, U, Q, (T)0);
+  put4(o + L::ND0 + 4 * a, ga[0], ga[1], ga[2], U);
+  tq[a] = Tn;
+  tq[4 + a] = Q;
 }
 
 // all four rows of the element (one thread per element)
 template <typename T, int KIND>
 __device__ __forceinline__ void block_sums(const T (&q)[4][Lay<KIND>::GQ], const T (&g)[4][3], T w, T fact1,
                                            T fact2, T rho_ns, T* o) {
+  T tq[8];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) block_sums_row<T, KIND>(q, g, w, fact1, fact2, rho_ns, a, o);
+  for (int a = 0; a < 4; ++a) block_sums_row<T, KIND>(q, g, w, fact1, fact2, rho_ns, a, o, tq);
+  put4(o + Lay<KIND>::T0, tq[0], tq[1], tq[2], tq[3]);
+  put4(o + Lay<KIND>::T0 + 4, tq[4], tq[5], tq[6], tq[7]);
 }
 
 // The CFL number delt sqrt(taua), largest over an element's points: the
@@ -490,7 +497,7 @@ __device__ void summarize_ns(const SumArgs& a, const RA& r, const LA& lo, bool t
   T* orh = o + (MAT ? L::RHS0 : 0);
 #pragma unroll
   for (int n = 0; n < 4; ++n) put4(orh + 4 * n, ru[n][0], ru[n][1], ru[n][2], rp[n]);
-  if constexpr (MAT) put4(o + L::C0, KA, KB, MM, (T)0);
+  if constexpr (MAT) put4(o + L::C0, KA, KB, MM, target ? fact2 * w : (T)0);
   if constexpr (MAT)
     block_sums<T, OVS_ASM_NS>(q, g, target ? w : (T)0, (T)p.almi, fact2, rho, o);
 }
@@ -688,7 +695,13 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
                    q[gp], KA, KB, MM, KDP, ru, rp, rf, tamax, iv);
   }
   using L = Lay<OVS_ASM_NSVOF>;
-  {
+  if constexpr (MAT) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) put4(o + L::RHS0 + 4 * n, ru[n][0], ru[n][1], ru[n][2], rp[n]);
+    put4(o + L::RHS0 + 16, rf[0], rf[1], rf[2], rf[3]);
+    put4(o + L::C0, KA, KB, MM, KDP);
+    put4(o + L::C0 + 4, dphi[0], dphi[1], dphi[2], fluid ? (T)(p.alfi * p.delt * p.gami) * w : (T)0);
+  } else {   // 5 values per node
     T rh[20];
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -696,11 +709,7 @@ __device__ void summarize_nsvof(const SumArgs& a, const RA& r, const LA& lo, boo
       rh[5 * n + 3] = rp[n]; rh[5 * n + 4] = rf[n];
     }
 #pragma unroll
-    for (int k = 0; k < 20; k += 4) put4(o + (MAT ? L::RHS0 : 0) + k, rh[k], rh[k + 1], rh[k + 2], rh[k + 3]);
-  }
-  if constexpr (MAT) {
-    put4(o + L::C0, KA, KB, MM, KDP);
-    put4(o + L::C0 + 4, dphi[0], dphi[1], dphi[2], (T)0);
+    for (int k = 0; k < 20; k += 4) put4(o + k, rh[k], rh[k + 1], rh[k + 2], rh[k + 3]);
   }
   if constexpr (MAT)
     block_sums<T, OVS_ASM_NSVOF>(q, g, fluid ? w : (T)0, (T)p.almi, (T)(p.alfi * p.delt * p.gami), (T)0, o);
@@ -810,116 +819,94 @@ __device__ void summarize_tem(const SumArgs& a, const RA& r, const LA& lo, bool 
       for (int n = 0; n < 4; ++n) rt[n] += w * (-N[n] * rcp * rTi - hk * gdT[n]);
     }
   }
-  if constexpr (MAT) {
 #pragma unroll
-    for (int ia = 0; ia < 4; ++ia)
+  for (int ia = 0; ia < 4; ++ia) {
+    if constexpr (MAT) {
+      o[Lay<OVS_ASM_TEM>::RHS0 + 2 * ia + 1] = rt[ia];
 #pragma unroll
       for (int ib = 0; ib < 4; ++ib)
-        o[4 * ia + ib] = K[ia][ib] + HK * (g[ia][0] * g[ib][0] + g[ia][1] * g[ib][1] + g[ia][2] * g[ib][2]);
+        o[ia == ib ? Lay<OVS_ASM_TEM>::RHS0 + 2 * ia
+                   : 2 * (ia < ib ? tet_edge(ia, ib) : tet_edge(ib, ia)) + (ia < ib ? 0 : 1)] =
+            K[ia][ib] + HK * (g[ia][0] * g[ib][0] + g[ia][1] * g[ib][1] + g[ia][2] * g[ib][2]);
+    } else {
+      o[ia] = rt[ia];
+    }
   }
-#pragma unroll
-  for (int n = 0; n < 4; ++n) o[(MAT ? Lay<OVS_ASM_TEM>::RHS0 : 0) + n] = rt[n];
 }
 
 // -------------------------------------------------- pass 2: block expansion
-// Blocks of row A (local node la) of one element from its summary, for a
-// column node b (formulas factored from the reference's per Gauss point
-// sums, with the sums of block_sums):
-//   K(i,j) = KA ga_j gb_i + KB ga_i gb_j + delta_ij (KA gab + S_ab)
-//   G(i) = -ga_i PR_b + gb_i Q_a      D(i) = gb_i PR_a + ga_i T_b
-//   M = MM gab    LS = L1_ab + E_ab + KDP gab    ULS(i) = ga_i U_b
-//   PLS = PL_ab   LSU(i) = dphi_i V_ab - gb_i U_a
-// 4 consecutive values: read-only global loads (SMEM = false) or loads from
-// the warp's shared-memory stage (SMEM = true)
-template <typename T, bool SMEM = false>
-__device__ __forceinline__ void ldv4(const T* p, T* d) {
-  if constexpr (sizeof(T) == 4) {
-    const float4 v = SMEM ? *reinterpret_cast<const float4*>(p) : __ldg(reinterpret_cast<const float4*>(p));
-    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-  } else {
-    const double2 a = SMEM ? reinterpret_cast<const double2*>(p)[0] : __ldg(reinterpret_cast<const double2*>(p));
-    const double2 b = SMEM ? reinterpret_cast<const double2*>(p)[1] : __ldg(reinterpret_cast<const double2*>(p) + 1);
-    d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
-  }
+// 4 consecutive values with one read-only load (FP64: the 256-bit load of
+// sm_100; summary groups are 32-byte aligned there)
+__device__ __forceinline__ void ldv4(const float* p, float* d) {
+  const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+  d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
 }
-template <typename T, bool SMEM = false>
-__device__ __forceinline__ T ld1(const T* p) {
-  if constexpr (SMEM) return *p;
-  else return __ldg(p);
+__device__ __forceinline__ void ldv4(const double* p, double* d) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(d[0]), "=d"(d[1]), "=d"(d[2]), "=d"(d[3]) : "l"(p));
+}
+// 2 consecutive values
+__device__ __forceinline__ void ldv2(const float* p, float* d) {
+  const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+  d[0] = v.x; d[1] = v.y;
+}
+__device__ __forceinline__ void ldv2(const double* p, double* d) {
+  const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+  d[0] = v.x; d[1] = v.y;
 }
 
-// the summary values an NS/NS+VOF block (la, b) is formed from: node la's
-// record, the element constants, node b's record and the pair sums
+// the summary values an NS/NS+VOF block (row node a, column node b) is formed
+// from: the nodes' gradients and U, Q of the row, T of the column, the element
+// constants and the pair sums
 template <typename T> struct BlockIn {
-  T na[8], cs[8], nb[8], pr[4];
+  T ga[4], gb[4], Qa, Tb, cs[8], pr[4];
 };
 
-template <typename T, int KIND, bool SMEM>
-__device__ __forceinline__ void load_block(const T* sm, int la, int b, BlockIn<T>& in) {
+template <typename T, int KIND>
+__device__ __forceinline__ void load_block(const T* sm, int a, int b, BlockIn<T>& in) {
   using L = Lay<KIND>;
-  constexpr bool vof = KIND == OVS_ASM_NSVOF;
-  ldv4<T, SMEM>(sm + L::ND0 + 8 * la, in.na);
-  ldv4<T, SMEM>(sm + L::ND0 + 8 * la + 4, in.na + 4);
-  ldv4<T, SMEM>(sm + L::C0, in.cs);
-  ldv4<T, SMEM>(sm + L::ND0 + 8 * b, in.nb);
-  ldv4<T, SMEM>(sm + L::ND0 + 8 * b + 4, in.nb + 4);
-  if constexpr (vof) {
-    ldv4<T, SMEM>(sm + L::C0 + 4, in.cs + 4);
-    ldv4<T, SMEM>(sm + L::PW * (4 * la + b), in.pr);
+  ldv4(sm + L::ND0 + 4 * a, in.ga);
+  ldv4(sm + L::ND0 + 4 * b, in.gb);
+  ldv4(sm + L::C0, in.cs);
+  if constexpr (KIND == OVS_ASM_NSVOF) {
+    ldv4(sm + L::C0 + 4, in.cs + 4);
+    ldv4(sm + L::PW * (4 * a + b), in.pr);
   } else {
-    in.pr[0] = ld1<T, SMEM>(sm + L::PW * (4 * la + b));
+    in.pr[0] = __ldg(sm + L::PW * (4 * a + b));
   }
+  in.Tb = __ldg(sm + L::T0 + b);
+  in.Qa = __ldg(sm + L::T0 + 4 + a);
 }
 
+// Block of row node a, column node b added to o (formulas factored from the
+// reference's per Gauss point sums, with the sums of block_sums):
+//   K(i,j) = KA ga_j gb_i + KB ga_i gb_j + delta_ij (KA gab + S_ab)
+//   G(i) = -ga_i PR + gb_i Q_a      D(i) = gb_i PR + ga_i T_b
+//   M = MM gab    LS = L1_ab + E_ab + KDP gab    ULS(i) = ga_i U_b
+//   PLS = PL_ab   LSU(i) = dphi_i V_ab - gb_i U_a
 template <typename T, int KIND>
-__device__ __forceinline__ void form_block(const BlockIn<T>& in, T (&o)[Lay<KIND>::NV]) {
+__device__ __forceinline__ void add_block(const BlockIn<T>& in, T* o) {
   constexpr bool vof = KIND == OVS_ASM_NSVOF;
-  const T ga[3] = {in.na[0], in.na[1], in.na[2]};
-  const T Ra = in.na[3], Wa = in.na[5], Qa = in.na[6];
-  const T KA = in.cs[0], KB = in.cs[1], MM = in.cs[2];
-  const T gk[3] = {in.nb[0], in.nb[1], in.nb[2]};
-  const T Pb = in.nb[3], Tb = in.nb[4], Ub = in.nb[5];
-  const T gab = ga[0] * gk[0] + ga[1] * gk[1] + ga[2] * gk[2];
+  const T KA = in.cs[0], KB = in.cs[1], MM = in.cs[2], PR = vof ? in.cs[7] : in.cs[3];
+  const T gab = in.ga[0] * in.gb[0] + in.ga[1] * in.gb[1] + in.ga[2] * in.gb[2];
   const T dg = KA * gab + in.pr[0];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
+    const T ka = KA * in.gb[i], kb = KB * in.ga[i];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) o[4 * i + j] = KA * ga[j] * gk[i] + KB * ga[i] * gk[j] + (i == j ? dg : (T)0);
-    o[4 * i + 3] = -ga[i] * Pb + gk[i] * Qa;
+    for (int j = 0; j < 3; ++j) o[4 * i + j] += ka * in.ga[j] + kb * in.gb[j];
+    o[5 * i] += dg;
+    o[4 * i + 3] += in.gb[i] * in.Qa - in.ga[i] * PR;
+    o[12 + i] += in.gb[i] * PR + in.ga[i] * in.Tb;
   }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) o[12 + d] = gk[d] * Ra + ga[d] * Tb;
-  o[15] = MM * gab;
+  o[15] += MM * gab;
   if constexpr (vof) {
-    const T KDP = in.cs[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) o[16 + d] = in.cs[4 + d] * in.pr[3] - gk[d] * Wa;
-    o[19] = in.pr[1] + KDP * gab;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) o[20 + d] = ga[d] * Ub;
-    o[23] = in.pr[2];
-  }
-}
-
-// Blocks (row node la, column nodes b0 + k*BS, k < NC) of an element from
-// its summary.  The 4 lanes of an NS/NS+VOF element take one column each
-// (NC = 1); a T lane takes all four.  sm: the element's summary (global
-// memory, or its matrix part staged in shared memory with SMEM); the
-// residual rows behind it are read by the caller
-template <typename T, int KIND, int NC, bool SMEM = false>
-__device__ __forceinline__ void expand_block(const T* sm, int la, int b0, int BS,
-                                             T (&o)[NC][Lay<KIND>::NV < 4 ? 1 : Lay<KIND>::NV]) {
-  if constexpr (KIND == OVS_ASM_TEM) {
-    // the element pass stored the element matrix: row la, columns b
-#pragma unroll
-    for (int k = 0; k < NC; ++k) o[k][0] = sm[4 * la + b0 + k * BS];
-  } else {
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-      BlockIn<T> in;
-      load_block<T, KIND, SMEM>(sm, la, b0 + k * BS, in);
-      form_block<T, KIND>(in, o[k]);
+    for (int d = 0; d < 3; ++d) {
+      o[16 + d] += in.cs[4 + d] * in.pr[3] - in.gb[d] * in.ga[3];
+      o[20 + d] += in.ga[d] * in.gb[3];
     }
+    o[19] += in.pr[1] + in.cs[3] * gab;
+    o[23] += in.pr[2];
   }
 }
 
@@ -941,51 +928,6 @@ template <> struct Vec4<double> {
     reinterpret_cast<double2*>(dst)[1] = a1;
   }
 };
-
-// shared-memory layout per warp: the blocks of the chunk's elements
-// [CH elements][4 columns][BSTR] (stride padded so the 16-byte stores of a
-// quarter warp hit distinct banks), their RHS rows [CH][RSTR], the row
-// accumulator [max_deg][NVP], then the slot words of the chunk's elements
-// [CH], the columns [max_deg] and their Dirichlet masks [max_deg]
-template <typename T, int KIND> struct Smem {
-  static constexpr int NV = Lay<KIND>::NV, NF = Lay<KIND>::NF;
-  static constexpr int LPE = (NV < 4) ? 1 : 4;       // lanes per element
-  static constexpr int CH = 32 / LPE;                // elements per chunk
-  static constexpr int NVP = (NV < 4) ? 1 : NV;
-  static constexpr int BSTR = (NV < 4) ? 1 : NV + 16 / (int)sizeof(T);
-  static constexpr int RSTR = NF + 1;
-  // the stage buffer of the staged row pass: the chunk's CH element
-  // summaries, copied in with one round of asynchronous 16-byte copies
-  static constexpr int SW = Lay<KIND>::SW;
-  // values staged per element: the matrix part of the summary (the residual
-  // rows behind it are read from global memory by the lanes that need them)
-  static constexpr int SWS = (KIND == OVS_ASM_TEM) ? SW : Lay<KIND>::RHS0;
-  __host__ __device__ static size_t ints_offset(int max_deg) {
-    const size_t b = sizeof(T) * ((size_t)4 * CH * BSTR + (size_t)CH * RSTR + (size_t)max_deg * NVP);
-    return (b + 15) & ~(size_t)15;
-  }
-  __host__ __device__ static size_t bytes(int max_deg, bool staged = false) {
-    size_t b = ints_offset(max_deg) + sizeof(int) * ((size_t)CH + 2 * (size_t)max_deg);
-    b = (b + 15) & ~(size_t)15;
-    if (staged) b += sizeof(T) * (size_t)CH * SWS;
-    return b;
-  }
-  __host__ __device__ static size_t stage_offset(int max_deg) { return bytes(max_deg, false); }
-};
-
-// 16-byte asynchronous global -> shared copy (cp.async, no register
-// staging) and 4-byte variant; completion by cp_async_wait_all
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
 
 // ---------------------------------------------------------- pass 1 kernel
 // blocks per SM the element pass is compiled for: the FP32 NS+VOF pass at 3
@@ -1091,587 +1033,214 @@ __device__ __forceinline__ unsigned mask_of(int v) {
   return (unsigned)c_rowbits[v] | ((unsigned)c_colbits[v] << 8) | ((unsigned)c_diagbit[v] << 16);
 }
 
-// One warp per CSR row, the rows in the order of the row records (Morton
-// order of the nodes, so that the rows sharing an element run close
-// together in time and its summary comes from L2).  Per chunk of CH of the
-// row's elements: phase 1 expands block (A's row, column b) of each element
-// into shared memory (lane = element, column), phase 2 adds them into the
-// row accumulator, each lane owning value groups of whole slots and adding
-// the chunk's blocks that fall in its slot in ascending element order (so
-// every entry is summed in the same order on every run).  The next row's
-// record and its first element ids are loaded while the current row runs,
-// and the Dirichlet masks of the row's columns while its first chunk runs.
-// STAGED: the warp first copies the chunk's element summaries into its
-// shared-memory stage with one round of asynchronous 16-byte copies (all in
-// flight together, no registers held); the block expansion then reads
-// shared memory.  Otherwise every lane reads its element's summary from
-// global memory.
-template <typename T, int KIND, int WARPS, bool STAGED>
-__global__ void __launch_bounds__(WARPS * 32)
-assemble_rows_kernel(const AsmArgs a) {
-  using S = Smem<T, KIND>;
-  using L = Lay<KIND>;
-  constexpr int NV = S::NV, NF = S::NF, NVP = S::NVP, BSTR = S::BSTR, RSTR = S::RSTR, CH = S::CH;
-  constexpr int NG = (NV >= 4) ? NV / 4 : 1;   // value groups per slot: 4 values (T: the value)
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned masks[24];
-  if (threadIdx.x < 24) masks[threadIdx.x] = (KIND == OVS_ASM_TEM) ? (TB | (TB << 8) | (TB << 16)) : mask_of(threadIdx.x);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned char* base = smem_raw + (size_t)wid * S::bytes(a.max_deg, STAGED);
-  T* stage = reinterpret_cast<T*>(base + S::stage_offset(a.max_deg));   // [CH][SWS] (STAGED)
-  T* blk = reinterpret_cast<T*>(base);                 // [CH][4][BSTR]
-  T* rvs = blk + 4 * CH * BSTR;                        // [CH][RSTR]
-  T* acc = rvs + CH * RSTR;                            // [max_deg][NVP]
-  unsigned* sl4 = reinterpret_cast<unsigned*>(base + S::ints_offset(a.max_deg));   // [CH]
-  int* cols = reinterpret_cast<int*>(sl4 + CH);        // [max_deg]
-  unsigned* cib = reinterpret_cast<unsigned*>(cols + a.max_deg);                 // [max_deg]
-
-  const T* sum = reinterpret_cast<const T*>(a.rec);
-  const int W = gridDim.x * WARPS;
-  // lane = (element jl of the chunk, first column node bl0 of that element);
-  // with one lane per element (T) a lane takes all 4 columns
-  constexpr int LPE = S::LPE, CPL = 4 / LPE;
-  const int jl = lane / LPE, bl0 = lane % LPE;
-  constexpr int SWS = S::SWS;
-  constexpr int U16 = SWS * (int)sizeof(T) / 16;            // 16-byte units staged per summary
-  static_assert(SWS * sizeof(T) % 16 == 0, "staged summaries must be whole 16-byte units");
-  static_assert(L::SW * sizeof(T) % 16 == 0, "summaries must be whole 16-byte units");
-  int t = blockIdx.x * WARPS + wid;
-  // row record {A, rowptr[A], n2e_ptr[A], deg | sd << 8 | ne << 16} and the element
-  // ids of the first chunk (lanes j < nc hold entry j)
-  int4 rr = make_int4(0, 0, 0, 0);
-  if (t < a.nrows) rr = __ldg(a.row_rec + t);
-  int pk_n = 0;
-  unsigned s4_n = 0;
-  if (t < a.nrows && lane < min(CH, rr.w >> 16)) {
-    pk_n = __ldg(a.n2e + rr.z + lane);
-    s4_n = __ldg(a.n2s + rr.z + lane);
+// Edge pass (tets).  A block of 4 warps takes a tile of OVS_TILE_ROWS
+// consecutive rows of the row order (Morton order of the nodes, so that what
+// runs at a time shares its elements and reads their summaries from L2): the
+// diagonal blocks and residuals of the tile's rows, 8 lanes per row, then the
+// edges the tile owns (those whose other node comes later in the order), in
+// sets of 16, two lanes per edge: lane 0 the entry (A, B), lane 1 (B, A).
+// Every entry adds its elements in ascending order; a diagonal block adds
+// lane l's elements l, l + 8, ... and then the lanes by halving: orders fixed
+// by the mesh, the same on every run.
+// Bound: the summaries are read in scattered 32-byte pieces, which the L1
+// data path serves at a quarter of its rate, so what counts is the bytes a
+// block asks for and how many distinct elements a load touches: 22 values
+// per block, and the two lanes of an edge read the same element.  A warp per
+// row with one list per entry (28 values, 24 elements a load, an exchange
+// through shared memory) took 12.65 ms for the FP64 NS+VOF rows of the
+// 128^3 x6 tets and 6.91 ms in FP32; this takes 6.70 and 3.64 ms (T: 1.90 ->
+// 0.85 and 1.43 -> 0.47 ms).  A tile's edges are sorted by list
+// length, so the rounds of a set are nearly equal.
+template <typename T, int KIND>
+__device__ __forceinline__ void write_entry(T* dst, T* v, const unsigned* masks, unsigned ibA, unsigned ibB) {
+  constexpr int NV = Lay<KIND>::NV;
+  if ((ibA | ibB) != 0u) {
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+      const unsigned m = masks[u];
+      if ((ibA & m & 0xffu) || ((ibB << 8) & m & 0xff00u)) v[u] = (T)0;
+    }
   }
-  for (; t < a.nrows; t += W) {
-    const int A = rr.x, rp = rr.y, ep = rr.z, deg = rr.w & 0xff, ne = rr.w >> 16;
-    int4 rn = make_int4(0, 0, 0, 0);
-    if (t + W < a.nrows) rn = __ldg(a.row_rec + t + W);
-    const unsigned ibA = __ldg(a.ibc + A);
-    for (int s = lane; s < deg; s += 32) cp_async4(cols + s, a.colidx + rp + s);
-    for (int q = lane; q < deg * NVP; q += 32) acc[q] = (T)0;
-    T racc = (T)0;
-    unsigned ib0 = 0, ib1 = 0;   // masks of columns lane and lane + 32
-    __syncwarp();
-    for (int c0 = 0; c0 < ne; c0 += CH) {
-      const int nc = min(CH, ne - c0);
-      const int pk_c = pk_n;
-      const unsigned s4_c = s4_n;
-      // the next chunk's ids travel while this one is expanded
-      if (c0 + CH < ne && lane < min(CH, ne - c0 - CH)) {
-        pk_n = __ldg(a.n2e + ep + c0 + CH + lane);
-        s4_n = __ldg(a.n2s + ep + c0 + CH + lane);
-      }
-      if constexpr (STAGED) {
-        // every lane runs the same trip count: the shuffle needs the full warp
-        for (int it = 0; it < (CH * U16 + 31) / 32; ++it) {
-          const int u = lane + 32 * it;
-          const int j = min(u / U16, CH - 1);
-          const int e = __shfl_sync(0xffffffffu, pk_c, j) >> 3;
-          if (u < nc * U16) {
-            const int k = u - j * U16;
-            cp_async16(reinterpret_cast<unsigned char*>(stage + (size_t)j * SWS) + 16 * k,
-                       reinterpret_cast<const unsigned char*>(sum + (size_t)e * L::SW) + 16 * k);
-          }
-        }
-        cp_async_wait_all();
-        __syncwarp();
-      }
-      // ---------------- phase 1: block (A's row, column bl) of element jl
-      const int packed = __shfl_sync(0xffffffffu, pk_c, min(jl, CH - 1));
-      const unsigned slots4 = __shfl_sync(0xffffffffu, s4_c, min(jl, CH - 1));
-      if (jl < nc) {
-        const int e = packed >> 3, la = packed & 7;
-        T o[CPL][NVP];
-        if constexpr (STAGED)
-          expand_block<T, KIND, CPL, true>(stage + (size_t)jl * SWS, la, bl0, LPE, o);
-        else
-          expand_block<T, KIND, CPL>(sum + (size_t)e * L::SW, la, bl0, LPE, o);
 #pragma unroll
-        for (int k = 0; k < CPL; ++k) {
-          T* dst = blk + (jl * 4 + bl0 + k * LPE) * BSTR;
-          if constexpr (NV >= 4) {
-#pragma unroll
-            for (int v = 0; v < NV; v += 4) store_row<4>(dst + v, o[k] + v);
-          } else {
-            dst[0] = o[k][0];
-          }
-        }
-        if (bl0 == 0) {   // the element's slot word and residual rows of node la
-          sl4[jl] = slots4;
-          const T* r = sum + (size_t)e * L::SW + L::RHS0 + NF * la;
-#pragma unroll
-          for (int f = 0; f < NF; ++f) rvs[jl * RSTR + f] = r[f];
-        }
-      }
-      if (c0 == 0) {
-        // the columns have arrived (their copies were issued at the row's
-        // start); their masks travel while the row is assembled
-        if constexpr (!STAGED) cp_async_wait_all();
-        __syncwarp();
-        if (lane < deg) ib0 = __ldg(a.ibc + cols[lane]);
-        if (lane + 32 < deg) ib1 = __ldg(a.ibc + cols[lane + 32]);
-      }
-      __syncwarp();
-      // ---------------- phase 2: ordered reduction into acc
-      // task q = (slot s, value group g); the 4 blocks of one element go to
-      // distinct slots (elements with a repeated node are rejected at upload)
-      for (int q = lane; q < deg * NG; q += 32) {
-        const int s = q / NG, g = q - s * NG;
-        const unsigned key = (unsigned)s * 0x01010101u;
-        if constexpr (NV >= 4) {
-          T v[4];
-          ldv4<T, true>(acc + s * NVP + 4 * g, v);
-          for (int j = 0; j < nc; ++j) {
-            const unsigned m = __vcmpeq4(sl4[j], key);
-            if (m) {
-              const int b = (__ffs(m) - 1) >> 3;
-              T x[4];
-              ldv4<T, true>(blk + (j * 4 + b) * BSTR + 4 * g, x);
-              v[0] += x[0]; v[1] += x[1]; v[2] += x[2]; v[3] += x[3];
-            }
-          }
-          store_row<4>(acc + s * NVP + 4 * g, v);
-        } else {
-          T v = acc[s];
-          for (int j = 0; j < nc; ++j) {
-            const unsigned m = __vcmpeq4(sl4[j], key);
-            if (m) v += blk[j * 4 + ((__ffs(m) - 1) >> 3)];
-          }
-          acc[s] = v;
-        }
-      }
-      if (lane < NF)
-        for (int j = 0; j < nc; ++j) racc += rvs[j * RSTR + lane];
-      __syncwarp();
-    }
-    if (ne == 0) {   // a node without elements: only the Dirichlet rows
-      cp_async_wait_all();
-      __syncwarp();
-      if (lane < deg) ib0 = __ldg(a.ibc + cols[lane]);
-      if (lane + 32 < deg) ib1 = __ldg(a.ibc + cols[lane + 32]);
-    }
-    // the next row's first element ids travel while this row is written
-    pk_n = 0;
-    s4_n = 0;
-    if (t + W < a.nrows && lane < min(CH, rn.w >> 16)) {
-      pk_n = __ldg(a.n2e + rn.z + lane);
-      s4_n = __ldg(a.n2s + rn.z + lane);
-    }
-    // ---------------- row write with the Dirichlet treatment
-    {
-      if (lane < deg) cib[lane] = ib0;
-      if (lane + 32 < deg) cib[lane + 32] = ib1;
-      for (int s = lane + 64; s < deg; s += 32) cib[s] = __ldg(a.ibc + cols[s]);
-      __syncwarp();
-      T* out = reinterpret_cast<T*>(a.vals) + (size_t)rp * NV;
-      const T cnt = (T)ne;
-      if constexpr (NV >= 4) {
-        // one 4-value group per lane and step, 16-byte aligned (NV % 4 == 0)
-        for (int q = lane; q < deg * NG; q += 32) {
-          const int s = q / NG, gidx = q - s * NG;
-          const unsigned ibB = cib[s];
-          const bool dg = cols[s] == A;
-          T v4[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const unsigned m = masks[4 * gidx + u];
-            T val = acc[s * NVP + 4 * gidx + u];
-            if ((ibA & m & 0xffu) || ((ibB << 8) & m & 0xff00u)) val = (T)0;
-            if (dg && ((ibA << 16) & m & 0xff0000u)) val = cnt;
-            v4[u] = val;
-          }
-          store4_cs(out + (size_t)s * NV + 4 * gidx, v4);
-        }
-      } else {
-        for (int q = lane; q < deg; q += 32) {
-          const int B = cols[q];
-          const unsigned ibB = cib[q];
-          T val = acc[q];
-          if ((ibA & TB) || (ibB & TB)) val = (T)0;
-          if (B == A && (ibA & TB)) val = cnt;
-          __stcs(out + q, val);
-        }
-      }
-    }
-    if (a.vec && lane < NF) {
-      unsigned bit;
-      if (KIND == OVS_ASM_TEM) bit = TB;
-      else bit = (lane < 3) ? (1u << lane) : (lane == 3 ? PB : FB);
-      T v = (ibA & bit) ? (T)0 : racc;
-      if (!isfinite((double)v)) atomicOr(a.flags + 1, 1);
-      __stcs(reinterpret_cast<T*>(a.rhs) + (size_t)lane * a.N + A, v);
-    }
-    rr = rn;
-    __syncwarp();
-  }
+  for (int g = 0; g < NV; g += 4) store4_cs(dst + g, v + g);
 }
 
-// A block of NV values to its CSR slot with the Dirichlet treatment of the
-// row (ibA) and column (ibB) masks; dg: the diagonal entry (cnt, the row's
-// element count, on constrained diagonal positions)
-template <typename T, int NV>
-__device__ __forceinline__ void write_block(T* dst, const T* v, const unsigned* masks, unsigned ibA, unsigned ibB,
-                                            bool dg, T cnt) {
-  const bool plain = (ibA | ibB) == 0u;
-  if constexpr (NV >= 4) {
+// the diagonal block of row rr and its residual (8 lanes, l8 their index)
+template <typename T, int KIND>
+__device__ __forceinline__ void diag_row(const AsmArgs& a, const int4 rr, bool on, int l8, const unsigned* masks) {
+  using L = Lay<KIND>;
+  constexpr int NV = L::NV, NF = L::NF, NG = NV / 4;
+  const int A = rr.x, deg = rr.w & 0xff, sd = (rr.w >> 8) & 0xff, ne = on ? rr.w >> 16 : 0;
+  const T* sum = reinterpret_cast<const T*>(a.rec);
+  T v[32];
 #pragma unroll
-    for (int g = 0; g < NV; g += 4) {
-      T v4[4];
+  for (int k = 0; k < 32; ++k) v[k] = (T)0;
+  int pk = l8 < ne ? __ldg(a.n2e + rr.z + l8) : 0;
+  for (int q = l8; q < ne; q += 8) {
+    const int la = pk & 7;
+    const T* se = sum + (size_t)(pk >> 3) * L::SW;
+    if (q + 8 < ne) pk = __ldg(a.n2e + rr.z + q + 8);
+    BlockIn<T> in;
+    T r[4];
+    load_block<T, KIND>(se, la, la, in);
+    ldv4(se + L::RHS0 + 4 * la, r);
+    add_block<T, KIND>(in, v);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) v[NV + f] += r[f];
+    if constexpr (NF == 5) v[NV + 4] += __ldg(se + L::RHS0 + 16 + la);
+  }
+  // lane l ends up with values 4 l' .. 4 l' + 3, l' = l with its bits reversed
+#pragma unroll
+  for (int half = 16, off = 4; off >= 1; half >>= 1, off >>= 1) {
+    const bool up = l8 & off;
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const T send = up ? v[k] : v[k + half], keep = up ? v[k + half] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  if (!on) return;
+  const int g = ((l8 >> 2) & 1) * 4 + (l8 & 2) + (l8 & 1);
+  const unsigned ibA = __ldg(a.ibc + A);
+  if (g < NG) {
+    if (deg > 0) {
+      const T cnt = (T)(rr.w >> 16);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        T val = v[g + u];
-        if (!plain) {
-          const unsigned m = masks[g + u];
-          if ((ibA & m & 0xffu) || ((ibB << 8) & m & 0xff00u)) val = (T)0;
-          if (dg && ((ibA << 16) & m & 0xff0000u)) val = cnt;
-        }
-        v4[u] = val;
+        const unsigned m = masks[4 * g + u];
+        if ((ibA & m & 0xffu) || ((ibA << 8) & m & 0xff00u)) v[u] = (T)0;
+        if ((ibA << 16) & m & 0xff0000u) v[u] = cnt;
       }
-      store4_cs(dst + g, v4);
+      store4_cs(reinterpret_cast<T*>(a.vals) + ((size_t)rr.y + sd) * NV + 4 * g, v);
     }
-  } else {
-    T val = v[0];
-    if ((ibA & TB) || (ibB & TB)) val = (T)0;
-    if (dg && (ibA & TB)) val = cnt;
-    __stcs(dst, val);
-  }
-}
-
-// Gather row pass (tets): one warp per CSR row, every lane summing whole
-// blocks of the row in registers, so that no element block passes through
-// shared memory.  The work of a row is its off-diagonal entries'
-// contribution lists (the elements holding both nodes, ascending) and the
-// diagonal entry's list (all the row's elements, ascending, with the
-// residual rows).  Each list is cut into pieces of at most R consecutive
-// entries, R the fewest rounds for which the pieces fit the 32 lanes (an
-// interior Kuhn-mesh row: 96 entries, lists of 4, 6 and 24, R = 4); a lane
-// adds its piece one entry per round, loading the next entry while the
-// current block is expanded.  The pieces' sums then meet in the warp's
-// shared memory, and each output task (entry, 4-value group) adds its
-// entry's pieces in order and writes the group, consecutive lanes writing
-// consecutive groups.  Every entry is summed in an order fixed by the mesh,
-// the same on every run.  A row with more than 31 off-diagonal entries
-// takes further passes.  TILED: the element summaries come from the CTA's
-// shared-memory stage (tile-local element numbers in n2e_loc / clist_loc),
-// otherwise from global memory (element ids in n2e / clist).
-template <typename T, int KIND> struct GatherGeom {
-  static constexpr int NV = Lay<KIND>::NV, NF = Lay<KIND>::NF;
-  static constexpr int NVP = NV < 4 ? 1 : NV;
-  static constexpr int PSTR = ((NVP + NF) * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T);
-};
-// per warp: the lanes' piece sums and the pass's entry table (slot, first
-// lane, lanes, column mask; the diagonal last)
-template <typename T, int KIND> struct GatherSmem {
-  T part[32][GatherGeom<T, KIND>::PSTR];
-  int slot[33], first[33], nl[33];
-  unsigned ib[33];
-};
-
-__device__ __forceinline__ int warp_excl_scan(int v, int lane) {
-  int x = v;
+  } else if (a.vec) {
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, d);
-    if (lane >= d) x += y;
-  }
-  return x - v;
-}
-
-
-template <typename T, int KIND, bool TILED>
-__device__ __forceinline__ void gather_row(const AsmArgs& a, const int4 rr, const T* base, int str,
-                                           const uint16_t* n2e_loc, const uint16_t* clist_loc,
-                                           GatherSmem<T, KIND>& w, const unsigned* masks, int lane) {
-  using L = Lay<KIND>;
-  using Q = GatherGeom<T, KIND>;
-  constexpr int NV = Q::NV, NF = Q::NF, NVP = Q::NVP;
-  constexpr int NG = NV >= 4 ? NV / 4 : 1, GW = NV >= 4 ? 4 : 1;
-  constexpr unsigned FULL = 0xffffffffu;
-  const int A = rr.x, rp = rr.y, ep = rr.z, deg = rr.w & 0xff, sd = (rr.w >> 8) & 0xff, ne = rr.w >> 16;
-  const unsigned ibA = __ldg(a.ibc + A);
-  const int nod = deg > 0 ? deg - 1 : 0;
-  T* out = reinterpret_cast<T*>(a.vals) + (size_t)rp * NV;
-  const T cnt = (T)ne;
-  for (int o0 = 0; o0 == 0 || o0 < nod;) {
-    const bool wd = o0 == 0;                        // this pass also takes the diagonal and the residual
-    const int nsl = min(nod - o0, wd ? 31 : 32);    // the pass's off-diagonal entries
-    int s = 0, c0 = 0, len = 0;                     // lane j < nsl: entry j
-    unsigned ibB = 0;
-    if (lane < nsl) {
-      const int o = o0 + lane;
-      s = o < sd ? o : o + 1;
-      c0 = __ldg(a.cptr + rp + s);
-      len = __ldg(a.cptr + rp + s + 1) - c0;
-      ibB = __ldg(a.ibc + __ldg(a.colidx + rp + s));
-    }
-    const int nd = wd ? ne : 0;
-    int R = max(1, (__reduce_add_sync(FULL, len) + nd + 31) / 32);
-    while (__reduce_add_sync(FULL, (len + R - 1) / R) + (nd + R - 1) / R > 32) ++R;
-    const int P = (len + R - 1) / R;                // lanes of entry j
-    const int F = warp_excl_scan(P, lane);          // its first lane
-    const int Fd = __reduce_add_sync(FULL, P);      // the diagonal's first lane
-    const int PD = (nd + R - 1) / R;
-    if (lane < nsl) {
-      w.slot[lane] = s; w.first[lane] = F; w.nl[lane] = P; w.ib[lane] = ibB;
-    }
-    if (wd && lane == 0) {
-      w.slot[nsl] = sd; w.first[nsl] = Fd; w.nl[nsl] = PD; w.ib[nsl] = ibA;
-    }
-    // this lane's piece: of entry k (the last with first lane <= lane), or
-    // of the diagonal list
-    int k = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-      const int j = k + step;
-      const int Fj = __shfl_sync(FULL, F, j & 31);
-      if (j < nsl && Fj <= lane) k = j;
-    }
-    const int Fk = __shfl_sync(FULL, F, k), c0k = __shfl_sync(FULL, c0, k), lenk = __shfl_sync(FULL, len, k);
-    const bool dl = lane >= Fd && lane < Fd + PD;  // a diagonal piece
-    int pc0 = 0, plen = 0;
-    if (lane < Fd) {
-      pc0 = c0k + (lane - Fk) * R;
-      plen = min(R, lenk - (lane - Fk) * R);
-    } else if (dl) {
-      pc0 = ep + (lane - Fd) * R;
-      plen = min(R, ne - (lane - Fd) * R);
-    }
-    T acc[NVP], racc[NF];
-#pragma unroll
-    for (int v = 0; v < NVP; ++v) acc[v] = (T)0;
-#pragma unroll
-    for (int f = 0; f < NF; ++f) racc[f] = (T)0;
-    // entry i of the piece: off-diagonal (e << 4) | (la << 2) | b, diagonal
-    // (e << 3) | la (tiled: (tile-local element << 2) | la)
-    auto entry = [&](int i) -> int {
-      if constexpr (TILED) return dl ? (int)__ldg(n2e_loc + pc0 + i) : (int)__ldg(clist_loc + pc0 + i);
-      else return dl ? __ldg(a.n2e + pc0 + i) : __ldg(a.clist + pc0 + i);
-    };
-    // one entry per round, the next round's entry loaded ahead (a second
-    // buffer of summary loads in flight measured slower in FP64, 13.3 vs
-    // 12.7 ms at 128^3: 235 registers and 8 warps per SM against 128 and 16)
-    int ent = plen > 0 ? entry(0) : 0;
-    for (int r = 0; r < R; ++r) {
-      const int cur = ent;
-      if (r + 1 < plen) ent = entry(r + 1);
-      if (r < plen) {
-        int e, la, b;
-        if (!dl) {
-          e = cur >> 4; la = (cur >> 2) & 3; b = cur & 3;
-        } else if constexpr (TILED) {
-          e = cur >> 2; la = cur & 3; b = la;
-        } else {
-          e = cur >> 3; la = cur & 7; b = la;
-        }
-        const T* se = base + (size_t)e * str;
-        T ob[1][NVP];
-        expand_block<T, KIND, 1, TILED>(se, la, b, 0, ob);
-#pragma unroll
-        for (int v = 0; v < NVP; ++v) acc[v] += ob[0][v];
-        if (dl) {
-#pragma unroll
-          for (int f = 0; f < NF; ++f) racc[f] += ld1<T, TILED>(se + L::RHS0 + NF * la + f);
-        }
+    for (int u = 0; u < 4; ++u) {
+      const int f = 4 * (g - NG) + u;
+      if (f < NF) {
+        const T x = (ibA & (1u << f)) ? (T)0 : v[u];   // IBC bits 0-4: u1 u2 u3 p phi
+        if (!isfinite((double)x)) atomicOr(a.flags + 1, 1);
+        __stcs(reinterpret_cast<T*>(a.rhs) + (size_t)f * a.N + A, x);
       }
-    }
-    if (plen > 0) {
-#pragma unroll
-      for (int v = 0; v < NVP; ++v) w.part[lane][v] = acc[v];
-      if (dl) {
-#pragma unroll
-        for (int f = 0; f < NF; ++f) w.part[lane][NVP + f] = racc[f];
-      }
-    }
-    __syncwarp();
-    // output tasks (entry j, group g): the entry's pieces added in order
-    if (deg > 0) {
-      const int nt = (nsl + (wd ? 1 : 0)) * NG;
-      for (int q = lane; q < nt; q += 32) {
-        const int j = q / NG, g = q - j * NG;
-        const int f0 = w.first[j], n = w.nl[j];
-        const unsigned ib = w.ib[j];
-        const bool dg = wd && j == nsl;
-        T v[GW];
-#pragma unroll
-        for (int u = 0; u < GW; ++u) v[u] = (T)0;
-        for (int pp = 0; pp < n; ++pp)
-#pragma unroll
-          for (int u = 0; u < GW; ++u) v[u] += w.part[f0 + pp][GW * g + u];
-        T* dst = out + (size_t)w.slot[j] * NV + GW * g;
-        if constexpr (NV >= 4) {
-          if ((ibA | ib) != 0u) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const unsigned m = masks[4 * g + u];
-              if ((ibA & m & 0xffu) || ((ib << 8) & m & 0xff00u)) v[u] = (T)0;
-              if (dg && ((ibA << 16) & m & 0xff0000u)) v[u] = cnt;
-            }
-          }
-          store4_cs(dst, v);
-        } else {
-          if ((ibA & TB) || (ib & TB)) v[0] = (T)0;
-          if (dg && (ibA & TB)) v[0] = cnt;
-          __stcs(dst, v[0]);
-        }
-      }
-    }
-    if (wd && a.vec && lane < NF) {
-      T v = (T)0;
-      for (int pp = 0; pp < PD; ++pp) v += w.part[Fd + pp][NVP + lane];
-      unsigned bit;
-      if (KIND == OVS_ASM_TEM) bit = TB;
-      else bit = (lane < 3) ? (1u << lane) : (lane == 3 ? PB : FB);
-      if (ibA & bit) v = (T)0;
-      if (!isfinite((double)v)) atomicOr(a.flags + 1, 1);
-      __stcs(reinterpret_cast<T*>(a.rhs) + (size_t)lane * a.N + A, v);
-    }
-    __syncwarp();
-    o0 += nsl;
-  }
-}
-
-// Interleaved form of the gather scheme (the temperature rows, whose
-// blocks are single values: the piece bookkeeping above costs more than it
-// saves there).  Lanes 0..GD-1 take the off-diagonal entries (lane l the
-// l-th, counting past the diagonal slot; a row with more than GD of them
-// takes further passes) and add each entry's whole list, one block per
-// round; lanes GD..31 share the diagonal block and the residual rows, lane
-// GD + i taking the row's elements i, i + ND, ... in ascending order, the ND
-// partial sums then added in lane order.
-template <typename T, int KIND, bool TILED>
-__device__ __forceinline__ void gather_row_il(const AsmArgs& a, const int4 rr, const T* base, int str,
-                                              const uint16_t* n2e_loc, const uint16_t* clist_loc,
-                                              GatherSmem<T, KIND>& w, const unsigned* masks, int lane) {
-  using L = Lay<KIND>;
-  using Q = GatherGeom<T, KIND>;
-  constexpr int NV = Q::NV, NF = Q::NF, NVP = Q::NVP, ND = 8, GD = 32 - ND;
-  T(*pw)[Q::PSTR] = w.part;
-  const bool diagl = lane >= GD;
-  const int di = lane - GD;   // the diagonal lane's index
-  const int A = rr.x, rp = rr.y, ep = rr.z, deg = rr.w & 0xff, sd = (rr.w >> 8) & 0xff, ne = rr.w >> 16;
-  const unsigned ibA = __ldg(a.ibc + A);
-  const int nod = deg > 0 ? deg - 1 : 0;
-  T* out = reinterpret_cast<T*>(a.vals) + (size_t)rp * NV;
-  const T cnt = (T)ne;
-  for (int o0 = 0; o0 == 0 || o0 < nod; o0 += GD) {
-    const int o = o0 + lane;   // off-diagonal ordinal of the lane
-    const bool offl = !diagl && o < nod;
-    const int s = o < sd ? o : o + 1;
-    int c0 = 0, len = 0;
-    unsigned ibB = 0;
-    if (offl) {
-      c0 = __ldg(a.cptr + rp + s);
-      len = __ldg(a.cptr + rp + s + 1) - c0;
-      ibB = __ldg(a.ibc + __ldg(a.colidx + rp + s));
-    } else if (diagl && o0 == 0) {
-      len = ne > di ? (ne - di + ND - 1) / ND : 0;
-    }
-    const int rounds = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
-    T acc[NVP], racc[NF];
-#pragma unroll
-    for (int v = 0; v < NVP; ++v) acc[v] = (T)0;
-#pragma unroll
-    for (int f = 0; f < NF; ++f) racc[f] = (T)0;
-    // entry k of the lane's list: off-diagonal (e << 4) | (la << 2) | b,
-    // diagonal (e << 3) | la (tiled: the tile-local element number)
-    auto entry = [&](int k) -> int {
-      if constexpr (TILED) return offl ? (int)__ldg(clist_loc + c0 + k) : (int)__ldg(n2e_loc + ep + di + k * ND);
-      else return offl ? __ldg(a.clist + c0 + k) : __ldg(a.n2e + ep + di + k * ND);
-    };
-    int ent = len > 0 ? entry(0) : 0;
-    for (int k = 0; k < rounds; ++k) {
-      const int cur = ent;
-      if (k + 1 < len) ent = entry(k + 1);
-      if (k < len) {
-        int e, la, b;
-        if (offl) {
-          e = cur >> 4; la = (cur >> 2) & 3; b = cur & 3;
-        } else if constexpr (TILED) {
-          e = cur >> 2; la = cur & 3; b = la;
-        } else {
-          e = cur >> 3; la = cur & 7; b = la;
-        }
-        const T* se = base + (size_t)e * str;
-        T ob[1][NVP];
-        expand_block<T, KIND, 1, TILED>(se, la, b, 0, ob);
-#pragma unroll
-        for (int v = 0; v < NVP; ++v) acc[v] += ob[0][v];
-        if (diagl) {
-#pragma unroll
-          for (int f = 0; f < NF; ++f) racc[f] += ld1<T, TILED>(se + L::RHS0 + NF * la + f);
-        }
-      }
-    }
-    if (offl) write_block<T, NV>(out + (size_t)s * NV, acc, masks, ibA, ibB, false, cnt);
-    if (o0 == 0) {
-      if (diagl) {
-#pragma unroll
-        for (int v = 0; v < NVP; ++v) pw[di][v] = acc[v];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) pw[di][NVP + f] = racc[f];
-      }
-      __syncwarp();
-      constexpr int NG = NV >= 4 ? NV / 4 : 1;
-      if (deg > 0 && lane < NG) {
-        constexpr int GW = NV >= 4 ? 4 : 1;
-        T v4[GW];
-#pragma unroll
-        for (int u = 0; u < GW; ++u) v4[u] = pw[0][GW * lane + u];
-        for (int i = 1; i < ND; ++i)
-#pragma unroll
-          for (int u = 0; u < GW; ++u) v4[u] += pw[i][GW * lane + u];
-        if constexpr (NV >= 4) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const unsigned m = masks[4 * lane + u];
-            if (ibA & m & 0xffu) v4[u] = (T)0;
-            if ((ibA << 8) & m & 0xff00u) v4[u] = (T)0;
-            if ((ibA << 16) & m & 0xff0000u) v4[u] = cnt;
-          }
-          store4_cs(out + (size_t)sd * NV + 4 * lane, v4);
-        } else {
-          T val = v4[0];
-          if (ibA & TB) val = cnt;
-          __stcs(out + sd, val);
-        }
-      }
-      if (a.vec && lane >= 32 - NF) {
-        const int f = lane - (32 - NF);
-        T v = pw[0][NVP + f];
-        for (int i = 1; i < ND; ++i) v += pw[i][NVP + f];
-        unsigned bit;
-        if (KIND == OVS_ASM_TEM) bit = TB;
-        else bit = (f < 3) ? (1u << f) : (f == 3 ? PB : FB);
-        if (ibA & bit) v = (T)0;
-        if (!isfinite((double)v)) atomicOr(a.flags + 1, 1);
-        __stcs(reinterpret_cast<T*>(a.rhs) + (size_t)f * a.N + A, v);
-      }
-      __syncwarp();
     }
   }
 }
 
 template <typename T, int KIND>
-__global__ void __launch_bounds__(128) gather_rows_kernel(const AsmArgs a) {
+__global__ void __launch_bounds__(128, 4) edge_rows_kernel(const AsmArgs a) {
+  using L = Lay<KIND>;
+  constexpr int NV = L::NV;
   __shared__ unsigned masks[24];
-  __shared__ __align__(16) GatherSmem<T, KIND> gw[4];
-  if (threadIdx.x < 24) masks[threadIdx.x] = (KIND == OVS_ASM_TEM) ? (TB | (TB << 8) | (TB << 16)) : mask_of(threadIdx.x);
+  if (threadIdx.x < 24) masks[threadIdx.x] = mask_of(threadIdx.x);
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, tile = blockIdx.x;
+#pragma unroll 1
+  for (int r = 4 * wid; r < OVS_TILE_ROWS; r += 16) {
+    const int t = tile * OVS_TILE_ROWS + r + (lane >> 3);
+    const bool on = t < a.N;
+    const int4 rr = on ? __ldg(a.row_rec + t) : make_int4(0, 0, 0, 0);
+    diag_row<T, KIND>(a, rr, on, lane & 7, masks);
+  }
   const T* sum = reinterpret_cast<const T*>(a.rec);
-  const int W = gridDim.x * 4;
-  for (int t = blockIdx.x * 4 + wid; t < a.nrows; t += W)
-    if constexpr (KIND == OVS_ASM_TEM)
-      gather_row_il<T, KIND, false>(a, __ldg(a.row_rec + t), sum, Lay<KIND>::SW, nullptr, nullptr, gw[wid], masks,
-                                    lane);
-    else
-      gather_row<T, KIND, false>(a, __ldg(a.row_rec + t), sum, Lay<KIND>::SW, nullptr, nullptr, gw[wid], masks, lane);
+  T* vals = reinterpret_cast<T*>(a.vals);
+  const int p = lane & 1;
+  const unsigned e1 = __ldg(a.tile_edge + tile + 1);
+  unsigned i = __ldg(a.tile_edge + tile) + 16u * wid + (lane >> 1);
+  // the next set's records and first list entry travel while a set runs
+  int4 rec = make_int4(0, 0, 0, 0);
+  unsigned c = 0, c1 = 0, ent = 0;
+  if (i < e1) {
+    rec = __ldg(a.edge_rec + i);
+    c = __ldg(a.edge_ptr + i);
+    c1 = __ldg(a.edge_ptr + i + 1);
+    ent = __ldg(a.edge_list + c);
+  }
+  while (__any_sync(0xffffffffu, i < e1)) {
+    const bool on = i < e1;
+    const int4 cur = rec;
+    const unsigned end = c1;
+    unsigned pos = c, en = ent;
+    i += 64u;
+    c = c1 = 0;
+    if (i < e1) {
+      rec = __ldg(a.edge_rec + i);
+      c = __ldg(a.edge_ptr + i);
+      c1 = __ldg(a.edge_ptr + i + 1);
+    }
+    const unsigned ib = on ? __ldg(a.ibc + (p ? cur.y : cur.x)) : 0u;
+    T acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = (T)0;
+#pragma unroll 1
+    for (; pos < end; ++pos) {
+      const unsigned now = en;
+      if (pos + 1 < end) en = __ldg(a.edge_list + pos + 1);
+      const int la = (now >> 2) & 3, lb = now & 3;
+      BlockIn<T> in;
+      load_block<T, KIND>(sum + (size_t)(now >> 4) * L::SW, p ? lb : la, p ? la : lb, in);
+      add_block<T, KIND>(in, acc);
+    }
+    if (c < c1) ent = __ldg(a.edge_list + c);
+    const unsigned other = __shfl_xor_sync(0xffffffffu, ib, 1);
+    if (on) write_entry<T, KIND>(vals + (size_t)(p ? cur.w : cur.z) * NV, acc, masks, ib, other);
+  }
+}
+
+// the same for the temperature system: its blocks are single values, so one
+// lane takes both entries of an edge
+template <typename T>
+__global__ void __launch_bounds__(128) edge_rows_tem_kernel(const AsmArgs a) {
+  using L = Lay<OVS_ASM_TEM>;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, tile = blockIdx.x, l8 = lane & 7;
+  const T* sum = reinterpret_cast<const T*>(a.rec);
+  T* vals = reinterpret_cast<T*>(a.vals);
+#pragma unroll 1
+  for (int r = 4 * wid; r < OVS_TILE_ROWS; r += 16) {
+    const int t = tile * OVS_TILE_ROWS + r + (lane >> 3);
+    const bool on = t < a.N;
+    const int4 rr = on ? __ldg(a.row_rec + t) : make_int4(0, 0, 0, 0);
+    const int ne = rr.w >> 16;
+    T k = (T)0, f = (T)0;
+#pragma unroll 4
+    for (int q = l8; q < ne; q += 8) {
+      const int pk = __ldg(a.n2e + rr.z + q);
+      T x[2];
+      ldv2(sum + (size_t)(pk >> 3) * L::SW + L::RHS0 + 2 * (pk & 7), x);
+      k += x[0];
+      f += x[1];
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      k += __shfl_xor_sync(0xffffffffu, k, o);
+      f += __shfl_xor_sync(0xffffffffu, f, o);
+    }
+    if (!on || l8) continue;
+    const bool held = __ldg(a.ibc + rr.x) & TB;
+    if (rr.w & 0xff) __stcs(vals + rr.y + ((rr.w >> 8) & 0xff), held ? (T)ne : k);
+    if (a.vec) {
+      const T x = held ? (T)0 : f;
+      if (!isfinite((double)x)) atomicOr(a.flags + 1, 1);
+      __stcs(reinterpret_cast<T*>(a.rhs) + rr.x, x);
+    }
+  }
+  const unsigned e1 = __ldg(a.tile_edge + tile + 1);
+  for (unsigned i = __ldg(a.tile_edge + tile) + threadIdx.x; i < e1; i += blockDim.x) {
+    const int4 cur = __ldg(a.edge_rec + i);
+    const unsigned end = __ldg(a.edge_ptr + i + 1);
+    T kab = (T)0, kba = (T)0;
+#pragma unroll 4
+    for (unsigned q = __ldg(a.edge_ptr + i); q < end; ++q) {
+      const unsigned now = __ldg(a.edge_list + q);
+      const int la = (now >> 2) & 3, lb = now & 3;
+      T x[2];
+      ldv2(sum + (size_t)(now >> 4) * L::SW + 2 * (la < lb ? tet_edge(la, lb) : tet_edge(lb, la)), x);
+      kab += la < lb ? x[0] : x[1];
+      kba += la < lb ? x[1] : x[0];
+    }
+    const bool held = (__ldg(a.ibc + cur.x) | __ldg(a.ibc + cur.y)) & TB;
+    __stcs(vals + cur.z, held ? (T)0 : kab);
+    __stcs(vals + cur.w, held ? (T)0 : kba);
+  }
 }
 
 // Row pass of a vector-only assembly (tets and hexahedra): 8 lanes per node
@@ -1710,82 +1279,6 @@ __global__ void __launch_bounds__(256) residual_rows_kernel(const AsmArgs a, int
   if (__ldg(a.ibc + A) & bit) v = (T)0;
   if (!isfinite((double)v)) atomicOr(a.flags + 1, 1);
   reinterpret_cast<T*>(a.rhs)[(size_t)l8 * a.N + A] = v;
-}
-
-// ---------------------------------------------------------- tiled row pass
-// One CTA per row tile (ovs_tiles_build): the summaries of the tile's
-// elements are copied into shared memory by bulk asynchronous copies
-// (cp.async.bulk, completing on one mbarrier; from this GPU's own memory, no
-// multicast), then the four warps take the tile's rows by the gather scheme
-// above, reading the summaries from shared memory.  Each summary is fetched
-// in whole 16-byte units, once per tile that uses it, instead of lane by
-// lane in scattered 16-byte loads.
-struct TileArgs {
-  const int* rptr;
-  const int* rows;
-  const int* eptr;
-  const int* elems;
-  const uint16_t* n2e_loc;
-  const uint16_t* clist_loc;
-};
-
-// a staged summary's stride in shared memory: an odd number of 16-byte
-// units, so the lanes reading different elements spread over the banks
-template <typename T, int KIND> struct TileStage {
-  static constexpr int SWB = Lay<KIND>::SW * (int)sizeof(T);
-  static constexpr int STRB = 16 * ((SWB / 16) | 1);
-  static constexpr int STR = STRB / (int)sizeof(T);
-  static_assert(SWB % 16 == 0, "summaries must be whole 16-byte units");
-};
-
-constexpr long TILE_WAIT_LIMIT = 1L << 26;   // bounded mbarrier wait (polls)
-
-template <typename T, int KIND>
-__global__ void __launch_bounds__(128) tiled_rows_kernel(const AsmArgs a, const TileArgs ta) {
-  using G = TileStage<T, KIND>;
-  extern __shared__ __align__(128) unsigned char tile_smem[];
-  __shared__ __align__(8) unsigned long long bar;
-  __shared__ unsigned masks[24];
-  __shared__ __align__(16) GatherSmem<T, KIND> gw[4];
-  T* stage = reinterpret_cast<T*>(tile_smem);
-  const int tile = blockIdx.x;
-  const int k0 = __ldg(ta.eptr + tile), nel = __ldg(ta.eptr + tile + 1) - k0;
-  const unsigned barp = (unsigned)__cvta_generic_to_shared(&bar);
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barp));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (threadIdx.x < 24) masks[threadIdx.x] = (KIND == OVS_ASM_TEM) ? (TB | (TB << 8) | (TB << 16)) : mask_of(threadIdx.x);
-  __syncthreads();
-  if (threadIdx.x == 0)
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(barp), "r"((unsigned)(nel * G::SWB))
-                 : "memory");
-  __syncthreads();   // the expected bytes are registered before any copy completes
-  const T* sum = reinterpret_cast<const T*>(a.rec);
-  for (int k = threadIdx.x; k < nel; k += blockDim.x) {
-    const int e = __ldg(ta.elems + k0 + k);
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"((unsigned)__cvta_generic_to_shared(stage + (size_t)k * G::STR)), "l"(sum + (size_t)e * Lay<KIND>::SW),
-                 "r"((unsigned)G::SWB), "r"(barp)
-                 : "memory");
-  }
-  unsigned done = 0;
-  for (long it = 0; it < TILE_WAIT_LIMIT && !done; ++it)
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(done) : "r"(barp) : "memory");
-  if (!done) {   // the copies did not land: report, assemble nothing
-    if (threadIdx.x == 0) atomicOr(a.flags + 2, 1);
-    return;
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int r1 = __ldg(ta.rptr + tile + 1);
-  for (int r = __ldg(ta.rptr + tile) + wid; r < r1; r += 4) {
-    const int4 rr = __ldg(a.row_rec + __ldg(ta.rows + r));
-    if constexpr (KIND == OVS_ASM_TEM)
-      gather_row_il<T, KIND, true>(a, rr, stage, G::STR, ta.n2e_loc, ta.clist_loc, gw[wid], masks, lane);
-    else
-      gather_row<T, KIND, true>(a, rr, stage, G::STR, ta.n2e_loc, ta.clist_loc, gw[wid], masks, lane);
-  }
 }
 
 // ---------------------------------------------------- alpha-stage records
@@ -1838,61 +1331,13 @@ __global__ void alpha_records_kernel(const AlphaArgs a) {
   for (int k = 0; k < REC; ++k) o[k] = r[k];
 }
 
-template <typename T, int KIND, int WARPS, bool STAGED>
-int launch_rows(ovs_ctx* c, const AsmArgs& a) {
-  using S = Smem<T, KIND>;
-  const size_t smem = S::bytes(a.max_deg, STAGED) * WARPS;
-  auto kern = assemble_rows_kernel<T, KIND, WARPS, STAGED>;
-  OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem));
-  if (per_sm < 1) return OVS_ERR_ARG;
-  long need = ((long)c->N + WARPS - 1) / WARPS;
-  long grid = (long)per_sm * c->num_sms * 4;
-  if (grid > need) grid = need;
-  if (grid < 1) grid = 1;
-  kern<<<(int)grid, WARPS * 32, smem, c->stream>>>(a);
+template <typename T, int KIND>
+int launch_edges(ovs_ctx* c, const AsmArgs& a) {
+  const int tiles = (c->N + OVS_TILE_ROWS - 1) / OVS_TILE_ROWS;
+  if constexpr (KIND == OVS_ASM_TEM) edge_rows_tem_kernel<T><<<tiles, 128, 0, c->stream>>>(a);
+  else edge_rows_kernel<T, KIND><<<tiles, 128, 0, c->stream>>>(a);
   ++c->launches;
   OVS_CUDA_TRY(cudaGetLastError());
-  return OVS_OK;
-}
-
-template <typename T, int KIND>
-int launch_gather(ovs_ctx* c, const AsmArgs& a) {
-  auto kern = gather_rows_kernel<T, KIND>;
-  int per_sm = 0;
-  OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, 0));
-  if (per_sm < 1) return OVS_ERR_ARG;
-  long need = ((long)a.nrows + 3) / 4;
-  long grid = (long)per_sm * c->num_sms * 4;
-  if (grid > need) grid = need;
-  if (grid < 1) grid = 1;
-  kern<<<(int)grid, 128, 0, c->stream>>>(a);
-  ++c->launches;
-  OVS_CUDA_TRY(cudaGetLastError());
-  return OVS_OK;
-}
-
-template <typename T, int KIND>
-int launch_tiled(ovs_ctx* c, const AsmArgs& a) {
-  int st;
-  if ((st = ovs_tiles_build(c, c->tile_elems_opt))) return st;
-  using G = TileStage<T, KIND>;
-  const size_t smem = (size_t)c->tile_maxe * G::STRB;
-  auto kern = tiled_rows_kernel<T, KIND>;
-  OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const TileArgs ta{c->tile_rptr, c->tile_rows, c->tile_eptr, c->tile_elems, c->n2e_loc, c->clist_loc};
-  if (c->ntiles > 0) {
-    kern<<<c->ntiles, 128, smem, c->stream>>>(a, ta);
-    ++c->launches;
-    OVS_CUDA_TRY(cudaGetLastError());
-  }
-  if (c->nbig > 0) {   // rows with more elements than a tile holds
-    AsmArgs b = a;
-    b.row_rec = c->big_rec;
-    b.nrows = c->nbig;
-    return launch_gather<T, KIND>(c, b);
-  }
   return OVS_OK;
 }
 
@@ -1943,13 +1388,7 @@ int launch_assemble(ovs_ctx* c, const AsmArgs& a, const SumArgs& sa, int parts =
     OVS_CUDA_TRY(cudaGetLastError());
   }
   if (!(parts & 2)) return OVS_OK;
-  // pass 2: rows
-  // the temperature summaries (20 values, one lane per element) gain
-  // nothing from staging: measured slower, so it reads them directly
-  if (c->rows_tiled && c->cptr) return launch_tiled<T, KIND>(c, a);
-  if (c->rows_gather && c->cptr) return launch_gather<T, KIND>(c, a);
-  if (c->rows_staged && KIND != OVS_ASM_TEM) return launch_rows<T, KIND, 4, true>(c, a);
-  return launch_rows<T, KIND, 4, false>(c, a);
+  return launch_edges<T, KIND>(c, a);   // pass 2
 }
 
 
@@ -2523,13 +1962,14 @@ static void fill_args(ovs_ctx* c, int prec, SysStore& S, int tensor_flag, AsmArg
   a.flags = c->flags;
   a.cfl_bits = c->cfl_bits;
   a.N = c->N;
-  a.nrows = c->N;
   a.mat = (tensor_flag & OVS_TENSOR_MAT) != 0;
   a.vec = (tensor_flag & OVS_TENSOR_VEC) != 0;
   a.n2s = c->n2s;
   a.row_rec = c->row_rec;
-  a.cptr = c->cptr;
-  a.clist = c->clist;
+  a.edge_rec = c->edge_rec;
+  a.edge_ptr = c->edge_ptr;
+  a.edge_list = c->edge_list;
+  a.tile_edge = c->tile_edge;
   a.max_deg = c->max_deg;
   a.p = c->params;
   a.kbuf = nullptr;

@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(64) hex_element_kernel(const SumArgs a) {
 }
 
 // Block (row node la, column node b) of a hex from its records: the
-// per-point forms of the tet block sums (see expand_block), summed over the
+// per-point forms of the tet block sums (see add_block), summed over the
 // 8 points.
 template <typename T, int KIND>
 __device__ __forceinline__ void hex_expand_block(const ovs_params& p, const T* sm, int la, int b, T* o, T* rv) {

@@ -9,6 +9,7 @@
 
 #define OVS_MAX_DEG 128        // longest CSR row supported (27*nshl hex bound = 216 not needed)
 #define OVS_MAX_KSPACE 400     // largest Krylov space
+#define OVS_TILE_ROWS 32       // rows per tile of the tet edge pass (a multiple of 16)
 #define OVS_ASYNC_SLOTS 16     // assembly passes ovs_assemble_async queues before a wait
 #define OVS_RED_BLOCKS 592     // fixed grid of every deterministic reduction (4 x 148 SMs)
 #define OVS_RED_THREADS 256
@@ -98,20 +99,11 @@ struct ovs_ctx {
   double* vjp_grad = nullptr;
   int* row_order = nullptr;  // N: rows in Morton order of the node coordinates (the row pass's order)
   int4* row_rec = nullptr;   // N: per row in that order {A, rowptr[A], n2e_ptr[A], deg | sd << 8 | ne << 16}
-  int* cptr = nullptr;       // nnz + 1: off-diagonal contribution lists (tets), offsets into clist
-  int* clist = nullptr;      // 12 E entries (e << 4) | (la << 2) | b, ascending element per entry
-  // row tiles of the tiled row pass (tets; built at the first assembly that
-  // takes that pass, ovs_tiles_build): runs of consecutive rows of row_rec
-  // whose elements, at most tile_maxe of them, are staged in one CTA's
-  // shared memory
-  int ntiles = 0, nbig = 0, tile_maxe = 0;
-  int* tile_rptr = nullptr;  // ntiles + 1: offsets into tile_rows
-  int* tile_rows = nullptr;  // row positions t (into row_rec) of each tile
-  int* tile_eptr = nullptr;  // ntiles + 1: offsets into tile_elems
-  int* tile_elems = nullptr; // the tile's elements, in first-use order
-  uint16_t* n2e_loc = nullptr;   // per n2e entry: (tile-local element << 2) | la
-  uint16_t* clist_loc = nullptr; // per clist entry: (tile-local element << 4) | (la << 2) | b
-  int4* big_rec = nullptr;   // nbig row records of rows with more than tile_maxe elements
+  // edges of the tet edge pass (pattern.cu: build_edges)
+  int4* edge_rec = nullptr;      // per edge {A, B, slot of (A, B), slot of (B, A)}, tile by tile of rows
+  unsigned* edge_ptr = nullptr;  // edges + 1: offsets into edge_list
+  unsigned* edge_list = nullptr; // 6 E entries (e << 4) | (la << 2) | lb, ascending element per edge
+  unsigned* tile_edge = nullptr; // first edge of every tile of OVS_TILE_ROWS rows, and the end
   unsigned* n2s = nullptr;   // nshl*E entries: slots of the element's nodes in the row, one byte each
                              // (one word per entry for tets, two for hexahedra)
   int nnz = 0;
@@ -134,9 +126,6 @@ struct ovs_ctx {
   cudaEvent_t ev_rhs_out[4] = {};         // the last read-back of rhs_out[sys] done
   // hex tensor-core pass (FP32 NS+VOF): off unless OVS_HEX_TC=1 or OVS_OPT_HEX_TC
   int hex_tc = 0;
-  // tet row pass: element summaries staged through shared memory by
-  // asynchronous copies (1, default) or read by every lane from global memory
-  int rows_staged = 1;
   // FP64 element pass: node records in registers (0) or shared memory (1);
   // -1 (default): shared memory for NS+VOF, registers for the others, the
   // faster of the two measured for each
@@ -146,14 +135,6 @@ struct ovs_ctx {
   int mixed_outer = 30;
   void* fg_buf = nullptr;    // the flexible outer's basis and directions
   size_t fg_bytes = 0;
-  // tet row pass: lanes gather whole blocks by the contribution lists (1,
-  // default) or the chunked pass reduces element blocks in shared memory (0)
-  int rows_gather = 1;
-  // tet row pass: rows in CTA tiles with their element summaries staged in
-  // shared memory by bulk copies (1; default 0, measured slower than the
-  // gather pass), the element budget per tile
-  int rows_tiled = 0;
-  int tile_elems_opt = 96;
   void* hex_kbuf = nullptr;              // E x 64 x 24 block values
   float* hex_w = nullptr;                // W hi + lo, canonical layout
   // boundary-condition producers (ovs_set_bc_spec)
@@ -201,7 +182,6 @@ struct ovs_ctx {
 
 // ------------------------------------------------------------ helpers
 int ovs_ensure(void** p, size_t bytes);
-int ovs_tiles_build(ovs_ctx* c, int maxe);
 int ovs_activate(ovs_ctx* c);
 
 // pattern.cu

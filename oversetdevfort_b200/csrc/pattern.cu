@@ -406,165 +406,139 @@ static int build_row_rec(ovs_ctx* c) {
   return OVS_OK;
 }
 
-// Contribution lists of the off-diagonal entries (tets), the gather row
-// pass's input: for entry (A, B), B != A, the elements holding both nodes in
-// ascending element order, each as (e << 4) | (la << 2) | b with
-// A = ien[e][la], B = ien[e][b]; cptr[k]..cptr[k+1] delimits entry k's list
-// (diagonal entries have none: every element of the row adds to them).
-// One thread per row, the row's entries counted / filled in n2e order.
-__global__ void contrib_count_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ n2e_ptr,
-                                     const int* __restrict__ n2e, const unsigned* __restrict__ n2s,
-                                     int* __restrict__ cnt) {
-  const int A = blockIdx.x * blockDim.x + threadIdx.x;
-  if (A >= N) return;
-  const int rp = rowptr[A];
-  for (int k = n2e_ptr[A]; k < n2e_ptr[A + 1]; ++k) {
-    const int la = n2e[k] & 7;
-    const unsigned w = n2s[k];
-    for (int b = 0; b < 4; ++b)
-      if (b != la) ++cnt[rp + ((w >> (8 * b)) & 0xffu)];
+// Edges of the tet edge pass.  An edge is a pair of off-diagonal entries
+// (A, B), (B, A); it belongs to the row that comes first in the processing
+// order, and rows come in tiles of OVS_TILE_ROWS.  Within a tile the edges
+// are sorted by the length of their element list, longest first (stable), so
+// that the edges a warp takes together have lists of nearly equal length.
+__global__ void order_pos_kernel(const int4* __restrict__ rec, int N, int* __restrict__ pos) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < N) pos[rec[t].x] = t;
+}
+
+__global__ void edge_count_kernel(const int4* __restrict__ rec, const int* __restrict__ colidx,
+                                  const int* __restrict__ pos, int N, int* __restrict__ cnt) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= N) return;
+  const int4 r = rec[t];
+  int n = 0;
+  for (int s = 0; s < (r.w & 0xff); ++s) n += pos[colidx[r.y + s]] > t;
+  cnt[t] = n;
+}
+
+__global__ void edge_fill_kernel(const int4* __restrict__ rec, const int* __restrict__ rowptr,
+                                 const int* __restrict__ colidx, const int* __restrict__ pos,
+                                 const int* __restrict__ n2e, const unsigned* __restrict__ n2s, int N,
+                                 const int* __restrict__ off, int4* __restrict__ edge, int* __restrict__ len) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= N) return;
+  const int4 r = rec[t];
+  const int ne = r.w >> 16;
+  int i = off[t];
+  for (int s = 0; s < (r.w & 0xff); ++s) {
+    const int B = colidx[r.y + s];
+    if (pos[B] <= t) continue;
+    int lo = rowptr[B], hi = rowptr[B + 1];   // the pattern is symmetric: row B holds column A
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (colidx[mid] > r.x) hi = mid; else lo = mid;
+    }
+    int n = 0;
+    for (int k = 0; k < ne; ++k) {
+      const unsigned w = n2s[r.z + k];
+      n += __vcmpeq4(w, (unsigned)s * 0x01010101u) != 0u;
+    }
+    edge[i] = make_int4(r.x, B, r.y + s, lo);
+    len[i++] = n;
   }
 }
 
-__global__ void contrib_fill_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ n2e_ptr,
-                                    const int* __restrict__ n2e, const unsigned* __restrict__ n2s,
-                                    int* __restrict__ cursor, int* __restrict__ list) {
-  const int A = blockIdx.x * blockDim.x + threadIdx.x;
-  if (A >= N) return;
-  const int rp = rowptr[A];
-  for (int k = n2e_ptr[A]; k < n2e_ptr[A + 1]; ++k) {
-    const int e = n2e[k] >> 3, la = n2e[k] & 7;
-    const unsigned w = n2s[k];
-    for (int b = 0; b < 4; ++b)
-      if (b != la) list[cursor[rp + ((w >> (8 * b)) & 0xffu)]++] = (e << 4) | (la << 2) | b;
+// one block per tile: every edge's rank among the tile's, by descending length
+__global__ void edge_sort_kernel(const int* __restrict__ off, int N, const int4* __restrict__ in,
+                                 const int* __restrict__ len, int4* __restrict__ out, int* __restrict__ slen,
+                                 unsigned* __restrict__ tile_edge) {
+  const int t0 = blockIdx.x * OVS_TILE_ROWS, t1 = min(t0 + OVS_TILE_ROWS, N);
+  const int e0 = off[t0], e1 = off[t1];
+  for (int i = e0 + threadIdx.x; i < e1; i += blockDim.x) {
+    const int n = len[i];
+    int rank = 0;
+    for (int j = e0; j < e1; ++j) rank += len[j] > n || (len[j] == n && j < i);
+    out[e0 + rank] = in[i];
+    slen[e0 + rank] = n;
+  }
+  if (threadIdx.x == 0) {
+    tile_edge[blockIdx.x] = (unsigned)e0;
+    if (t1 == N) tile_edge[blockIdx.x + 1] = (unsigned)e1;
   }
 }
 
-static int build_contrib(ovs_ctx* c) {
+// the elements of every edge, ascending: (e << 4) | (la << 2) | lb with
+// A = ien[e][la], B = ien[e][lb]
+__global__ void edge_list_kernel(int nedge, const int4* __restrict__ edge, const unsigned* __restrict__ ptr,
+                                 const int* __restrict__ rowptr, const int* __restrict__ n2e_ptr,
+                                 const int* __restrict__ n2e, const unsigned* __restrict__ n2s,
+                                 unsigned* __restrict__ list) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nedge) return;
+  const int4 r = edge[i];
+  const unsigned key = (unsigned)(r.z - rowptr[r.x]) * 0x01010101u;
+  unsigned q = ptr[i];
+  for (int k = n2e_ptr[r.x]; k < n2e_ptr[r.x + 1]; ++k) {
+    const unsigned m = __vcmpeq4(n2s[k], key);
+    if (m) list[q++] = ((unsigned)(n2e[k] >> 3) << 4) | ((n2e[k] & 3) << 2) | ((__ffs(m) - 1) >> 3);
+  }
+}
+
+static int build_edges(ovs_ctx* c) {
   cudaStream_t s = c->stream;
-  const int N = c->N, nnz = c->nnz;
-  if (c->nshl != 4 || N < 1 || nnz < 1) return OVS_OK;
-  if (c->E >= (1 << 27)) return OVS_OK;   // (e << 4) must fit an int: the chunked row pass serves
-  const size_t ents = (size_t)12 * c->E;  // 3 off-diagonal blocks per element row
-  int st;
-  if ((st = ovs_ensure((void**)&c->cptr, sizeof(int) * ((size_t)nnz + 1)))) return st;
-  if ((st = ovs_ensure((void**)&c->clist, sizeof(int) * (ents > 0 ? ents : 1)))) return st;
-  int *cnt = nullptr, *tmp = nullptr;
-  const int nb = (nnz + 1 + SCAN_T - 1) / SCAN_T;
-  OVS_CUDA_TRY(cudaMallocAsync(&cnt, sizeof(int) * ((size_t)nnz + 1), s));
-  OVS_CUDA_TRY(cudaMallocAsync(&tmp, sizeof(int) * (4 * (size_t)nb + 64), s));
-  OVS_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)nnz + 1), s));
-  contrib_count_kernel<<<ovs_grid(N, 128, 1 << 30), 128, 0, s>>>(N, c->rowptr, c->n2e_ptr, c->n2e, c->n2s, cnt);
-  ++c->launches;
-  if ((st = exclusive_scan(cnt, c->cptr, nnz + 1, tmp, s, &c->launches))) return st;
-  OVS_CUDA_TRY(cudaMemcpyAsync(cnt, c->cptr, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToDevice, s));
-  contrib_fill_kernel<<<ovs_grid(N, 128, 1 << 30), 128, 0, s>>>(N, c->rowptr, c->n2e_ptr, c->n2e, c->n2s, cnt,
-                                                                c->clist);
-  ++c->launches;
-  OVS_CUDA_TRY(cudaFreeAsync(cnt, s));
+  const int N = c->N;
+  if (c->nshl != 4 || N < 1) return OVS_OK;
+  const int tiles = (N + OVS_TILE_ROWS - 1) / OVS_TILE_ROWS;
+  int *pos = nullptr, *cnt = nullptr, *off = nullptr, *tmp = nullptr, *len = nullptr, *slen = nullptr;
+  int4* raw = nullptr;
+  const size_t nb = ((size_t)N + 1 + SCAN_T - 1) / SCAN_T;
+  OVS_CUDA_TRY(cudaMallocAsync(&pos, sizeof(int) * (size_t)N, s));
+  OVS_CUDA_TRY(cudaMallocAsync(&cnt, sizeof(int) * ((size_t)N + 1), s));
+  OVS_CUDA_TRY(cudaMallocAsync(&off, sizeof(int) * ((size_t)N + 1), s));
+  OVS_CUDA_TRY(cudaMallocAsync(&tmp, sizeof(int) * (4 * nb + 64), s));
+  order_pos_kernel<<<ovs_grid(N, 256, 1 << 30), 256, 0, s>>>(c->row_rec, N, pos);
+  edge_count_kernel<<<ovs_grid(N, 128, 1 << 30), 128, 0, s>>>(c->row_rec, c->colidx, pos, N, cnt);
+  c->launches += 2;
+  OVS_CUDA_TRY(cudaMemsetAsync(cnt + N, 0, sizeof(int), s));
+  int st, ne = 0;
+  if ((st = exclusive_scan(cnt, off, N + 1, tmp, s, &c->launches))) return st;
+  OVS_CUDA_TRY(cudaMemcpyAsync(&ne, off + N, sizeof(int), cudaMemcpyDeviceToHost, s));
   OVS_CUDA_TRY(cudaFreeAsync(tmp, s));
-  OVS_CUDA_TRY(cudaGetLastError());
-  return OVS_OK;
-}
-
-// Row tiles of the tiled row pass, built on the host from the row records,
-// the node-to-element lists and the contribution lists: consecutive rows of
-// the row order (Morton order of the nodes, so a tile is a compact cluster
-// of nodes) are added to a tile while its distinct elements stay within
-// maxe and its rows within 16.  For every row entry the element is
-// renumbered to its place in the tile's element list (n2e_loc, clist_loc).
-// A row with more than maxe elements takes no tile (big_rec lists them for
-// the gather pass).
-int ovs_tiles_build(ovs_ctx* c, int maxe) {
-  constexpr int RMAX = 16;
-  cudaStream_t s = c->stream;
-  const int N = c->N, E = c->E;
-  if (c->nshl != 4 || !c->cptr || !c->row_rec || N < 1) return OVS_ERR_STATE;
-  if (maxe < 4 || maxe > 4000) return OVS_ERR_ARG;
-  if (c->tile_maxe == maxe && c->tile_rptr) return OVS_OK;
-  void** olds[] = {(void**)&c->tile_rptr, (void**)&c->tile_rows, (void**)&c->tile_eptr, (void**)&c->tile_elems,
-                   (void**)&c->n2e_loc, (void**)&c->clist_loc, (void**)&c->big_rec};
+  OVS_CUDA_TRY(cudaStreamSynchronize(s));
+  // sized for this pattern: a rebuilt one may have more edges
+  void** olds[] = {(void**)&c->edge_rec, (void**)&c->edge_ptr, (void**)&c->edge_list, (void**)&c->tile_edge};
   for (void** q : olds) {
     if (*q) cudaFree(*q);
     *q = nullptr;
   }
-  c->ntiles = c->nbig = c->tile_maxe = 0;
-  const size_t EN = (size_t)E * 4, NC = (size_t)12 * E, nnz = (size_t)c->nnz;
-  std::vector<int4> rec(N);
-  std::vector<int> n2e(EN), cptr(nnz + 1), clist(NC > 0 ? NC : 1);
-  OVS_CUDA_TRY(cudaMemcpyAsync(rec.data(), c->row_rec, sizeof(int4) * N, cudaMemcpyDeviceToHost, s));
-  OVS_CUDA_TRY(cudaMemcpyAsync(n2e.data(), c->n2e, sizeof(int) * EN, cudaMemcpyDeviceToHost, s));
-  OVS_CUDA_TRY(cudaMemcpyAsync(cptr.data(), c->cptr, sizeof(int) * (nnz + 1), cudaMemcpyDeviceToHost, s));
-  if (NC) OVS_CUDA_TRY(cudaMemcpyAsync(clist.data(), c->clist, sizeof(int) * NC, cudaMemcpyDeviceToHost, s));
-  OVS_CUDA_TRY(cudaStreamSynchronize(s));
-  std::vector<int> stamp(E, -1), loc(E, 0), trptr{0}, trows, teptr{0}, telems;
-  std::vector<uint16_t> n2e_loc(EN, 0), clist_loc(NC > 0 ? NC : 1, 0);
-  std::vector<int4> big;
-  trows.reserve(N);
-  telems.reserve((size_t)N * 20);
-  int tile = 0, cnt = 0, rows = 0;
-  for (int t = 0; t < N; ++t) {
-    const int4 r = rec[t];
-    const int rp = r.y, ep = r.z, deg = r.w & 0xff, sd = (r.w >> 8) & 0xff, ne = r.w >> 16;
-    if (ne > maxe) {
-      big.push_back(r);
-      continue;
-    }
-    int nnew = 0;
-    for (int j = 0; j < ne; ++j) nnew += stamp[n2e[ep + j] >> 3] != tile;
-    if (rows > 0 && (cnt + nnew > maxe || rows >= RMAX)) {   // close the tile
-      trptr.push_back((int)trows.size());
-      teptr.push_back((int)telems.size());
-      ++tile;
-      cnt = rows = 0;
-    }
-    for (int j = 0; j < ne; ++j) {
-      const int e = n2e[ep + j] >> 3, la = n2e[ep + j] & 7;
-      if (stamp[e] != tile) {
-        stamp[e] = tile;
-        loc[e] = cnt++;
-        telems.push_back(e);
-      }
-      n2e_loc[ep + j] = (uint16_t)((loc[e] << 2) | la);
-    }
-    for (int q = 0; q < deg; ++q) {
-      if (q == sd) continue;
-      for (int k = cptr[rp + q]; k < cptr[rp + q + 1]; ++k)
-        clist_loc[k] = (uint16_t)((loc[clist[k] >> 4] << 4) | (clist[k] & 15));
-    }
-    trows.push_back(t);
-    ++rows;
+  if ((st = ovs_ensure((void**)&c->edge_rec, sizeof(int4) * (size_t)ne))) return st;
+  if ((st = ovs_ensure((void**)&c->edge_ptr, sizeof(unsigned) * ((size_t)ne + 1)))) return st;
+  if ((st = ovs_ensure((void**)&c->edge_list, sizeof(unsigned) * 6 * (size_t)c->E))) return st;
+  if ((st = ovs_ensure((void**)&c->tile_edge, sizeof(unsigned) * ((size_t)tiles + 1)))) return st;
+  const size_t eb = ((size_t)ne + 1 + SCAN_T - 1) / SCAN_T;
+  OVS_CUDA_TRY(cudaMallocAsync(&raw, sizeof(int4) * (size_t)(ne + 1), s));
+  OVS_CUDA_TRY(cudaMallocAsync(&len, sizeof(int) * ((size_t)ne + 1), s));
+  OVS_CUDA_TRY(cudaMallocAsync(&slen, sizeof(int) * ((size_t)ne + 1), s));
+  OVS_CUDA_TRY(cudaMallocAsync(&tmp, sizeof(int) * (4 * eb + 64), s));
+  edge_fill_kernel<<<ovs_grid(N, 128, 1 << 30), 128, 0, s>>>(c->row_rec, c->rowptr, c->colidx, pos, c->n2e, c->n2s, N,
+                                                            off, raw, len);
+  edge_sort_kernel<<<tiles, 256, 0, s>>>(off, N, raw, len, c->edge_rec, slen, c->tile_edge);
+  c->launches += 2;
+  OVS_CUDA_TRY(cudaMemsetAsync(slen + ne, 0, sizeof(int), s));
+  if ((st = exclusive_scan(slen, reinterpret_cast<int*>(c->edge_ptr), ne + 1, tmp, s, &c->launches))) return st;
+  if (ne > 0) {
+    edge_list_kernel<<<ovs_grid(ne, 256, 1 << 30), 256, 0, s>>>(ne, c->edge_rec, c->edge_ptr, c->rowptr, c->n2e_ptr,
+                                                               c->n2e, c->n2s, c->edge_list);
+    ++c->launches;
   }
-  if (rows > 0) {
-    trptr.push_back((int)trows.size());
-    teptr.push_back((int)telems.size());
-    ++tile;
-  }
-  int st;
-  const int nt = tile;
-  if ((st = ovs_ensure((void**)&c->tile_rptr, sizeof(int) * (nt + 1)))) return st;
-  if ((st = ovs_ensure((void**)&c->tile_rows, sizeof(int) * (trows.size() + 1)))) return st;
-  if ((st = ovs_ensure((void**)&c->tile_eptr, sizeof(int) * (nt + 1)))) return st;
-  if ((st = ovs_ensure((void**)&c->tile_elems, sizeof(int) * (telems.size() + 1)))) return st;
-  if ((st = ovs_ensure((void**)&c->n2e_loc, sizeof(uint16_t) * EN))) return st;
-  if ((st = ovs_ensure((void**)&c->clist_loc, sizeof(uint16_t) * clist_loc.size()))) return st;
-  if ((st = ovs_ensure((void**)&c->big_rec, sizeof(int4) * (big.size() + 1)))) return st;
-  OVS_CUDA_TRY(cudaMemcpyAsync(c->tile_rptr, trptr.data(), sizeof(int) * (nt + 1), cudaMemcpyHostToDevice, s));
-  if (!trows.empty())
-    OVS_CUDA_TRY(cudaMemcpyAsync(c->tile_rows, trows.data(), sizeof(int) * trows.size(), cudaMemcpyHostToDevice, s));
-  OVS_CUDA_TRY(cudaMemcpyAsync(c->tile_eptr, teptr.data(), sizeof(int) * (nt + 1), cudaMemcpyHostToDevice, s));
-  if (!telems.empty())
-    OVS_CUDA_TRY(
-        cudaMemcpyAsync(c->tile_elems, telems.data(), sizeof(int) * telems.size(), cudaMemcpyHostToDevice, s));
-  OVS_CUDA_TRY(cudaMemcpyAsync(c->n2e_loc, n2e_loc.data(), sizeof(uint16_t) * EN, cudaMemcpyHostToDevice, s));
-  OVS_CUDA_TRY(cudaMemcpyAsync(c->clist_loc, clist_loc.data(), sizeof(uint16_t) * clist_loc.size(),
-                               cudaMemcpyHostToDevice, s));
-  if (!big.empty())
-    OVS_CUDA_TRY(cudaMemcpyAsync(c->big_rec, big.data(), sizeof(int4) * big.size(), cudaMemcpyHostToDevice, s));
-  OVS_CUDA_TRY(cudaStreamSynchronize(s));
-  c->ntiles = nt;
-  c->nbig = (int)big.size();
-  c->tile_maxe = maxe;
+  for (void* q : {(void*)pos, (void*)cnt, (void*)off, (void*)tmp, (void*)raw, (void*)len, (void*)slen})
+    OVS_CUDA_TRY(cudaFreeAsync(q, s));
+  OVS_CUDA_TRY(cudaGetLastError());
   return OVS_OK;
 }
 
@@ -629,7 +603,7 @@ int ovs_pattern_build(ovs_ctx* c) {
   OVS_CUDA_TRY(cudaFreeAsync(stats, s));
   if ((st = build_row_order(c))) return st;
   if ((st = build_row_rec(c))) return st;
-  if ((st = build_contrib(c))) return st;
+  if ((st = build_edges(c))) return st;
   OVS_CUDA_TRY(cudaStreamSynchronize(s));
   OVS_CUDA_TRY(cudaGetLastError());
   c->have_pattern = true;
