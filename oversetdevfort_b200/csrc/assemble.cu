@@ -41,12 +41,12 @@ struct AsmArgs {
   const int* rowptr;
   const int* colidx;
   const int* n2e_ptr;
-  const int* n2e;
+  const int* n2e;         // node's elements as places of their summaries, by ascending id: (t << 3) | local node
   const unsigned* n2s;    // slots of each entry's element nodes in the row
   const int4* row_rec;    // per row in processing order: {A, rowptr[A], n2e_ptr[A], deg | sd << 8 | ne << 16}
   const int4* edge_rec;   // edges (tets): {A, B, slot of (A, B), slot of (B, A)}, tile by tile of rows
   const unsigned* edge_ptr;   //   offsets into edge_list, one per edge and the end
-  const unsigned* edge_list;  //   (e << 4) | (local node of A << 2) | local node of B
+  const unsigned* edge_list;  //   (t << 4) | (local node of A << 2) | local node of B
   const unsigned* tile_edge;  // first edge of every tile of OVS_TILE_ROWS rows, and the end
   void* vals;             // nnz*NV
   void* rhs;              // NF*N field-major
@@ -401,7 +401,7 @@ __device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
 
 struct SumArgs {
   const void* rec;
-  const int* ien;
+  const int* ien;      // in storage order, as elm_id and the summaries
   const int* elm_id;
   void* sum;
   int* flags;
@@ -952,14 +952,14 @@ __global__ void __launch_bounds__(128, (MAT ? SumBlocks<T, KIND, SMEMREC>::v : S
 element_summary_kernel(const SumArgs a) {
   using L = Lay<KIND>;
   constexpr int SW = MAT ? L::SW : 4 * L::NF;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   double tamax = 0.0;   // the element's largest taua over its points (CflPerPoint: largest CFL number)
   int nbad = 0;
-  if (e < a.E) {
-    const int4 nd = __ldg(reinterpret_cast<const int4*>(a.ien) + e);
+  if (t < a.E) {
+    const int4 nd = __ldg(reinterpret_cast<const int4*>(a.ien) + t);
     const int nodes[4] = {nd.x, nd.y, nd.z, nd.w};
     const T* rec = reinterpret_cast<const T*>(a.rec);
-    const int eid = __ldg(a.elm_id + e);
+    const int eid = __ldg(a.elm_id + t);
     T detj;
     auto run = [&](const auto& r, const auto& lo, T* o) {
       if constexpr (KIND == OVS_ASM_NS) {
@@ -987,7 +987,7 @@ element_summary_kernel(const SumArgs a) {
           col[(size_t)(n * 16 + 2 * k + 1) * 128] = v.y;
         }
       }
-      run(SmemRecs<T>{col}, ZeroRecs<T>{}, reinterpret_cast<T*>(a.sum) + (size_t)e * SW);
+      run(SmemRecs<T>{col}, ZeroRecs<T>{}, reinterpret_cast<T*>(a.sum) + (size_t)t * SW);
     } else {
       T r[4][16], lo[4][4];
 #pragma unroll
@@ -997,7 +997,7 @@ element_summary_kernel(const SumArgs a) {
         run(r, lo, o);
         // 20 values per tet (vector-only: 4): groups of 4 (256-bit stores in FP64, the
         // summary 32-byte aligned; 2.45 against 2.52 ms at 128^3)
-        T* dst = reinterpret_cast<T*>(a.sum) + (size_t)e * SW;
+        T* dst = reinterpret_cast<T*>(a.sum) + (size_t)t * SW;
         if constexpr (sizeof(T) == 8) {
 #pragma unroll
           for (int k = 0; k < SW; k += 4) put4(dst + k, o[k], o[k + 1], o[k + 2], o[k + 3]);
@@ -1007,7 +1007,7 @@ element_summary_kernel(const SumArgs a) {
       } else {
         // NS / NS+VOF write their summary with vector stores as its parts
         // are formed
-        run(r, lo, reinterpret_cast<T*>(a.sum) + (size_t)e * SW);
+        run(r, lo, reinterpret_cast<T*>(a.sum) + (size_t)t * SW);
       }
     }
     if (!(detj > (T)0)) nbad = 1;
@@ -1942,8 +1942,8 @@ static int dispatch_assemble(ovs_ctx* c, int kernel, int prec, const AsmArgs& a,
 
 static void fill_args(ovs_ctx* c, int prec, SysStore& S, int tensor_flag, AsmArgs& a, SumArgs& sa) {
   sa.rec = c->rec[prec];
-  sa.ien = c->ien;
-  sa.elm_id = c->elm_id;
+  sa.ien = c->ien_t;
+  sa.elm_id = c->elm_t;
   sa.sum = c->esum[prec];
   sa.flags = c->flags;
   sa.cfl_bits = c->cfl_bits;
@@ -1956,7 +1956,7 @@ static void fill_args(ovs_ctx* c, int prec, SysStore& S, int tensor_flag, AsmArg
   a.rowptr = c->rowptr;
   a.colidx = c->colidx;
   a.n2e_ptr = c->n2e_ptr;
-  a.n2e = c->n2e;
+  a.n2e = c->n2e_t;
   a.vals = S.vals;
   a.rhs = S.rhs;
   a.flags = c->flags;

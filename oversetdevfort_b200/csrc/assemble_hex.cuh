@@ -400,16 +400,16 @@ template <typename T, int KIND, bool TC = false, bool MAT = true>
 __global__ void __launch_bounds__(64) hex_element_kernel(const SumArgs a) {
   using L = HexLay<KIND>;
   constexpr int SW = !MAT ? 8 * L::NF : TC ? HexTcLay::SW : L::SW;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   double tamax = 0.0;   // the element's largest taua over its points
   int nbad = 0;
-  if (e < a.E) {
+  if (t < a.E) {
     T r[8][16], lo[8][4];
     const T* rec = reinterpret_cast<const T*>(a.rec);
 #pragma unroll
-    for (int n = 0; n < 8; ++n) load_rec(rec, a.ien[8 * (size_t)e + n], r[n], lo[n]);
-    const bool fluid = __ldg(a.elm_id + e) == a.p.fluid_elm_id;
-    T* out = reinterpret_cast<T*>(a.sum) + (size_t)e * SW;
+    for (int n = 0; n < 8; ++n) load_rec(rec, a.ien[8 * (size_t)t + n], r[n], lo[n]);
+    const bool fluid = __ldg(a.elm_id + t) == a.p.fluid_elm_id;
+    T* out = reinterpret_cast<T*>(a.sum) + (size_t)t * SW;
     if constexpr (KIND == OVS_ASM_NSVOF) hex_summarize_nsvof<T, TC, MAT>(a.p, r, lo, fluid, out, tamax, nbad);
     else hex_summarize_tem<T, MAT>(a.p, r, lo, fluid, out, tamax, nbad);
   }

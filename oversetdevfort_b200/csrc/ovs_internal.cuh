@@ -99,10 +99,14 @@ struct ovs_ctx {
   double* vjp_grad = nullptr;
   int* row_order = nullptr;  // N: rows in Morton order of the node coordinates (the row pass's order)
   int4* row_rec = nullptr;   // N: per row in that order {A, rowptr[A], n2e_ptr[A], deg | sd << 8 | ne << 16}
+  int* row_pos = nullptr;    // N: the place of a node's row in that order
+  int* ien_t = nullptr;      // ien and elm_id in the storage order of the element summaries
+  int* elm_t = nullptr;      //   (pattern.cu: build_elem_order)
+  int* n2e_t = nullptr;      // n2e with the place t of the element for its id
   // edges of the tet edge pass (pattern.cu: build_edges)
   int4* edge_rec = nullptr;      // per edge {A, B, slot of (A, B), slot of (B, A)}, tile by tile of rows
   unsigned* edge_ptr = nullptr;  // edges + 1: offsets into edge_list
-  unsigned* edge_list = nullptr; // 6 E entries (e << 4) | (la << 2) | lb, ascending element per edge
+  unsigned* edge_list = nullptr; // 6 E entries (t << 4) | (la << 2) | lb, ascending element id per edge
   unsigned* tile_edge = nullptr; // first edge of every tile of OVS_TILE_ROWS rows, and the end
   unsigned* n2s = nullptr;   // nshl*E entries: slots of the element's nodes in the row, one byte each
                              // (one word per entry for tets, two for hexahedra)
