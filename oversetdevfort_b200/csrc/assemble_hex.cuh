@@ -26,10 +26,12 @@ __device__ __forceinline__ T hex_N(int g, int a) {
 }
 
 template <int KIND> struct HexLay;
-//   NS+VOF record per point: g(8x3) w KA KB MM KDP dphi(3) uadv(3) rho rt
-//   tauLS src eps ufac plfac pad(2); then the residual rows 8x5
+//   NS+VOF record per point, with c_n = uadv . grad N_n: (grad N_n, c_n) of the
+//   8 nodes, then the factors of the block formulas (hex_point): w rho, rt, w,
+//   w tauLS | fact2 w, fact2 w rt, w rt, fact2 src | KA KB MM KDP |
+//   dphi(3) ufac | eps plfac pad(2); then the residual rows 8x5
 template <> struct HexLay<OVS_ASM_NSVOF> {
-  static constexpr int GPW = 44, RHS0 = 8 * 44, NF = 5, SW = 8 * 44 + 40, NV = 24;
+  static constexpr int GPW = 52, RHS0 = 8 * 52, NF = 5, SW = 8 * 52 + 40, NV = 24;
 };
 //   T record per point: g(8x3) w HK uadv(3) rcp dSe trc; then 8 residuals
 template <> struct HexLay<OVS_ASM_TEM> {
@@ -242,25 +244,16 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
       rec[27] = 0;
       store_n(out + gp * HexTcLay::GPW, rec, HexTcLay::GPW);
     } else {
-      T rec[L::GPW];
+      T* rec = out + gp * L::GPW;
 #pragma unroll
       for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) rec[3 * a + d] = g[a][d];
-      rec[24] = wf;
-      rec[25] = fluid ? fact2 * mupk * w : (T)0;
-      rec[26] = fluid ? fact2 * (tauC + lambda) * w : (T)0;
-      rec[27] = fluid ? fact2 * w * tauM : (T)0;
-      rec[28] = fluid ? fact2 * w * kdphi : (T)0;
-      rec[29] = dphi[0]; rec[30] = dphi[1]; rec[31] = dphi[2];
-      rec[32] = uadv[0]; rec[33] = uadv[1]; rec[34] = uadv[2];
-      rec[35] = rho; rec[36] = rho * tauM; rec[37] = tauLS;
-      rec[38] = vdot + phii * ira * dmd - dmd * irhoa;
-      rec[39] = fact2 * wf * tauC * dmdi * dmdi;
-      rec[40] = fact2 * tauC * dmdi * wf;
-      rec[41] = fact2 * dmdi * wf;
-      rec[42] = 0; rec[43] = 0;
-      store_n(out + gp * L::GPW, rec, L::GPW);
+        put4(rec + 4 * a, g[a][0], g[a][1], g[a][2], uadv[0] * g[a][0] + uadv[1] * g[a][1] + uadv[2] * g[a][2]);
+      const T rt = rho * tauM, fw = fact2 * wf;
+      put4(rec + 32, wf * rho, rt, wf, wf * tauLS);
+      put4(rec + 36, fw, fw * rt, wf * rt, fact2 * (vdot + phii * ira * dmd - dmd * irhoa));
+      put4(rec + 40, fw * mupk, fw * (tauC + lambda), fw * tauM, fw * kdphi);
+      put4(rec + 44, dphi[0], dphi[1], dphi[2], fw * tauC * dmdi);
+      put4(rec + 48, fw * tauC * dmdi * dmdi, fw * dmdi, (T)0, (T)0);
     }
     if (!fluid) continue;
     T svis[8], gdphi[8], c[8];
@@ -425,70 +418,53 @@ __global__ void __launch_bounds__(64) hex_element_kernel(const SumArgs a) {
   }
 }
 
-// Block (row node la, column node b) of a hex from its records: the
-// per-point forms of the tet block sums (see add_block), summed over the
-// 8 points.
-template <typename T, int KIND>
-__device__ __forceinline__ void hex_expand_block(const ovs_params& p, const T* sm, int la, int b, T* o, T* rv) {
-  using L = HexLay<KIND>;
-  if constexpr (KIND == OVS_ASM_TEM) {
-    const T fact1 = (T)p.almi, fact2 = (T)(p.alfi * p.gami * p.delt);
-    T X = 0;
-    for (int gp = 0; gp < 8; ++gp) {
-      const T* q = sm + gp * L::GPW;
-      const T ga[3] = {q[3 * la], q[3 * la + 1], q[3 * la + 2]};
-      const T gb[3] = {q[3 * b], q[3 * b + 1], q[3 * b + 2]};
-      const T w = q[24], HK = q[25], rcp = q[29], dSe = q[30], trc = q[31];
-      const T uadv[3] = {q[26], q[27], q[28]};
-      const T Na = hex_N<T>(gp, la), Nb = hex_N<T>(gp, b);
-      const T ca = ga[0] * uadv[0] + ga[1] * uadv[1] + ga[2] * uadv[2];
-      const T cb = gb[0] * uadv[0] + gb[1] * uadv[1] + gb[2] * uadv[2];
-      const T aw = w * (Na + trc * ca);
-      X += aw * (rcp * (fact1 * Nb + fact2 * cb) - fact2 * dSe * Nb) + HK * (ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2]);
-    }
-    o[0] = X;
-    rv[0] = sm[L::RHS0 + la];
-  } else {
-    const T fact1 = (T)p.almi, fact2 = (T)(p.alfi * p.delt * p.gami);
-#pragma unroll
-    for (int v = 0; v < 24; ++v) o[v] = 0;
-    for (int gp = 0; gp < 8; ++gp) {
-      const T* q = sm + gp * L::GPW;
-      const T ga[3] = {q[3 * la], q[3 * la + 1], q[3 * la + 2]};
-      const T gb[3] = {q[3 * b], q[3 * b + 1], q[3 * b + 2]};
-      T s[20];
-#pragma unroll
-      for (int k = 0; k < 20; k += 4) ldv4(q + 24 + k, s + k);
-      const T w = s[0], KA = s[1], KB = s[2], MM = s[3], KDP = s[4];
-      const T dphi[3] = {s[5], s[6], s[7]}, uadv[3] = {s[8], s[9], s[10]};
-      const T rho = s[11], rt = s[12], tls = s[13], src = s[14], eps = s[15], ufac = s[16], plfac = s[17];
-      const T Na = hex_N<T>(gp, la), Nb = hex_N<T>(gp, b);
-      const T ca = uadv[0] * ga[0] + uadv[1] * ga[1] + uadv[2] * ga[2];
-      const T cb = uadv[0] * gb[0] + uadv[1] * gb[1] + uadv[2] * gb[2];
-      const T gab = ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2];
-      const T beta = fact1 * Nb + fact2 * cb;
-      const T S = w * rho * (Na + rt * ca) * beta;
-      const T P = fact2 * w * Nb, Q = fact2 * w * rt * ca, R = fact2 * w * Na, Tt = w * rt * beta;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) o[4 * i + j] += KA * ga[j] * gb[i] + KB * ga[i] * gb[j] + (i == j ? KA * gab + S : (T)0);
-        o[4 * i + 3] += -ga[i] * P + gb[i] * Q;
-      }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) o[12 + d] += gb[d] * R + ga[d] * Tt;
-      o[15] += MM * gab;
-      const T gam = w * (Na + tls * ca);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) o[16 + d] += dphi[d] * (fact2 * gam * Nb) - gb[d] * (ufac * Na);
-      o[19] += gam * (beta + fact2 * Nb * src) + KDP * gab + eps * Na * Nb;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) o[20 + d] += ga[d] * (ufac * Nb);
-      o[23] += -plfac * Na * Nb;
-    }
-#pragma unroll
-    for (int f = 0; f < 5; ++f) rv[f] = sm[L::RHS0 + 5 * la + f];
+// Entry (row node la, column node b) of a hex temperature matrix from its
+// records, summed over the 8 points.
+template <typename T>
+__device__ __forceinline__ T hex_tem_entry(const ovs_params& p, const T* sm, int la, int b) {
+  using L = HexLay<OVS_ASM_TEM>;
+  const T fact1 = (T)p.almi, fact2 = (T)(p.alfi * p.gami * p.delt);
+  T X = 0;
+  for (int gp = 0; gp < 8; ++gp) {
+    const T* q = sm + gp * L::GPW;
+    const T ga[3] = {q[3 * la], q[3 * la + 1], q[3 * la + 2]};
+    const T gb[3] = {q[3 * b], q[3 * b + 1], q[3 * b + 2]};
+    const T w = q[24], HK = q[25], rcp = q[29], dSe = q[30], trc = q[31];
+    const T uadv[3] = {q[26], q[27], q[28]};
+    const T Na = hex_N<T>(gp, la), Nb = hex_N<T>(gp, b);
+    const T ca = ga[0] * uadv[0] + ga[1] * uadv[1] + ga[2] * uadv[2];
+    const T cb = gb[0] * uadv[0] + gb[1] * uadv[1] + gb[2] * uadv[2];
+    const T aw = w * (Na + trc * ca);
+    X += aw * (rcp * (fact1 * Nb + fact2 * cb) - fact2 * dSe * Nb) + HK * (ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2]);
   }
+  return X;
+}
+
+// The block (row node a, column node b) of one Gauss point added to o, the
+// per-point forms of the tet block sums (add_block): ga, gb the nodes' gradients
+// and c, Na, Nb their shape values, s the point's factors (HexLay).
+template <typename T>
+__device__ __forceinline__ void hex_point(const T (&ga)[4], const T (&gb)[4], T Na, T Nb, T f1, T f2,
+                                          const T (&s)[20], T (&o)[24]) {
+  const T gab = ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2];
+  const T beta = f1 * Nb + f2 * gb[3];
+  const T P = s[4] * Nb, Q = s[5] * ga[3], R = s[4] * Na, Tt = s[6] * beta;
+  const T dg = s[8] * gab + s[0] * (Na + s[1] * ga[3]) * beta;
+  const T gam = s[2] * Na + s[3] * ga[3], V = f2 * Nb * gam, uNa = s[15] * Na, uNb = s[15] * Nb, NN = Na * Nb;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const T ka = s[8] * gb[i], kb = s[9] * ga[i];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) o[4 * i + j] += ka * ga[j] + kb * gb[j];
+    o[5 * i] += dg;
+    o[4 * i + 3] += gb[i] * Q - ga[i] * P;
+    o[12 + i] += gb[i] * R + ga[i] * Tt;
+    o[16 + i] += s[12 + i] * V - gb[i] * uNa;
+    o[20 + i] += ga[i] * uNb;
+  }
+  o[15] += s[10] * gab;
+  o[19] += gam * (beta + s[7] * Nb) + s[11] * gab + s[16] * NN;
+  o[23] -= s[17] * NN;
 }
 
 // ------------------------------------------------------------------------
@@ -880,7 +856,8 @@ __global__ void __launch_bounds__(128) hex_rows_kernel(const AsmArgs a) {
 #pragma unroll
           for (int f = 0; f < NF; ++f) rv[f] = sum[(size_t)e * HexTcLay::SW + HexTcLay::RHS0 + 5 * la + f];
         } else {
-          hex_expand_block<T, KIND>(a.p, sum + (size_t)e * L::SW, la, bl, o, rv);
+          o[0] = hex_tem_entry<T>(a.p, sum + (size_t)e * L::SW, la, bl);
+          rv[0] = sum[(size_t)e * L::SW + L::RHS0 + la];
         }
         T* dst = blk + (jl * 8 + bl) * BSTR;
         if constexpr (NV >= 4) {
@@ -963,6 +940,227 @@ __global__ void __launch_bounds__(128) hex_rows_kernel(const AsmArgs a) {
   }
 }
 
+// Row pass of the NS+VOF hexahedra: one warp per CSR row, in the order of the
+// row records.  A chunk is 4 of the row's elements, 8 lanes per element, a
+// column per lane.  The elements' point records pass through shared memory two
+// points at a time, copied asynchronously ahead of the points being summed, and
+// a lane sums its block over the 8 points in registers.  Then the chunk's 32
+// blocks meet in the same shared memory, and each output task (slot, 4-value
+// group) adds the blocks of its slot in ascending element order (`has` and
+// `colof` name them; `acc` carries the sums between chunks) and in the last
+// chunk writes the group, consecutive lanes writing consecutive groups.
+// Bound: latency at 16 (FP64) and 20 (FP32) warps per SM; the FP64 pipe is a
+// third busy (74 operations per block and point), the shared-memory reads that
+// feed it another third.  96^3 hexahedra: FP64 11.03 -> 6.62 ms, FP32 5.42 ->
+// 4.01 ms against records read from global memory at every point, one point
+// after the other, with the shape values recomputed; two columns per lane and 8
+// elements per chunk took 7.31 and 4.23 ms (254 and 166 registers).
+template <typename T> struct HexRows {
+  static constexpr int GPS = 2;                                        // points per stage
+  static constexpr int EPC = 4, LPE = 8;                               // elements per chunk, lanes per element
+  static constexpr int GPW = HexLay<OVS_ASM_NSVOF>::GPW;
+  static constexpr int ES = GPS * GPW + (sizeof(T) == 8 ? 2 : 8);      // element stride: quarter warps spread over the banks
+  static constexpr int BST = sizeof(T) == 8 ? 26 : 28;                 // block stride
+  static constexpr int UNITS = GPS * GPW * (int)sizeof(T) / 16;        // 16-byte copies per element and stage
+  static constexpr size_t stage = sizeof(T) * (size_t)(2 * EPC * ES > 8 * EPC * BST ? 2 * EPC * ES : 8 * EPC * BST);
+  static_assert(GPS * GPW * sizeof(T) % 16 == 0 && ES * sizeof(T) % 16 == 0 && BST * sizeof(T) % 16 == 0, "16-byte units");
+  // per warp: stages (then blocks), per slot the columns of the chunk's
+  // elements, which of them hold the slot, the Dirichlet mask; carried sums
+  __host__ __device__ static size_t slots(int max_deg) { return ((size_t)max_deg + 3) & ~(size_t)3; }
+  __host__ __device__ static size_t bytes(int max_deg, bool carry) {
+    return stage + (EPC + 8) * slots(max_deg) + (carry ? sizeof(T) * 24 * (size_t)max_deg : 0);
+  }
+};
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
+__device__ __forceinline__ void lds4(const float* p, float* d) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+}
+__device__ __forceinline__ void lds4(const double* p, double* d) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128, (sizeof(T) == 8 ? 4 : 5)) hex_block_rows_kernel(const AsmArgs a, int carry) {
+  using L = HexLay<OVS_ASM_NSVOF>;
+  using H = HexRows<T>;
+  constexpr int EPC = H::EPC, LPE = H::LPE;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned masks[24];
+  __shared__ T Nt[8][8];
+  if (threadIdx.x < 24) masks[threadIdx.x] = mask_of(threadIdx.x);
+  if (threadIdx.x < 64) Nt[threadIdx.x >> 3][threadIdx.x & 7] = hex_N<T>(threadIdx.x >> 3, threadIdx.x & 7);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, el = lane / LPE, cp = lane % LPE;
+  unsigned char* base = smem_raw + (size_t)wid * H::bytes(a.max_deg, carry);
+  T* st = reinterpret_cast<T*>(base);
+  const int ns = (int)H::slots(a.max_deg);
+  uint8_t* colof = base + H::stage;                            // [ns][EPC]: column of element j in slot s
+  unsigned* has = reinterpret_cast<unsigned*>(colof + EPC * ns);   // [ns]: bit j, element j holds slot s
+  unsigned* cib = has + ns;                                    // [ns]
+  T* acc = reinterpret_cast<T*>(cib + ns);
+  const T* sum = reinterpret_cast<const T*>(a.rec);
+  const uint2* n2s8 = reinterpret_cast<const uint2*>(a.n2s);
+  const T f1 = (T)a.p.almi, f2 = (T)(a.p.alfi * a.p.delt * a.p.gami);
+  // a row's record, and element ids and slots of its first chunk, travel while
+  // the row before it is summed
+  int t = blockIdx.x * 4 + wid;
+  const int step = gridDim.x * 4;
+  int4 rn = t < a.N ? __ldg(a.row_rec + t) : make_int4(0, 0, 0, 0);
+  int pkn = 0;
+  uint2 wn = make_uint2(0u, 0u);
+  if (el < rn.w >> 16) {
+    pkn = __ldg(a.n2e + rn.z + el);
+    wn = __ldg(n2s8 + rn.z + el);
+  }
+  for (; t < a.N; t += step) {
+    const int4 rr = rn;
+    const int A = rr.x, deg = rr.w & 0xff, sd = (rr.w >> 8) & 0xff, ne = rr.w >> 16;
+    T* out = reinterpret_cast<T*>(a.vals) + (size_t)rr.y * 24;
+    T res[2] = {(T)0, (T)0};   // residual fields cp and (lane 0 of an element) 4
+    unsigned ibA = 0;
+    for (int c0 = 0; c0 == 0 || c0 < ne; c0 += EPC) {
+      const int nc = min(EPC, ne - c0);
+      const bool on = el < nc;
+      int pk = pkn;
+      uint2 w = wn;
+      if (c0 > 0 && on) {
+        pk = __ldg(a.n2e + rr.z + c0 + el);
+        w = __ldg(n2s8 + rr.z + c0 + el);
+      }
+      const int la = pk & 7;
+      const T* mine = sum + (size_t)(pk >> 3) * L::SW;
+      auto fetch = [&](int k) {   // stage k: points 2 k, 2 k + 1 of the chunk's elements, an element by its 4 lanes
+        if (on) {
+          unsigned char* dst = reinterpret_cast<unsigned char*>(st + ((k & 1) * EPC + el) * H::ES) + 16 * cp;
+          const unsigned char* src = reinterpret_cast<const unsigned char*>(mine + k * H::GPS * H::GPW) + 16 * cp;
+#pragma unroll
+          for (int u = 0; u < H::UNITS; u += LPE)
+            if (u + LPE <= H::UNITS || cp < H::UNITS - u) cp_async16(dst + 16 * u, src + 16 * u);
+        }
+        cp_async_commit();
+      };
+      fetch(0);
+      fetch(1);
+      int col = 0;
+      unsigned ibB = 0;
+      T r0 = (T)0, r1 = (T)0;
+      if (c0 == 0) {
+        if (lane < deg) col = __ldg(a.colidx + rr.y + lane);
+        ibA = __ldg(a.ibc + A);
+        rn = t + step < a.N ? __ldg(a.row_rec + t + step) : make_int4(0, 0, 0, 0);
+      }
+      for (int s = lane; s < deg; s += 32) has[s] = 0u;
+      __syncwarp();
+      if (on) {   // the lane's column
+        const unsigned s = ((cp < 4 ? w.x : w.y) >> (8 * (cp & 3))) & 0xffu;
+        colof[EPC * s + el] = (uint8_t)cp;
+        atomicOr(has + s, 1u << el);
+        if (cp < 4) r0 = __ldg(mine + L::RHS0 + 5 * la + cp);
+        if (cp == 0) r1 = __ldg(mine + L::RHS0 + 5 * la + 4);
+      }
+      T o[24];
+#pragma unroll
+      for (int v = 0; v < 24; ++v) o[v] = (T)0;
+#pragma unroll 1
+      for (int k = 0; k < 4; ++k) {
+        if (k < 3) cp_async_wait<1>(); else cp_async_wait<0>();
+        __syncwarp();
+        if (k == 1 && c0 == 0) {
+          if (lane < deg) ibB = __ldg(a.ibc + col);
+          pkn = 0;
+          if (el < rn.w >> 16) {
+            pkn = __ldg(a.n2e + rn.z + el);
+            wn = __ldg(n2s8 + rn.z + el);
+          }
+        }
+        if (on) {
+#pragma unroll 1
+          for (int h = 0; h < H::GPS; ++h) {
+            const T* q = st + ((k & 1) * EPC + el) * H::ES + h * H::GPW;
+            const T* N = Nt[H::GPS * k + h];
+            T s[20], ga[4], gb[4];
+#pragma unroll
+            for (int v = 0; v < 20; v += 4) lds4(q + 32 + v, s + v);
+            lds4(q + 4 * la, ga);
+            lds4(q + 4 * cp, gb);
+            hex_point<T>(ga, gb, N[la], N[cp], f1, f2, s, o);
+          }
+        }
+        __syncwarp();
+        if (k < 2) fetch(k + 2);
+      }
+      if (c0 == 0) {
+        if (lane < deg) cib[lane] = ibB;
+        for (int s = lane + 32; s < deg; s += 32) cib[s] = __ldg(a.ibc + __ldg(a.colidx + rr.y + s));
+      }
+      res[0] += r0;
+      res[1] += r1;
+      // the chunk's blocks, in the stages' place
+      if (on) {
+#pragma unroll
+        for (int v = 0; v < 24; v += 4) store_row<4>(st + lane * H::BST + v, o + v);
+      }
+      __syncwarp();
+      const bool last = c0 + EPC >= ne;
+      for (int q = lane; q < deg * 6; q += 32) {
+        const int s = q / 6, g = q - 6 * s;
+        if (!last && c0 > 0 && has[s] == 0u) continue;   // nothing of this chunk
+        T v[4] = {(T)0, (T)0, (T)0, (T)0};
+        if (c0 > 0) lds4(acc + 24 * s + 4 * g, v);
+        const T* blk = st + 4 * g;
+        for (unsigned m = has[s]; m; m &= m - 1) {   // ascending elements; an element's 8 columns have distinct slots
+          const int j = __ffs(m) - 1;
+          T x[4];
+          lds4(blk + (j * 8 + colof[EPC * s + j]) * H::BST, x);
+          v[0] += x[0]; v[1] += x[1]; v[2] += x[2]; v[3] += x[3];
+        }
+        if (!last) {
+          store_row<4>(acc + 24 * s + 4 * g, v);
+          continue;
+        }
+        const unsigned ib = cib[s];
+        if ((ibA | ib) != 0u) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const unsigned m = masks[4 * g + u];
+            if ((ibA & m & 0xffu) || ((ib << 8) & m & 0xff00u)) v[u] = (T)0;
+            if (s == sd && ((ibA << 16) & m & 0xff0000u)) v[u] = (T)ne;
+          }
+        }
+        store4_cs(out + 24 * (size_t)s + 4 * g, v);
+      }
+      __syncwarp();
+    }
+    // residual: the elements' lanes added by halving (fields 0-3 and 4)
+#pragma unroll
+    for (int o = 16; o >= LPE; o >>= 1) {
+      res[0] += __shfl_xor_sync(0xffffffffu, res[0], o);
+      res[1] += __shfl_xor_sync(0xffffffffu, res[1], o);
+    }
+    if (a.vec && lane < 4) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int f = u ? 4 : lane;
+        if (u && lane) break;
+        const T v = (ibA & (1u << f)) ? (T)0 : res[u];   // IBC bits 0-4: u1 u2 u3 p phi
+        if (!isfinite((double)v)) atomicOr(a.flags + 1, 1);
+        reinterpret_cast<T*>(a.rhs)[(size_t)f * a.N + A] = v;
+      }
+    }
+  }
+}
+
 template <typename T, int KIND>
 int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int parts) {
   if (!a0.mat) {   // vector-only pass, as for the tets
@@ -1009,19 +1207,28 @@ int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int pa
     }
   }
   if (!(parts & 2)) return OVS_OK;
-  using S = HexSmem<T, KIND>;
-  const size_t smem = S::bytes(a.max_deg) * 4;
-  auto kern = tc ? hex_rows_kernel<T, KIND, can_tc> : hex_rows_kernel<T, KIND, false>;
-  OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem));
-  if (per_sm < 1) return OVS_ERR_ARG;
-  long need = ((long)c->N + 3) / 4;
-  long grid = (long)per_sm * c->num_sms * 4;
-  if (grid > need) grid = need;
-  if (grid < 1) grid = 1;
-  kern<<<(int)grid, 128, smem, c->stream>>>(a);
-  ++c->launches;
-  OVS_CUDA_TRY(cudaGetLastError());
-  return OVS_OK;
+  auto launch = [&](auto kern, size_t smem, auto... more) -> int {
+    OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem));
+    if (per_sm < 1) return OVS_ERR_ARG;
+    long need = ((long)c->N + 3) / 4;
+    long grid = (long)per_sm * c->num_sms * 4;
+    if (grid > need) grid = need;
+    if (grid < 1) grid = 1;
+    kern<<<(int)grid, 128, smem, c->stream>>>(a, more...);
+    ++c->launches;
+    OVS_CUDA_TRY(cudaGetLastError());
+    return OVS_OK;
+  };
+  if constexpr (KIND == OVS_ASM_NSVOF) {
+    if (!tc) {
+      const int carry = c->max_elem > HexRows<T>::EPC;
+      return launch(hex_block_rows_kernel<T>, HexRows<T>::bytes(a.max_deg, carry) * 4, carry);
+    }
+    if constexpr (can_tc) return launch(hex_rows_kernel<T, KIND, true>, HexSmem<T, KIND>::bytes(a.max_deg) * 4);
+    return OVS_ERR_ARG;
+  } else {
+    return launch(hex_rows_kernel<T, KIND, false>, HexSmem<T, KIND>::bytes(a.max_deg) * 4);
+  }
 }
