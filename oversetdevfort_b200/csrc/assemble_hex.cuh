@@ -1,28 +1,33 @@
 // Trilinear hexahedra (nshl = 8): the NS+VOF quench and temperature
 // element routines (src/solveQuenching.f90:122-882) with the 2x2x2 rule
 // (src/genGP_GW.f90:355-389) and linhexshl (src/eval_shape_FEM.f90:148-196),
-// assembled like the tets: an element pass writes per-Gauss-point records
-// and the element's residual rows, a row pass (one warp per CSR row) expands
-// the blocks of A's row and adds them in ascending element id.  Unlike a
-// linear tet, a hex has different gradients at every Gauss point, so the
-// row pass sums each block over the 8 points.  Included into assemble.cu's
+// assembled like the tets: an element pass writes per-Gauss-point records (T:
+// the element matrix) and the element's residual rows, a row pass (one warp per
+// CSR row) forms the blocks of A's row and adds them in ascending element id.
+// Unlike a linear tet, a hex has different gradients at every Gauss point, so
+// the row pass sums each block over the 8 points.  Included into assemble.cu's
 // anonymous namespace (it uses its helpers).
 
-// node signs of linhexshl: N_a = (1 + sx xi)(1 + sy eta)(1 + sz zeta) / 8
-__constant__ signed char c_hex_sign[8][3] = {{-1, 1, -1}, {1, 1, -1}, {1, 1, 1}, {-1, 1, 1},
-                                             {-1, -1, -1}, {1, -1, -1}, {1, -1, 1}, {-1, -1, 1}};
-// 2x2x2 points (genGPandGW, weights 1)
-__device__ __forceinline__ void hex_gp(int g, double& xi, double& eta, double& ze) {
-  const double q = 0.57735026918963;
-  xi = (g & 1) ? q : -q;
-  eta = (g & 2) ? q : -q;
-  ze = (g & 4) ? q : -q;
+// Node signs of linhexshl, N_a = (1 + sx xi)(1 + sy eta)(1 + sz zeta) / 8: bit
+// set where the node sits at +1 along axis d.  The points are at +-q, so every
+// shape value and derivative is one of a few constants, picked by how many of
+// the node's signs match the point's.
+__host__ __device__ constexpr int hex_bit(int a, int d) {
+  return d == 0 ? ((a ^ (a >> 1)) & 1) : (d == 1 ? (a < 4) : ((a >> 1) & 1));
+}
+constexpr double HEX_P = 1.0 + 0.57735026918963, HEX_M = 1.0 - 0.57735026918963;   // 2x2x2 points (genGPandGW, weights 1)
+template <typename T> __device__ __forceinline__ T hex_n3(int m) {   // N by matching signs
+  constexpr double c0 = HEX_M * HEX_M * HEX_M * 0.125, c1 = HEX_P * HEX_M * HEX_M * 0.125,
+                   c2 = HEX_P * HEX_P * HEX_M * 0.125, c3 = HEX_P * HEX_P * HEX_P * 0.125;
+  return m == 0 ? (T)c0 : (m == 1 ? (T)c1 : (m == 2 ? (T)c2 : (T)c3));
+}
+template <typename T> __device__ __forceinline__ T hex_n2(int m) {   // |dN/dxi| by matching signs of the other two axes
+  constexpr double c0 = HEX_M * HEX_M * 0.125, c1 = HEX_P * HEX_M * 0.125, c2 = HEX_P * HEX_P * 0.125;
+  return m == 0 ? (T)c0 : (m == 1 ? (T)c1 : (T)c2);
 }
 template <typename T>
 __device__ __forceinline__ T hex_N(int g, int a) {
-  double xi, eta, ze;
-  hex_gp(g, xi, eta, ze);
-  return (T)((1.0 + c_hex_sign[a][0] * xi) * (1.0 + c_hex_sign[a][1] * eta) * (1.0 + c_hex_sign[a][2] * ze) * 0.125);
+  return hex_n3<T>((hex_bit(a, 0) == (g & 1)) + (hex_bit(a, 1) == ((g >> 1) & 1)) + (hex_bit(a, 2) == ((g >> 2) & 1)));
 }
 
 template <int KIND> struct HexLay;
@@ -33,9 +38,10 @@ template <int KIND> struct HexLay;
 template <> struct HexLay<OVS_ASM_NSVOF> {
   static constexpr int GPW = 52, RHS0 = 8 * 52, NF = 5, SW = 8 * 52 + 40, NV = 24;
 };
-//   T record per point: g(8x3) w HK uadv(3) rcp dSe trc; then 8 residuals
+//   T: the 8x8 element matrix itself, row-major (a scalar system: smaller than
+//   the records it would be summed from), then 8 residuals
 template <> struct HexLay<OVS_ASM_TEM> {
-  static constexpr int GPW = 32, RHS0 = 8 * 32, NF = 1, SW = 8 * 32 + 8, NV = 1;
+  static constexpr int RHS0 = 64, NF = 1, SW = 72, NV = 1;
 };
 
 //   NS+VOF record per point for the tensor-core path: dxi/dx (3x3, row k =
@@ -45,136 +51,173 @@ struct HexTcLay {
   static constexpr int GPW = 28, RHS0 = 8 * 28, SW = 8 * 28 + 40;
 };
 
-// eval_shape_fem for a hex at point g on x+d: global gradients, DetJ, G
-template <typename T>
-__device__ __forceinline__ T hex_geometry(int gp, const T r[8][16], const T lo[8][4], T g[8][3], T G[3][3],
-                                          T (*Aio)[3] = nullptr) {
-  double xi, eta, ze;
-  hex_gp(gp, xi, eta, ze);
-  T dN[8][3];
+__device__ __forceinline__ void lds4(const float* p, float* d) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+}
+__device__ __forceinline__ void lds4(const double* p, double* d) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
+}
+
+// Element pass: 8 lanes per element, lane g evaluates Gauss point g.  A lane
+// walks the element's 8 node records once (the 8 lanes read the same address)
+// and keeps the sums it needs: values at the point and derivatives along the
+// reference axes, which the inverse Jacobian then turns into gradients.  The
+// residual rows are added over the lanes by halving, which leaves lane n with
+// node n's.  NS+VOF: every lane writes its point's record (MAT) or the compact
+// one of the tensor-core pass (TC).  T: the points meet in shared memory and
+// lane a sums row a of the element matrix.  MAT false (vector-only pass): the
+// residual rows alone.
+// One thread per element held 8 records and 40 residual sums (255 registers,
+// 1.4 KB of spills in FP64): 96^3 hexahedra, NS+VOF 1.78 -> 1.20 ms in FP64 and
+// 0.82 -> 0.80 in FP32, T, which wrote point records for the row pass to sum,
+// 1.47 -> 1.09 and 1.12 -> 0.55 ms (T rows 3.08 -> 0.59 and 2.39 -> 0.54 ms).
+// Blocks per SM: 3 in FP64 (2: 1.48 ms, no spills), 6 in FP32 (4: 0.97, 5: 0.84).
+template <typename T> struct HexTemStage {
+  static constexpr int GPW = 44;                                       // per point: (grad, B) of 8 nodes, A of 8, HK
+  static constexpr int ES = 8 * GPW + (sizeof(T) == 8 ? 2 : 4);        // element stride: elements of a warp spread over the banks
+  static constexpr int bytes = 16 * ES * (int)sizeof(T);
+};
+
+// values summed over the 8 lanes of an element by halving: v holds NV values
+// per node, lane n ends up with node n's in v[0..NV)
+template <typename T, int NV>
+__device__ __forceinline__ void hex_sum_nodes(T (&v)[8 * NV], int lane) {
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const double sx = c_hex_sign[a][0], sy = c_hex_sign[a][1], sz = c_hex_sign[a][2];
-    dN[a][0] = (T)(sx * (1.0 + sy * eta) * (1.0 + sz * ze) * 0.125);
-    dN[a][1] = (T)(sy * (1.0 + sx * xi) * (1.0 + sz * ze) * 0.125);
-    dN[a][2] = (T)(sz * (1.0 + sx * xi) * (1.0 + sy * eta) * 0.125);
+  for (int half = 4, off = 4; off >= 1; half >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int k = 0; k < half * NV; ++k) {
+      const T send = up ? v[k] : v[k + half * NV], keep = up ? v[k + half * NV] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
   }
-  // dx/dxi from coordinates relative to node 0 (sum_a dN_a = 0), so the
-  // FP32 path keeps the edge lengths to full precision
-  T A[3][3], Ai[3][3];
+}
+
+template <typename T, int KIND, bool TC = false, bool MAT = true>
+__global__ void __launch_bounds__(128, (sizeof(T) == 8 ? 3 : 6)) hex_element_kernel(const SumArgs a) {
+  constexpr bool vof = KIND == OVS_ASM_NSVOF;
+  using L = HexLay<KIND>;
+  constexpr int NF = L::NF;
+  constexpr int SW = !MAT ? 8 * NF : TC ? HexTcLay::SW : L::SW;
+  constexpr int RHS0 = !MAT ? 0 : TC ? HexTcLay::RHS0 : L::RHS0;
+  const ovs_params& p = a.p;
+  const int lane = threadIdx.x & 31, gp = lane & 7;
+  const int tt = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 3);
+  const bool on = tt < a.E;
+  const int t = on ? tt : a.E - 1;
+  const T* rec = reinterpret_cast<const T*>(a.rec);
+  const int mynode = __ldg(a.ien + 8 * (size_t)t + gp);
+  const bool fluid = __ldg(a.elm_id + t) == p.fluid_elm_id;
+  const int g0 = gp & 1, g1 = (gp >> 1) & 1, g2 = (gp >> 2) & 1;
+  // shape values and reference derivatives of node n at this lane's point
+  auto shape = [&](int n, T& N, T (&dN)[3]) {
+    const int m0 = hex_bit(n, 0) == g0, m1 = hex_bit(n, 1) == g1, m2 = hex_bit(n, 2) == g2;
+    N = hex_n3<T>(m0 + m1 + m2);
+    const T d0 = hex_n2<T>(m1 + m2), d1 = hex_n2<T>(m0 + m2), d2 = hex_n2<T>(m0 + m1);
+    dN[0] = hex_bit(n, 0) ? d0 : -d0;
+    dN[1] = hex_bit(n, 1) ? d1 : -d1;
+    dN[2] = hex_bit(n, 2) ? d2 : -d2;
+  };
+  T J[3][3], ur[3][3], pr[3], fr[3];   // T pass: fr holds the temperature's derivatives, ur and pr are unused
+  T ui[3], umi[3], aci[3], pri = 0, rphii = 0, Ti = 0, rTi = 0;
+  double phid = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    ui[i] = umi[i] = aci[i] = pr[i] = fr[i] = 0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) J[i][j] = ur[i][j] = 0;
+  }
+  T x0[3], l0[3];
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    T r[16], lo[4], N, dN[3];
+    load_rec(rec, __shfl_sync(0xffffffffu, mynode, (lane & 24) + n), r, lo);
+    shape(n, N, dN);
+    if (n == 0) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) { x0[i] = r[i]; l0[i] = lo[i]; }
+    } else {
+      // dx/dxi from coordinates relative to node 0 (sum_a dN_a = 0), so the
+      // FP32 path keeps the edge lengths to full precision
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const T d = (r[i] - x0[i]) + (lo[i] - l0[i]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) J[i][j] += d * dN[j];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      ui[i] += r[3 + i] * N;
+      umi[i] += r[6 + i] * N;
+      if constexpr (vof) {
+        aci[i] += r[9 + i] * N;
+        pr[i] += r[12] * dN[i];
+        fr[i] += r[13] * dN[i];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) ur[i][j] += r[3 + i] * dN[j];
+      } else {
+        fr[i] += r[10] * dN[i];
+      }
+    }
+    phid += ((double)r[vof ? 13 : 9] + (double)lo[3]) * hex_n3<double>((hex_bit(n, 0) == g0) + (hex_bit(n, 1) == g1) +
+                                                                      (hex_bit(n, 2) == g2));
+    if constexpr (vof) {
+      pri += r[12] * N;
+      rphii += r[14] * N;
+      Ti += r[15] * N;
+    } else {
+      Ti += r[10] * N;
+      rTi += r[11] * N;
+    }
+  }
+  // inverse Jacobian, DetJ (eval_shape_fem), G
+  T Ai[3][3], G[3][3];
+  Ai[0][0] = J[1][1] * J[2][2] - J[2][1] * J[1][2];
+  Ai[0][1] = J[2][1] * J[0][2] - J[0][1] * J[2][2];
+  Ai[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
+  const T tmp = (T)1.0 / (Ai[0][0] * J[0][0] + Ai[0][1] * J[1][0] + Ai[0][2] * J[2][0]);
+  Ai[0][0] *= tmp; Ai[0][1] *= tmp; Ai[0][2] *= tmp;
+  Ai[1][0] = (J[1][2] * J[2][0] - J[1][0] * J[2][2]) * tmp;
+  Ai[1][1] = (J[0][0] * J[2][2] - J[2][0] * J[0][2]) * tmp;
+  Ai[1][2] = (J[1][0] * J[0][2] - J[0][0] * J[1][2]) * tmp;
+  Ai[2][0] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]) * tmp;
+  Ai[2][1] = (J[2][0] * J[0][1] - J[0][0] * J[2][1]) * tmp;
+  Ai[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * tmp;
+  const T w = (T)1.0 / tmp;   // hex weights are 1
+  T GG = 0;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      T s = 0;
-#pragma unroll
-      for (int a = 1; a < 8; ++a) s += ((r[a][i] - r[0][i]) + (lo[a][i] - lo[0][i])) * dN[a][j];
-      A[i][j] = s;
+      G[i][j] = Ai[0][i] * Ai[0][j] + Ai[1][i] * Ai[1][j] + Ai[2][i] * Ai[2][j];
+      GG += G[i][j] * G[i][j];
     }
-  Ai[0][0] = A[1][1] * A[2][2] - A[2][1] * A[1][2];
-  Ai[0][1] = A[2][1] * A[0][2] - A[0][1] * A[2][2];
-  Ai[0][2] = A[0][1] * A[1][2] - A[0][2] * A[1][1];
-  T tmp = (T)1.0 / (Ai[0][0] * A[0][0] + Ai[0][1] * A[1][0] + Ai[0][2] * A[2][0]);
-  Ai[0][0] *= tmp; Ai[0][1] *= tmp; Ai[0][2] *= tmp;
-  Ai[1][0] = (A[1][2] * A[2][0] - A[1][0] * A[2][2]) * tmp;
-  Ai[1][1] = (A[0][0] * A[2][2] - A[2][0] * A[0][2]) * tmp;
-  Ai[1][2] = (A[1][0] * A[0][2] - A[0][0] * A[1][2]) * tmp;
-  Ai[2][0] = (A[1][0] * A[2][1] - A[1][1] * A[2][0]) * tmp;
-  Ai[2][1] = (A[2][0] * A[0][1] - A[0][0] * A[2][1]) * tmp;
-  Ai[2][2] = (A[0][0] * A[1][1] - A[0][1] * A[1][0]) * tmp;
+  auto grad = [&](const T (&d)[3], T (&g)[3]) {
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) g[a][j] = dN[a][0] * Ai[0][j] + dN[a][1] * Ai[1][j] + dN[a][2] * Ai[2][j];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) G[i][j] = Ai[0][i] * Ai[0][j] + Ai[1][i] * Ai[1][j] + Ai[2][i] * Ai[2][j];
-  if (Aio)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) Aio[i][j] = Ai[i][j];
-  return (T)1.0 / tmp;
-}
-
-template <typename T>
-__device__ __forceinline__ double hex_phi(const T r[8][16], const T lo[8][4], int k, int gp) {
-  double s = 0.0;
-#pragma unroll
-  for (int a = 0; a < 8; ++a) s += ((double)r[a][k] + (double)lo[a][3]) * hex_N<double>(gp, a);
-  return s;
-}
-
-template <typename T>
-__device__ __forceinline__ void store_n(T* dst, const T* v, int n) {
-  for (int k = 0; k < n; ++k) dst[k] = v[k];
-}
-
-// element pass, NS+VOF quench on a hex (src/solveQuenching.f90:295-523);
-// TC: write the compact records of the tensor-core matrix pass instead; MAT
-// false (vector-only pass): the residual rows alone
-template <typename T, bool TC = false, bool MAT = true>
-__device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const T lo[8][4], bool fluid,
-                                    T* out, double& tamax, int& nbad) {
-  using L = HexLay<OVS_ASM_NSVOF>;
-  constexpr int RHS0 = !MAT ? 0 : TC ? HexTcLay::RHS0 : L::RHS0;
-  const T fact2 = (T)(p.alfi * p.delt * p.gami);
-  const T taut = (T)(4.0 / (p.delt * p.delt));
-  const T rhoa = (T)p.rhoa, rhow = (T)p.rhow, ts = (T)p.ts;
-  // reciprocals of the launch constants, taken once: the point formulas
-  // multiply by them where the reference divides (as the tet routines)
-  const T its = (T)(1.0 / p.ts), irhoa = (T)(1.0 / p.rhoa), irhow = (T)(1.0 / p.rhow);
-  const T ira = irhoa - irhow;
-  const bool kdc_on = fabs(p.ns_kdc_w) + fabs(p.ns_kdc_a) > 0.0;
-  const bool kdcphi_on = fabs(p.lsc_kdc) > 0.0;
-  T ru[8][3], rp[8], rf[8];
-#pragma unroll
-  for (int n = 0; n < 8; ++n) { ru[n][0] = ru[n][1] = ru[n][2] = 0; rp[n] = 0; rf[n] = 0; }
-  for (int gp = 0; gp < 8; ++gp) {
-    T g[8][3], G[3][3], Ai[3][3];
-    const T detj = hex_geometry<T>(gp, r, lo, g, G, Ai);
-    if (!(detj > (T)0)) nbad = 1;
-    const T w = detj;   // hex weights are 1
-    T GG = 0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int i = 0; i < 3; ++i) GG += G[i][j] * G[i][j];
+    for (int j = 0; j < 3; ++j) g[j] = d[0] * Ai[0][j] + d[1] * Ai[1][j] + d[2] * Ai[2][j];
+  };
+  const T fact2 = (T)(p.alfi * p.delt * p.gami), taut = (T)(4.0 / (p.delt * p.delt)), ts = (T)p.ts;
+  const double phicd = clamp01(phid);
+  const T phic = (T)phicd;
+  const T uadv[3] = {ui[0] - umi[0], ui[1] - umi[1], ui[2] - umi[2]};
+  const T taua = quad_uGu<T>(uadv, G);
+  T* out = reinterpret_cast<T*>(a.sum) + (size_t)t * SW;
+  T rr[8 * NF];
+  if constexpr (vof) {   // src/solveQuenching.f90:295-523
     const T trG = G[0][0] + G[1][1] + G[2][2];
-    T N[8];
+    T du[3][3], dp[3], dphi[3];
 #pragma unroll
-    for (int a = 0; a < 8; ++a) N[a] = hex_N<T>(gp, a);
-    T du[3][3], dp[3], dphi[3], ui[3], umi[3], aci[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      ui[i] = umi[i] = aci[i] = 0;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) du[i][j] = 0;
-      dp[i] = dphi[i] = 0;
-    }
-    T pri = 0, rphii = 0, Ti = 0;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        ui[i] += r[a][3 + i] * N[a];
-        umi[i] += r[a][6 + i] * N[a];
-        aci[i] += r[a][9 + i] * N[a];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) du[i][j] += r[a][3 + i] * g[a][j];
-        dp[i] += r[a][12] * g[a][i];
-        dphi[i] += r[a][13] * g[a][i];
-      }
-      pri += r[a][12] * N[a];
-      rphii += r[a][14] * N[a];
-      Ti += r[a][15] * N[a];
-    }
-    const T divu = du[0][0] + du[1][1] + du[2][2];
-    const double phid = hex_phi<T>(r, lo, 13, gp);
-    const T phii = (T)phid;
-    const double phicd = clamp01(phid);
-    const T phic = (T)phicd;
+    for (int i = 0; i < 3; ++i) grad(ur[i], du[i]);
+    grad(pr, dp);
+    grad(fr, dphi);
+    const T rhoa = (T)p.rhoa, rhow = (T)p.rhow;
+    // reciprocals of the launch constants: the point formulas multiply by
+    // them where the reference divides (as the tet routines)
+    const T its = (T)(1.0 / p.ts), irhoa = (T)(1.0 / p.rhoa), irhow = (T)(1.0 / p.rhow), ira = irhoa - irhow;
+    const T divu = du[0][0] + du[1][1] + du[2][2], phii = (T)phid;
     T mdot, dmd;
     if (Ti > ts) {
       mdot = (T)p.c_evap * (T)(1.0 - phicd) * rhow * (Ti - ts) * its;
@@ -193,7 +236,6 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
     }
     const T lambda = (T)(-2.0 / 3.0) * mu;
     if (phid < 0.0 || phid > 1.0) dmd = 0;
-    const T uadv[3] = {ui[0] - umi[0], ui[1] - umi[1], ui[2] - umi[2]};
     T tmp1[3], rL[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -202,134 +244,70 @@ __device__ void hex_summarize_nsvof(const ovs_params& p, const T r[8][16], const
       rL[i] = tmp1[i] + dp[i];
     }
     const T res_phi = rphii + (uadv[0] * dphi[0] + uadv[1] * dphi[1] + uadv[2] * dphi[2]) + phii * vdot - mdot * irhoa;
-    const T taua = quad_uGu<T>(uadv, G);
     const T irho = (T)1.0 / rho;
     const T nu = mu * irho;
     const T taud = nu * nu * (T)12.0 * GG;
     const T tauM = irho * inv_sqrt(taut + taua + taud);
     const T tauLS = inv_sqrt(taut + taua);
     const T tauC = rho * sqrt(taua + taud) / trG;
-    if ((double)taua > tamax) tamax = (double)taua;   // CFL number: delt sqrt(max taua), in the kernel
     T kdc = 0;
-    if (kdc_on) {
+    if (fabs(p.ns_kdc_w) + fabs(p.ns_kdc_a) > 0.0) {
       const double nk = (double)(p.ns_kdc_w * (1.0 - phicd) + p.ns_kdc_a * phicd);
-      const T rr = rL[0] * rL[0] + rL[1] * rL[1] + rL[2] * rL[2];
-      kdc = (T)low_word(nk) * sqrt(rr / GG);
+      kdc = (T)low_word(nk) * sqrt((rL[0] * rL[0] + rL[1] * rL[1] + rL[2] * rL[2]) / GG);
     }
     T kdphi = 0;
-    if (kdcphi_on) kdphi = (T)p.lsc_kdc * fabs(res_phi) / sqrt(GG);
-    const T mupk = mu + kdc;
-    const T dmdi = dmd * ira;
+    if (fabs(p.lsc_kdc) > 0.0) kdphi = (T)p.lsc_kdc * fabs(res_phi) / sqrt(GG);
+    const T mupk = mu + kdc, dmdi = dmd * ira;
     const T wf = fluid ? w : (T)0;   // solid elements contribute nothing
-    if constexpr (!MAT) {
-    } else if constexpr (TC) {
-      T rec[HexTcLay::GPW];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) rec[3 * k + j] = Ai[k][j];
-      rec[9] = wf;
-      rec[10] = fluid ? fact2 * mupk * w : (T)0;
-      rec[11] = fluid ? fact2 * (tauC + lambda) * w : (T)0;
-      rec[12] = fluid ? fact2 * w * tauM : (T)0;
-      rec[13] = fluid ? fact2 * w * kdphi : (T)0;
-      rec[14] = dphi[0]; rec[15] = dphi[1]; rec[16] = dphi[2];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) rec[17 + k] = Ai[k][0] * uadv[0] + Ai[k][1] * uadv[1] + Ai[k][2] * uadv[2];
-      rec[20] = rho; rec[21] = rho * tauM; rec[22] = tauLS;
-      rec[23] = vdot + phii * ira * dmd - dmd * irhoa;
-      rec[24] = fact2 * wf * tauC * dmdi * dmdi;
-      rec[25] = fact2 * tauC * dmdi * wf;
-      rec[26] = fact2 * dmdi * wf;
-      rec[27] = 0;
-      store_n(out + gp * HexTcLay::GPW, rec, HexTcLay::GPW);
-    } else {
-      T* rec = out + gp * L::GPW;
-#pragma unroll
-      for (int a = 0; a < 8; ++a)
-        put4(rec + 4 * a, g[a][0], g[a][1], g[a][2], uadv[0] * g[a][0] + uadv[1] * g[a][1] + uadv[2] * g[a][2]);
-      const T rt = rho * tauM, fw = fact2 * wf;
-      put4(rec + 32, wf * rho, rt, wf, wf * tauLS);
-      put4(rec + 36, fw, fw * rt, wf * rt, fact2 * (vdot + phii * ira * dmd - dmd * irhoa));
-      put4(rec + 40, fw * mupk, fw * (tauC + lambda), fw * tauM, fw * kdphi);
-      put4(rec + 44, dphi[0], dphi[1], dphi[2], fw * tauC * dmdi);
-      put4(rec + 48, fw * tauC * dmdi * dmdi, fw * dmdi, (T)0, (T)0);
+    const T src = vdot + phii * ira * dmd - dmd * irhoa, fw = fact2 * wf;
+    T* prec = out + gp * (TC ? HexTcLay::GPW : L::GPW);
+    if constexpr (MAT && TC) {
+      if (on) {
+        put4(prec, Ai[0][0], Ai[0][1], Ai[0][2], Ai[1][0]);
+        put4(prec + 4, Ai[1][1], Ai[1][2], Ai[2][0], Ai[2][1]);
+        put4(prec + 8, Ai[2][2], wf, fw * mupk, fw * (tauC + lambda));
+        put4(prec + 12, fw * tauM, fw * kdphi, dphi[0], dphi[1]);
+        put4(prec + 16, dphi[2], Ai[0][0] * uadv[0] + Ai[0][1] * uadv[1] + Ai[0][2] * uadv[2],
+             Ai[1][0] * uadv[0] + Ai[1][1] * uadv[1] + Ai[1][2] * uadv[2],
+             Ai[2][0] * uadv[0] + Ai[2][1] * uadv[1] + Ai[2][2] * uadv[2]);
+        put4(prec + 20, rho, rho * tauM, tauLS, src);
+        put4(prec + 24, fw * tauC * dmdi * dmdi, fw * tauC * dmdi, fw * dmdi, (T)0);
+      }
+    } else if constexpr (MAT) {
+      const T rt = rho * tauM;
+      if (on) {
+        put4(prec + 32, wf * rho, rt, wf, wf * tauLS);
+        put4(prec + 36, fw, fw * rt, wf * rt, fact2 * src);
+        put4(prec + 40, fw * mupk, fw * (tauC + lambda), fw * tauM, fw * kdphi);
+        put4(prec + 44, dphi[0], dphi[1], dphi[2], fw * tauC * dmdi);
+        put4(prec + 48, fw * tauC * dmdi * dmdi, fw * dmdi, (T)0, (T)0);
+      }
     }
-    if (!fluid) continue;
-    T svis[8], gdphi[8], c[8];
+    T h[3];   // the viscous broadcast (:508-510) as one vector: svis_n = grad N_n . h
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      T sv = 0;
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-        sv += g[n][0] * (du[0][k] + du[k][0]) + g[n][1] * (du[1][k] + du[k][1]) + g[n][2] * (du[2][k] + du[k][2]);
-      svis[n] = sv;
-      gdphi[n] = g[n][0] * dphi[0] + g[n][1] * dphi[1] + g[n][2] * dphi[2];
-      c[n] = uadv[0] * g[n][0] + uadv[1] * g[n][1] + uadv[2] * g[n][2];
-    }
+    for (int j = 0; j < 3; ++j) h[j] = (du[j][0] + du[0][j]) + (du[j][1] + du[1][j]) + (du[j][2] + du[2][j]);
     const T tdiv = -pri + tauC * divu;
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
+      T N, dN[3], g[3];
+      shape(n, N, dN);
+      grad(dN, g);
+      const T c = uadv[0] * g[0] + uadv[1] * g[1] + uadv[2] * g[2];
+      if constexpr (MAT && !TC)
+        if (on) put4(prec + 4 * n, g[0], g[1], g[2], c);
+      const T sv = g[0] * h[0] + g[1] * h[1] + g[2] * h[2];
 #pragma unroll
       for (int i = 0; i < 3; ++i)
-        ru[n][i] += w * (-N[n] * tmp1[i] - g[n][i] * tdiv + g[n][i] * tauC * vdot - g[n][i] * lambda * divu -
-                         mupk * svis[n] + rho * c[n] * (-tauM * rL[i]));
-      rp[n] += w * (-N[n] * (divu - vdot) + (g[n][0] * rL[0] + g[n][1] * rL[1] + g[n][2] * rL[2]) * (-tauM));
-      rf[n] += w * (-(N[n] + tauLS * c[n]) * res_phi - kdphi * gdphi[n] + N[n] * dmdi * tauC * (divu - vdot));
+        rr[5 * n + i] = wf * (-N * tmp1[i] - g[i] * tdiv + g[i] * tauC * vdot - g[i] * lambda * divu - mupk * sv +
+                              rho * c * (-tauM * rL[i]));
+      rr[5 * n + 3] = wf * (-N * (divu - vdot) + (g[0] * rL[0] + g[1] * rL[1] + g[2] * rL[2]) * (-tauM));
+      rr[5 * n + 4] = wf * (-(N + tauLS * c) * res_phi - kdphi * (g[0] * dphi[0] + g[1] * dphi[1] + g[2] * dphi[2]) +
+                            N * dmdi * tauC * (divu - vdot));
     }
-  }
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    T* orh = out + RHS0 + 5 * n;
-    orh[0] = ru[n][0]; orh[1] = ru[n][1]; orh[2] = ru[n][2]; orh[3] = rp[n]; orh[4] = rf[n];
-  }
-}
-
-// element pass, temperature on a hex (src/solveQuenching.f90:712-856);
-// record layout of this pass: xd(0:2) u(3:5) um(6:8) phi(9) T(10) rT(11)
-template <typename T, bool MAT = true>
-__device__ void hex_summarize_tem(const ovs_params& p, const T r[8][16], const T lo[8][4], bool fluid, T* out,
-                                  double& tamax, int& nbad) {
-  using L = HexLay<OVS_ASM_TEM>;
-  const T fact2 = (T)(p.alfi * p.gami * p.delt);
-  const T ts = (T)p.ts, cpw = (T)p.cpw, cpa = (T)p.cpa, lh = (T)p.lh;
-  const T its = (T)(1.0 / p.ts), itref = (T)(1.0 / p.tref), taut = (T)(4.0 / (p.delt * p.delt));
-  const bool kdc_on = fabs(p.tem_kdc) > 0.0;
-  T rt[8];
-#pragma unroll
-  for (int n = 0; n < 8; ++n) rt[n] = 0;
-  for (int gp = 0; gp < 8; ++gp) {
-    T g[8][3], G[3][3];
-    const T detj = hex_geometry<T>(gp, r, lo, g, G);
-    if (!(detj > (T)0)) nbad = 1;
-    const T w = detj;
-    T GG = 0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int i = 0; i < 3; ++i) GG += G[i][j] * G[i][j];
-    T N[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) N[a] = hex_N<T>(gp, a);
-    T dT[3] = {0, 0, 0}, ui[3] = {0, 0, 0}, umi[3] = {0, 0, 0};
-    T Ti = 0, rTi = 0;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        dT[j] += r[a][10] * g[a][j];
-        ui[j] += r[a][3 + j] * N[a];
-        umi[j] += r[a][6 + j] * N[a];
-      }
-      Ti += r[a][10] * N[a];
-      rTi += r[a][11] * N[a];
-    }
-    T gdT[8];
-#pragma unroll
-    for (int n = 0; n < 8; ++n) gdT[n] = g[n][0] * dT[0] + g[n][1] * dT[1] + g[n][2] * dT[2];
-    const double phid = hex_phi<T>(r, lo, 9, gp);
-    const double phicd = clamp01(phid);
-    const T phic = (T)phicd;
+  } else {   // src/solveQuenching.f90:712-856
+    const T cpw = (T)p.cpw, cpa = (T)p.cpa, lh = (T)p.lh, its = (T)(1.0 / p.ts), itref = (T)(1.0 / p.tref);
+    T dT[3];
+    grad(fr, dT);
     T mdot, dmdT;
     if (Ti > ts) {
       mdot = (T)p.c_evap * (T)(1.0 - phicd) * (T)p.rhow * (Ti - ts) * its;
@@ -347,97 +325,76 @@ __device__ void hex_summarize_tem(const ovs_params& p, const T r[8][16], const T
     } else {
       rho = (T)p.rhos; cp = (T)p.cps; hk = (T)p.kappas; rcp = (T)(p.rhos * p.cps);
     }
-    const T uadv[3] = {ui[0] - umi[0], ui[1] - umi[1], ui[2] - umi[2]};
     const T Se = ((cpw - cpa) * (Ti - ts) - lh) * mdot;
     const T udT = uadv[0] * dT[0] + uadv[1] * dT[1] + uadv[2] * dT[2];
     const T res = rcp * (rTi + udT) - Se;
-    const T taua = quad_uGu<T>(uadv, G);
-    T tt = taua + taut;
-    const T ircp = (T)1.0 / (rho * cp);
-    const T kk = hk * ircp;
-    tt = tt + kk * kk * (T)12.0 * GG;
-    const T tauT = ircp * inv_sqrt(tt);
-    if ((double)taua > tamax) tamax = (double)taua;   // CFL number: delt sqrt(max taua), in the kernel
+    const T ircp = (T)1.0 / (rho * cp), kk = hk * ircp;
+    const T tauT = ircp * inv_sqrt(taua + taut + kk * kk * (T)12.0 * GG);
     T kdcT = 0;
-    if (kdc_on && fluid) kdcT = (T)p.tem_kdc * fabs(res) * inv_sqrt(GG) * itref;
+    if (fabs(p.tem_kdc) > 0.0 && fluid) kdcT = (T)p.tem_kdc * fabs(res) * inv_sqrt(GG) * itref;
     const T dSe = (cpw - cpa) * mdot + ((cpw - cpa) * (Ti - ts) - lh) * dmdT;
-    T rec[L::GPW];
+    // solid: no advection, no source
+    const T fl = fluid ? (T)1 : (T)0, trq = fl * tauT * rcp, dSq = fl * dSe, HK = hk + kdcT;
+    const T rmass = fluid ? res : rcp * rTi;
+    extern __shared__ __align__(16) unsigned char hex_sm[];
+    using HT = HexTemStage<T>;
+    T* eb = reinterpret_cast<T*>(hex_sm) + (threadIdx.x >> 3) * HT::ES;   // this element's points
+    T* q = eb + gp * HT::GPW;
+    const T fact1 = (T)p.almi;
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) rec[3 * a + d] = g[a][d];
-    rec[24] = w;
-    rec[29] = rcp;
-    if (fluid) {
-      rec[25] = fact2 * (hk + kdcT) * w;
-      rec[26] = uadv[0]; rec[27] = uadv[1]; rec[28] = uadv[2];
-      rec[30] = dSe; rec[31] = tauT * rcp;
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const T cn = uadv[0] * g[n][0] + uadv[1] * g[n][1] + uadv[2] * g[n][2];
-        rt[n] += w * (-N[n] * rcp * (rTi + udT) + N[n] * Se - rcp * tauT * cn * res - (hk + kdcT) * gdT[n]);
+    for (int n = 0; n < 8; ++n) {
+      T N, dN[3], g[3];
+      shape(n, N, dN);
+      grad(dN, g);
+      const T c = fl * (uadv[0] * g[0] + uadv[1] * g[1] + uadv[2] * g[2]);
+      rr[n] = w * (-N * rmass - trq * c * res - HK * (g[0] * dT[0] + g[1] * dT[1] + g[2] * dT[2]));
+      if constexpr (MAT) {
+        const T v[4] = {g[0], g[1], g[2], rcp * (fact1 * N + fact2 * c) - fact2 * dSq * N};
+        store_row<4>(q + 4 * n, v);
+        q[32 + n] = w * (N + trq * c);
       }
-    } else {
-      rec[25] = fact2 * hk * w;
-      rec[26] = rec[27] = rec[28] = 0; rec[30] = 0; rec[31] = 0;
-#pragma unroll
-      for (int n = 0; n < 8; ++n) rt[n] += w * (-N[n] * rcp * rTi - hk * gdT[n]);
     }
-    if constexpr (MAT) store_n(out + gp * L::GPW, rec, L::GPW);
-  }
+    if constexpr (MAT) {
+      q[40] = fact2 * HK * w;
+      __syncwarp();
+      T K[8];
 #pragma unroll
-  for (int n = 0; n < 8; ++n) out[(MAT ? L::RHS0 : 0) + n] = rt[n];
-}
-
-template <typename T, int KIND, bool TC = false, bool MAT = true>
-__global__ void __launch_bounds__(64) hex_element_kernel(const SumArgs a) {
-  using L = HexLay<KIND>;
-  constexpr int SW = !MAT ? 8 * L::NF : TC ? HexTcLay::SW : L::SW;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  double tamax = 0.0;   // the element's largest taua over its points
+      for (int b = 0; b < 8; ++b) K[b] = (T)0;
+#pragma unroll 1
+      for (int k = 0; k < 8; ++k) {   // row gp of the matrix, point k
+        const T* z = eb + k * HT::GPW;
+        T ga[4];
+        lds4(z + 4 * gp, ga);
+        const T A = z[32 + gp], hk2 = z[40];
+        ga[0] *= hk2; ga[1] *= hk2; ga[2] *= hk2;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          T gb[4];
+          lds4(z + 4 * b, gb);
+          K[b] += A * gb[3] + (ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2]);
+        }
+      }
+      if (on) {
+        put4(out + 8 * gp, K[0], K[1], K[2], K[3]);
+        put4(out + 8 * gp + 4, K[4], K[5], K[6], K[7]);
+      }
+    }
+  }
+  hex_sum_nodes<T, NF>(rr, lane);
+  if (on)
+#pragma unroll
+    for (int f = 0; f < NF; ++f) out[RHS0 + NF * gp + f] = rr[f];
+  double cfl = (double)p.delt * sqrt((double)taua);   // the largest over the warp's points
   int nbad = 0;
-  if (t < a.E) {
-    T r[8][16], lo[8][4];
-    const T* rec = reinterpret_cast<const T*>(a.rec);
+  const unsigned bad = __ballot_sync(0xffffffffu, on && !(w > (T)0));
+  // an element counts once
+  for (int e = 0; e < 4; ++e) nbad += ((bad >> (8 * e)) & 0xffu) != 0u;
 #pragma unroll
-    for (int n = 0; n < 8; ++n) load_rec(rec, a.ien[8 * (size_t)t + n], r[n], lo[n]);
-    const bool fluid = __ldg(a.elm_id + t) == a.p.fluid_elm_id;
-    T* out = reinterpret_cast<T*>(a.sum) + (size_t)t * SW;
-    if constexpr (KIND == OVS_ASM_NSVOF) hex_summarize_nsvof<T, TC, MAT>(a.p, r, lo, fluid, out, tamax, nbad);
-    else hex_summarize_tem<T, MAT>(a.p, r, lo, fluid, out, tamax, nbad);
-  }
-  double cfl = (double)a.p.delt * sqrt(tamax);   // as the tet element pass
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    cfl = fmax(cfl, __shfl_xor_sync(0xffffffffu, cfl, off));
-    nbad += __shfl_xor_sync(0xffffffffu, nbad, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
+  for (int off = 16; off > 0; off >>= 1) cfl = fmax(cfl, __shfl_xor_sync(0xffffffffu, cfl, off));
+  if (lane == 0) {
     cfl_max(a.cfl_bits, cfl);
     if (nbad) atomicAdd(a.flags, nbad);
   }
-}
-
-// Entry (row node la, column node b) of a hex temperature matrix from its
-// records, summed over the 8 points.
-template <typename T>
-__device__ __forceinline__ T hex_tem_entry(const ovs_params& p, const T* sm, int la, int b) {
-  using L = HexLay<OVS_ASM_TEM>;
-  const T fact1 = (T)p.almi, fact2 = (T)(p.alfi * p.gami * p.delt);
-  T X = 0;
-  for (int gp = 0; gp < 8; ++gp) {
-    const T* q = sm + gp * L::GPW;
-    const T ga[3] = {q[3 * la], q[3 * la + 1], q[3 * la + 2]};
-    const T gb[3] = {q[3 * b], q[3 * b + 1], q[3 * b + 2]};
-    const T w = q[24], HK = q[25], rcp = q[29], dSe = q[30], trc = q[31];
-    const T uadv[3] = {q[26], q[27], q[28]};
-    const T Na = hex_N<T>(gp, la), Nb = hex_N<T>(gp, b);
-    const T ca = ga[0] * uadv[0] + ga[1] * uadv[1] + ga[2] * uadv[2];
-    const T cb = gb[0] * uadv[0] + gb[1] * uadv[1] + gb[2] * uadv[2];
-    const T aw = w * (Na + trc * ca);
-    X += aw * (rcp * (fact1 * Nb + fact2 * cb) - fact2 * dSe * Nb) + HK * (ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2]);
-  }
-  return X;
 }
 
 // The block (row node a, column node b) of one Gauss point added to o, the
@@ -856,7 +813,7 @@ __global__ void __launch_bounds__(128) hex_rows_kernel(const AsmArgs a) {
 #pragma unroll
           for (int f = 0; f < NF; ++f) rv[f] = sum[(size_t)e * HexTcLay::SW + HexTcLay::RHS0 + 5 * la + f];
         } else {
-          o[0] = hex_tem_entry<T>(a.p, sum + (size_t)e * L::SW, la, bl);
+          o[0] = __ldg(sum + (size_t)e * L::SW + 8 * la + bl);
           rv[0] = sum[(size_t)e * L::SW + L::RHS0 + la];
         }
         T* dst = blk + (jl * 8 + bl) * BSTR;
@@ -979,15 +936,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int LEFT> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
-}
-
-__device__ __forceinline__ void lds4(const float* p, float* d) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-}
-__device__ __forceinline__ void lds4(const double* p, double* d) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
-  d[0] = a.x; d[1] = a.y; d[2] = b.x; d[3] = b.y;
 }
 
 template <typename T>
@@ -1164,7 +1112,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 8 ? 4 : 5)) hex_block_rows_
 template <typename T, int KIND>
 int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int parts) {
   if (!a0.mat) {   // vector-only pass, as for the tets
-    hex_element_kernel<T, KIND, false, false><<<(sa.E + 63) / 64, 64, 0, c->stream>>>(sa);
+    hex_element_kernel<T, KIND, false, false><<<(sa.E + 15) / 16, 128, 0, c->stream>>>(sa);
     ++c->launches;
     OVS_CUDA_TRY(cudaGetLastError());
     return launch_residual_rows<T, HexLay<KIND>::NF>(c, a0, KIND == OVS_ASM_TEM);
@@ -1180,7 +1128,7 @@ int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int pa
   if (parts & 1) {
     if (tc) {
       if constexpr (can_tc) {
-        hex_element_kernel<T, KIND, true><<<(sa.E + 63) / 64, 64, 0, c->stream>>>(sa);
+        hex_element_kernel<T, KIND, true><<<(sa.E + 15) / 16, 128, 0, c->stream>>>(sa);
         ++c->launches;
         OVS_CUDA_TRY(cudaGetLastError());
         HexTcArgs ta;
@@ -1201,7 +1149,7 @@ int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int pa
         }
       }
     } else {
-      hex_element_kernel<T, KIND><<<(sa.E + 63) / 64, 64, 0, c->stream>>>(sa);
+      hex_element_kernel<T, KIND><<<(sa.E + 15) / 16, 128, KIND == OVS_ASM_TEM ? HexTemStage<T>::bytes : 0, c->stream>>>(sa);
       ++c->launches;
       OVS_CUDA_TRY(cudaGetLastError());
     }
