@@ -56,8 +56,7 @@ __device__ __forceinline__ void ld4(const double* p, double v[4]) {
 template <typename A, typename B, bool ACC64> struct AccT { using type = double; };
 template <> struct AccT<float, float, false> { using type = float; };
 
-// MODE 0: y = A x ; MODE 1: y = P^-1 A x (times *scale, if given) ; MODE 2:
-// y = b - A x
+// MODE 0: y = A x ; MODE 1: y = P^-1 A x ; MODE 2: y = b - A x
 // Block systems: NG groups of 4 values per slot, one lane per group.
 //   NS   (NG=4): groups rows u1,u2,u3,p over columns (u1,u2,u3,p)
 //   NSVOF(NG=6): + row phi over (u1,u2,u3,phi), + column phi into (u1,u2,u3,p)
@@ -71,8 +70,7 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
                                                 const int* __restrict__ colidx, const TM* __restrict__ vals,
                                                 const TX* __restrict__ x, TY* __restrict__ y,
                                                 const TM* __restrict__ pre, const double* __restrict__ b,
-                                                const int* __restrict__ rows = nullptr, long nrows = 0,
-                                                const double* __restrict__ scale = nullptr) {
+                                                const int* __restrict__ rows = nullptr, long nrows = 0) {
   using AT = typename AccT<TM, TX, ACC64>::type;
   constexpr int NV = 4 * NG;
   constexpr int RPW = 32 / NG;  // rows per warp
@@ -175,7 +173,6 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
     } else {
       z = yv * (AT)pre[(size_t)10 * N + row];
     }
-    if (scale) z *= (AT)__ldg(scale);
   } else if (MODE == 2) {
     z = (AT)b[(size_t)g * N + row] - yv;
   }
@@ -187,10 +184,10 @@ __global__ void __launch_bounds__(SPMV_THREADS)
 spmv_block_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                   const TM* __restrict__ vals, const TX* __restrict__ x, TY* __restrict__ y,
                   const TM* __restrict__ pre, const double* __restrict__ b,
-                  const int* __restrict__ done, const double* __restrict__ scale) {
+                  const int* __restrict__ done) {
   if (done && *done) return;
   const long wglob = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  spmv_block_warp<NG, TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b, nullptr, 0, scale);
+  spmv_block_warp<NG, TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b);
 }
 
 // the same product over a list of rows (a partition's interior or boundary
@@ -211,8 +208,7 @@ __device__ __forceinline__ void spmv_scalar_warp(long wglob, int N, const int* _
                                                  const int* __restrict__ colidx, const TM* __restrict__ vals,
                                                  const TX* __restrict__ x, TY* __restrict__ y,
                                                  const TM* __restrict__ pre, const double* __restrict__ b,
-                                                 const int* __restrict__ rows = nullptr, long nrows = 0,
-                                                 const double* __restrict__ scale = nullptr) {
+                                                 const int* __restrict__ rows = nullptr, long nrows = 0) {
   using AT = typename AccT<TM, TX, ACC64>::type;
   const int lane = threadIdx.x & 31;
   const int sub = lane >> 3, k = lane & 7;
@@ -237,12 +233,8 @@ __device__ __forceinline__ void spmv_scalar_warp(long wglob, int N, const int* _
   a += __shfl_xor_sync(0xffffffffu, a, 1);
   if (!active || k != 0) return;
   AT z = a;
-  if (MODE == 1) {
-    z = a * (AT)pre[row];
-    if (scale) z *= (AT)__ldg(scale);
-  } else if (MODE == 2) {
-    z = (AT)b[row] - a;
-  }
+  if (MODE == 1) z = a * (AT)pre[row];
+  else if (MODE == 2) z = (AT)b[row] - a;
   y[row] = (TY)z;
 }
 
@@ -251,10 +243,10 @@ __global__ void __launch_bounds__(SPMV_THREADS)
 spmv_scalar_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                    const TM* __restrict__ vals, const TX* __restrict__ x, TY* __restrict__ y,
                    const TM* __restrict__ pre, const double* __restrict__ b,
-                   const int* __restrict__ done, const double* __restrict__ scale) {
+                   const int* __restrict__ done) {
   if (done && *done) return;
   const long wglob = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  spmv_scalar_warp<TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b, nullptr, 0, scale);
+  spmv_scalar_warp<TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b);
 }
 
 template <typename TM, typename TX, typename TY, int MODE>
@@ -292,7 +284,7 @@ int launch_spmv_rows(ovs_ctx* c, int sys, const TM* vals, const double* x, doubl
 
 template <typename TM, typename TX, typename TY, int MODE, bool ACC64 = true>
 int launch_spmv(ovs_ctx* c, int sys, const TM* vals, const TX* x, TY* y, const TM* pre,
-                const double* b, const int* done, const double* scale = nullptr) {
+                const double* b, const int* done) {
   const int N = c->N;
   int rpw = sys == OVS_SYS_NS ? 8 : (sys == OVS_SYS_NSVOF ? 5 : 4);
   long warps = ((long)N + rpw - 1) / rpw;
@@ -300,19 +292,19 @@ int launch_spmv(ovs_ctx* c, int sys, const TM* vals, const TX* x, TY* y, const T
   if (sys == OVS_SYS_NS)
     {
       spmv_block_kernel<4, TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
-          N, c->rowptr, c->colidx, vals, x, y, pre, b, done, scale);
+          N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
       ++c->launches;
     }
   else if (sys == OVS_SYS_NSVOF)
     {
       spmv_block_kernel<6, TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
-          N, c->rowptr, c->colidx, vals, x, y, pre, b, done, scale);
+          N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
       ++c->launches;
     }
   else
     {
       spmv_scalar_kernel<TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
-          N, c->rowptr, c->colidx, vals, x, y, pre, b, done, scale);
+          N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
       ++c->launches;
     }
   OVS_CUDA_TRY(cudaGetLastError());
@@ -465,7 +457,7 @@ gm_start_kernel(int N, int nf, int sys, const double* __restrict__ rhs, const TM
     gm->e[0] = un;
     gm->sc[0] = 1.0;
     gm->iks = 0;
-    gm->done = (un == 0.0) ? 1 : 0;
+    gm->done = (un == 0.0) ? -1 : 0;
     gm->breakdown = (un == 0.0) ? 1 : 0;
     gm->converged = (un == 0.0) ? 1 : 0;
     gm->ercheck = un;
@@ -515,15 +507,20 @@ gm_normalize_kernel(const TW* w, TV* v, size_t n, GmresDev* gm, int first) {
   for (size_t i = 4 * n4 + t0; i < n; i += stride) v[i] = (TV)((double)w[i] / d);
 }
 
-// H(k+1,k) = unorm, Givens rotations of column k (Hk[0..k), rotated in
-// place; cs, sn: the earlier rotations), e update, exit test
-// (SparseGMRES_NS.f90:289-327); one thread
-__device__ void givens_step(GmresDev* gm, int k, double unorm, double* Hk, const double* cs, const double* sn) {
+// H(k+1,k) = unorm, Givens rotations of column k (Hk[0..k) in, its rotated form
+// out in Ho; cs, sn: the earlier rotations; ek: e(k)), e update, exit test
+// (SparseGMRES_NS.f90:289-327); one thread.  The arrays do not overlap, so that
+// the loads of several rotations go ahead of the chain.
+__device__ void givens_step(GmresDev* gm, int k, double unorm, const double* __restrict__ Hk, double* __restrict__ Ho,
+                            const double* __restrict__ cs, const double* __restrict__ sn, double ek) {
+  const double epsnrm = gm->epsnrm;
+  const int kmin = gm->kmin, kspace = gm->kspace;
   double cur = Hk[0];
+#pragma unroll 8
   for (int jk = 1; jk <= k - 1; ++jk) {
-    const double nxt = Hk[jk];
-    Hk[jk - 1] = cs[jk - 1] * cur + sn[jk - 1] * nxt;
-    cur = -sn[jk - 1] * cur + cs[jk - 1] * nxt;
+    const double nxt = Hk[jk], c = cs[jk - 1], q = sn[jk - 1];
+    Ho[jk - 1] = c * cur + q * nxt;
+    cur = -q * cur + c * nxt;
   }
   const double a = cur, b = unorm;
   const double tmp = sqrt(a * a + b * b);
@@ -532,28 +529,27 @@ __device__ void givens_step(GmresDev* gm, int k, double unorm, double* Hk, const
     // v_1..v_{k-1}): the rotation would be 0/0 and the reference carries NaN
     // on; the cycle ends with the solution of the first k-1 columns
     gm->iks = k - 1;
-    gm->ercheck = fabs(gm->e[k - 1]);
-    gm->done = 1;
-    gm->converged = gm->ercheck <= gm->epsnrm;
+    gm->ercheck = fabs(ek);
+    gm->done = k;
+    gm->converged = fabs(ek) <= epsnrm;
     gm->breakdown = 1;
     return;
   }
   const double c = a / tmp, sg = b / tmp;
   gm->cs[k - 1] = c;
   gm->sn[k - 1] = sg;
-  Hk[k - 1] = tmp;
-  const double ek = gm->e[k - 1];
-  gm->e[k - 1] = c * ek + sg * gm->e[k];
-  const double en = -sg * ek + c * gm->e[k];
+  Ho[k - 1] = tmp;
+  gm->e[k - 1] = c * ek;   // e(k+1) was 0
+  const double en = -sg * ek;
   gm->e[k] = en;
   const double er = fabs(en);
   gm->ercheck = er;
   gm->iks = k;
-  const bool conv = (er <= gm->epsnrm) && (k >= gm->kmin);
+  const bool conv = (er <= epsnrm) && (k >= kmin);
   const bool brk = unorm == 0.0;  // exact breakdown; NaN propagates as in the reference
-  if (conv || brk || k >= gm->kspace) {
-    gm->done = 1;
-    gm->converged = er <= gm->epsnrm;
+  if (conv || brk || k >= kspace) {
+    gm->done = k;
+    gm->converged = er <= epsnrm;
     gm->breakdown = brk;
   }
 }
@@ -651,7 +647,9 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     gm->sc[k] = 1.0;
-    givens_step(gm, k, unorm, gm->H + (size_t)(k - 1) * (gm->kspace + 1), gm->cs, gm->sn);
+    double* Hk = gm->H + (size_t)(k - 1) * (gm->kspace + 1);
+    givens_step(gm, k, unorm, Hk, gm->y, gm->cs, gm->sn, gm->e[k - 1]);   // (y is free until the cycle ends)
+    for (int j = 0; j < k; ++j) Hk[j] = gm->y[j];
   }
 }
 
@@ -667,14 +665,20 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
 // residual algorithms", 2021).  T = (I + L)^-1 grows by a row per step.
 //   phase A  every v_j is read once, for both dots (FP64 products and sums);
 //   barrier  every block adds the partial dots in the same order and forms h;
-//   phase B  w -= sum_j h_j v_j and |w|^2, the last block to finish adds the
-//            norm and does the Givens step and T's new row.
-// w stays unnormalized: gm->sc[j] = 1 / |w| belongs to slot j, and the SpMV
-// (linear in its vector), the dots and the coefficients carry it, which
-// saves the barrier and the pass over w that a division would need.
+//   phase B  w -= sum_j h_j v_j and the partial sums of |w|^2.
+// What the step leaves over is done where nothing waits for it: block G, beside
+// the others' phase A, finishes the step before (norm, Givens rotations, exit
+// test) and adds the row of T that the next step will use (the newest two rows
+// of the triangular solve are done directly); every other block adds the norm
+// partials itself.  w stays unnormalized: gm->sc[j] = 1 / |w| belongs to slot j,
+// and the product (linear in its vector), the dots and the coefficients carry
+// it, which saves the barrier and the pass over w that a division would need.
 // Each basis vector is read twice per step, as in MGS; the bound is that
 // traffic (two vectors a step at 6.4 TB/s) for long vectors and the chain
-// launch - dots - barrier - h - update - tail for short ones.
+// launch - dots - barrier - h - update for short ones.  Per iteration at k = 25
+// (FP64, SpMV included; in brackets with the leftovers before the barrier of
+// the same step): 4.9K nodes 21 us (28), 31K nodes 54 (57), 236K nodes 0.207 ms
+// (0.213), 2.1M nodes 1.78 ms (1.80).
 //
 // A warp owns sub-chunks of 32 V values.  Phase A takes JG vectors at a
 // time: all their loads in flight, 2 JG sums per lane, reduced over the
@@ -687,10 +691,10 @@ constexpr int ORTH_THREADS = 512;
 constexpr int ORTH_WARPS = ORTH_THREADS / 32;
 constexpr int JG = 8;
 
-// V values at index i (a multiple of V), zero at and beyond n.  Plain loads:
-// the slot being orthogonalized is rewritten by the thread that reads it.
+// V values at index i (a multiple of V), zero at and beyond n (plain loads: the
+// slot being orthogonalized is rewritten by the same thread)
 template <int V, typename TV>
-__device__ __forceinline__ void orth_ld(const TV* __restrict__ p, size_t i, size_t n, TV (&x)[V]) {
+__device__ __forceinline__ void orth_ld(const TV* p, size_t i, size_t n, TV (&x)[V]) {
   if (V == 4 && i + 4 <= n) {
     if constexpr (V == 4 && sizeof(TV) == 8) {
       asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p + i));
@@ -725,43 +729,127 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// shared memory of a step: the warps' sums (2 kk each), a, g, h, h sc, cs, sn
+// shared memory of a step: the warps' sums (2 kk each), a, g, g of the step
+// before, h, h sc, sc
 inline size_t orth_smem(int k) {
   const size_t kk = ((size_t)k + JG - 1) / JG * JG;
   return sizeof(double) * ((2 * ORTH_WARPS + 6) * kk + 2);
 }
 
+// four sums over the lanes at a time (their chains overlap)
+__device__ __forceinline__ void warp_sum4(double (&v)[4]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] += __shfl_xor_sync(0xffffffffu, v[u], o);
+}
+
+// the sum of G values by one warp, all its loads in flight (G <= 160: one
+// block per SM), the same on every block
+__device__ __forceinline__ double warp_gather(const double* p, int G, int lane) {
+  double s[5], t = 0.0;
+#pragma unroll
+  for (int u = 0; u < 5; ++u) s[u] = lane + 32 * u < G ? __ldcg(p + lane + 32 * u) : 0.0;
+  for (int q = lane + 160; q < G; q += 32) t += __ldcg(p + q);
+#pragma unroll
+  for (int u = 0; u < 5; ++u) t += s[u];
+  return warp_sum(t);
+}
+
+// part: partial norms (G) and dots with v_k (kspace) of step k and the step
+// before, by the parity of k, then [2 k - 1][G] partial dots
+__device__ __forceinline__ void orth_part(double* part, int k, int G, int ks, double*& nrm, double*& gsave) {
+  nrm = part + (size_t)(k & 1) * (G + ks);
+  gsave = nrm + G;
+}
+
+// What step k leaves over, by one block (sm: 12 k values of shared memory): the
+// norm of slot k, the Givens rotations of column k and the exit test (one
+// thread, its data staged in shared memory), and, by the other warps, row k - 1
+// of T from the dots of v_k with the vectors before it.
+__device__ void finish_step(GmresDev* gm, int k, double* part, int G, double* T, double* sm) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, ks = gm->kspace;
+  double *acc = sm, *Hs = acc + 8 * k, *cs = Hs + k, *sn = cs + k, *Ho = sn + k, *nrm, *gk;
+  orth_part(part, k, G, ks, nrm, gk);
+  double* Hk = gm->H + (size_t)(k - 1) * (ks + 1);
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    Hs[j] = __ldcg(Hk + j);
+    if (j < k - 1) { cs[j] = __ldcg(gm->cs + j); sn[j] = __ldcg(gm->sn + j); }
+  }
+  __shared__ double total;
+  const double ek = threadIdx.x == 0 ? __ldcg(gm->e + (k - 1)) : 0.0;
+  if (wid == 0) {
+    const double t = warp_gather(nrm, G, lane);
+    if (lane == 0) total = t;
+  }
+  __syncthreads();
+  const int cols = k - 1, nt = blockDim.x - 32, parts = cols ? max(1, min(8, nt / cols)) : 0;
+  if (threadIdx.x == 0) {
+    const double unorm = sqrt(total);
+    gm->beta = total;
+    gm->sc[k] = unorm != 0.0 ? 1.0 / unorm : 1.0;
+    givens_step(gm, k, unorm, Hs, Ho, cs, sn, ek);
+  } else if (wid > 0) {
+    // t_c = -(g_c + sum_{j>c} g_j T_jc), T's diagonal being 1; up to eight
+    // threads share a column's sum
+    for (int u = threadIdx.x - 32; u < cols * parts; u += nt) {
+      const int q = u / cols, c = u - q * cols;
+      double s = q == 0 ? __ldcg(gk + c) : 0.0;
+#pragma unroll 4
+      for (int j = c + 1 + q; j < cols; j += parts) s += __ldcg(gk + j) * __ldcg(T + (size_t)j * ks + c);
+      acc[u] = s;
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += blockDim.x) Hk[j] = Ho[j];
+  for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+    double s = 0.0;
+    for (int q = 0; q < parts; ++q) s += acc[q * cols + c];
+    T[(size_t)(k - 1) * ks + c] = -s;
+  }
+}
+
+// Step k by the blocks b < G of the grid (blockIdx G is finish_step's; it takes
+// part in the barrier).
+// part: partial norms (G) and dots with v_k (kspace) of step k and the step
+// before, by the parity of k, then [2 k - 1][G] partial dots.
 template <typename TV, int V>
-__global__ void __launch_bounds__(ORTH_THREADS, 1)
-gm_orthog_kernel(TV* basis, size_t ld, size_t n, int k, GmresDev* gm, double* part, double* T, int nsc, int js) {
-  cg::grid_group grid = cg::this_grid();
-  if (gm->done) return;
-  extern __shared__ __align__(16) double orth_sm[];
+__device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_t ld, size_t n, int k, int ks,
+                                          GmresDev* gm, double* part, double* T, int nsc, int js, double* orth_sm) {
   __shared__ double sh[ORTH_WARPS];
-  __shared__ int is_last;
   const int kk = (k + JG - 1) / JG * JG, ncol = 2 * k - 1;   // columns: k dots with w, k - 1 with v_k
   double* acc = orth_sm;                    // [ORTH_WARPS][2 kk]
   double* as = acc + 2 * ORTH_WARPS * kk;   // V^T w
-  double* gs = as + kk;                     // row k of L
-  double* hh = gs + kk;                     // the coefficients
+  double* gs = as + kk;                     // v_k . v_j
+  double* gp = gs + kk;                     // v_{k-1} . v_j
+  double* hh = gp + kk;                     // the coefficients
   double* hs = hh + kk;                     // times the slots' scales
-  double* cs = hs + kk;
-  double* sn = cs + kk;
+  double* sc = hs + kk;                     // the slots' scales
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int G = gridDim.x, b = blockIdx.x, W = G * ORTH_WARPS;
+  const int G = gridDim.x - 1, b = blockIdx.x, W = G * ORTH_WARPS;
+  double *nrm, *gsave;
+  orth_part(part, k, G, ks, nrm, gsave);
+  double *nrm1, *gsave1;                    // of the step before
+  orth_part(part, k - 1, G, ks, nrm1, gsave1);
+  double* col = part + 2 * (G + ks);
   const int gw = wid * G + b;               // short vectors spread over the blocks first
   const TV* vk = basis + ld * (size_t)(k - 1);
   TV* w = basis + ld * (size_t)k;
-  double* nrm = part;                       // G partial norms
-  double* col = part + G;                   // [ncol][G] partial dots
   double* my = acc + 2 * kk * wid;
   for (int c = lane; c < 2 * kk; c += 32) my[c] = 0.0;
+  // the scales and the older dots travel while phase A runs
+  const int t = threadIdx.x;
+  const double sct = t < k - 1 ? __ldcg(gm->sc + t) : 0.0, gpt = t < k - 2 ? __ldcg(gsave1 + t) : 0.0;
+  if (wid == ORTH_WARPS - 1) {              // 1 / |v_k| from the norm partials
+    const double u = k > 1 ? sqrt(warp_gather(nrm1, G, lane)) : 1.0;
+    if (lane == 0) sc[k - 1] = u != 0.0 ? 1.0 / u : 1.0;
+  }
   __syncwarp();
   // ---- phase A
   const int slot = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
   for (long it = gw; it < (long)nsc * js; it += W) {
-    const int sc = (int)(it / js), jj = (int)(it - (long)sc * js);
-    const size_t i = ((size_t)sc * 32 + lane) * V;
+    const int si = (int)(it / js), jj = (int)(it - (long)si * js);
+    const size_t i = ((size_t)si * 32 + lane) * V;
     TV wv[V], kv[V];
     orth_ld<V>(w, i, n, wv);
     orth_ld<V>(vk, i, n, kv);
@@ -783,6 +871,8 @@ gm_orthog_kernel(TV* basis, size_t ld, size_t n, int k, GmresDev* gm, double* pa
       if (!(lane & 1)) my[(slot < JG ? 0 : kk - JG) + j0 + slot] += s;
     }
   }
+  if (t < k - 1) sc[t] = sct;
+  if (t < k - 2) gp[t] = gpt;
   __syncthreads();
   for (int c = threadIdx.x; c < ncol; c += ORTH_THREADS) {
     const int o = c < k ? c : kk + c - k;
@@ -792,68 +882,101 @@ gm_orthog_kernel(TV* basis, size_t ld, size_t n, int k, GmresDev* gm, double* pa
     col[(size_t)c * G + b] = s;
   }
   grid.sync();
+  const int done = *(volatile int*)&gm->done;   // the step before may have ended the cycle
   // ---- the dots, added over the blocks in the same order everywhere (four
   // columns of a warp's share in flight)
-  const double sk = gm->sc[k - 1];
+  const double sk = sc[k - 1];
   for (int c0 = wid; c0 < ncol; c0 += 4 * ORTH_WARPS) {
-    double s[4];
+    double s[4][5];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int c = c0 + u * ORTH_WARPS;
-      s[u] = 0.0;
-      if (c < ncol)
-        for (int q = lane; q < G; q += 32) s[u] += __ldcg(col + (size_t)c * G + q);
+      const int c = min(c0 + u * ORTH_WARPS, ncol - 1);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) s[u][v] = lane + 32 * v < G ? __ldcg(col + (size_t)c * G + lane + 32 * v) : 0.0;
     }
+    double r[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int c = c0 + u * ORTH_WARPS;
-      const double t = warp_sum(s[u]);
-      if (lane == 0 && c < ncol) {
-        if (c < k) as[c] = t * gm->sc[c];
-        else gs[c - k] = t * sk * gm->sc[c - k];
-      }
+      r[u] = 0.0;
+      for (int q = lane + 160; q < G; q += 32) r[u] += __ldcg(col + (size_t)min(c0 + u * ORTH_WARPS, ncol - 1) * G + q);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) r[u] += s[u][v];
+    }
+    warp_sum4(r);
+    if (lane < 4) {
+      const double v = (lane & 2) ? ((lane & 1) ? r[3] : r[2]) : ((lane & 1) ? r[1] : r[0]);
+      const int c = c0 + lane * ORTH_WARPS;
+      if (c < k) as[c] = v * sk * sc[c];
+      else if (c < ncol) gs[c - k] = v * sk * sc[c - k];
     }
   }
+  if (done) return;
   __syncthreads();
-  // ---- h = T V^T w (rows 0..k-2 of T; the last row is direct)
-  const int ks = gm->kspace;
-  for (int j0 = wid; j0 < k - 1; j0 += 4 * ORTH_WARPS) {
+  // ---- h = T V^T w for rows 0..k-3 of T; the last two rows are direct
+  // (four rows of a warp's share in flight)
+  for (int j0 = wid; j0 < k - 2; j0 += 4 * ORTH_WARPS) {
     double s[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int j = j0 + u * ORTH_WARPS;
-      s[u] = 0.0;
-      if (j < k - 1)
-        for (int c = lane; c < j; c += 32) s[u] += __ldcg(T + (size_t)j * ks + c) * as[c];
+      const bool in0 = j < k - 2 && lane < j, in1 = j < k - 2 && lane + 32 < j;
+      const double* Tj = T + (size_t)j * ks + lane;
+      const double x0 = in0 ? __ldcg(Tj) : 0.0, x1 = in1 ? __ldcg(Tj + 32) : 0.0;
+      s[u] = (in0 ? x0 * as[lane] : 0.0) + (in1 ? x1 * as[lane + 32] : 0.0);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int j = j0 + u * ORTH_WARPS;
-      const double t = warp_sum(s[u]);
-      if (lane == 0 && j < k - 1) {
-        hh[j] = as[j] + t;
-        hs[j] = hh[j] * gm->sc[j];
+      if (j < k - 2)
+        for (int c = lane + 64; c < j; c += 32) s[u] += __ldcg(T + (size_t)j * ks + c) * as[c];
+    }
+    warp_sum4(s);
+    if (lane < 4) {
+      const double v = (lane & 2) ? ((lane & 1) ? s[3] : s[2]) : ((lane & 1) ? s[1] : s[0]);
+      const int j = j0 + lane * ORTH_WARPS;
+      if (j < k - 2) {
+        hh[j] = as[j] + v;
+        hs[j] = hh[j] * sc[j];
       }
     }
   }
   __syncthreads();
   if (wid == 0) {
-    double t = 0.0;
-    for (int j = lane; j < k - 1; j += 32) t += gs[j] * hh[j];
-    t = warp_sum(t);
+    double t1 = 0.0, t2 = 0.0;
+    for (int j = lane; j < k - 2; j += 32) { t1 += gp[j] * hh[j]; t2 += gs[j] * hh[j]; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+    }
     if (lane == 0) {
-      hh[k - 1] = as[k - 1] - t;
+      if (k > 1) {
+        const double h = as[k - 2] - t1;
+        hh[k - 2] = h;
+        hs[k - 2] = h * sc[k - 2];
+        t2 += gs[k - 2] * h;
+      }
+      hh[k - 1] = as[k - 1] - t2;
       hs[k - 1] = hh[k - 1] * sk;
     }
   }
   __syncthreads();
+  if (b == 0) {   // for finish_step and the next step
+    for (int j = threadIdx.x; j < k; j += ORTH_THREADS) {
+      gm->H[(size_t)(k - 1) * (ks + 1) + j] = hh[j];
+      if (j < k - 1) gsave[j] = gs[j];
+    }
+  }
   // ---- phase B: the update and its norm
   double na = 0.0;
+  const TV skv = (TV)sk;
   const int cnt = gw < nsc ? (nsc - gw + W - 1) / W : 0;
   for (int r = cnt - 1; r >= 0; --r) {
     const size_t i = ((size_t)(gw + (long)r * W) * 32 + lane) * V;
     TV wv[V];
     orth_ld<V>(w, i, n, wv);
+#pragma unroll
+    for (int q = 0; q < V; ++q) wv[q] *= skv;
     constexpr int JB = V == 1 ? 2 * JG : JG;
     for (int j0 = 0; j0 < k; j0 += JB) {
       TV x[JB][V];
@@ -886,66 +1009,51 @@ gm_orthog_kernel(TV* basis, size_t ld, size_t n, int k, GmresDev* gm, double* pa
     double s = 0.0;
     for (int q = 0; q < ORTH_WARPS; ++q) s += sh[q];
     nrm[b] = s;
-    __threadfence();
-    is_last = atomicAdd(&gm->counter, 1) == G - 1;
   }
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  // ---- the last block: norm, Givens rotations (one thread, its data staged
-  // in shared memory) and the new row of T (the other warps)
-  double* Hk = gm->H + (size_t)(k - 1) * (ks + 1);
-  for (int j = threadIdx.x; j < k - 1; j += ORTH_THREADS) { cs[j] = gm->cs[j]; sn[j] = gm->sn[j]; }
-  if (wid == 0) {
-    double s = 0.0;
-    for (int q = lane; q < G; q += 32) s += __ldcg(nrm + q);
-    s = warp_sum(s);
-    if (lane == 0) sh[0] = s;
+}
+
+// one step per launch (after the SpMV that wrote slot k)
+template <typename TV, int V>
+__global__ void __launch_bounds__(ORTH_THREADS, 1)
+gm_orthog_kernel(TV* basis, size_t ld, size_t n, int k, GmresDev* gm, double* part, double* T, int nsc, int js) {
+  cg::grid_group grid = cg::this_grid();
+  // ended by a step before the one that block G finishes here (the same answer
+  // on every block, whenever it starts)
+  const int ended = *(volatile int*)&gm->done;
+  if (ended != 0 && ended < k - 1) return;
+  extern __shared__ __align__(16) double orth_sm[];
+  const int G = gridDim.x - 1;
+  if (blockIdx.x == G) {
+    if (k > 1) finish_step(gm, k - 1, part, G, T, orth_sm);
+    grid.sync();
+    return;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double unorm = sqrt(sh[0]);
-    gm->counter = 0;
-    gm->beta = sh[0];
-    gm->sc[k] = unorm != 0.0 ? 1.0 / unorm : 1.0;
-    givens_step(gm, k, unorm, hh, cs, sn);
-  } else if (wid > 0 && k > 1) {
-    // t_c = -(g_c + sum_{j>c} g_j T_jc), T's diagonal being 1; up to eight
-    // threads share a column's sum
-    const int cols = k - 1, t = threadIdx.x - 32, parts = max(1, min(8, (ORTH_THREADS - 32) / cols));
-    for (int u = t; u < cols * parts; u += ORTH_THREADS - 32) {
-      const int q = u / cols, c = u - q * cols;
-      double s = q == 0 ? gs[c] : 0.0;
-#pragma unroll 4
-      for (int j = c + 1 + q; j < cols; j += parts) s += gs[j] * __ldcg(T + (size_t)j * ks + c);
-      acc[u] = s;
-    }
-  }
-  __syncthreads();
-  for (int j = threadIdx.x; j < k; j += ORTH_THREADS) Hk[j] = hh[j];
-  const int parts = k > 1 ? max(1, min(8, (ORTH_THREADS - 32) / (k - 1))) : 0;
-  for (int c = threadIdx.x; c < k - 1; c += ORTH_THREADS) {
-    double s = 0.0;
-    for (int q = 0; q < parts; ++q) s += acc[q * (k - 1) + c];
-    T[(size_t)(k - 1) * ks + c] = -s;
-  }
+  orth_step<TV, V>(grid, basis, ld, n, k, gm->kspace, gm, part, T, nsc, js, orth_sm);
 }
 
 // back-substitution (SparseGMRES_NS.f90:341-346): one block, thread l holds
 // e(l); the columns of H are loaded eight at a time ahead of the steps that
-// use them.  y_j comes out times the scale of slot j.
+// use them.  y_j comes out times the scale of slot j.  A cycle that ran all its
+// steps first finishes the last one (part, T, G: of gm_orthog_kernel).
 constexpr int BACKSUB_THREADS = 416;
 static_assert(BACKSUB_THREADS >= OVS_MAX_KSPACE, "one thread per unknown");
-__global__ void __launch_bounds__(BACKSUB_THREADS) gm_backsub_kernel(GmresDev* gm) {
+__global__ void __launch_bounds__(BACKSUB_THREADS) gm_backsub_kernel(GmresDev* gm, double* part, double* T, int G) {
   __shared__ double ys;
-  const int iks = gm->iks, ld = gm->kspace + 1, t = threadIdx.x;
-  double e = t < iks ? gm->e[t] : 0.0;
+  extern __shared__ __align__(16) double bs_sm[];
+  if (!gm->done) {
+    const int k = gm->kspace;
+    finish_step(gm, k, part, G, T, bs_sm);
+    __threadfence();
+    __syncthreads();
+  }
+  const int iks = *(volatile int*)&gm->iks, ld = gm->kspace + 1, t = threadIdx.x;
+  double e = t < iks ? __ldcg(gm->e + t) : 0.0;
   for (int j1 = iks; j1 > 0; j1 -= 8) {
     double h[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int j = j1 - 1 - u;
-      h[u] = j >= 0 && t <= j ? gm->H[(size_t)j * ld + t] : 0.0;
+      h[u] = j >= 0 && t <= j ? __ldcg(gm->H + (size_t)j * ld + t) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -954,7 +1062,7 @@ __global__ void __launch_bounds__(BACKSUB_THREADS) gm_backsub_kernel(GmresDev* g
       if (t == j) ys = e / h[u];
       __syncthreads();
       const double y = ys;
-      if (t == j) gm->y[j] = y * gm->sc[j];
+      if (t == j) gm->y[j] = y * __ldcg(gm->sc + j);
       else if (t < j) e = e - y * h[u];
       __syncthreads();
     }
@@ -1048,8 +1156,9 @@ template <typename TM, typename TV, bool ACC64>
 int plan_arnoldi(ovs_ctx* c, int sys, size_t n, int kspace, bool want_fused, ArnoldiPlan* pl) {
   int st;
   // the partial sums (fused variant: two per block; gm_orthog_kernel: 2 k per
-  // block), then T, kspace x kspace; kept by the context, grown when needed
-  const size_t parts = std::max((size_t)2 * OVS_COOP_MAX_BLOCKS, (size_t)2 * kspace * c->num_sms);
+  // block and two rows of dots), then T, kspace x kspace; kept by the context,
+  // grown when needed
+  const size_t parts = std::max((size_t)2 * OVS_COOP_MAX_BLOCKS, (size_t)2 * (kspace + 1) * (c->num_sms + 1));
   const size_t need = sizeof(double) * (parts + (size_t)kspace * kspace);
   if (c->coop_bytes < need) {
     if (c->coop_part) cudaFree(c->coop_part);
@@ -1069,10 +1178,11 @@ int plan_arnoldi(ovs_ctx* c, int sys, size_t n, int kspace, bool want_fused, Arn
     int per_sm = 0;
     OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ORTH_THREADS, bytes));
-    if (per_sm >= 1 && nsc < ((size_t)1 << 31)) {
+    if (per_sm >= 1 && c->num_sms >= 2 && nsc < ((size_t)1 << 31)) {
       pl->nsc = (int)nsc;
       const long items = (long)nsc * orth_split(*pl, kspace, c->num_sms);
-      pl->grid = (int)std::min((long)c->num_sms, (items + ORTH_WARPS - 1) / ORTH_WARPS);
+      // one SM is left for the block that finishes the step before
+      pl->grid = (int)std::min((long)c->num_sms - 1, (items + ORTH_WARPS - 1) / ORTH_WARPS);
       return OVS_OK;
     }
     pl->fused = true;
@@ -1103,13 +1213,13 @@ int launch_arnoldi(ovs_ctx* c, int sys, const ArnoldiPlan& pl, const TM* vals, c
     return OVS_OK;
   }
   int st = launch_spmv<TM, TV, TV, 1, ACC64>(c, sys, vals, V + ld * (size_t)(k - 1), V + ld * (size_t)k, pre,
-                                               nullptr, &gm->done, gm->sc + (k - 1));
+                                               nullptr, &gm->done);
   if (st) return st;
   int kk = k, nsc = pl.nsc, js = orth_split(pl, k, c->num_sms);
   size_t ldv = ld, nn = n;
   double* T = pl.T;
   void* args[] = {&V, &ldv, &nn, &kk, &gm, &part, &T, &nsc, &js};
-  OVS_CUDA_TRY(cudaLaunchCooperativeKernel((void*)orthog_kernel<TV>(pl.wide), pl.grid, ORTH_THREADS, args,
+  OVS_CUDA_TRY(cudaLaunchCooperativeKernel((void*)orthog_kernel<TV>(pl.wide), pl.grid + 1, ORTH_THREADS, args,
                                            orth_smem(k), c->stream));
   ++c->launches;
   return OVS_OK;
@@ -1170,7 +1280,7 @@ int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol,
       if (c->h_pinned[(q - 1) & 1]) break;
     }
   }
-  gm_backsub_kernel<<<1, BACKSUB_THREADS, 0, s>>>(gm);
+  gm_backsub_kernel<<<1, BACKSUB_THREADS, sizeof(double) * 12 * kspace, s>>>(gm, c->coop_part, pl.T, pl.grid);
   ++c->launches;
   gm_update_kernel<TV><<<ovs_grid(n, 256, 8 * c->num_sms), 256, 0, s>>>(sol, V, n, ld, gm);
   ++c->launches;
@@ -1236,6 +1346,7 @@ int profile_krylov_t(ovs_ctx* c, int what, int sys, int reps, double* ms) {
   ArnoldiPlan pl;
   if ((st = plan_arnoldi<TM, TM, ACC64>(c, sys, n, kspace, what == OVS_PROF_ARNOLDI_FUSED, &pl))) return st;
   OVS_CUDA_TRY(cudaMemsetAsync(pl.T, 0, sizeof(double) * kspace * kspace, c->stream));
+  fill_kernel<double><<<1, 256, 0, c->stream>>>(c->coop_part, 2 * ((size_t)pl.grid + kspace), 1.0);   // a norm before
   auto run = [&]() -> int {
     if (what == OVS_PROF_SPMV) {
       st = launch_spmv<TM, TM, TM, 1, ACC64>(c, sys, vals, V, V + ld, pre, nullptr, nullptr);

@@ -43,7 +43,7 @@ struct GmresDev {
   double unorm0;      // |P^-1 b|
   double ercheck;
   int iks;            // iterations completed
-  int done;           // cycle finished (converged, breakdown or kspace)
+  int done;           // the step that ended the cycle (converged, breakdown or kspace), -1: a zero start; 0: running
   int breakdown;
   int converged;
   int kspace, kmin;
