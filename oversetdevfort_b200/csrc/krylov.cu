@@ -1347,6 +1347,7 @@ int profile_krylov_t(ovs_ctx* c, int what, int sys, int reps, double* ms) {
   if ((st = plan_arnoldi<TM, TM, ACC64>(c, sys, n, kspace, what == OVS_PROF_ARNOLDI_FUSED, &pl))) return st;
   OVS_CUDA_TRY(cudaMemsetAsync(pl.T, 0, sizeof(double) * kspace * kspace, c->stream));
   fill_kernel<double><<<1, 256, 0, c->stream>>>(c->coop_part, 2 * ((size_t)pl.grid + kspace), 1.0);   // a norm before
+  ++c->launches;
   auto run = [&]() -> int {
     if (what == OVS_PROF_SPMV) {
       st = launch_spmv<TM, TM, TM, 1, ACC64>(c, sys, vals, V, V + ld, pre, nullptr, nullptr);

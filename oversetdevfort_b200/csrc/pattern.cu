@@ -541,6 +541,7 @@ static int build_elem_order(ovs_ctx* c) {
   if ((st = ovs_ensure((void**)&c->elm_t, sizeof(int) * (size_t)E))) return st;
   if ((st = ovs_ensure((void**)&c->n2e_t, sizeof(int) * EN))) return st;
   order_pos_kernel<<<ovs_grid(N, 256, 1 << 30), 256, 0, s>>>(c->row_rec, N, c->row_pos);
+  ++c->launches;
   unsigned *k0 = nullptr, *k1 = nullptr;
   int *id = nullptr, *order = nullptr;
   OVS_CUDA_TRY(cudaMallocAsync(&k0, sizeof(unsigned) * (size_t)E, s));
@@ -548,6 +549,7 @@ static int build_elem_order(ovs_ctx* c) {
   OVS_CUDA_TRY(cudaMallocAsync(&id, sizeof(int) * (size_t)E, s));
   OVS_CUDA_TRY(cudaMallocAsync(&order, sizeof(int) * (size_t)E, s));
   elem_key_kernel<<<ovs_grid(E, 256, 1 << 30), 256, 0, s>>>(c->ien, E, c->nshl, c->row_pos, k0, id);
+  ++c->launches;
   int bits = 1;
   while (bits < 31 && ((N - 1) >> ELEM_TILE_SHIFT) >= (1 << bits)) ++bits;
   size_t tbytes = 0;
@@ -559,7 +561,7 @@ static int build_elem_order(ovs_ctx* c) {
                                                              c->elm_id, reinterpret_cast<int4*>(c->ien_t), c->elm_t,
                                                              id);
   n2e_place_kernel<<<ovs_grid(EN, 256, 1 << 30), 256, 0, s>>>(c->n2e, id, EN, c->n2e_t);
-  c->launches += 7;   // with the radix sort's passes (counted approximately)
+  c->launches += 5;   // with the radix sort's passes (counted approximately)
   for (void* q : {(void*)k0, (void*)k1, (void*)id, (void*)order, tmp}) OVS_CUDA_TRY(cudaFreeAsync(q, s));
   OVS_CUDA_TRY(cudaGetLastError());
   return OVS_OK;
