@@ -385,6 +385,11 @@ int ovs_sync_copies(ovs_ctx* ctx);
  * layout) is accumulated into: sol += sum_j y_j v_j. */
 int ovs_gmres(ovs_ctx* ctx, int system, double tol, int kspace,
               int kspace_min, double* sol, ovs_gmres_info* info);
+/* The same with the start vector in columns of N values (one host pointer per
+ * field of the system; not written) and the result alone in sol, whose contents
+ * on entry do not matter and which overlaps no column. */
+int ovs_gmres_from(ovs_ctx* ctx, int system, double tol, int kspace, int kspace_min,
+                   const double* const* start, double* sol, ovs_gmres_info* info);
 
 /* Solve A x = b to ||b - A x||_2 <= rtol ||b||_2 (true residual, FP64).
  * mode OVS_FP64: restarted FP64 GMRES(kspace) on the FP64 system.

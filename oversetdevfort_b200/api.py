@@ -285,10 +285,19 @@ class Context:
         return y
 
     def gmres(self, system: int, tol: float, kspace: int, kspace_min: int, sol: np.ndarray):
-        s = _f64(np.reshape(sol, (self.N, NF[system]), order="F")).copy(order="F")
+        start = _f64(np.reshape(sol, (self.N, NF[system]), order="F"))
+        return self._gmres_columns(system, tol, kspace, kspace_min, [start[:, k] for k in range(NF[system])])
+
+    def _gmres_columns(self, system: int, tol: float, kspace: int, kspace_min: int, cols):
+        """One cycle from the start vector's columns (nf contiguous FP64 arrays of N, not written); returns the
+        new solution (N, nf) and the info."""
+        if [c.shape for c in cols] != [(self.N,)] * NF[system]:
+            raise ValueError(f"start vector: {NF[system]} columns of {self.N} values expected")
+        s = np.empty((self.N, NF[system]), order="F")
         info = F.OvsGmresInfo()
-        F.check(self.lib.ovs_gmres(self.h, system, tol, kspace, kspace_min, _dptr(s), C.byref(info)),
-                "ovs_gmres")
+        F.check(self.lib.ovs_gmres_from(self.h, system, tol, kspace, kspace_min,
+                                        (C.POINTER(C.c_double) * len(cols))(*(_dptr(c) for c in cols)), _dptr(s),
+                                        C.byref(info)), "ovs_gmres")
         return s, info
 
     def solve(self, system: int, mode: int, rtol: float, kspace: int = 50, max_cycles: int = 100,
@@ -496,24 +505,25 @@ def SparseGMRES_up(ctx: Context, Utol: float, Kspaceu: int, Kspaceu_mn: int,
                    solu: np.ndarray, solp: np.ndarray):
     """src/SparseGMRES_NS.f90:4-369 on the resident FP64 (u,p) system; solu
     (N,3) and solp (N) are accumulated into and returned with the info."""
-    sol = np.concatenate([_f64(solu).reshape(-1, 3, order="F"), _f64(solp).reshape(-1, 1)], axis=1)
-    s, info = ctx.gmres(F.OVS_SYS_NS, Utol, Kspaceu, Kspaceu_mn, sol)
-    return np.asfortranarray(s[:, :3]), s[:, 3].copy(), info
+    u = _f64(solu).reshape(-1, 3, order="F")
+    s, info = ctx._gmres_columns(F.OVS_SYS_NS, Utol, Kspaceu, Kspaceu_mn,
+                                 [u[:, 0], u[:, 1], u[:, 2], _f64(solp).reshape(-1)])
+    return s[:, :3], s[:, 3], info
 
 
 def SparseGMRES_ns_conv(ctx: Context, Utol: float, Kspaceu: int, Kspaceu_mn: int,
                         solu: np.ndarray, solp: np.ndarray, solls: np.ndarray):
     """src/SparseGMRES_NS_conv.f:1-406 on the resident FP64 (u,p,phi) system."""
-    sol = np.concatenate([_f64(solu).reshape(-1, 3, order="F"), _f64(solp).reshape(-1, 1),
-                          _f64(solls).reshape(-1, 1)], axis=1)
-    s, info = ctx.gmres(F.OVS_SYS_NSVOF, Utol, Kspaceu, Kspaceu_mn, sol)
-    return np.asfortranarray(s[:, :3]), s[:, 3].copy(), s[:, 4].copy(), info
+    u = _f64(solu).reshape(-1, 3, order="F")
+    s, info = ctx._gmres_columns(F.OVS_SYS_NSVOF, Utol, Kspaceu, Kspaceu_mn,
+                                 [u[:, 0], u[:, 1], u[:, 2], _f64(solp).reshape(-1), _f64(solls).reshape(-1)])
+    return s[:, :3], s[:, 3], s[:, 4], info
 
 
 def SparseGMRES_tem(ctx: Context, Utol: float, Kspaceu: int, Kspaceu_mn: int, sol: np.ndarray):
     """src/SparseGMRES_tem.f90:1-256 on the resident FP64 temperature system."""
-    s, info = ctx.gmres(F.OVS_SYS_TEM, Utol, Kspaceu, Kspaceu_mn, _f64(sol).reshape(-1, 1))
-    return s[:, 0].copy(), info
+    s, info = ctx._gmres_columns(F.OVS_SYS_TEM, Utol, Kspaceu, Kspaceu_mn, [_f64(sol).reshape(-1)])
+    return s[:, 0], info
 
 
 def calculate_residual(ctx: Context, precision: int = F.OVS_FP64) -> np.ndarray:

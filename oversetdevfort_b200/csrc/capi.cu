@@ -207,6 +207,8 @@ int create_resources(ovs_ctx* c, const ovs_dims* dims) {
   OVS_CUDA_TRY(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   OVS_CUDA_TRY(cudaEventCreate(&c->ev0));
   OVS_CUDA_TRY(cudaEventCreate(&c->ev1));
+  OVS_CUDA_TRY(cudaStreamCreateWithFlags(&c->sol_stream, cudaStreamNonBlocking));
+  OVS_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_sol, cudaEventDisableTiming));
   for (cudaEvent_t& e : c->ev_poll) OVS_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   int st;
   const size_t N = c->N;
@@ -281,6 +283,8 @@ int ovs_destroy(ovs_ctx* c) {
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t e : c->ev_poll) if (e) cudaEventDestroy(e);
+  if (c->ev_sol) cudaEventDestroy(c->ev_sol);
+  if (c->sol_stream) cudaStreamDestroy(c->sol_stream);
   if (c->stream) cudaStreamDestroy(c->stream);
   cudaGetLastError();
   delete c;
@@ -686,19 +690,29 @@ int ovs_precond_device(ovs_ctx* c, int sys, int prec, const double* dx, double* 
   return OVS_OK;
 }
 
-int ovs_gmres(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, double* sol, ovs_gmres_info* info) {
-  if (!sys_ok(c, sys, OVS_FP64) || !sol) return OVS_ERR_ARG;
-  if (kspace < 1 || kspace > OVS_MAX_KSPACE) return OVS_ERR_ARG;
+// One cycle from the host columns `cols` (the start vector), the result to `out`
+// (host, N x nf column-major), which may be the columns themselves.  The upload
+// and the first touch of `out` go on while the device iterates: the copies in
+// front of and behind a cycle took 30 of 121 ms at 2.1M nodes (50 steps).
+static int gmres_host(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, const double* const* cols,
+                      double* out, bool touch, ovs_gmres_info* info) {
   int st;
   if ((st = ovs_activate(c))) return st;
-  const size_t n = (size_t)c->N * ovs_sys_nf(sys);
+  const int nf = ovs_sys_nf(sys);
+  const size_t n = (size_t)c->N * nf;
   if ((st = ovs_ensure((void**)&c->sol[sys], sizeof(double) * 5 * (size_t)c->N))) return st;
-  OVS_CUDA_TRY(cudaMemcpyAsync(c->sol[sys], sol, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+  // earlier work on sol (a queued update) comes first
+  OVS_CUDA_TRY(cudaEventRecord(c->ev_sol, c->stream));
+  OVS_CUDA_TRY(cudaStreamWaitEvent(c->sol_stream, c->ev_sol, 0));
+  SolFeed feed{cols, nf, (size_t)c->N, c->sol[sys], touch ? out : nullptr};
   ovs_gmres_info gi;
   memset(&gi, 0, sizeof(gi));
   OVS_CUDA_TRY(cudaEventRecord(c->ev0, c->stream));
-  st = ovs_gmres_ref_impl(c, sys, tol, kspace, kspace_min, c->sol[sys], &gi);
-  if (st) return st;
+  st = ovs_gmres_ref_impl(c, sys, tol, kspace, kspace_min, c->sol[sys], &gi, &feed);
+  if (st) {
+    cudaStreamSynchronize(c->sol_stream);   // no copy from the caller's memory outlives the call
+    return st;
+  }
   OVS_CUDA_TRY(cudaEventRecord(c->ev1, c->stream));
   OVS_CUDA_TRY(cudaEventSynchronize(c->ev1));
   {
@@ -706,10 +720,27 @@ int ovs_gmres(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, doubl
     OVS_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     c->last_ms = ms;
   }
-  OVS_CUDA_TRY(cudaMemcpyAsync(sol, c->sol[sys], sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  OVS_CUDA_TRY(cudaMemcpyAsync(out, c->sol[sys], sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
   OVS_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (info) *info = gi;
   return OVS_OK;
+}
+
+int ovs_gmres(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, double* sol, ovs_gmres_info* info) {
+  if (!sys_ok(c, sys, OVS_FP64) || !sol) return OVS_ERR_ARG;
+  if (kspace < 1 || kspace > OVS_MAX_KSPACE) return OVS_ERR_ARG;
+  const double* cols[5];
+  for (int f = 0; f < 5; ++f) cols[f] = sol + (size_t)f * (f < ovs_sys_nf(sys) ? c->N : 0);
+  return gmres_host(c, sys, tol, kspace, kspace_min, cols, sol, false, info);
+}
+
+int ovs_gmres_from(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, const double* const* start,
+                   double* sol, ovs_gmres_info* info) {
+  if (!sys_ok(c, sys, OVS_FP64) || !start || !sol) return OVS_ERR_ARG;
+  if (kspace < 1 || kspace > OVS_MAX_KSPACE) return OVS_ERR_ARG;
+  for (int f = 0; f < ovs_sys_nf(sys); ++f)
+    if (!start[f]) return OVS_ERR_ARG;
+  return gmres_host(c, sys, tol, kspace, kspace_min, start, sol, true, info);
 }
 
 int ovs_solve(ovs_ctx* c, int sys, int mode, double rtol, int kspace, int max_cycles, double* sol,

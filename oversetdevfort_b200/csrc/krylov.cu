@@ -1229,9 +1229,10 @@ int launch_arnoldi(ovs_ctx* c, int sys, const ArnoldiPlan& pl, const TM* vals, c
 // and basis precision TV.  rhs and sol are FP64 device vectors (nf*N).
 // rhs_pre: rhs is P^-1 times the right-hand side already (the cycle then
 // solves P^-1 A x = rhs)
+// feed: sol is still on its way from the host (SolFeed)
 template <typename TM, typename TV, bool ACC64 = true>
 int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol, int kspace,
-                int kmin, ovs_gmres_info* info, bool rhs_pre = false) {
+                int kmin, ovs_gmres_info* info, bool rhs_pre = false, SolFeed* feed = nullptr) {
   const int N = c->N, nf = ovs_sys_nf(sys);
   const size_t n = (size_t)N * nf;
   const int prec = sizeof(TM) == 8 ? OVS_FP64 : OVS_FP32;
@@ -1272,6 +1273,9 @@ int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol,
     const int kend = (k + batch - 1 < kspace) ? k + batch - 1 : kspace;
     for (; k <= kend; ++k)
       if ((st = launch_arnoldi<TM, TV, ACC64>(c, sys, pl, vals, pre, V, ld, n, k))) return st;
+    // a piece takes the host less time than the device has work queued (27 ms for
+    // all five columns of 2.1M nodes, 7 ms for four steps)
+    if (feed && (st = ovs_feed(c, feed, feed->n * feed->ncol / 5 + 1))) return st;
     if (k > kspace) break;
     OVS_CUDA_TRY(cudaMemcpyAsync(c->h_pinned + (q & 1), &gm->done, sizeof(int), cudaMemcpyDeviceToHost, s));
     OVS_CUDA_TRY(cudaEventRecord(c->ev_poll[q & 1], s));
@@ -1279,6 +1283,11 @@ int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol,
       OVS_CUDA_TRY(cudaEventSynchronize(c->ev_poll[(q - 1) & 1]));
       if (c->h_pinned[(q - 1) & 1]) break;
     }
+  }
+  if (feed) {
+    if ((st = ovs_feed(c, feed, 0))) return st;
+    OVS_CUDA_TRY(cudaEventRecord(c->ev_sol, c->sol_stream));
+    OVS_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_sol, 0));
   }
   gm_backsub_kernel<<<1, BACKSUB_THREADS, sizeof(double) * 12 * kspace, s>>>(gm, c->coop_part, pl.T, pl.grid);
   ++c->launches;
@@ -1520,8 +1529,26 @@ int ovs_spmv_impl(ovs_ctx* c, int sys, int prec, const double* dx, double* dy) {
 }
 
 // Reference-semantics single cycle in FP64 (SparseGMRES_up / _ns_conv / _tem)
+int ovs_feed(ovs_ctx* c, SolFeed* f, size_t count) {
+  const size_t total = f->n * f->ncol;
+  const size_t end = count == 0 || count >= total - f->at ? total : f->at + count;
+  while (f->at < end) {
+    const size_t col = f->at / f->n, off = f->at - col * f->n;
+    const size_t m = std::min(end - f->at, f->n - off);
+    OVS_CUDA_TRY(cudaMemcpyAsync(f->dst + f->at, f->cols[col] + off, sizeof(double) * m, cudaMemcpyHostToDevice,
+                                 c->sol_stream));
+    if (f->out) {
+      constexpr size_t PAGE = 4096 / sizeof(double);
+      volatile double* o = f->out + f->at;
+      for (size_t i = 0; i < m; i += PAGE) o[i] = 0.0;
+    }
+    f->at += m;
+  }
+  return OVS_OK;
+}
+
 int ovs_gmres_ref_impl(ovs_ctx* c, int sys, double tol, int kspace, int kmin, double* dsol,
-                       ovs_gmres_info* info) {
+                       ovs_gmres_info* info, SolFeed* feed) {
   SysStore& S = c->sys[sys][OVS_FP64];
   if (!S.vals || !S.rhs) return OVS_ERR_STATE;
   int st;
@@ -1538,7 +1565,7 @@ int ovs_gmres_ref_impl(ovs_ctx* c, int sys, double tol, int kspace, int kmin, do
       return OVS_OK;
     }
   }
-  st = gmres_cycle<double, double>(c, sys, rhs, dsol, tol, kspace, kmin, info);
+  st = gmres_cycle<double, double>(c, sys, rhs, dsol, tol, kspace, kmin, info, false, feed);
   if (st) return st;
   OVS_CUDA_TRY(cudaStreamSynchronize(c->stream));
   return OVS_OK;

@@ -80,6 +80,8 @@ struct ovs_ctx {
   int num_sms = 148;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaStream_t sol_stream = nullptr;             // uploads of a start vector beside the Krylov cycle (SolFeed)
+  cudaEvent_t ev_sol = nullptr;
   cudaEvent_t ev_poll[2] = {nullptr, nullptr};   // the done word of a batch of Krylov iterations has arrived
   int N = 0, E = 0, nshl = 0;
   // mesh
@@ -221,8 +223,22 @@ int ovs_spmv_pre_impl(ovs_ctx* c, int sys, int prec, const double* dx, double* d
 int ovs_spmv_rows_impl(ovs_ctx* c, int sys, int prec, bool precond, const double* dx, double* dy, const int* rows,
                        int nrows);
 int ovs_precond_apply_impl(ovs_ctx* c, int sys, int prec, const double* dx, double* dy);
+// The start vector of a cycle on its way from the host: columns of N values, in
+// any memory, to dst (column-major).  A cycle needs it for the last update only,
+// so the host copies it in pieces between the launches of the cycle's steps
+// (sol_stream), and touches the pages of `out`, where the result will land.
+struct SolFeed {
+  const double* const* cols;
+  int ncol;
+  size_t n;            // values per column
+  double* dst;
+  double* out;         // host pages to touch (null: none)
+  size_t at = 0;       // values sent so far
+};
+// queue the next `count` values (of n * ncol; every one left for 0)
+int ovs_feed(ovs_ctx* c, SolFeed* f, size_t count);
 int ovs_gmres_ref_impl(ovs_ctx* c, int sys, double tol, int kspace, int kmin,
-                       double* dsol, ovs_gmres_info* info);
+                       double* dsol, ovs_gmres_info* info, SolFeed* feed = nullptr);
 int ovs_solve_impl(ovs_ctx* c, int sys, int mode, double rtol, int kspace,
                    int max_cycles, ovs_solve_info* info);
 int ovs_round_impl(ovs_ctx* c, int sys);
