@@ -683,10 +683,15 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
 // A warp owns sub-chunks of 32 V values.  Phase A takes JG vectors at a
 // time: all their loads in flight, 2 JG sums per lane, reduced over the
 // lanes by halving (16 shuffles for 16 sums) into the warp's accumulators in
-// shared memory.  Phase B visits the sub-chunks in reverse, so that what
-// phase A read last is still in L2.  V = 4 (256-bit loads in FP64) where it
-// gives every warp of the grid a sub-chunk, V = 1 for shorter vectors; there
-// the JG groups of a sub-chunk are also spread over `js` warps.
+// shared memory.  With 32-byte loads (V = 4 in FP64, 8 in FP32) a sub-chunk
+// takes all its vectors in turn, and phase B visits the sub-chunks in reverse, so
+// that what phase A read last is still in L2; with shorter ones the sums over
+// the lanes would cost more than that saves, and a group of vectors goes through
+// all the warp's sub-chunks first (Gram-Schmidt at k = 25: 153K values 25 against
+// 28 us; FP32, 1.2M values 64 against 66; FP64, 1.2M values 103 against 90 the
+// other way round).  V = 1 for vectors that would not give every warp of the grid
+// a sub-chunk of four; where they leave warps idle even so, the JG groups of a
+// sub-chunk are spread over `js` warps.
 constexpr int ORTH_THREADS = 512;
 constexpr int ORTH_WARPS = ORTH_THREADS / 32;
 constexpr int JG = 8;
@@ -695,9 +700,13 @@ constexpr int JG = 8;
 // slot being orthogonalized is rewritten by the same thread)
 template <int V, typename TV>
 __device__ __forceinline__ void orth_ld(const TV* p, size_t i, size_t n, TV (&x)[V]) {
-  if (V == 4 && i + 4 <= n) {
+  if (V >= 4 && i + V <= n) {
     if constexpr (V == 4 && sizeof(TV) == 8) {
       asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p + i));
+    } else if constexpr (V == 8 && sizeof(TV) == 4) {
+      asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+          : "l"(p + i));
     } else if constexpr (V == 4) {
       const float4 v = *reinterpret_cast<const float4*>(p + i);
       x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
@@ -847,28 +856,48 @@ __device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_
   __syncwarp();
   // ---- phase A
   const int slot = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
-  for (long it = gw; it < (long)nsc * js; it += W) {
-    const int si = (int)(it / js), jj = (int)(it - (long)si * js);
-    const size_t i = ((size_t)si * 32 + lane) * V;
-    TV wv[V], kv[V];
-    orth_ld<V>(w, i, n, wv);
-    orth_ld<V>(vk, i, n, kv);
-    for (int j0 = jj * JG; j0 < k; j0 += js * JG) {
-      TV x[JG][V];
+  auto dots = [&](int j0, size_t i, const TV (&wv)[V], const TV (&kv)[V], double (&p)[2 * JG]) {
+    TV x[JG][V];
 #pragma unroll
-      for (int u = 0; u < JG; ++u) orth_ld<V>(basis + ld * (size_t)min(j0 + u, k - 1), i, n, x[u]);
-      double p[2 * JG];
+    for (int u = 0; u < JG; ++u) orth_ld<V>(basis + ld * (size_t)min(j0 + u, k - 1), i, n, x[u]);
 #pragma unroll
-      for (int u = 0; u < JG; ++u) {
-        p[u] = p[JG + u] = 0.0;
+    for (int u = 0; u < JG; ++u) {
 #pragma unroll
-        for (int q = 0; q < V; ++q) {
-          p[u] += (double)wv[q] * (double)x[u][q];
-          p[JG + u] += (double)kv[q] * (double)x[u][q];
-        }
+      for (int q = 0; q < V; ++q) {
+        p[u] += (double)wv[q] * (double)x[u][q];
+        p[JG + u] += (double)kv[q] * (double)x[u][q];
       }
-      const double s = lanes_sum16(p, lane);
-      if (!(lane & 1)) my[(slot < JG ? 0 : kk - JG) + j0 + slot] += s;
+    }
+  };
+  auto add = [&](int j0, double (&p)[2 * JG]) {
+    const double s = lanes_sum16(p, lane);
+    if (!(lane & 1)) my[(slot < JG ? 0 : kk - JG) + j0 + slot] += s;
+  };
+  if (V == 1 || (V == 4 && sizeof(TV) == 4)) {   // short vectors: a warp's sub-chunks inside a group, one sum over the lanes per group
+    // (js > 1: a warp has one sub-chunk at most, nsc js <= W)
+    const int jj = js == 1 ? 0 : gw % js, si0 = js == 1 ? gw : gw / js;
+    for (int j0 = jj * JG; j0 < k && si0 < nsc; j0 += js * JG) {
+      double p[2 * JG] = {};
+      for (long si = si0; si < nsc; si += W) {
+        const size_t i = ((size_t)si * 32 + lane) * V;
+        TV wv[V], kv[V];
+        orth_ld<V>(w, i, n, wv);
+        orth_ld<V>(vk, i, n, kv);
+        dots(j0, i, wv, kv, p);
+      }
+      add(j0, p);
+    }
+  } else {
+    for (long si = gw; si < nsc; si += W) {
+      const size_t i = ((size_t)si * 32 + lane) * V;
+      TV wv[V], kv[V];
+      orth_ld<V>(w, i, n, wv);
+      orth_ld<V>(vk, i, n, kv);
+      for (int j0 = 0; j0 < k; j0 += JG) {
+        double p[2 * JG] = {};
+        dots(j0, i, wv, kv, p);
+        add(j0, p);
+      }
     }
   }
   if (t < k - 1) sc[t] = sct;
@@ -989,10 +1018,11 @@ __device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_
         for (int q = 0; q < V; ++q) wv[q] = fma(-h, x[u][q], wv[q]);
       }
     }
-    if (V == 4 && i + 4 <= n) {
-      if constexpr (V == 4) {
-        const double d[4] = {(double)wv[0], (double)wv[1], (double)wv[2], (double)wv[3]};
-        st4v(w + i, d);
+    if (V >= 4 && i + V <= n) {
+#pragma unroll
+      for (int q = 0; q + 4 <= V; q += 4) {
+        const double d[4] = {(double)wv[q], (double)wv[q + 1], (double)wv[q + 2], (double)wv[q + 3]};
+        st4v(w + i + q, d);
       }
     } else {
 #pragma unroll
@@ -1125,7 +1155,7 @@ int ensure_basis(ovs_ctx* c, int prec, size_t bytes) {
 struct ArnoldiPlan {
   bool fused = false;
   int grid = 0;
-  bool wide = false;   // V = 4
+  int v = 1;           // values per lane (1, 4 or 8)
   int nsc = 0;         // sub-chunks of 32 V values
   double* T = nullptr;
 };
@@ -1142,13 +1172,16 @@ ArnoldiKern<TM, TV, ACC64> fused_kernel(int sys) {
 }
 
 template <typename TV>
-auto orthog_kernel(bool wide) {
-  return wide ? gm_orthog_kernel<TV, 4> : gm_orthog_kernel<TV, 1>;
+auto orthog_kernel(int v) {
+  using Kern = void (*)(TV*, size_t, size_t, int, GmresDev*, double*, double*, int, int);
+  if constexpr (sizeof(TV) == 4)
+    if (v == 8) return (Kern)gm_orthog_kernel<TV, 8>;
+  return v == 4 ? (Kern)gm_orthog_kernel<TV, 4> : (Kern)gm_orthog_kernel<TV, 1>;
 }
 
 // warps that share a sub-chunk's groups of vectors at step k
 inline int orth_split(const ArnoldiPlan& pl, int k, int sms) {
-  const int groups = (k + JG - 1) / JG, room = std::max(1, sms * ORTH_WARPS / std::max(1, pl.nsc));
+  const int groups = (k + JG - 1) / JG, room = std::max(1, (sms - 1) * ORTH_WARPS / std::max(1, pl.nsc));
   return std::min(groups, room);
 }
 
@@ -1170,10 +1203,14 @@ int plan_arnoldi(ovs_ctx* c, int sys, size_t n, int kspace, bool want_fused, Arn
   pl->T = c->coop_part + parts;
   pl->fused = want_fused;
   if (!want_fused) {
-    // V = 4 once it gives every warp of the chip a sub-chunk
-    pl->wide = n >= (size_t)128 * ORTH_WARPS * c->num_sms;
-    const size_t per = pl->wide ? 128 : 32, nsc = (n + per - 1) / per;
-    auto kern = orthog_kernel<TV>(pl->wide);
+    // V = 4 once it gives every warp of the chip a sub-chunk; FP32 V = 8 (32-byte
+    // loads, as V = 4 in FP64) once it gives every warp four: Gram-Schmidt at k = 25
+    // 0.132 against 0.139 ms at 3.2M values, 0.180 against 0.192 at 4.6M, but 0.110
+    // against 0.104 at 2.1M
+    const size_t chip = (size_t)32 * ORTH_WARPS * c->num_sms;
+    pl->v = sizeof(TV) == 4 && n >= 32 * chip ? 8 : (n >= 4 * chip ? 4 : 1);
+    const size_t per = 32 * pl->v, nsc = (n + per - 1) / per;
+    auto kern = orthog_kernel<TV>(pl->v);
     const size_t bytes = orth_smem(kspace);
     int per_sm = 0;
     OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
@@ -1219,7 +1256,7 @@ int launch_arnoldi(ovs_ctx* c, int sys, const ArnoldiPlan& pl, const TM* vals, c
   size_t ldv = ld, nn = n;
   double* T = pl.T;
   void* args[] = {&V, &ldv, &nn, &kk, &gm, &part, &T, &nsc, &js};
-  OVS_CUDA_TRY(cudaLaunchCooperativeKernel((void*)orthog_kernel<TV>(pl.wide), pl.grid + 1, ORTH_THREADS, args,
+  OVS_CUDA_TRY(cudaLaunchCooperativeKernel((void*)orthog_kernel<TV>(pl.v), pl.grid + 1, ORTH_THREADS, args,
                                            orth_smem(k), c->stream));
   ++c->launches;
   return OVS_OK;

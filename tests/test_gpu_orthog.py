@@ -67,3 +67,21 @@ def test_orthog_at_the_switch_of_values_per_lane(dims):
         out.append(ctx.solve(F.OVS_SYS_NSVOF, F.OVS_FP32, 1e-30, kspace=20, max_cycles=1)[0])
     assert np.abs(out[0] - out[1]).max() <= 1e-4 * np.abs(out[1]).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("dims", [(77, 78, 77), (78, 78, 77)])
+def test_orthog_at_the_switch_to_eight_values_per_lane(dims):
+    """FP32: 2,424,832 values on 148 SMs, ragged lengths on both sides.  Four
+    steps: the variants then differ by a few roundings of the basis vectors
+    (6e-8 each) times the condition of a 4x4 Hessenberg matrix, below 1e-5 of
+    the largest entry; over 20 steps the one-launch variant's own error against
+    FP64 reaches 9e-5 at this size."""
+    ctx = Context.from_case(M.quench_case(M.box_tet(*dims), "orthog_switch8", seed=3))
+    ctx.assemble(F.OVS_ASM_NSVOF, 6, F.OVS_FP32)
+    out = []
+    for fused in (0, 1):
+        ctx.set_option(F.OVS_OPT_ARNOLDI_FUSED, fused)
+        out.append(ctx.solve(F.OVS_SYS_NSVOF, F.OVS_FP32, 1e-30, kspace=4, max_cycles=1)[0])
+    assert np.abs(out[1]).max() > 0.0
+    assert np.abs(out[0] - out[1]).max() <= 1e-5 * np.abs(out[1]).max()
+    ctx.close()
