@@ -34,17 +34,24 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr int SPMV_THREADS = 256;
+// threads of a block row product: 64 but for FP64 matrices with vectors by fields
+// (see spmv_block_warp)
+template <typename TM, bool AOS>
+__host__ __device__ constexpr int spmv_threads() { return AOS || sizeof(TM) == 4 ? 64 : SPMV_THREADS; }
 
 template <typename T> __device__ __forceinline__ T ldm(const T* p) { return __ldcs(p); }
 
+// Four matrix values.  FP64: one 32-byte load instead of two of 16 (1.09 -> 1.02
+// ms at 2.1M nodes, 25 -> 17 us at 31K), evicted first from L2, where the Krylov
+// basis is worth more: per iteration at k = 25 31K nodes 46 us (51 without the
+// hint, 49 before), 236K nodes 199 (202, 207), 2.1M nodes 1.73 ms (1.71, 1.83).
+// FP32: no hint (a streaming load costs 0.57 -> 0.61 ms at 2.1M nodes).
 __device__ __forceinline__ void ld4(const float* p, float v[4]) {
-  float4 q = __ldcs(reinterpret_cast<const float4*>(p));
-  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
 __device__ __forceinline__ void ld4(const double* p, double v[4]) {
-  double2 a = __ldcs(reinterpret_cast<const double2*>(p));
-  double2 b = __ldcs(reinterpret_cast<const double2*>(p) + 1);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  asm("ld.global.nc.L2::evict_first.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
 }
 
 // Accumulation precision of the SpMV: FP32 storage accumulates in FP32 on
@@ -62,17 +69,26 @@ template <> struct AccT<float, float, false> { using type = float; };
 //   NSVOF(NG=6): + row phi over (u1,u2,u3,phi), + column phi into (u1,u2,u3,p)
 // The RPW = 32/NG rows of warp chunk `wglob` (all 32 lanes take part in
 // the shuffles).
+// AOS: x and y by nodes (x[node nf + field]), as the Krylov basis holds its
+// vectors, instead of by fields: a slot's gathers fall into one or two sectors
+// instead of one per field (FP32 66.0 -> 62.1 us at 236K nodes, 0.627 -> 0.597 ms
+// at 2.1M).  The kernel waits for its loads (20 stalled warps per issue), so the
+// warps in flight decide: blocks of 64 threads, whose places are refilled sooner
+// than those of 256, gain 1 to 8% there and for FP32 matrices by fields, and lose
+// 7% for FP64 by fields.  With the loads of ld4, at 236K and 2.1M nodes: by nodes
+// FP64 0.109 and 1.05 ms, FP32 0.069 (0.061 with the basis out of L2) and 0.57; its
+// bytes at 6.45 TB/s: 0.106 and 0.98, 0.053 and 0.50.
 // LIST: the warp chunks run over the row list rows[0, nrows) (local row
 // indices; an index outside [0, N) is skipped) instead of rows 0..N-1;
 // each listed row is computed exactly as in the full product.
-template <int NG, typename TM, typename TX, typename TY, int MODE, bool ACC64, bool LIST = false>
+template <int NG, typename TM, typename TX, typename TY, int MODE, bool ACC64, bool LIST = false, bool AOS = false>
 __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __restrict__ rowptr,
                                                 const int* __restrict__ colidx, const TM* __restrict__ vals,
                                                 const TX* __restrict__ x, TY* __restrict__ y,
                                                 const TM* __restrict__ pre, const double* __restrict__ b,
                                                 const int* __restrict__ rows = nullptr, long nrows = 0) {
   using AT = typename AccT<TM, TX, ACC64>::type;
-  constexpr int NV = 4 * NG;
+  constexpr int NV = 4 * NG, NFX = NG == 6 ? 5 : 4;
   constexpr int RPW = 32 / NG;  // rows per warp
   const int lane = threadIdx.x & 31;
   const int sub = lane / NG;
@@ -99,10 +115,10 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
     // u,v,w,p,phi in lanes 0-4) and the row's lanes exchange them by
     // shuffles: 4-5 gathers per slot instead of 4 per lane
     int s = s0;
-    constexpr int NFX = NG == 6 ? 5 : 4;
     const unsigned gmask = ((1u << NG) - 1u) << (sub * NG);
     const int base = sub * NG;
-    const TX* xg = x + (size_t)(g < NFX ? g : 0) * N;
+    const TX* xg = x + (AOS ? (size_t)(g < NFX ? g : 0) : (size_t)(g < NFX ? g : 0) * N);
+    constexpr int XS = AOS ? NFX : 1;   // stride between nodes
     // FP32 values: 4 slots in flight per lane (measured 0.63 vs 0.72 ms at
     // 2.1M nodes); FP64 values already move 32 bytes per lane and slot, and
     // run faster with 2
@@ -115,7 +131,7 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
         ld4(vals + (size_t)(s + 1) * NV + 4 * g, w);
         ld4(vals + (size_t)(s + 2) * NV + 4 * g, y);
         ld4(vals + (size_t)(s + 3) * NV + 4 * g, z);
-        const AT f0 = (AT)__ldg(xg + c0), f1 = (AT)__ldg(xg + c1), f2 = (AT)__ldg(xg + c2), f3 = (AT)__ldg(xg + c3);
+        const AT f0 = (AT)__ldg(xg + (size_t)c0 * XS), f1 = (AT)__ldg(xg + (size_t)c1 * XS), f2 = (AT)__ldg(xg + (size_t)c2 * XS), f3 = (AT)__ldg(xg + (size_t)c3 * XS);
         a0 += (AT)v[0] * __shfl_sync(gmask, f0, base + cf0); a1 += (AT)v[1] * __shfl_sync(gmask, f0, base + cf1);
         a2 += (AT)v[2] * __shfl_sync(gmask, f0, base + cf2); a3 += (AT)v[3] * __shfl_sync(gmask, f0, base + cf3);
         a0 += (AT)w[0] * __shfl_sync(gmask, f1, base + cf0); a1 += (AT)w[1] * __shfl_sync(gmask, f1, base + cf1);
@@ -131,7 +147,7 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
       TM v[4], w[4];
       ld4(vals + (size_t)s * NV + 4 * g, v);
       ld4(vals + (size_t)(s + 1) * NV + 4 * g, w);
-      const AT f0 = (AT)__ldg(xg + c0), f1 = (AT)__ldg(xg + c1);
+      const AT f0 = (AT)__ldg(xg + (size_t)c0 * XS), f1 = (AT)__ldg(xg + (size_t)c1 * XS);
       a0 += (AT)v[0] * __shfl_sync(gmask, f0, base + cf0); a1 += (AT)v[1] * __shfl_sync(gmask, f0, base + cf1);
       a2 += (AT)v[2] * __shfl_sync(gmask, f0, base + cf2); a3 += (AT)v[3] * __shfl_sync(gmask, f0, base + cf3);
       a0 += (AT)w[0] * __shfl_sync(gmask, f1, base + cf0); a1 += (AT)w[1] * __shfl_sync(gmask, f1, base + cf1);
@@ -141,7 +157,7 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
       const int c0 = __ldg(colidx + s);
       TM v[4];
       ld4(vals + (size_t)s * NV + 4 * g, v);
-      const AT f0 = (AT)__ldg(xg + c0);
+      const AT f0 = (AT)__ldg(xg + (size_t)c0 * XS);
       a0 += (AT)v[0] * __shfl_sync(gmask, f0, base + cf0); a1 += (AT)v[1] * __shfl_sync(gmask, f0, base + cf1);
       a2 += (AT)v[2] * __shfl_sync(gmask, f0, base + cf2); a3 += (AT)v[3] * __shfl_sync(gmask, f0, base + cf3);
     }
@@ -176,18 +192,18 @@ __device__ __forceinline__ void spmv_block_warp(long wglob, int N, const int* __
   } else if (MODE == 2) {
     z = (AT)b[(size_t)g * N + row] - yv;
   }
-  y[(size_t)g * N + row] = (TY)z;
+  y[AOS ? (size_t)row * NFX + g : (size_t)g * N + row] = (TY)z;
 }
 
-template <int NG, typename TM, typename TX, typename TY, int MODE, bool ACC64>
-__global__ void __launch_bounds__(SPMV_THREADS)
+template <int NG, typename TM, typename TX, typename TY, int MODE, bool ACC64, bool AOS>
+__global__ void __launch_bounds__(spmv_threads<TM, AOS>())
 spmv_block_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__ colidx,
                   const TM* __restrict__ vals, const TX* __restrict__ x, TY* __restrict__ y,
                   const TM* __restrict__ pre, const double* __restrict__ b,
                   const int* __restrict__ done) {
   if (done && *done) return;
   const long wglob = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  spmv_block_warp<NG, TM, TX, TY, MODE, ACC64>(wglob, N, rowptr, colidx, vals, x, y, pre, b);
+  spmv_block_warp<NG, TM, TX, TY, MODE, ACC64, false, AOS>(wglob, N, rowptr, colidx, vals, x, y, pre, b);
 }
 
 // the same product over a list of rows (a partition's interior or boundary
@@ -282,28 +298,29 @@ int launch_spmv_rows(ovs_ctx* c, int sys, const TM* vals, const double* x, doubl
   return OVS_OK;
 }
 
-template <typename TM, typename TX, typename TY, int MODE, bool ACC64 = true>
+template <typename TM, typename TX, typename TY, int MODE, bool ACC64 = true, bool AOS = false>
 int launch_spmv(ovs_ctx* c, int sys, const TM* vals, const TX* x, TY* y, const TM* pre,
                 const double* b, const int* done) {
   const int N = c->N;
   int rpw = sys == OVS_SYS_NS ? 8 : (sys == OVS_SYS_NSVOF ? 5 : 4);
   long warps = ((long)N + rpw - 1) / rpw;
-  long blocks = (warps * 32 + SPMV_THREADS - 1) / SPMV_THREADS;
+  const int threads = sys != OVS_SYS_TEM ? spmv_threads<TM, AOS>() : SPMV_THREADS;
+  long blocks = (warps * 32 + threads - 1) / threads;
   if (sys == OVS_SYS_NS)
     {
-      spmv_block_kernel<4, TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
+      spmv_block_kernel<4, TM, TX, TY, MODE, ACC64, AOS><<<(int)blocks, threads, 0, c->stream>>>(
           N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
       ++c->launches;
     }
   else if (sys == OVS_SYS_NSVOF)
     {
-      spmv_block_kernel<6, TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
+      spmv_block_kernel<6, TM, TX, TY, MODE, ACC64, AOS><<<(int)blocks, threads, 0, c->stream>>>(
           N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
       ++c->launches;
     }
   else
     {
-      spmv_scalar_kernel<TM, TX, TY, MODE, ACC64><<<(int)blocks, SPMV_THREADS, 0, c->stream>>>(
+      spmv_scalar_kernel<TM, TX, TY, MODE, ACC64><<<(int)blocks, threads, 0, c->stream>>>(
           N, c->rowptr, c->colidx, vals, x, y, pre, b, done);
       ++c->launches;
     }
@@ -424,7 +441,7 @@ gm_start_kernel(int N, int nf, int sys, const double* __restrict__ rhs, const TM
     if (raw) {   // rhs is already preconditioned
       for (int f = 0; f < nf; ++f) {
         const double z = rhs[(size_t)f * N + i];
-        v0[(size_t)f * N + i] = (TV)z;
+        v0[i * nf + f] = (TV)z;
         s += z * z;
       }
     } else if (sys == OVS_SYS_TEM) {
@@ -438,12 +455,12 @@ gm_start_kernel(int N, int nf, int sys, const double* __restrict__ rhs, const TM
       const double z1 = (double)B[3] * r0 + (double)B[4] * r1 + (double)B[5] * r2;
       const double z2 = (double)B[6] * r0 + (double)B[7] * r1 + (double)B[8] * r2;
       const double z3 = rhs[3 * (size_t)N + i] * (double)pre[(size_t)9 * N + i];
-      v0[i] = (TV)z0; v0[(size_t)N + i] = (TV)z1; v0[2 * (size_t)N + i] = (TV)z2;
-      v0[3 * (size_t)N + i] = (TV)z3;
+      TV* v = v0 + i * nf;
+      v[0] = (TV)z0; v[1] = (TV)z1; v[2] = (TV)z2; v[3] = (TV)z3;
       s += z0 * z0 + z1 * z1 + z2 * z2 + z3 * z3;
       if (nf == 5) {
         const double z4 = rhs[4 * (size_t)N + i] * (double)pre[(size_t)10 * N + i];
-        v0[4 * (size_t)N + i] = (TV)z4;
+        v[4] = (TV)z4;
         s += z4 * z4;
       }
     }
@@ -466,7 +483,8 @@ gm_start_kernel(int N, int nf, int sys, const double* __restrict__ rhs, const TM
 }
 
 // Krylov vectors are stored with a padded leading dimension (multiple of
-// 64 values) so every basis vector starts 256-byte aligned.  The vector
+// 64 values) so every basis vector starts 256-byte aligned, by nodes (the nf
+// values of a node side by side; start and update convert).  The vector
 // being orthogonalized, w, is kept in FP64 whatever the basis precision, so
 // the projections of Gram-Schmidt do not lose the small remainder to FP32
 // rounding; only normalized vectors are rounded into the basis.
@@ -579,9 +597,9 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
     const long nchunks = ((long)N + RPW - 1) / RPW;
     for (long c = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nwarps) {
       if constexpr (SYS == OVS_SYS_NS)
-        spmv_block_warp<4, TM, TV, TV, 1, ACC64>(c, N, rowptr, colidx, vals, vk, w, pre, nullptr);
+        spmv_block_warp<4, TM, TV, TV, 1, ACC64, false, true>(c, N, rowptr, colidx, vals, vk, w, pre, nullptr);
       else if constexpr (SYS == OVS_SYS_NSVOF)
-        spmv_block_warp<6, TM, TV, TV, 1, ACC64>(c, N, rowptr, colidx, vals, vk, w, pre, nullptr);
+        spmv_block_warp<6, TM, TV, TV, 1, ACC64, false, true>(c, N, rowptr, colidx, vals, vk, w, pre, nullptr);
       else
         spmv_scalar_warp<TM, TV, TV, 1, ACC64>(c, N, rowptr, colidx, vals, vk, w, pre, nullptr);
     }
@@ -1100,17 +1118,18 @@ __global__ void __launch_bounds__(BACKSUB_THREADS) gm_backsub_kernel(GmresDev* g
 }
 
 // sol += sum_j y_j v_j (SparseGMRES_NS.f90:349-352), eight vectors' loads in
-// flight per value
+// flight per value; sol is by fields, the basis by nodes
 template <typename TV>
 __global__ void __launch_bounds__(256)
-gm_update_kernel(double* __restrict__ sol, const TV* __restrict__ basis, size_t n, size_t ld,
+gm_update_kernel(double* __restrict__ sol, const TV* __restrict__ basis, size_t n, size_t ld, int nf,
                  const GmresDev* __restrict__ gm) {
   __shared__ double y[OVS_MAX_KSPACE];
   const int iks = gm->iks;
   for (int j = threadIdx.x; j < iks; j += blockDim.x) y[j] = gm->y[j];
   __syncthreads();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double s = sol[i];
+    const size_t node = i / (unsigned)nf, o = (i - node * nf) * (n / (unsigned)nf) + node;
+    double s = sol[o];
     int j = 0;
     for (; j + 8 <= iks; j += 8) {
       TV x[8];
@@ -1120,7 +1139,7 @@ gm_update_kernel(double* __restrict__ sol, const TV* __restrict__ basis, size_t 
       for (int u = 0; u < 8; ++u) s = s + y[j + u] * (double)x[u];
     }
     for (; j < iks; ++j) s = s + y[j] * (double)basis[(size_t)j * ld + i];
-    sol[i] = s;
+    sol[o] = s;
   }
 }
 
@@ -1249,7 +1268,7 @@ int launch_arnoldi(ovs_ctx* c, int sys, const ArnoldiPlan& pl, const TM* vals, c
     ++c->launches;
     return OVS_OK;
   }
-  int st = launch_spmv<TM, TV, TV, 1, ACC64>(c, sys, vals, V + ld * (size_t)(k - 1), V + ld * (size_t)k, pre,
+  int st = launch_spmv<TM, TV, TV, 1, ACC64, true>(c, sys, vals, V + ld * (size_t)(k - 1), V + ld * (size_t)k, pre,
                                                nullptr, &gm->done);
   if (st) return st;
   int kk = k, nsc = pl.nsc, js = orth_split(pl, k, c->num_sms);
@@ -1328,7 +1347,7 @@ int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol,
   }
   gm_backsub_kernel<<<1, BACKSUB_THREADS, sizeof(double) * 12 * kspace, s>>>(gm, c->coop_part, pl.T, pl.grid);
   ++c->launches;
-  gm_update_kernel<TV><<<ovs_grid(n, 256, 8 * c->num_sms), 256, 0, s>>>(sol, V, n, ld, gm);
+  gm_update_kernel<TV><<<ovs_grid(n, 256, 8 * c->num_sms), 256, 0, s>>>(sol, V, n, ld, nf, gm);
   ++c->launches;
   OVS_CUDA_TRY(cudaGetLastError());
   if (info) {
@@ -1396,7 +1415,7 @@ int profile_krylov_t(ovs_ctx* c, int what, int sys, int reps, double* ms) {
   ++c->launches;
   auto run = [&]() -> int {
     if (what == OVS_PROF_SPMV) {
-      st = launch_spmv<TM, TM, TM, 1, ACC64>(c, sys, vals, V, V + ld, pre, nullptr, nullptr);
+      st = launch_spmv<TM, TM, TM, 1, ACC64, true>(c, sys, vals, V, V + ld, pre, nullptr, nullptr);
       return st;
     }
     return launch_arnoldi<TM, TM, ACC64>(c, sys, pl, vals, pre, V, ld, n, k);

@@ -85,3 +85,22 @@ def test_orthog_at_the_switch_to_eight_values_per_lane(dims):
     assert np.abs(out[1]).max() > 0.0
     assert np.abs(out[0] - out[1]).max() <= 1e-5 * np.abs(out[1]).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("n,kspace", [(1, 4), (2, 9), (4, 12)])
+def test_ns_rows_by_nodes_match_the_oracle(oracle, n, kspace):
+    """The (u,p) system's product with vectors by nodes: 8, 27 and 125 rows, one
+    warp of eight rows, a ragged last one, several blocks of 64 threads.  The
+    enclosed cavity leaves the pressure's constant to rounding: compared without."""
+    case = M.config1(n)
+    ctx = Context.from_case(case)
+    oc = oracle.OracleCase(case)
+    oc.assemble_navsto(6)
+    ctx.assemble(F.OVS_ASM_NS, 6, F.OVS_FP64)
+    ref, it, _, _ = oc.gmres("ns", 1e-12, kspace, 1)
+    s, info = ctx.gmres(F.OVS_SYS_NS, 1e-12, kspace, 1, np.zeros((ctx.N, 4)))
+    assert info.iterations == it
+    d = s - ref
+    d[:, 3] -= d[:, 3].mean()
+    assert np.abs(d).max() <= TOL * np.abs(ref).max()
+    ctx.close()
