@@ -1048,8 +1048,8 @@ __device__ __forceinline__ unsigned mask_of(int v) {
 // per block, and the two lanes of an edge read the same element.  A warp per
 // row with one list per entry (28 values, 24 elements a load, an exchange
 // through shared memory) took 12.65 ms for the FP64 NS+VOF rows of the
-// 128^3 x6 tets and 6.91 ms in FP32; this takes 6.70 and 3.64 ms (T: 1.90 ->
-// 0.85 and 1.43 -> 0.47 ms).  A tile's edges are sorted by list
+// 128^3 x6 tets and 6.91 ms in FP32; this takes 6.29 and 3.34 ms (T: 1.90 ->
+// 0.81 and 1.43 -> 0.46 ms).  A tile's edges are sorted by list
 // length, so the rounds of a set are nearly equal.
 template <typename T, int KIND>
 __device__ __forceinline__ void write_entry(T* dst, T* v, const unsigned* masks, unsigned ibA, unsigned ibB) {
@@ -1127,7 +1127,7 @@ __device__ __forceinline__ void diag_row(const AsmArgs& a, const int4 rr, bool o
 }
 
 template <typename T, int KIND>
-__global__ void __launch_bounds__(128, 4) edge_rows_kernel(const AsmArgs a) {
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4) edge_rows_kernel(const AsmArgs a) {
   using L = Lay<KIND>;
   constexpr int NV = L::NV;
   __shared__ unsigned masks[24];
@@ -1171,7 +1171,12 @@ __global__ void __launch_bounds__(128, 4) edge_rows_kernel(const AsmArgs a) {
     T acc[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = (T)0;
-#pragma unroll 1
+    // several elements' loads in flight (lists of 4 to 8 are the rule): FP64 four
+    // at 3 blocks per SM, 6.63 -> 6.29 ms at 128^3 x6 (two or three 6.60 and 6.49,
+    // six 6.51; 4 blocks: 7.23 with two), FP32 three at 4 blocks, 3.56 -> 3.34 (two
+    // 3.37, four 3.38, 5 blocks 3.47)
+    constexpr int UNR = sizeof(T) == 8 ? 4 : 3;
+#pragma unroll UNR
     for (; pos < end; ++pos) {
       const unsigned now = en;
       if (pos + 1 < end) en = __ldg(a.edge_list + pos + 1);
