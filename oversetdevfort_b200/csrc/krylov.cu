@@ -26,6 +26,7 @@
 #include <vector>
 
 #include <cooperative_groups.h>
+#include <type_traits>
 #include <math.h>
 #include <string.h>
 
@@ -708,8 +709,8 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
 // all the warp's sub-chunks first (Gram-Schmidt at k = 25: 153K values 25 against
 // 28 us; FP32, 1.2M values 64 against 66; FP64, 1.2M values 103 against 90 the
 // other way round).  V = 1 for vectors that would not give every warp of the grid
-// a sub-chunk of four; where they leave warps idle even so, the JG groups of a
-// sub-chunk are spread over `js` warps.
+// a sub-chunk of four; the groups of vectors are split over `js` shares of the
+// warps (orth_split).
 constexpr int ORTH_THREADS = 512;
 constexpr int ORTH_WARPS = ORTH_THREADS / 32;
 constexpr int JG = 8;
@@ -892,11 +893,10 @@ __device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_
     if (!(lane & 1)) my[(slot < JG ? 0 : kk - JG) + j0 + slot] += s;
   };
   if (V == 1 || (V == 4 && sizeof(TV) == 4)) {   // short vectors: a warp's sub-chunks inside a group, one sum over the lanes per group
-    // (js > 1: a warp has one sub-chunk at most, nsc js <= W)
-    const int jj = js == 1 ? 0 : gw % js, si0 = js == 1 ? gw : gw / js;
-    for (int j0 = jj * JG; j0 < k && si0 < nsc; j0 += js * JG) {
+    const int Wj = W / js, jj = gw % js, si0 = gw / js;   // Wj warps per share of the groups
+    for (int j0 = jj * JG; j0 < k && si0 < min(Wj, nsc); j0 += js * JG) {
       double p[2 * JG] = {};
-      for (long si = si0; si < nsc; si += W) {
+      for (long si = si0; si < nsc; si += Wj) {
         const size_t i = ((size_t)si * 32 + lane) * V;
         TV wv[V], kv[V];
         orth_ld<V>(w, i, n, wv);
@@ -1018,38 +1018,53 @@ __device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_
   double na = 0.0;
   const TV skv = (TV)sk;
   const int cnt = gw < nsc ? (nsc - gw + W - 1) / W : 0;
-  for (int r = cnt - 1; r >= 0; --r) {
-    const size_t i = ((size_t)(gw + (long)r * W) * 32 + lane) * V;
-    TV wv[V];
-    orth_ld<V>(w, i, n, wv);
+  auto update = [&](auto nb, int r) {   // sub-chunks r, r - 1, .. of the warp's, their loads in flight together
+    constexpr int NB = decltype(nb)::value, JB = V == 1 ? 2 * JG : JG;
+    size_t i[NB];
+    TV wv[NB][V];
 #pragma unroll
-    for (int q = 0; q < V; ++q) wv[q] *= skv;
-    constexpr int JB = V == 1 ? 2 * JG : JG;
+    for (int m = 0; m < NB; ++m) {
+      i[m] = ((size_t)(gw + (long)(r - m) * W) * 32 + lane) * V;
+      orth_ld<V>(w, i[m], n, wv[m]);
+#pragma unroll
+      for (int q = 0; q < V; ++q) wv[m][q] *= skv;
+    }
     for (int j0 = 0; j0 < k; j0 += JB) {
-      TV x[JB][V];
+      TV x[NB][JB][V];
 #pragma unroll
-      for (int u = 0; u < JB; ++u) orth_ld<V>(basis + ld * (size_t)min(j0 + u, k - 1), i, n, x[u]);
+      for (int m = 0; m < NB; ++m)
+#pragma unroll
+        for (int u = 0; u < JB; ++u) orth_ld<V>(basis + ld * (size_t)min(j0 + u, k - 1), i[m], n, x[m][u]);
 #pragma unroll
       for (int u = 0; u < JB; ++u) {
         const TV h = j0 + u < k ? (TV)hs[j0 + u] : (TV)0;
 #pragma unroll
-        for (int q = 0; q < V; ++q) wv[q] = fma(-h, x[u][q], wv[q]);
+        for (int m = 0; m < NB; ++m)
+#pragma unroll
+          for (int q = 0; q < V; ++q) wv[m][q] = fma(-h, x[m][u][q], wv[m][q]);
       }
     }
-    if (V >= 4 && i + V <= n) {
 #pragma unroll
-      for (int q = 0; q + 4 <= V; q += 4) {
-        const double d[4] = {(double)wv[q], (double)wv[q + 1], (double)wv[q + 2], (double)wv[q + 3]};
-        st4v(w + i + q, d);
+    for (int m = 0; m < NB; ++m) {
+      if (V >= 4 && i[m] + V <= n) {
+#pragma unroll
+        for (int q = 0; q + 4 <= V; q += 4) {
+          const double d[4] = {(double)wv[m][q], (double)wv[m][q + 1], (double)wv[m][q + 2], (double)wv[m][q + 3]};
+          st4v(w + i[m] + q, d);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+          if (i[m] + q < n) w[i[m] + q] = wv[m][q];
       }
-    } else {
 #pragma unroll
-      for (int q = 0; q < V; ++q)
-        if (i + q < n) w[i + q] = wv[q];
+      for (int q = 0; q < V; ++q) na += (double)wv[m][q] * (double)wv[m][q];
     }
-#pragma unroll
-    for (int q = 0; q < V; ++q) na += (double)wv[q] * (double)wv[q];
-  }
+  };
+  int r = cnt - 1;
+  if constexpr (V == 1 && sizeof(TV) == 4)
+    for (; r >= 1; r -= 2) update(std::integral_constant<int, 2>(), r);
+  for (; r >= 0; --r) update(std::integral_constant<int, 1>(), r);
   na = warp_sum(na);
   if (lane == 0) sh[wid] = na;
   __syncthreads();
@@ -1198,10 +1213,25 @@ auto orthog_kernel(int v) {
   return v == 4 ? (Kern)gm_orthog_kernel<TV, 4> : (Kern)gm_orthog_kernel<TV, 1>;
 }
 
-// warps that share a sub-chunk's groups of vectors at step k
-inline int orth_split(const ArnoldiPlan& pl, int k, int sms) {
-  const int groups = (k + JG - 1) / JG, room = std::max(1, (sms - 1) * ORTH_WARPS / std::max(1, pl.nsc));
-  return std::min(groups, room);
+// Shares into which the groups of vectors of step k are split over the warps of
+// the grid (a share's warps take a group through all their sub-chunks).  FP64: as
+// many as leave every warp one sub-chunk at most; more shares than that even out
+// the warps' rounds but read w and v_k once more each, which long FP64 vectors pay
+// for (296K values 37 against 33 us).  FP32: the fewest rounds of eight loads for
+// the warp that has the most, a sum over the lanes counted as two rounds (Gram-
+// Schmidt at k = 25, with two sub-chunks at a time in phase B: 78K values 22.5 ->
+// 18.8 us, 176K 29.5 -> 27.6, 345K 36 -> 32).
+template <typename TV>
+int orth_split(const ArnoldiPlan& pl, int k) {
+  const int groups = (k + JG - 1) / JG, W = pl.grid * ORTH_WARPS;
+  if (sizeof(TV) == 8) return std::min(groups, std::max(1, W / std::max(1, pl.nsc)));
+  int best = 1;
+  long cost = 0;
+  for (int js = 1; js <= groups && js <= W; ++js) {
+    const long wj = W / js, c = ((pl.nsc + wj - 1) / wj + 2) * ((groups + js - 1) / js);
+    if (js == 1 || c < cost) { best = js; cost = c; }
+  }
+  return best;
 }
 
 template <typename TM, typename TV, bool ACC64>
@@ -1236,9 +1266,10 @@ int plan_arnoldi(ovs_ctx* c, int sys, size_t n, int kspace, bool want_fused, Arn
     OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ORTH_THREADS, bytes));
     if (per_sm >= 1 && c->num_sms >= 2 && nsc < ((size_t)1 << 31)) {
       pl->nsc = (int)nsc;
-      const long items = (long)nsc * orth_split(*pl, kspace, c->num_sms);
       // one SM is left for the block that finishes the step before
-      pl->grid = (int)std::min((long)c->num_sms - 1, (items + ORTH_WARPS - 1) / ORTH_WARPS);
+      pl->grid = c->num_sms - 1;
+      const int shares = sizeof(TV) == 8 ? orth_split<TV>(*pl, kspace) : (kspace + JG - 1) / JG;
+      pl->grid = (int)std::min((long)pl->grid, ((long)nsc * shares + ORTH_WARPS - 1) / ORTH_WARPS);
       return OVS_OK;
     }
     pl->fused = true;
@@ -1271,7 +1302,7 @@ int launch_arnoldi(ovs_ctx* c, int sys, const ArnoldiPlan& pl, const TM* vals, c
   int st = launch_spmv<TM, TV, TV, 1, ACC64, true>(c, sys, vals, V + ld * (size_t)(k - 1), V + ld * (size_t)k, pre,
                                                nullptr, &gm->done);
   if (st) return st;
-  int kk = k, nsc = pl.nsc, js = orth_split(pl, k, c->num_sms);
+  int kk = k, nsc = pl.nsc, js = orth_split<TV>(pl, k);
   size_t ldv = ld, nn = n;
   double* T = pl.T;
   void* args[] = {&V, &ldv, &nn, &kk, &gm, &part, &T, &nsc, &js};
