@@ -516,7 +516,7 @@ enum { OVS_PROF_SPMV = 1, OVS_PROF_ASSEMBLE = 2, OVS_PROF_ARNOLDI = 3, OVS_PROF_
  *                      Gram-Schmidt steps, normalization, Givens) at k = 25
  *                      of a 50-vector cycle, `system` in `precision`, as
  *                      the solvers run it (SpMV launch, then Gram-Schmidt
- *                      with the new vector held on chip);
+ *                      in one cooperative launch);
  *   OVS_PROF_ARNOLDI_FUSED  the same iteration as one cooperative launch
  *                      (the variant selected by OVS_ARNOLDI_FUSED=1). */
 int ovs_profile(ovs_ctx* ctx, int what, int system, int precision, int reps,
@@ -543,10 +543,9 @@ enum { OVS_VJP_XG = 0, OVS_VJP_UG = 3, OVS_VJP_PG = 6, OVS_VJP_PHIG = 7, OVS_VJP
  * ovs_assemble(kernel, OVS_TENSOR_VEC, OVS_FP64) would write for the current
  * state, parameters and IBC (kernel OVS_ASM_NSVOF: cot is N x 5 field-major
  * u1 u2 u3 p phi; OVS_ASM_TEM: N x 1), the state the nodal fields above.
- * Each element's Gauss-point quantities are recomputed in forward-mode
- * dual arithmetic per nodal input (nothing is stored between assembly and
- * adjoint); the node sums run in ascending element id, so the result is
- * deterministic.  grad is N x OVS_VJP_COUNT (fields the kernel does not
+ * Each element's Gauss-point quantities are recomputed and walked back
+ * (reverse mode; nothing is stored between assembly and adjoint); the node
+ * sums run in a fixed order, so the result is deterministic.  grad is N x OVS_VJP_COUNT (fields the kernel does not
  * depend on come back 0).  Host arrays; synchronous. */
 int ovs_residual_vjp(ovs_ctx* ctx, int kernel, const double* cot, double* grad);
 /* Solve A^T x = rhs by GMRES (the reference-semantics cycle of ovs_gmres,

@@ -8,9 +8,8 @@ for the NS+VOF pass (RHSGu, RHSGp, RHSGls: (N, 5)) and the temperature pass
 (RHSGtem: (N,)), as a function of the nodal velocity ug, pressure pg, VOF
 field phig, temperature Tg and node coordinates xg, all other state held
 fixed.  Its vector-Jacobian product is the CUDA kernel behind
-``ovs_residual_vjp``: the element's Gauss-point quantities are recomputed in
-forward-mode dual arithmetic for each nodal input; nothing is stored by the
-forward pass.
+``ovs_residual_vjp``: the element's Gauss-point quantities are recomputed and
+walked back in reverse mode; nothing is stored by the forward pass.
 """
 from __future__ import annotations
 

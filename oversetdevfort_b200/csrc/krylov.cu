@@ -485,10 +485,9 @@ gm_start_kernel(int N, int nf, int sys, const double* __restrict__ rhs, const TM
 
 // Krylov vectors are stored with a padded leading dimension (multiple of
 // 64 values) so every basis vector starts 256-byte aligned, by nodes (the nf
-// values of a node side by side; start and update convert).  The vector
-// being orthogonalized, w, is kept in FP64 whatever the basis precision, so
-// the projections of Gram-Schmidt do not lose the small remainder to FP32
-// rounding; only normalized vectors are rounded into the basis.
+// values of a node side by side; start and update convert).  The product
+// is written to its slot and orthogonalized there; dots are formed and added in
+// FP64 for either precision.
 inline size_t basis_ld(size_t n) { return (n + 63) & ~(size_t)63; }
 
 __device__ __forceinline__ void ld4v(const float* p, double v[4]) {
