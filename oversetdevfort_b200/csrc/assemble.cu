@@ -1048,8 +1048,8 @@ __device__ __forceinline__ unsigned mask_of(int v) {
 // per block, and the two lanes of an edge read the same element.  A warp per
 // row with one list per entry (28 values, 24 elements a load, an exchange
 // through shared memory) took 12.65 ms for the FP64 NS+VOF rows of the
-// 128^3 x6 tets and 6.91 ms in FP32; this takes 6.29 and 3.34 ms (T: 1.90 ->
-// 0.81 and 1.43 -> 0.46 ms).  A tile's edges are sorted by list
+// 128^3 x6 tets and 6.91 ms in FP32; this takes 5.91 and 3.35 ms (T: 1.90 ->
+// 0.66 and 1.43 -> 0.48 ms).  A tile's edges are sorted by list
 // length, so the rounds of a set are nearly equal.
 template <typename T, int KIND>
 __device__ __forceinline__ void write_entry(T* dst, T* v, const unsigned* masks, unsigned ibA, unsigned ibB) {
@@ -1172,7 +1172,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 3 : 4) edge_rows_kernel(
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[v] = (T)0;
     // several elements' loads in flight (lists of 4 to 8 are the rule): FP64 four
-    // at 3 blocks per SM, 6.63 -> 6.29 ms at 128^3 x6 (two or three 6.60 and 6.49,
+    // at 3 blocks per SM, 6.63 -> 6.29 ms at 128^3 x6 with tiles of 32 rows (two or three 6.60 and 6.49,
     // six 6.51; 4 blocks: 7.23 with two), FP32 three at 4 blocks, 3.56 -> 3.34 (two
     // 3.37, four 3.38, 5 blocks 3.47)
     constexpr int UNR = sizeof(T) == 8 ? 4 : 3;

@@ -9,7 +9,12 @@
 
 #define OVS_MAX_DEG 128        // longest CSR row supported (27*nshl hex bound = 216 not needed)
 #define OVS_MAX_KSPACE 400     // largest Krylov space
-#define OVS_TILE_ROWS 32       // rows per tile of the tet edge pass (a multiple of 16)
+// rows per tile of the tet edge pass: one round of its diagonal blocks, and about
+// two rounds of its edges.  FP64 NS+VOF rows at 128^3 x6 with tiles of 8, 16, 32:
+// 6.73, 5.91, 6.29 ms (T 0.66, 0.66, 0.81), FP32 3.72, 3.35, 3.34 (T 0.49, 0.48,
+// 0.46); 48x48x96 0.733, 0.655, 0.704 and 0.407, 0.374, 0.387; tiles of 64 rows
+// 0.818 and 0.459
+#define OVS_TILE_ROWS 16
 #define OVS_ASYNC_SLOTS 16     // assembly passes ovs_assemble_async queues before a wait
 #define OVS_RED_BLOCKS 592     // fixed grid of every deterministic reduction (4 x 148 SMs)
 #define OVS_RED_THREADS 256

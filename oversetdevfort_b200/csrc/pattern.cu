@@ -501,7 +501,7 @@ __global__ void edge_list_kernel(int nedge, const int4* __restrict__ edge, const
 // Tiles of 32, 128, 512 and 4096 rows: 2.98, 3.00, 3.01 and 3.08 ms for that
 // pass; without tiles (by the first row alone) a numbering along the mesh loses
 // its runs (128^3: elements 2.78 -> 3.34 ms).
-constexpr int ELEM_TILE_SHIFT = 5;
+constexpr int ELEM_TILE_SHIFT = 4;
 static_assert(OVS_TILE_ROWS == 1 << ELEM_TILE_SHIFT, "one tile size");
 
 __global__ void elem_key_kernel(const int* __restrict__ ien, int E, int nshl, const int* __restrict__ pos,
