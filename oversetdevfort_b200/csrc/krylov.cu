@@ -691,6 +691,10 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
 // partials itself.  w stays unnormalized: gm->sc[j] = 1 / |w| belongs to slot j,
 // and the product (linear in its vector), the dots and the coefficients carry
 // it, which saves the barrier and the pass over w that a division would need.
+// (FP32: the new vector takes the scale in FP64 and is rounded once.  With the
+// scale rounded to FP32 first, all of it was off by up to 2^-25 from what h
+// belongs to; the two conversions cost nothing, 126.7 us either way for an
+// iteration at 1.2M values, 980 at 10.7M.)
 // Each basis vector is read twice per step, as in MGS; the bound is that
 // traffic (two vectors a step at 6.4 TB/s) for long vectors and the chain
 // launch - dots - barrier - h - update for short ones.  Per iteration at k = 25
@@ -1015,7 +1019,6 @@ __device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_
   }
   // ---- phase B: the update and its norm
   double na = 0.0;
-  const TV skv = (TV)sk;
   const int cnt = gw < nsc ? (nsc - gw + W - 1) / W : 0;
   auto update = [&](auto nb, int r) {   // sub-chunks r, r - 1, .. of the warp's, their loads in flight together
     constexpr int NB = decltype(nb)::value, JB = V == 1 ? 2 * JG : JG;
@@ -1026,7 +1029,7 @@ __device__ __forceinline__ void orth_step(cg::grid_group& grid, TV* basis, size_
       i[m] = ((size_t)(gw + (long)(r - m) * W) * 32 + lane) * V;
       orth_ld<V>(w, i[m], n, wv[m]);
 #pragma unroll
-      for (int q = 0; q < V; ++q) wv[m][q] *= skv;
+      for (int q = 0; q < V; ++q) wv[m][q] = (TV)((double)wv[m][q] * sk);   // the coefficients' own sk, not its FP32 rounding
     }
     for (int j0 = 0; j0 < k; j0 += JB) {
       TV x[NB][JB][V];
