@@ -1264,7 +1264,10 @@ int plan_arnoldi(ovs_ctx* c, int sys, size_t n, int kspace, bool want_fused, Arn
     auto kern = orthog_kernel<TV>(pl->v);
     const size_t bytes = orth_smem(kspace);
     int per_sm = 0;
-    OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // the limit belongs to the kernel, whatever the context: always the largest
+    // space's (121,616 bytes), so that no call lowers it under another thread's cycle
+    OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)orth_smem(OVS_MAX_KSPACE)));
     OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ORTH_THREADS, bytes));
     if (per_sm >= 1 && c->num_sms >= 2 && nsc < ((size_t)1 << 31)) {
       pl->nsc = (int)nsc;
