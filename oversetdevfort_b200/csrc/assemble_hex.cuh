@@ -1155,8 +1155,11 @@ int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int pa
     }
   }
   if (!(parts & 2)) return OVS_OK;
-  auto launch = [&](auto kern, size_t smem, auto... more) -> int {
-    OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // most: the bytes for the longest row there is.  The limit belongs to the kernel,
+  // whatever the context, so it is always that: no call lowers it under another
+  // thread's launch
+  auto launch = [&](auto kern, size_t smem, size_t most, auto... more) -> int {
+    OVS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     int per_sm = 0;
     OVS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem));
     if (per_sm < 1) return OVS_ERR_ARG;
@@ -1172,11 +1175,15 @@ int launch_assemble_hex(ovs_ctx* c, const AsmArgs& a0, const SumArgs& sa, int pa
   if constexpr (KIND == OVS_ASM_NSVOF) {
     if (!tc) {
       const int carry = c->max_elem > HexRows<T>::EPC;
-      return launch(hex_block_rows_kernel<T>, HexRows<T>::bytes(a.max_deg, carry) * 4, carry);
+      return launch(hex_block_rows_kernel<T>, HexRows<T>::bytes(a.max_deg, carry) * 4,
+                    HexRows<T>::bytes(OVS_MAX_DEG, true) * 4, carry);
     }
-    if constexpr (can_tc) return launch(hex_rows_kernel<T, KIND, true>, HexSmem<T, KIND>::bytes(a.max_deg) * 4);
+    if constexpr (can_tc)
+      return launch(hex_rows_kernel<T, KIND, true>, HexSmem<T, KIND>::bytes(a.max_deg) * 4,
+                    HexSmem<T, KIND>::bytes(OVS_MAX_DEG) * 4);
     return OVS_ERR_ARG;
   } else {
-    return launch(hex_rows_kernel<T, KIND, false>, HexSmem<T, KIND>::bytes(a.max_deg) * 4);
+    return launch(hex_rows_kernel<T, KIND, false>, HexSmem<T, KIND>::bytes(a.max_deg) * 4,
+                  HexSmem<T, KIND>::bytes(OVS_MAX_DEG) * 4);
   }
 }

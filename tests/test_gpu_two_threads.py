@@ -2,8 +2,8 @@
 of one need more dynamic shared memory than calls of the other: that limit
 belongs to the kernel, not to the context, so a call must not lower it under
 another thread's launches.  Krylov spaces of 200 and 3 (a 200-step cycle asks
-for 60.8 KB in its last steps).  Every call runs to its end and gives the bits
-it gives alone.
+for 60.8 KB in its last steps), and hexahedral row passes of rows of 27 and of
+8 columns.  Every call runs to its end and gives the bits it gives alone.
 The systems are small: all blocks of both threads fit the device at once."""
 import threading
 
@@ -60,3 +60,24 @@ def test_krylov_spaces_of_two_threads():
     _beside(large, small)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("kernel,system", [(F.OVS_ASM_NSVOF, F.OVS_SYS_NSVOF), (F.OVS_ASM_TEM, F.OVS_SYS_TEM)])
+def test_hexahedral_rows_of_two_threads(kernel, system):
+    a = Context.from_case(M.random_case(3, 3, 3, seed=5, kernel=kernel, hex=True))
+    b = Context.from_case(M.random_case(1, 1, 1, seed=6, kernel=kernel, hex=True))
+    refs = []
+    for c in (a, b):
+        c.assemble(kernel, 6, F.OVS_FP64)
+        refs.append(c.get_system(system))
+
+    def large():
+        for _ in range(1000):
+            a.assemble(kernel, 6, F.OVS_FP64)
+
+    _beside(large, lambda: b.assemble(kernel, 6, F.OVS_FP64))
+    for c, ref in zip((a, b), refs):
+        got = c.get_system(system)
+        for k in ref:
+            np.testing.assert_array_equal(got[k], ref[k], err_msg=k)
+        c.close()
