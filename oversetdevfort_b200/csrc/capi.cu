@@ -310,6 +310,10 @@ int ovs_upload_mesh(ovs_ctx* c, const double* xg, const int* ien, const int* elm
   cudaStream_t s = c->stream;
   const size_t EN = (size_t)c->E * c->nshl;
   if (xg) OVS_CUDA_TRY(cudaMemcpyAsync(c->field[OVS_F_XG], xg, sizeof(double) * 3 * (size_t)c->N, cudaMemcpyHostToDevice, s));
+  // until this one is accepted there is no mesh: its connectivity replaces an
+  // earlier mesh's before it is checked
+  c->have_mesh = false;
+  c->have_pattern = false;
   int *tmp = nullptr, *bad = nullptr;
   OVS_CUDA_TRY(cudaMallocAsync(&tmp, sizeof(int) * EN, s));
   OVS_CUDA_TRY(cudaMallocAsync(&bad, sizeof(int), s));
@@ -331,7 +335,6 @@ int ovs_upload_mesh(ovs_ctx* c, const double* xg, const int* ien, const int* elm
   OVS_CUDA_TRY(cudaStreamSynchronize(s));
   if (hbad) return OVS_ERR_ARG;
   c->have_mesh = true;
-  c->have_pattern = false;
   return OVS_OK;
 }
 
