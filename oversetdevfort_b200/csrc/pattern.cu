@@ -619,8 +619,29 @@ static int build_edges(ovs_ctx* c) {
   return OVS_OK;
 }
 
+// what an earlier pattern sized by its entries: columns, matrices, transpose
+static void drop_entries(ovs_ctx* c) {
+  void** p[] = {(void**)&c->colidx, (void**)&c->tmap, (void**)&c->vals_t};
+  for (void** q : p) {
+    if (*q) cudaFree(*q);
+    *q = nullptr;
+  }
+  for (auto& sys : c->sys)
+    for (SysStore& S : sys) {
+      if (S.vals) cudaFree(S.vals);
+      S.vals = nullptr;
+      S.have_mat = false;
+    }
+  c->nnz = 0;
+}
+
+// A context may build a pattern again, on the same mesh (matrices stay) or on
+// another one of as many nodes and elements.  A pattern of another length drops
+// what the earlier one sized, and so does a build that is refused, since the row
+// pointers are then no longer those of the matrices.
 int ovs_pattern_build(ovs_ctx* c) {
   cudaStream_t s = c->stream;
+  c->have_pattern = false;   // until this one is whole
   const int N = c->N, E = c->E, nshl = c->nshl;
   const size_t EN = (size_t)E * nshl;
   int st;
@@ -653,6 +674,7 @@ int ovs_pattern_build(ovs_ctx* c) {
   int nnz = 0;
   OVS_CUDA_TRY(cudaMemcpyAsync(&nnz, c->rowptr + N, sizeof(int), cudaMemcpyDeviceToHost, s));
   OVS_CUDA_TRY(cudaStreamSynchronize(s));
+  if (h[0] != 0 || h[1] != 0 || nnz != c->nnz) drop_entries(c);
   if (h[0] != 0) { cudaFreeAsync(cnt, s); cudaFreeAsync(tmp, s); cudaFreeAsync(stats, s); return OVS_ERR_ARG; }
   if (h[1] != 0) { cudaFreeAsync(cnt, s); cudaFreeAsync(tmp, s); cudaFreeAsync(stats, s); return OVS_ERR_PATTERN; }
   c->max_elem = h[2];
