@@ -390,6 +390,10 @@ int ovs_gmres(ovs_ctx* ctx, int system, double tol, int kspace,
  * on entry do not matter and which overlaps no column. */
 int ovs_gmres_from(ovs_ctx* ctx, int system, double tol, int kspace, int kspace_min,
                    const double* const* start, double* sol, ovs_gmres_info* info);
+/* The same with the result in columns of N values too (one host pointer per
+ * field), which overlap neither one another nor the start's. */
+int ovs_gmres_columns(ovs_ctx* ctx, int system, double tol, int kspace, int kspace_min,
+                      const double* const* start, double* const* sol, ovs_gmres_info* info);
 
 /* Solve A x = b to ||b - A x||_2 <= rtol ||b||_2 (true residual, FP64).
  * mode OVS_FP64: restarted FP64 GMRES(kspace) on the FP64 system.

@@ -286,19 +286,18 @@ class Context:
 
     def gmres(self, system: int, tol: float, kspace: int, kspace_min: int, sol: np.ndarray):
         start = _f64(np.reshape(sol, (self.N, NF[system]), order="F"))
-        return self._gmres_columns(system, tol, kspace, kspace_min, [start[:, k] for k in range(NF[system])])
-
-    def _gmres_columns(self, system: int, tol: float, kspace: int, kspace_min: int, cols):
-        """One cycle from the start vector's columns (nf contiguous FP64 arrays of N, not written); returns the
-        new solution (N, nf) and the info."""
-        if [c.shape for c in cols] != [(self.N,)] * NF[system]:
-            raise ValueError(f"start vector: {NF[system]} columns of {self.N} values expected")
         s = np.empty((self.N, NF[system]), order="F")
+        return s, self._gmres_columns(system, tol, kspace, kspace_min, start.T, s.T)
+
+    def _gmres_columns(self, system: int, tol: float, kspace: int, kspace_min: int, start, sol):
+        """One cycle from the start vector's columns (nf contiguous FP64 arrays of N, not written), the new
+        solution to the columns `sol` (the same; they overlap nothing); returns the info."""
+        if [c.shape for c in start] != [(self.N,)] * NF[system]:
+            raise ValueError(f"start vector: {NF[system]} columns of {self.N} values expected")
         info = F.OvsGmresInfo()
-        F.check(self.lib.ovs_gmres_from(self.h, system, tol, kspace, kspace_min,
-                                        (C.POINTER(C.c_double) * len(cols))(*(_dptr(c) for c in cols)), _dptr(s),
-                                        C.byref(info)), "ovs_gmres")
-        return s, info
+        cols = [(C.POINTER(C.c_double) * NF[system])(*(_dptr(c) for c in a)) for a in (start, sol)]
+        F.check(self.lib.ovs_gmres_columns(self.h, system, tol, kspace, kspace_min, *cols, C.byref(info)), "ovs_gmres")
+        return info
 
     def solve(self, system: int, mode: int, rtol: float, kspace: int = 50, max_cycles: int = 100,
               want_solution: bool = True):
@@ -505,25 +504,26 @@ def SparseGMRES_up(ctx: Context, Utol: float, Kspaceu: int, Kspaceu_mn: int,
                    solu: np.ndarray, solp: np.ndarray):
     """src/SparseGMRES_NS.f90:4-369 on the resident FP64 (u,p) system; solu
     (N,3) and solp (N) are accumulated into and returned with the info."""
-    u = _f64(solu).reshape(-1, 3, order="F")
-    s, info = ctx._gmres_columns(F.OVS_SYS_NS, Utol, Kspaceu, Kspaceu_mn,
-                                 [u[:, 0], u[:, 1], u[:, 2], _f64(solp).reshape(-1)])
-    return s[:, :3], s[:, 3], info
+    start = _f64(solu).reshape(-1, 3, order="F")
+    u, p = np.empty((ctx.N, 3), order="F"), np.empty(ctx.N)
+    info = ctx._gmres_columns(F.OVS_SYS_NS, Utol, Kspaceu, Kspaceu_mn, [*start.T, _f64(solp).reshape(-1)], [*u.T, p])
+    return u, p, info
 
 
 def SparseGMRES_ns_conv(ctx: Context, Utol: float, Kspaceu: int, Kspaceu_mn: int,
                         solu: np.ndarray, solp: np.ndarray, solls: np.ndarray):
     """src/SparseGMRES_NS_conv.f:1-406 on the resident FP64 (u,p,phi) system."""
-    u = _f64(solu).reshape(-1, 3, order="F")
-    s, info = ctx._gmres_columns(F.OVS_SYS_NSVOF, Utol, Kspaceu, Kspaceu_mn,
-                                 [u[:, 0], u[:, 1], u[:, 2], _f64(solp).reshape(-1), _f64(solls).reshape(-1)])
-    return s[:, :3], s[:, 3], s[:, 4], info
+    start = _f64(solu).reshape(-1, 3, order="F")
+    u, p, ls = np.empty((ctx.N, 3), order="F"), np.empty(ctx.N), np.empty(ctx.N)
+    info = ctx._gmres_columns(F.OVS_SYS_NSVOF, Utol, Kspaceu, Kspaceu_mn,
+                              [*start.T, _f64(solp).reshape(-1), _f64(solls).reshape(-1)], [*u.T, p, ls])
+    return u, p, ls, info
 
 
 def SparseGMRES_tem(ctx: Context, Utol: float, Kspaceu: int, Kspaceu_mn: int, sol: np.ndarray):
     """src/SparseGMRES_tem.f90:1-256 on the resident FP64 temperature system."""
-    s, info = ctx._gmres_columns(F.OVS_SYS_TEM, Utol, Kspaceu, Kspaceu_mn, [_f64(sol).reshape(-1)])
-    return s[:, 0], info
+    t = np.empty(ctx.N)
+    return t, ctx._gmres_columns(F.OVS_SYS_TEM, Utol, Kspaceu, Kspaceu_mn, [_f64(sol).reshape(-1)], [t])
 
 
 def calculate_residual(ctx: Context, precision: int = F.OVS_FP64) -> np.ndarray:

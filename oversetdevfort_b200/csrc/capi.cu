@@ -693,16 +693,16 @@ int ovs_precond_device(ovs_ctx* c, int sys, int prec, const double* dx, double* 
   return OVS_OK;
 }
 
-// One cycle from the host columns `cols` (the start vector), the result to `out`
-// (host, N x nf column-major), which may be the columns themselves.  The upload
-// and the first touch of `out` go on while the device iterates: the copies in
-// front of and behind a cycle took 30 of 121 ms at 2.1M nodes (50 steps).
+// One cycle from the host columns `cols` (the start vector), the result to the
+// host columns `out`, which may be the same ones.  The upload and the first touch
+// of `out` go on while the device iterates: the copies in front of and behind a
+// cycle took 30 of 121 ms at 2.1M nodes (50 steps).
 static int gmres_host(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, const double* const* cols,
-                      double* out, bool touch, ovs_gmres_info* info) {
+                      double* const* out, bool touch, ovs_gmres_info* info) {
+  if (kspace < 1 || kspace > OVS_MAX_KSPACE) return OVS_ERR_ARG;
   int st;
   if ((st = ovs_activate(c))) return st;
   const int nf = ovs_sys_nf(sys);
-  const size_t n = (size_t)c->N * nf;
   if ((st = ovs_ensure((void**)&c->sol[sys], sizeof(double) * 5 * (size_t)c->N))) return st;
   // earlier work on sol (a queued update) comes first
   OVS_CUDA_TRY(cudaEventRecord(c->ev_sol, c->stream));
@@ -723,26 +723,41 @@ static int gmres_host(ovs_ctx* c, int sys, double tol, int kspace, int kspace_mi
     OVS_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     c->last_ms = ms;
   }
-  OVS_CUDA_TRY(cudaMemcpyAsync(out, c->sol[sys], sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+  for (int f = 0, m; f < nf; f += m) {   // columns that follow one another in one copy
+    for (m = 1; f + m < nf && out[f + m] == out[f] + (size_t)m * c->N; ++m) {}
+    OVS_CUDA_TRY(cudaMemcpyAsync(out[f], c->sol[sys] + (size_t)f * c->N, sizeof(double) * m * (size_t)c->N,
+                                 cudaMemcpyDeviceToHost, c->stream));
+  }
   OVS_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (info) *info = gi;
   return OVS_OK;
 }
 
+// the columns of an N x nf array
+static void columns_of(const ovs_ctx* c, int sys, double* a, double* col[5]) {
+  for (int f = 0; f < 5; ++f) col[f] = f < ovs_sys_nf(sys) ? a + (size_t)f * c->N : nullptr;
+}
+
 int ovs_gmres(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, double* sol, ovs_gmres_info* info) {
   if (!sys_ok(c, sys, OVS_FP64) || !sol) return OVS_ERR_ARG;
-  if (kspace < 1 || kspace > OVS_MAX_KSPACE) return OVS_ERR_ARG;
-  const double* cols[5];
-  for (int f = 0; f < 5; ++f) cols[f] = sol + (size_t)f * (f < ovs_sys_nf(sys) ? c->N : 0);
-  return gmres_host(c, sys, tol, kspace, kspace_min, cols, sol, false, info);
+  double* cols[5];
+  columns_of(c, sys, sol, cols);
+  return gmres_host(c, sys, tol, kspace, kspace_min, cols, cols, false, info);
 }
 
 int ovs_gmres_from(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, const double* const* start,
                    double* sol, ovs_gmres_info* info) {
   if (!sys_ok(c, sys, OVS_FP64) || !start || !sol) return OVS_ERR_ARG;
-  if (kspace < 1 || kspace > OVS_MAX_KSPACE) return OVS_ERR_ARG;
+  double* cols[5];
+  columns_of(c, sys, sol, cols);
+  return ovs_gmres_columns(c, sys, tol, kspace, kspace_min, start, cols, info);
+}
+
+int ovs_gmres_columns(ovs_ctx* c, int sys, double tol, int kspace, int kspace_min, const double* const* start,
+                      double* const* sol, ovs_gmres_info* info) {
+  if (!sys_ok(c, sys, OVS_FP64) || !start || !sol) return OVS_ERR_ARG;
   for (int f = 0; f < ovs_sys_nf(sys); ++f)
-    if (!start[f]) return OVS_ERR_ARG;
+    if (!start[f] || !sol[f]) return OVS_ERR_ARG;
   return gmres_host(c, sys, tol, kspace, kspace_min, start, sol, true, info);
 }
 

@@ -1631,7 +1631,7 @@ int ovs_feed(ovs_ctx* c, SolFeed* f, size_t count) {
                                  c->sol_stream));
     if (f->out) {
       constexpr size_t PAGE = 4096 / sizeof(double);
-      volatile double* o = f->out + f->at;
+      volatile double* o = f->out[col] + off;
       for (size_t i = 0; i < m; i += PAGE) o[i] = 0.0;
     }
     f->at += m;

@@ -231,13 +231,13 @@ int ovs_precond_apply_impl(ovs_ctx* c, int sys, int prec, const double* dx, doub
 // The start vector of a cycle on its way from the host: columns of N values, in
 // any memory, to dst (column-major).  A cycle needs it for the last update only,
 // so the host copies it in pieces between the launches of the cycle's steps
-// (sol_stream), and touches the pages of `out`, where the result will land.
+// (sol_stream), and touches the pages of `out`, the columns where the result will land.
 struct SolFeed {
   const double* const* cols;
   int ncol;
   size_t n;            // values per column
   double* dst;
-  double* out;         // host pages to touch (null: none)
+  double* const* out;  // host columns whose pages to touch (null: none)
   size_t at = 0;       // values sent so far
 };
 // queue the next `count` values (of n * ncol; every one left for 0)
