@@ -35,8 +35,6 @@ namespace {
 // ------------------------------------------------------------------ params
 struct AsmArgs {
   const void* rec;        // alpha-stage node records, REC values per node
-  const int* ien;         // E*nshl element-major, 0-based
-  const int* elm_id;      // E
   const uint8_t* ibc;     // N
   const int* rowptr;
   const int* colidx;
@@ -52,7 +50,6 @@ struct AsmArgs {
   void* rhs;              // NF*N field-major
   const void* kbuf;       // hex tensor-core block values (E x 64 x 24), or null
   int* flags;             // [0] non-positive DetJ count, [1] non-finite residual
-  unsigned long long* cfl_bits;
   int N;
   int mat, vec;
   int max_deg;
@@ -1089,7 +1086,7 @@ __device__ __forceinline__ void diag_row(const AsmArgs& a, const int4 rr, bool o
     for (int f = 0; f < 4; ++f) v[NV + f] += r[f];
     if constexpr (NF == 5) v[NV + 4] += __ldg(se + L::RHS0 + 16 + la);
   }
-  // lane l ends up with values 4 l' .. 4 l' + 3, l' = l with its bits reversed
+  // lane l ends up with group l, the values 4 l .. 4 l + 3
 #pragma unroll
   for (int half = 16, off = 4; off >= 1; half >>= 1, off >>= 1) {
     const bool up = l8 & off;
@@ -1100,7 +1097,7 @@ __device__ __forceinline__ void diag_row(const AsmArgs& a, const int4 rr, bool o
     }
   }
   if (!on) return;
-  const int g = ((l8 >> 2) & 1) * 4 + (l8 & 2) + (l8 & 1);
+  const int g = l8;
   const unsigned ibA = __ldg(a.ibc + A);
   if (g < NG) {
     if (deg > 0) {
@@ -1955,8 +1952,6 @@ static void fill_args(ovs_ctx* c, int prec, SysStore& S, int tensor_flag, AsmArg
   sa.E = c->E;
   sa.p = c->params;
   a.rec = c->esum[prec];     // pass 2 reads the summaries
-  a.ien = c->ien;
-  a.elm_id = c->elm_id;
   a.ibc = c->ibc;
   a.rowptr = c->rowptr;
   a.colidx = c->colidx;
@@ -1965,7 +1960,6 @@ static void fill_args(ovs_ctx* c, int prec, SysStore& S, int tensor_flag, AsmArg
   a.vals = S.vals;
   a.rhs = S.rhs;
   a.flags = c->flags;
-  a.cfl_bits = c->cfl_bits;
   a.N = c->N;
   a.mat = (tensor_flag & OVS_TENSOR_MAT) != 0;
   a.vec = (tensor_flag & OVS_TENSOR_VEC) != 0;

@@ -506,13 +506,12 @@ __device__ __forceinline__ void st4v(double* p, const double v[4]) {
   reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
 }
 
-// v = w / d with d = unorm0 (first vector) or sqrt(beta) (later vectors):
-// the normalization of SparseGMRES_NS.f90:159-160,291-294
-template <typename TV, typename TW>
+// the first vector: v = w / unorm0 (SparseGMRES_NS.f90:159-160; later vectors
+// stay unnormalized, see gm_orthog_kernel)
+template <typename TV>
 __global__ void __launch_bounds__(OVS_RED_THREADS)
-gm_normalize_kernel(const TW* w, TV* v, size_t n, GmresDev* gm, int first) {
-  if (gm->done && !first) return;
-  const double d = first ? gm->unorm0 : sqrt(gm->beta);
+gm_normalize_kernel(const double* w, TV* v, size_t n, const GmresDev* gm) {
+  const double d = gm->unorm0;
   if (!(d != 0.0)) return;
   const size_t n4 = n >> 2, stride = (size_t)gridDim.x * blockDim.x;
   const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -522,7 +521,7 @@ gm_normalize_kernel(const TW* w, TV* v, size_t n, GmresDev* gm, int first) {
     a[0] /= d; a[1] /= d; a[2] /= d; a[3] /= d;
     st4v(v + 4 * q, a);
   }
-  for (size_t i = 4 * n4 + t0; i < n; i += stride) v[i] = (TV)((double)w[i] / d);
+  for (size_t i = 4 * n4 + t0; i < n; i += stride) v[i] = (TV)(w[i] / d);
 }
 
 // H(k+1,k) = unorm, Givens rotations of column k (Hk[0..k) in, its rotated form
@@ -1351,7 +1350,7 @@ int gmres_cycle(ovs_ctx* c, int sys, const double* rhs, double* sol, double tol,
   OVS_CUDA_TRY(cudaMemsetAsync(gm->e, 0, sizeof(double) * (size_t)(kspace + 1), s));
   gm_start_kernel<TM, double><<<OVS_RED_BLOCKS, OVS_RED_THREADS, 0, s>>>(N, nf, sys, rhs, pre, wd, tol, gm,
                                                                          rhs_pre ? 1 : 0);
-  gm_normalize_kernel<TV, double><<<OVS_RED_BLOCKS, OVS_RED_THREADS, 0, s>>>(wd, V, n, gm, 1);
+  gm_normalize_kernel<TV><<<OVS_RED_BLOCKS, OVS_RED_THREADS, 0, s>>>(wd, V, n, gm);
   c->launches += 2;
   OVS_CUDA_TRY(cudaGetLastError());
   // one Arnoldi iteration per step (see ArnoldiPlan)

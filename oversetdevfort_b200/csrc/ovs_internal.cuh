@@ -168,7 +168,6 @@ struct ovs_ctx {
   void* basis[2] = {nullptr, nullptr};   // Krylov basis per precision
   size_t basis_bytes[2] = {0, 0};
   double* work64 = nullptr;              // 3 vectors of 5N doubles (b, r, x)
-  float* work32 = nullptr;               // 1 vector of 5N floats
   double* wvec = nullptr;                // FP64 vector under orthogonalization
   double* coop_part = nullptr;           // partial sums of the cooperative Arnoldi kernels, then T = (I + L)^-1
   size_t coop_bytes = 0;                 //   (rows of kspace, strictly lower part)
