@@ -717,18 +717,15 @@ static int gmres_host(ovs_ctx* c, int sys, double tol, int kspace, int kspace_mi
     return st;
   }
   OVS_CUDA_TRY(cudaEventRecord(c->ev1, c->stream));
-  OVS_CUDA_TRY(cudaEventSynchronize(c->ev1));
-  {
-    float ms = 0.f;
-    OVS_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    c->last_ms = ms;
-  }
   for (int f = 0, m; f < nf; f += m) {   // columns that follow one another in one copy
     for (m = 1; f + m < nf && out[f + m] == out[f] + (size_t)m * c->N; ++m) {}
     OVS_CUDA_TRY(cudaMemcpyAsync(out[f], c->sol[sys] + (size_t)f * c->N, sizeof(double) * m * (size_t)c->N,
                                  cudaMemcpyDeviceToHost, c->stream));
   }
   OVS_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  float ms = 0.f;
+  OVS_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+  c->last_ms = ms;
   if (info) *info = gi;
   return OVS_OK;
 }
