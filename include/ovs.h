@@ -202,10 +202,13 @@ int ovs_synchronize(ovs_ctx* ctx);
 /* the cudaStream_t every call of this context is issued on */
 int ovs_get_stream(ovs_ctx* ctx, void** stream);
 
-/* mesh: xg(N,3), IEN(E,nshl) 1-based, ELM_ID(E) (may be NULL: all 102) */
+/* mesh: xg(N,3), IEN(E,nshl) 1-based, ELM_ID(E) (may be NULL: all 102).  May be
+ * called again, with ovs_build_pattern after it; a refused mesh leaves none. */
 int ovs_upload_mesh(ovs_ctx* ctx, const double* xg, const int* ien,
                     const int* elm_id);
-/* genSparStruc on the resident mesh; *icnt receives the entry count */
+/* genSparStruc on the resident mesh; *icnt receives the entry count.  Matrices of
+ * an earlier pattern stay if its entry count was the same, and go otherwise and
+ * when the build is refused. */
 int ovs_build_pattern(ovs_ctx* ctx, int* icnt);
 /* copy the pattern out (1-based, reference layout), col(N+1), row(icnt) */
 int ovs_get_pattern(ovs_ctx* ctx, int* col, int* row);

@@ -108,8 +108,6 @@ template <typename T> struct ZeroRecs {
   __device__ __forceinline__ ZeroRow<T> operator[](int) const { return ZeroRow<T>{}; }
 };
 
-// SMEMREC (FP64 only): the node records through shared memory (a 3-block
-// register bound) instead of registers (255 registers, 2 blocks)
 // VOF field at tet Gauss point g in FP64 from the record value (slot k)
 // plus its rounding remainder (lo[.][3]): sum_a N_a phi_a, in node order
 template <typename T, typename RA, typename LA>
@@ -242,11 +240,11 @@ __device__ __forceinline__ void cfl_max(unsigned long long* bits, double v) {
 // ----------------------------------------------------- element summaries
 // Pass 1 (one thread per element) evaluates everything the element matrix
 // needs from its Gauss points, once, plus the element's residual rows, and
-// stores it as a compact summary of SW values.  Pass 2 (one warp per CSR
-// row) expands A's row of each element matrix from the summaries.  Inactive
+// stores it as a compact summary of SW values.  Pass 2 (the edge pass) forms
+// the blocks of each element matrix from the summaries.  Inactive
 // elements (solid on the NS+VOF pass, non-target on the NS pass) store zero
 // sums and zero residuals, which makes every expanded block exactly zero.
-// NS / NS+VOF: the Gauss-point sums of the block formulas (see form_block),
+// NS / NS+VOF: the Gauss-point sums of the block formulas (see add_block),
 // which pass 1 forms once per element, in groups of 4 values that a lane of
 // the edge pass reads with one load each:
 //   [0, ND0)    per (row node a, column node b), PW values at PW (4a + b):
@@ -282,7 +280,7 @@ __device__ __forceinline__ constexpr int tet_edge(int a, int b) { return a * (5 
 // a 32-byte boundary) with one vector store.  FP64 uses the 256-bit global
 // store of sm_100: one instruction instead of two 128-bit stores, measured
 // 5.9 against 7.1 ms for the FP64 NS+VOF element pass at 128^3 (the pass
-// writes 31 such groups per tet).  The asm carries no memory clobber: the
+// writes 29 such groups per tet).  The asm carries no memory clobber: the
 // element pass never reads a summary it writes, and the row pass that
 // reads it is a later launch
 template <typename T>
@@ -296,7 +294,7 @@ __device__ __forceinline__ void put4(double* d, double a, double b, double c, do
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(d), "d"(a), "d"(b), "d"(c), "d"(e));
 }
 
-// The Gauss-point sums of the NS / NS+VOF block formulas (form_block)
+// The Gauss-point sums of the NS / NS+VOF block formulas (add_block)
 // from the per-point values q (layout GQ above), the shape gradients g and
 // the weight w, written to the summary o: with c_n = uadv . grad N_n,
 //   S_ab  = sum w rho (Na + rt ca)(fact1 Nb + fact2 cb)
@@ -1040,9 +1038,11 @@ __device__ __forceinline__ unsigned mask_of(int v) {
 // lane l's elements l, l + 8, ... and then the lanes by halving: orders fixed
 // by the mesh, the same on every run.
 // Bound: the summaries are read in scattered 32-byte pieces, which the L1
-// data path serves at a quarter of its rate, so what counts is the bytes a
-// block asks for and how many distinct elements a load touches: 22 values
-// per block, and the two lanes of an edge read the same element.  A warp per
+// data path serves at a quarter of its rate (L1 67% busy in FP64), and the loads'
+// latency at 10.6 warps per SM (12.6 cycles of waiting per instruction).  So what
+// counts is the bytes a block asks for, how many distinct elements a load touches
+// and how many loads are in flight: 22 values per block, and the two lanes of an
+// edge read the same element.  A warp per
 // row with one list per entry (28 values, 24 elements a load, an exchange
 // through shared memory) took 12.65 ms for the FP64 NS+VOF rows of the
 // 128^3 x6 tets and 6.91 ms in FP32; this takes 5.91 and 3.35 ms (T: 1.90 ->

@@ -439,8 +439,8 @@ __device__ __forceinline__ void hex_point(const T (&ga)[4], const T (&gb)[4], T 
 // the constant W = f_g (x) f_g shared by all elements, on tcgen05 (kind::tf32,
 // A and W K-major in shared memory without swizzle, D in TMEM).  FP32
 // accuracy comes from the 3xTF32 split A_hi W_hi + A_hi W_lo + A_lo W_hi
-// (W's split precomputed on the host).  One CTA of 128 threads per SM loops
-// over tiles of 16 elements with 256 threads; thread (element el, point g)
+// (W's split precomputed on the host).  One CTA of 256 threads per SM loops
+// over tiles of 16 elements; thread (element el, point g)
 // of each half builds its point's 4x4 C' for 4 of a group's 8 slot values
 // (three groups of 8 cover the 24; the value is a template parameter),
 // thread 0 issues the 48 MMAs of a group into its 64 TMEM columns and
@@ -501,7 +501,7 @@ __device__ __forceinline__ void tc_ld16(uint32_t addr, float* v) {
 
 // C' (reference features, row-major 4x4: [r][s], r on the row node a) of slot
 // value t at one point, from the point record q (HexTcLay): the per-point
-// forms of hex_expand_block with u.grad N = v . dN/dxi (v = dxi/dx uadv),
+// forms of hex_point with u.grad N = v . dN/dxi (v = dxi/dx uadv),
 // grad N_a . grad N_b = dN_a/dxi Gh dN_b/dxi (Gh = dxi/dx dxi/dx^T) and the
 // physical derivative j = dN/dxi . a_j (a_j column j of dxi/dx).
 template <int t>
@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 8 ? 4 : 5)) hex_block_rows_
       }
       const int la = pk & 7;
       const T* mine = sum + (size_t)(pk >> 3) * L::SW;
-      auto fetch = [&](int k) {   // stage k: points 2 k, 2 k + 1 of the chunk's elements, an element by its 4 lanes
+      auto fetch = [&](int k) {   // stage k: points 2 k, 2 k + 1 of the chunk's elements, an element by its 8 lanes
         if (on) {
           unsigned char* dst = reinterpret_cast<unsigned char*>(st + ((k & 1) * EPC + el) * H::ES) + 16 * cp;
           const unsigned char* src = reinterpret_cast<const unsigned char*>(mine + k * H::GPS * H::GPW) + 16 * cp;

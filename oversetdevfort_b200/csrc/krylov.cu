@@ -6,19 +6,21 @@
 // src/SparseGMRES_NS_conv.f:1-406, src/SparseGMRES_tem.f90:1-256).
 //
 // SpMV: a group of lanes owns one CSR row.  The slot values of a row are
-// contiguous (24/16/1 per slot), so the lanes of a group read one 16-byte
-// group each per slot and the whole row streams with full sectors; the x
-// gathers hit L2.  The preconditioner (exact 3x3 inverse of the velocity
+// contiguous (24/16/1 per slot), so the lanes of a group read four values each
+// per slot (16 bytes in FP32, 32 in FP64) and the whole row streams with full
+// sectors; the x gathers hit L2.  The preconditioner (exact 3x3 inverse of the velocity
 // diagonal block, reciprocal diagonal for p / phi / T) is applied to the row
 // result before the store, so one pass produces P^-1 A x.
 //
 // GMRES: one Arnoldi cycle follows the reference step by step (left
-// preconditioning, modified Gram-Schmidt with the reference's fused
-// "project off j-1, dot with j" order, Givens rotations, exit rule
-// |e(k+1)| <= tol |P^-1 b| and k >= kspace_min, back-substitution,
-// sol += sum y_j v_j).  All scalars live on the device; every dot product is
-// a fixed-grid, fixed-order FP64 reduction (last-block-done), so results are
-// bit-identical from run to run.  The host only polls the "done" word once
+// preconditioning, the coefficients of modified Gram-Schmidt, Givens rotations,
+// exit rule |e(k+1)| <= tol |P^-1 b| and k >= kspace_min, back-substitution,
+// sol += sum y_j v_j).  The coefficients of a step come from one pass of dots
+// and a triangular product (gm_orthog_kernel); the one-launch variant
+// (gm_arnoldi_kernel) takes them one after another in the reference's "project
+// off j-1, dot with j" order.  All scalars live on the device; every dot product
+// is added in FP64 in an order fixed by the grid, so results are bit-identical
+// from run to run.  The host only polls the "done" word once
 // per batch of iterations, a batch behind the launches.
 #include "ovs_internal.cuh"
 
@@ -42,11 +44,15 @@ __host__ __device__ constexpr int spmv_threads() { return AOS || sizeof(TM) == 4
 
 template <typename T> __device__ __forceinline__ T ldm(const T* p) { return __ldcs(p); }
 
-// Four matrix values.  FP64: one 32-byte load instead of two of 16 (1.09 -> 1.02
-// ms at 2.1M nodes, 25 -> 17 us at 31K), evicted first from L2, where the Krylov
-// basis is worth more: per iteration at k = 25 31K nodes 46 us (51 without the
-// hint, 49 before), 236K nodes 199 (202, 207), 2.1M nodes 1.73 ms (1.71, 1.83).
-// FP32: no hint (a streaming load costs 0.57 -> 0.61 ms at 2.1M nodes).
+// Four matrix values.  FP64: one 32-byte load instead of two streaming ones of 16,
+// evicted first from L2, where the Krylov basis is worth more.  FP32: no hint.
+// NS+VOF product with vectors by nodes, and in brackets the whole iteration at
+// k = 25, at 31K, 233K and 2.1M nodes:
+//   FP64  two of 16, streaming     24.4 (49.2), 111 (202), 1113 us (1765)
+//         one of 32                16.6 (51.3), 119 (199), 1035    (1687)
+//         one of 32, evict first   20.7 (45.4), 107 (196), 1060    (1711)
+//   FP32  one of 16, streaming     12.4 (37.7),  60 (127),  611    (972)
+//         one of 16                10.5 (36.8),  69 (126),  576    (938)
 __device__ __forceinline__ void ld4(const float* p, float v[4]) {
   asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
@@ -72,13 +78,13 @@ template <> struct AccT<float, float, false> { using type = float; };
 // the shuffles).
 // AOS: x and y by nodes (x[node nf + field]), as the Krylov basis holds its
 // vectors, instead of by fields: a slot's gathers fall into one or two sectors
-// instead of one per field (FP32 66.0 -> 62.1 us at 236K nodes, 0.627 -> 0.597 ms
+// instead of one per field (FP32 66.0 -> 62.1 us at 233K nodes, 0.627 -> 0.597 ms
 // at 2.1M).  The kernel waits for its loads (20 stalled warps per issue), so the
 // warps in flight decide: blocks of 64 threads, whose places are refilled sooner
 // than those of 256, gain 1 to 8% there and for FP32 matrices by fields, and lose
-// 7% for FP64 by fields.  With the loads of ld4, at 236K and 2.1M nodes: by nodes
-// FP64 0.109 and 1.05 ms, FP32 0.069 (0.061 with the basis out of L2) and 0.57; its
-// bytes at 6.45 TB/s: 0.106 and 0.98, 0.053 and 0.50.
+// 7% for FP64 by fields.  Times: ld4.  Its bytes with the preconditioner's at 6.45
+// TB/s, at 233K and 2.1M nodes: FP64 110 and 1024 us, FP32 56 and 522; with the
+// benchmark's system at 2.1M nodes it takes 1051 and 557, 97% and 94% of that rate.
 // LIST: the warp chunks run over the row list rows[0, nrows) (local row
 // indices; an index outside [0, N) is skipped) instead of rows 0..N-1;
 // each listed row is computed exactly as in the full product.
@@ -696,10 +702,13 @@ gm_arnoldi_kernel(int N, const int* __restrict__ rowptr, const int* __restrict__
 // iteration at 1.2M values, 980 at 10.7M.)
 // Each basis vector is read twice per step, as in MGS; the bound is that
 // traffic (two vectors a step at 6.4 TB/s) for long vectors and the chain
-// launch - dots - barrier - h - update for short ones.  Per iteration at k = 25
-// (FP64, SpMV included; in brackets with the leftovers before the barrier of
-// the same step): 4.9K nodes 21 us (28), 31K nodes 54 (57), 236K nodes 0.207 ms
-// (0.213), 2.1M nodes 1.78 ms (1.80).
+// launch - dots - barrier - h - update for short ones.  One iteration at k = 25,
+// product included, in FP64: 4.9K nodes 27 us ((u,p) system 22), 31K nodes 45, 233K
+// nodes 0.196 ms, 2.1M nodes 1.71 ms; a step of a whole cycle of 50, host polls,
+// start and update included: 31 (28), 52, 207 us and 1.76 ms.  With the leftovers
+// in front of the barrier of their own step, the step of a cycle was 32 against 27,
+// 61 against 58 and 232 against 227 us at the first three sizes when that was
+// changed.
 //
 // A warp owns sub-chunks of 32 V values.  Phase A takes JG vectors at a
 // time: all their loads in flight, 2 JG sums per lane, reduced over the

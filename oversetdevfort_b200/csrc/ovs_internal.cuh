@@ -168,7 +168,7 @@ struct ovs_ctx {
   void* basis[2] = {nullptr, nullptr};   // Krylov basis per precision
   size_t basis_bytes[2] = {0, 0};
   double* work64 = nullptr;              // 3 vectors of 5N doubles (b, r, x)
-  double* wvec = nullptr;                // FP64 vector under orthogonalization
+  double* wvec = nullptr;                // P^-1 rhs in FP64, before it becomes the first basis vector
   double* coop_part = nullptr;           // partial sums of the cooperative Arnoldi kernels, then T = (I + L)^-1
   size_t coop_bytes = 0;                 //   (rows of kspace, strictly lower part)
   bool arnoldi_fused = false;            // one-launch Arnoldi variant (env OVS_ARNOLDI_FUSED=1)
